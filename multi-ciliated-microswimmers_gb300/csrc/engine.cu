@@ -91,6 +91,7 @@ struct mpcd_engine {
   MDState md;
   long md_nsp = 0;  // springs in the device layout
   bool md_dirty = true;
+  uint32_t md_tag = 1;  // the next force evaluation's packet tag (double-float MD kernel)
 
   // profiling: event pairs per launch, resolved on query
   bool profiling = false;
@@ -218,7 +219,10 @@ void free_md(MDState& m) {
   cudaFree(m.newlen);
   cudaFree(m.oldlen);
   cudaFree(m.tile_cil);
-  for (int b = 0; b < 2; ++b) cudaFree(m.q[b]);
+  for (int b = 0; b < 2; ++b) {
+    cudaFree(m.q[b]);
+    cudaFree(m.qp[b]);
+  }
   cudaFree(m.sp_rest2);
   cudaFree(m.sp_m2k2);
   cudaFree(m.sp_code);
@@ -516,9 +520,8 @@ int build_md(mpcd_engine* h) {
     if (m.ntr) CK(up(m.tr_list, pl.tr_list.data(), m.ntr * sizeof(int)));
   }
   if (m.df || m.pair) {
-    // float pairs of the spring data and the packed layout; the position pair
-    // buffers are filled by the kernel (the pair kernel's four float64 per
-    // slot take the same 32 bytes)
+    // float pairs of the spring data and the packed layout; the position
+    // buffers are filled by the kernels
     std::vector<float2> r2(nspk), k2(nspk);
     for (long i = 0; i < nspk; ++i) {
       const dfloat a = df_from_double(pl.srest[i]), b = df_from_double(pl.sm2k[i]);
@@ -529,7 +532,15 @@ int build_md(mpcd_engine* h) {
     m.df_nb_max = pl.df_nb_max;
     m.df_nrun_max = pl.df_nrun_max;
     m.df_nsingle_max = pl.df_nsingle_max;
-    for (int b = 0; b < 2; ++b) CK(dalloc(&m.q[b], 2 * (size_t)ns));
+    for (int b = 0; b < 2; ++b) {
+      if (m.pair) {
+        CK(dalloc(&m.q[b], 2 * (size_t)ns));
+      } else {  // tag 0: no evaluation's packet
+        CK(dalloc(&m.qp[b], 3 * (size_t)ns));
+        CK(cudaMemset(m.qp[b], 0, 3 * (size_t)ns * sizeof(uint4)));
+      }
+    }
+    h->md_tag = 1;
     CK(dalloc(&m.sp_rest2, nspk));
     CK(dalloc(&m.sp_m2k2, nspk));
     CK(dalloc(&m.sp_code, nspk));
@@ -1176,6 +1187,8 @@ int mpcd_step(mpcd_engine* h, const mpcd_inject* inj) {
   }
   ma.bead_mass = h->p.bead_mass;
   ma.err = h->d_err;
+  ma.tag0 = h->md_tag;
+  h->md_tag += (uint32_t)h->nsub + 1u;
   cudaError_t coop = cudaSuccess;
   const bool f64 = h->p.precision == MPCD_FP64;
   const bool md = h->md.nslots > 0;

@@ -158,8 +158,7 @@ struct MDState {
   // double-float arithmetic (md_df.cu): float pairs of the spring data,
   // packed spring codes (other bead's staged index | kind << 16 | bond index
   // within the tile << 18), per slot the end of its in-tile springs, per tile
-  // its bond range, and two position buffers of pairs, two float4 per slot
-  // ({hx, hy, hz, lx}, {ly, lz, 0, 0})
+  // its bond range
   int df = 0;          // 1: double-float springs, 2: float springs (split arithmetic) on this layout
   int df_nsp_max = 0;  // most springs of one tile
   int df_nb_max = 0;   // most bonds of one tile
@@ -175,7 +174,10 @@ struct MDState {
   int* halo_run_start = nullptr;   // ntiles + 1
   int2* halo_single = nullptr;     // per tile: halo entries outside long runs {slot, rank}
   int* halo_single_start = nullptr;
-  float4* q[2] = {nullptr, nullptr};
+  float4* q[2] = {nullptr, nullptr};  // pair kernel: two buffers of positions, 32 bytes per slot
+  // double-float kernel: two buffers of position packets, three per slot
+  // (one per coordinate: offset pair, cell, tag of the force evaluation)
+  uint4* qp[2] = {nullptr, nullptr};
   // pair kernel (md_pair.cu), on the layout above with one slot per bead:
   // per tile its force entries (a spring and its exact reverse inside the
   // tile form one entry; code {a | b << 16, kind | both << 2 | react << 3 |
@@ -237,6 +239,9 @@ struct MDStepArgs {
   double a_cur[3], a_next[3];
   double bead_mass;
   unsigned* err;
+  // double-float kernel: tag of the launch's first force evaluation; the tags
+  // of successive launches do not repeat until the counter wraps
+  uint32_t tag0 = 0;
   // 1: the MD launch first applies the beads' collision (their cells' maps,
   // as the separate bead kernel would) and subtracts their m v'^2 from *diss
   int collide = 0;

@@ -667,9 +667,33 @@ std::string plan_md(const MDInput& in, const MDForce& force, bool allow_cluster,
   out.df_single.clear();
   out.df_single_start.assign(1, 0);
   int hmax = 0;
+  // The double-float grid kernel has no grid barrier: a tile may overwrite a
+  // position buffer once it has received the next evaluation from every tile
+  // that reads it, so every tile must read something of each of its readers.
+  // Spring networks made in both directions (every reference object) are so by
+  // themselves; for one-sided lists each missing direction gets one bead.
+  std::vector<std::vector<int>> answer(out.ntiles);  // per tile: its readers' beads to receive as well
+  if (out.df && !in.pair && !out.cluster) {
+    std::vector<std::vector<std::pair<int, int>>> reads(out.ntiles);  // (tile read, a primary slot of the reader)
+    std::vector<int> stamp(out.ntiles, -1);
+    for (int t = 0; t < out.ntiles; ++t)
+      for (int s2 = t * tile; s2 < (t + 1) * tile; ++s2)
+        for (int d = start[s2]; d < start[s2 + 1]; ++d) {
+          const int u = out.so[d] / tile;
+          if (u == t || stamp[u] == t) continue;
+          stamp[u] = t;
+          reads[t].push_back({u, out.prim[s2]});
+        }
+    for (int t = 0; t < out.ntiles; ++t)
+      for (const auto& r : reads[t]) {
+        bool back = false;
+        for (const auto& w : reads[r.first]) back = back || w.first == t;
+        if (!back) answer[r.first].push_back(r.second);
+      }
+  }
   for (int t = 0; t < out.ntiles; ++t) {
     const int b0 = t * tile, b1 = b0 + tile;
-    std::vector<int> ext;
+    std::vector<int> ext = answer[t];
     for (int s2 = start[b0]; s2 < start[b1]; ++s2)
       if (out.so[s2] < b0 || out.so[s2] >= b1) ext.push_back(out.so[s2]);
     std::sort(ext.begin(), ext.end());
