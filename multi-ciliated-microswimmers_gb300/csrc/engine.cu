@@ -233,6 +233,12 @@ void free_md(MDState& m) {
   cudaFree(m.halo_run_start);
   cudaFree(m.halo_single);
   cudaFree(m.halo_single_start);
+  cudaFree(m.de_start);
+  cudaFree(m.de_local_end);
+  cudaFree(m.de_solo);
+  cudaFree(m.de_nslot);
+  cudaFree(m.de_code);
+  cudaFree(m.de_rk);
   cudaFree(m.pr_start);
   cudaFree(m.pr_local_end);
   cudaFree(m.pr_hub_begin);
@@ -376,8 +382,14 @@ int build_md(mpcd_engine* h) {
   // MPCD_MD_MIN_TILE: narrowest grid-layout tile (tests of the wide layouts on small bead sets)
   const char* mt = std::getenv("MPCD_MD_MIN_TILE");
   const int min_tile = mt ? std::max(0, std::min(256, std::atoi(mt))) : 0;
-  const std::string why =
-      plan_md(in, MDForce{}, allow_cluster, false, h->p.precision == MPCD_FP32 ? 1 : 0, pl, min_tile);
+  const int f32cells = h->p.precision == MPCD_FP32 ? 1 : 0;
+  // double-float arithmetic: the entries layout (md_entries.cu) where the bead
+  // set fits it, else the slot layouts of plan_md.  MPCD_MD_SLOTS=1 keeps the
+  // slot layout (tests of that kernel)
+  const char* slots = std::getenv("MPCD_MD_SLOTS");
+  const bool entries = in.df && !in.pair && !(slots && std::atoi(slots) != 0) &&
+                       plan_entries(in, f32cells, pl, min_tile).empty();
+  const std::string why = entries ? "" : plan_md(in, MDForce{}, allow_cluster, false, f32cells, pl, min_tile);
   if (!why.empty()) return fail(h, MPCD_EINVAL, why);
   if (const char* ps = std::getenv("MPCD_MD_PLAN_STATS"); ps && std::atoi(ps) && pl.pair) {
     // the pair layout's per-tile sizes: force entries (of them reaching only
@@ -393,6 +405,7 @@ int build_md(mpcd_engine* h) {
   m.split = pl.split;
   m.pair = pl.pair;
   m.df = pl.df && !pl.pair ? (arith == 3 ? 2 : 1) : 0;
+  m.de = pl.de;
   m.cluster = pl.cluster;
   m.cl_lanes = pl.cl_lanes;
   m.cl_nsp_max = pl.cl_nsp_max;
@@ -420,15 +433,9 @@ int build_md(mpcd_engine* h) {
   CK(dalloc(&m.nhelp, ns));
   CK(dalloc(&m.tile_help, m.ntiles));
   CK(dalloc(&m.sp_start, ns + 1));
-  CK(dalloc(&m.sp_other, nspk));
-  CK(dalloc(&m.sp_local, nspk));
   CK(dalloc(&m.halo, pl.halo.size()));
   CK(dalloc(&m.halo_start, m.ntiles + 1));
   CK(dalloc(&m.diag, nbond));
-  CK(dalloc(&m.sp_kind, nspk));
-  CK(dalloc(&m.sp_ref, nspk));
-  CK(dalloc(&m.sp_rest, nspk));
-  CK(dalloc(&m.sp_m2k, nspk));
   CK(dalloc(&m.tile_react, m.ntiles));
   m.ncil = (int)ncil;
   CK(dalloc(&m.cil, ncil));
@@ -451,7 +458,13 @@ int build_md(mpcd_engine* h) {
   CK(up(m.nhelp, pl.nhelp.data(), ns * 4));
   CK(up(m.tile_help, pl.thelp.data(), m.ntiles * 4));
   CK(up(m.sp_start, pl.start.data(), (ns + 1) * 4));
-  if (nspk) {
+  if (nspk && !m.de) {  // the entries kernel keeps them in its own tables
+    CK(dalloc(&m.sp_other, nspk));
+    CK(dalloc(&m.sp_local, nspk));
+    CK(dalloc(&m.sp_kind, nspk));
+    CK(dalloc(&m.sp_ref, nspk));
+    CK(dalloc(&m.sp_rest, nspk));
+    CK(dalloc(&m.sp_m2k, nspk));
     CK(up(m.sp_other, pl.so.data(), nspk * 4));
     CK(up(m.sp_local, pl.sl.data(), nspk * 4));
     CK(up(m.sp_kind, pl.sk.data(), nspk * 4));
@@ -520,18 +533,7 @@ int build_md(mpcd_engine* h) {
     if (m.ntr) CK(up(m.tr_list, pl.tr_list.data(), m.ntr * sizeof(int)));
   }
   if (m.df || m.pair) {
-    // float pairs of the spring data and the packed layout; the position
-    // buffers are filled by the kernels
-    std::vector<float2> r2(nspk), k2(nspk);
-    for (long i = 0; i < nspk; ++i) {
-      const dfloat a = df_from_double(pl.srest[i]), b = df_from_double(pl.sm2k[i]);
-      r2[i] = make_float2(a.h, a.l);
-      k2[i] = make_float2(b.h, b.l);
-    }
-    m.df_nsp_max = pl.df_nsp_max;
     m.df_nb_max = pl.df_nb_max;
-    m.df_nrun_max = pl.df_nrun_max;
-    m.df_nsingle_max = pl.df_nsingle_max;
     for (int b = 0; b < 2; ++b) {
       if (m.pair) {
         CK(dalloc(&m.q[b], 2 * (size_t)ns));
@@ -541,20 +543,58 @@ int build_md(mpcd_engine* h) {
       }
     }
     h->md_tag = 1;
+    CK(dalloc(&m.tile_b0, m.ntiles));
+    CK(dalloc(&m.tile_nb, m.ntiles));
+    CK(up(m.tile_b0, pl.df_b0.data(), m.ntiles * sizeof(int)));
+    CK(up(m.tile_nb, pl.df_nb.data(), m.ntiles * sizeof(int)));
+  }
+  if (m.de) {
+    // force entries: codes, and {rest length, -2k} as float pairs
+    const size_t ne = pl.de_code.size();
+    std::vector<float4> rk(ne);
+    for (size_t i = 0; i < ne; ++i) {
+      const dfloat r = df_from_double(pl.de_rest[i]), k = df_from_double(pl.de_m2k[i]);
+      rk[i] = make_float4(r.h, r.l, k.h, k.l);
+    }
+    m.de_nent_max = pl.de_nent_max;
+    m.de_ninc_max = pl.de_ninc_max;
+    m.de_step = pl.de_step;
+    CK(dalloc(&m.de_start, m.ntiles + 1));
+    CK(dalloc(&m.de_local_end, m.ntiles));
+    CK(dalloc(&m.de_solo, m.ntiles));
+    CK(dalloc(&m.de_nslot, m.ntiles));
+    CK(up(m.de_nslot, pl.de_nslot.data(), m.ntiles * sizeof(int)));
+    CK(dalloc(&m.de_code, ne));
+    CK(dalloc(&m.de_rk, ne));
+    CK(up(m.de_start, pl.de_start.data(), (m.ntiles + 1) * sizeof(int)));
+    CK(up(m.de_local_end, pl.de_local_end.data(), m.ntiles * sizeof(int)));
+    CK(up(m.de_solo, pl.de_solo.data(), m.ntiles * sizeof(int)));
+    if (ne) {
+      CK(up(m.de_code, pl.de_code.data(), ne * sizeof(uint4)));
+      CK(up(m.de_rk, rk.data(), ne * sizeof(float4)));
+    }
+  } else if (m.df || m.pair) {
+    // float pairs of the spring data and the packed layout; the position
+    // buffers are filled by the kernels
+    std::vector<float2> r2(nspk), k2(nspk);
+    for (long i = 0; i < nspk; ++i) {
+      const dfloat a = df_from_double(pl.srest[i]), b = df_from_double(pl.sm2k[i]);
+      r2[i] = make_float2(a.h, a.l);
+      k2[i] = make_float2(b.h, b.l);
+    }
+    m.df_nsp_max = pl.df_nsp_max;
+    m.df_nrun_max = pl.df_nrun_max;
+    m.df_nsingle_max = pl.df_nsingle_max;
     CK(dalloc(&m.sp_rest2, nspk));
     CK(dalloc(&m.sp_m2k2, nspk));
     CK(dalloc(&m.sp_code, nspk));
     CK(dalloc(&m.sp_split, ns));
-    CK(dalloc(&m.tile_b0, m.ntiles));
-    CK(dalloc(&m.tile_nb, m.ntiles));
     if (nspk) {
       CK(up(m.sp_rest2, r2.data(), nspk * sizeof(float2)));
       CK(up(m.sp_m2k2, k2.data(), nspk * sizeof(float2)));
       CK(up(m.sp_code, pl.df_code.data(), nspk * sizeof(uint32_t)));
     }
     CK(up(m.sp_split, pl.df_split.data(), ns * sizeof(int)));
-    CK(up(m.tile_b0, pl.df_b0.data(), m.ntiles * sizeof(int)));
-    CK(up(m.tile_nb, pl.df_nb.data(), m.ntiles * sizeof(int)));
     CK(dalloc(&m.halo_run, std::max<size_t>(1, pl.df_runs.size())));
     CK(dalloc(&m.halo_run_start, m.ntiles + 1));
     if (!pl.df_runs.empty()) CK(up(m.halo_run, pl.df_runs.data(), pl.df_runs.size() * sizeof(int4)));
@@ -1239,6 +1279,9 @@ int mpcd_step(mpcd_engine* h, const mpcd_inject* inj) {
     else if (h->md.pair)
       h->launches += f64 ? launch_md_pair_f64cells(h->md, h->c64, ma, sm, &coop)
                          : launch_md_pair_f32cells(h->md, h->c32, ma, sm, &coop);
+    else if (h->md.de)
+      h->launches += f64 ? launch_md_entries_f64cells(h->md, h->c64, ma, sm, &coop)
+                         : launch_md_entries_f32cells(h->md, h->c32, ma, sm, &coop);
     else if (h->md.df)
       h->launches += f64 ? launch_md_df_f64cells(h->md, h->c64, ma, sm, &coop)
                          : launch_md_df_f32cells(h->md, h->c32, ma, sm, &coop);
@@ -1760,7 +1803,7 @@ int mpcd_md_layout(mpcd_engine* h, int* info) {
   }
   const MDState& m = h->md;
   info[0] = m.cluster;
-  info[1] = m.cluster ? m.cl_lanes : (m.pair ? md_pair_threads(m.tile) / m.tile : (m.df ? md_df_lanes(m.tile) : 4));
+  info[1] = m.cluster ? m.cl_lanes : (m.pair ? md_pair_threads(m.tile) / m.tile : (m.de ? md_entries_threads(m.tile) / m.tile : (m.df ? md_df_lanes(m.tile) : 4)));
   info[2] = m.tile;
   info[3] = m.ntiles;
   info[4] = m.nslots;

@@ -175,9 +175,22 @@ struct MDState {
   int2* halo_single = nullptr;     // per tile: halo entries outside long runs {slot, rank}
   int* halo_single_start = nullptr;
   float4* q[2] = {nullptr, nullptr};  // pair kernel: two buffers of positions, 32 bytes per slot
-  // double-float kernel: two buffers of position packets, three per slot
-  // (one per coordinate: offset pair, cell, tag of the force evaluation)
+  // double-float kernels: two buffers of position packets, one per coordinate
+  // and slot (coordinate-major: offset pair, cell, tag of the force evaluation)
   uint4* qp[2] = {nullptr, nullptr};
+  // entries kernel (md_entries.cu; de = 1), one slot per bead: per tile its
+  // force entries, those between its own beads first (codes as the kernel
+  // stages them, {rest length, -2k} as float pairs); a bead's incidences are
+  // its springs (sp_start).  de_solo: the tile holds one bead with a long list
+  int de = 0;
+  int de_nent_max = 0, de_ninc_max = 0;
+  int* de_start = nullptr;      // ntiles + 1
+  int* de_local_end = nullptr;  // ntiles
+  int* de_solo = nullptr;       // ntiles
+  int* de_nslot = nullptr;      // ntiles: incidence words of the tile
+  int de_step = 1;  // words between a bead's incidences: 1 (bead after bead) or the tile width (transposed)
+  uint4* de_code = nullptr;
+  float4* de_rk = nullptr;
   // pair kernel (md_pair.cu), on the layout above with one slot per bead:
   // per tile its force entries (a spring and its exact reverse inside the
   // tile form one entry; code {a | b << 16, kind | both << 2 | react << 3 |
@@ -242,6 +255,10 @@ struct MDStepArgs {
   // double-float kernel: tag of the launch's first force evaluation; the tags
   // of successive launches do not repeat until the counter wraps
   uint32_t tag0 = 0;
+  // dt and dt / 2 as float pairs (high, low), set by the double-float kernels'
+  // launchers: computed in the kernel, the compiler repeats the float64
+  // conversions in every substep (about 700 cycles of its dependent chain)
+  float2 dt_pair = {0.f, 0.f}, dt2_pair = {0.f, 0.f};
   // 1: the MD launch first applies the beads' collision (their cells' maps,
   // as the separate bead kernel would) and subtracts their m v'^2 from *diss
   int collide = 0;
@@ -267,6 +284,12 @@ int launch_md_f64(const MDState& m, const CellsF64& c, const MDStepArgs& a, cuda
 int launch_md_df_f64cells(const MDState& m, const CellsF64& c, const MDStepArgs& a, cudaStream_t s, cudaError_t* st);
 int launch_md_df_f32cells(const MDState& m, const CellsF32& c, const MDStepArgs& a, cudaStream_t s, cudaError_t* st);
 int md_df_max_coresident_blocks(const MDState& m, int f32cells);
+int launch_md_entries_f64cells(const MDState& m, const CellsF64& c, const MDStepArgs& a, cudaStream_t s,
+                               cudaError_t* st);
+int launch_md_entries_f32cells(const MDState& m, const CellsF32& c, const MDStepArgs& a, cudaStream_t s,
+                               cudaError_t* st);
+int md_entries_max_coresident_blocks(const MDState& m, int f32cells);
+int md_entries_threads(int tile);  // threads per CTA of the entries kernel
 int md_df_lanes(int tile);  // threads per slot of the double-float kernel
 int launch_md_pair_f64cells(const MDState& m, const CellsF64& c, const MDStepArgs& a, cudaStream_t s, cudaError_t* st);
 int launch_md_pair_f32cells(const MDState& m, const CellsF32& c, const MDStepArgs& a, cudaStream_t s, cudaError_t* st);

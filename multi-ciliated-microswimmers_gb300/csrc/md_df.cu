@@ -1,6 +1,10 @@
 // MD substeps of one MPC step for the float64 path, in double-float
 // arithmetic on the FP32 pipes.
 //
+// The general form of the double-float MD: every bead set whose layout fits the
+// device runs here; those that fit the layout of md_entries.cu (a thread per
+// spring pair, less than half the time on large swimmers) run there.
+//
 // Same integrator and forces as md_kernels.cu (velocity Verlet of
 // src/libcilia/mdobject.cpp:36-72 inside the loop of src/simulation.cpp:217-265;
 // springs of src/cilia.cpp:127-239, src/sphere.cpp:87-119, src/clami.cpp:188-198)
@@ -46,42 +50,11 @@
 #include "df32.cuh"
 #include "md_common.cuh"
 #include "md_df_coord.cuh"
+#include "md_packets.cuh"
 
 namespace mpcd {
 
 namespace {
-
-// polls of a packet before giving up (each an L2 round trip: a second or two)
-constexpr uint32_t kPollLimit = 1u << 21;
-// packets one thread polls at a time (their loads in flight together): the
-// sphere centre's tile takes its 661 x 3 packets in one round of 384 threads
-constexpr int kPollBatch = 6;
-
-// One coordinate of a bead as it travels between tiles: the offset's pair,
-// the cell, and the tag of the evaluation; stored and loaded by single
-// 128-bit accesses (single-copy atomic), so that the tag vouches for the rest.
-struct Packet {
-  uint32_t h, l, c, tag;
-};
-__device__ __forceinline__ void packet_store(uint4* p, const Packet& k) {
-  asm volatile(
-      "{\n\t.reg .b64 a, b;\n\t.reg .b128 t;\n\t"
-      "mov.b64 a, {%1, %2};\n\tmov.b64 b, {%3, %4};\n\tmov.b128 t, {a, b};\n\t"
-      "st.relaxed.gpu.global.b128 [%0], t;\n\t}" ::"l"(p),
-      "r"(k.h), "r"(k.l), "r"(k.c), "r"(k.tag)
-      : "memory");
-}
-__device__ __forceinline__ Packet packet_load(const uint4* p) {
-  Packet k;
-  asm volatile(
-      "{\n\t.reg .b64 a, b;\n\t.reg .b128 t;\n\t"
-      "ld.relaxed.gpu.global.b128 t, [%4];\n\tmov.b128 {a, b}, t;\n\t"
-      "mov.b64 {%0, %1}, a;\n\tmov.b64 {%2, %3}, b;\n\t}"
-      : "=r"(k.h), "=r"(k.l), "=r"(k.c), "=r"(k.tag)
-      : "l"(p)
-      : "memory");
-  return k;
-}
 
 // Tile-resident spring and bond tables in shared memory.
 struct Tables {
@@ -183,33 +156,6 @@ struct DfSmem {
   }
 };
 
-// a pair-wise exchange step: keeps `mine`, sends `give` to the lane `o` away,
-// and adds what comes back
-__device__ __forceinline__ void exchange_add(float& mh, float& ml, float gh, float gl, int o) {
-  const float bh = __shfl_xor_sync(0xffffffffu, gh, o), bl = __shfl_xor_sync(0xffffffffu, gl, o);
-  df_acc(mh, ml, bh, bl);
-}
-
-// The sum over groups of G lanes (G = 4, 8 or 32) of (x, y, z): the two top
-// levels trade components instead of summing all three in every lane, so that
-// the quarter of the group with index k ends with component k, summed over
-// the group (quarter 3 holds nothing).  A fixed order.
-template <int G>
-__device__ __forceinline__ void group_sum_xyz(int lane, float fxh, float fxl, float fyh, float fyl, float fzh, float fzl,
-                                              float& h, float& l) {
-  const bool up = (lane & (G / 2)) != 0, odd = (lane & (G / 4)) != 0;
-  // lower half keeps x and y, the upper half z
-  float ah = up ? fzh : fxh, al = up ? fzl : fxl, bh = up ? 0.0f : fyh, bl = up ? 0.0f : fyl;
-  exchange_add(ah, al, up ? fxh : fzh, up ? fxl : fzl, G / 2);
-  exchange_add(bh, bl, up ? fyh : 0.0f, up ? fyl : 0.0f, G / 2);
-  // the even quarter keeps the first, the odd one the second
-  h = odd ? bh : ah;
-  l = odd ? bl : al;
-  exchange_add(h, l, odd ? ah : bh, odd ? al : bl, G / 4);
-#pragma unroll
-  for (int o = G / 8; o > 0; o >>= 1) exchange_add(h, l, h, l, o);
-}
-
 template <int LANES, bool kFloat, typename Bin>
 __device__ void md_df_body(const MDState& m, const MDStepArgs& a, Bin bin) {
   extern __shared__ __align__(16) unsigned char smem[];
@@ -255,7 +201,7 @@ __device__ void md_df_body(const MDState& m, const MDStepArgs& a, Bin bin) {
   const int c0 = m.tile_cil[tile], c1 = m.tile_cil[tile + 1];
   const int b0 = m.tile_b0[tile], nb = m.tile_nb[tile];
   const int nsp = m.sp_start[base + T] - S0;
-  const dfloat dt = df_from_double(a.dt), dt2 = df_from_double(a.dt / 2.0);
+  const dfloat dt{a.dt_pair.x, a.dt_pair.y}, dt2{a.dt2_pair.x, a.dt2_pair.y};
 
   // the halo's slots; every one must lie in the packet buffers
   if (tid == 0) *s_fail = hn0 > m.hmax;
@@ -342,7 +288,7 @@ __device__ void md_df_body(const MDState& m, const MDStepArgs& a, Bin bin) {
         const int k = lane + j * LANES;
         if (k < 3) {
           const Packet pk{__float_as_uint(x[j].o.h), __float_as_uint(x[j].o.l), (uint32_t)x[j].c, a.tag0 + (uint32_t)e};
-          packet_store(m.qp[e & 1] + 3 * (size_t)slot + k, pk);
+          packet_store(m.qp[e & 1] + (size_t)k * m.nslots + slot, pk);
           stage_coord(own0 + 2 * ((size_t)T * (e & 1) + q), k, x[j].o.h, x[j].o.l, x[j].c);
         }
       }
@@ -353,35 +299,10 @@ __device__ void md_df_body(const MDState& m, const MDStepArgs& a, Bin bin) {
   // evaluation's packets of every tile that reads it (the planner makes the
   // halo relation symmetric), and those are published after this read.
   auto receive = [&](int e) {
-    const uint4* src = m.qp[e & 1];
-    const uint32_t tag = a.tag0 + (uint32_t)e;
-    const int np = 3 * hn;
-    for (int p0 = tid; p0 < np; p0 += kPollBatch * nthr) {
-      unsigned need = 0;
-#pragma unroll
-      for (int u = 0; u < kPollBatch; ++u) need |= p0 + u * nthr < np ? 1u << u : 0u;
-      for (uint32_t spins = 0; need; ++spins) {
-        Packet d[kPollBatch];
-#pragma unroll
-        for (int u = 0; u < kPollBatch; ++u)
-          if (need >> u & 1u) {
-            const int p = p0 + u * nthr;
-            d[u] = packet_load(src + 3 * (size_t)s_hslot[p / 3] + p % 3);
-          }
-#pragma unroll
-        for (int u = 0; u < kPollBatch; ++u)
-          if ((need >> u & 1u) && d[u].tag == tag) {
-            const int p = p0 + u * nthr;
-            stage_coord(halo + 2 * (p / 3), p % 3, __uint_as_float(d[u].h), __uint_as_float(d[u].l), (int)d[u].c);
-            need &= ~(1u << u);
-          }
-        if (need && spins > kPollLimit) {  // bounded: report, and leave the launch
-          atomicOr(a.err, kErrBarrier);
-          *s_fail = 1;
-          break;
-        }
-      }
-    }
+    receive_packets(m.qp[e & 1], m.nslots, a.tag0 + (uint32_t)e, hn, s_hslot, tid, nthr, a.err, s_fail,
+                    [&](int p, int k, const Packet& d) {
+                      stage_coord(halo + 2 * p, k, __uint_as_float(d.h), __uint_as_float(d.l), (int)d.c);
+                    });
   };
   // forces on the owned beads at evaluation e; false when a packet never came
   auto evaluate = [&](int e) -> bool {
@@ -617,6 +538,7 @@ int launch_df(const MDState& m, const typename Bin::Cells& c, const MDStepArgs& 
   MDState mm = m;
   typename Bin::Cells cc = c;
   MDStepArgs aa = a;
+  md_set_dt_pairs(aa);
   void* args[] = {&mm, &cc, &aa};
   const size_t smem = md_df_smem(m);
   const int lanes = md_df_lanes(m.tile);

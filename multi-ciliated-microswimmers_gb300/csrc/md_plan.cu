@@ -880,4 +880,364 @@ std::string plan_md(const MDInput& in, const MDForce& force, bool allow_cluster,
   return "";
 }
 
+// ------------------------------------------------ layout of md_entries.cu ---
+
+namespace {
+
+// A bead outside the cilia with more springs than this gets a tile of its own
+// (at most kMaxSolo of them), whose threads share its list: a sphere's centre
+// has hundreds, an ordinary bead at most about twenty.
+constexpr int kSoloSprings = 64;
+constexpr int kMaxSolo = 4;
+// Beads of a patch of non-cilium beads, if there are SMs for that many tiles:
+// about sixty entries and twenty halo beads, so that a substep's dependent
+// chain (entry, sum, Verlet) runs once through on a few warps (swimmer64 MD per
+// launch: 8 beads 127 us, 16 123, 24 128, 32 130, 43 138).
+constexpr int kPatchBeads = 16;
+constexpr long kMaxForceBytes = 96 * 1024;
+
+int device_sms() {
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  return sms > 0 ? sms : 152;
+}
+
+// Cuts `beads` into groups of at most cap by recursive coordinate bisection
+// (the longest extent halved), in a fixed order; calls leaf(first, last).
+template <typename Leaf>
+void bisect_beads(std::vector<long>& idx, const double* pos, int cap, Leaf&& leaf) {
+  std::vector<std::pair<size_t, size_t>> todo;
+  if (!idx.empty()) todo.push_back({0, idx.size()});
+  while (!todo.empty()) {  // depth first, left part first
+    const auto [lo, hi] = todo.back();
+    todo.pop_back();
+    const size_t n = hi - lo;
+    if (n <= (size_t)cap) {
+      leaf(lo, hi);
+      continue;
+    }
+    double mn[3] = {1e300, 1e300, 1e300}, mx[3] = {-1e300, -1e300, -1e300};
+    for (size_t k = lo; k < hi; ++k)
+      for (int d = 0; d < 3; ++d) {
+        mn[d] = std::min(mn[d], pos[3 * idx[k] + d]);
+        mx[d] = std::max(mx[d], pos[3 * idx[k] + d]);
+      }
+    int ax = 0;
+    for (int d = 1; d < 3; ++d)
+      if (mx[d] - mn[d] > mx[ax] - mn[ax]) ax = d;
+    // whole leaves on the left, so that the leaves are ceil(n / cap) in all
+    const size_t parts = (n + cap - 1) / cap, left = std::min(n - 1, (parts / 2) * (size_t)cap);
+    std::nth_element(idx.begin() + lo, idx.begin() + lo + left, idx.begin() + hi, [&](long p, long q) {
+      const double u = pos[3 * p + ax], w = pos[3 * q + ax];
+      return u < w || (u == w && p < q);
+    });
+    todo.push_back({lo + left, hi});
+    todo.push_back({lo, lo + left});
+  }
+}
+
+// the tables of a chosen tiling (tile of every bead's slot in slot_of)
+std::string fill_entries(const MDInput& in, const std::vector<int>& bstart, const std::vector<int>& blist,
+                         const std::vector<int>& cil_tile, const std::vector<char>& solo_bead,
+                         const std::vector<int>& slot_of, int tile, int ntiles, MDPlan& out) {
+  const long nb = in.nb;
+  const int ns = ntiles * tile;
+  out = MDPlan{};
+  out.df = out.de = 1;
+  out.tile = tile;
+  out.ntiles = ntiles;
+  out.nslots = ns;
+  out.slot_of = slot_of;
+  for (std::vector<double>* p : {&out.X, &out.Y, &out.Z, &out.VX, &out.VY, &out.VZ}) p->assign(ns, 0.0);
+  out.mv.assign(ns, -1);
+  out.prim.assign(ns, 0);
+  out.nhelp.assign(ns, 0);
+  out.thelp.assign(ntiles, 0);
+  out.tile_react.assign(ntiles, -1);
+  out.de_solo.assign(ntiles, 0);
+  std::vector<long> bead_at(ns, -1);
+  for (long b = 0; b < nb; ++b) {
+    const int s = slot_of[b];
+    bead_at[s] = b;
+    out.X[s] = in.bpos[3 * b];
+    out.Y[s] = in.bpos[3 * b + 1];
+    out.Z[s] = in.bpos[3 * b + 2];
+    out.VX[s] = in.bvel[3 * b];
+    out.VY[s] = in.bvel[3 * b + 1];
+    out.VZ[s] = in.bvel[3 * b + 2];
+    out.mv[s] = in.bmoves[b] ? 1 : 0;
+    out.prim[s] = s;
+    if (solo_bead[b]) out.de_solo[s / tile] = 1;
+  }
+  // springs by slot, every bead's in its input order: the incidences
+  out.start.assign(ns + 1, 0);
+  for (int s = 0; s < ns; ++s)
+    out.start[s + 1] = out.start[s] + (bead_at[s] >= 0 ? bstart[bead_at[s] + 1] - bstart[bead_at[s]] : 0);
+  const int nsp = out.start[ns];
+  out.so.resize(nsp);
+  out.sl.resize(nsp);
+  std::vector<int> src(nsp);  // input index
+  for (int s = 0; s < ns; ++s)
+    for (int d = out.start[s]; d < out.start[s + 1]; ++d) {
+      src[d] = blist[bstart[bead_at[s]] + d - out.start[s]];
+      out.so[d] = slot_of[in.sp_o[src[d]]];
+    }
+  // bonds of each tile's cilia
+  out.df_b0.assign(ntiles, 0);
+  out.df_nb.assign(ntiles, 0);
+  {
+    std::vector<int> lo(ntiles, INT_MAX), hi(ntiles, 0);
+    for (int c = 0; c < in.ncil; ++c) {
+      const int t = cil_tile[c];
+      lo[t] = std::min(lo[t], in.cil[c].bond_base);
+      hi[t] = std::max(hi[t], in.cil[c].bond_base + in.cil[c].rodlength);
+    }
+    for (int t = 0; t < ntiles; ++t) {
+      if (lo[t] > hi[t]) continue;
+      out.df_b0[t] = lo[t];
+      out.df_nb[t] = hi[t] - lo[t];
+      out.df_nb_max = std::max(out.df_nb_max, out.df_nb[t]);
+    }
+  }
+  // every tile has to read something of each of its readers (the position
+  // buffers are reused without a grid barrier; see plan_md)
+  std::vector<std::vector<int>> reads(ntiles), answer(ntiles);
+  {
+    std::vector<int> stamp(ntiles, -1);
+    for (int t = 0; t < ntiles; ++t)
+      for (int d = out.start[t * tile]; d < out.start[(t + 1) * tile]; ++d) {
+        const int u = out.so[d] / tile;
+        if (u == t || stamp[u] == t) continue;
+        stamp[u] = t;
+        reads[t].push_back(u);
+      }
+    for (int t = 0; t < ntiles; ++t) std::sort(reads[t].begin(), reads[t].end());
+    for (int t = 0; t < ntiles; ++t)
+      for (int u : reads[t])
+        if (!std::binary_search(reads[u].begin(), reads[u].end(), t)) {
+          int s = t * tile;  // a bead of the reader
+          while (out.mv[s] < 0) ++s;
+          answer[u].push_back(s);
+        }
+  }
+  out.hstart.assign(1, 0);
+  out.de_start.assign(1, 0);
+  // the forces of a tile's incidences, 24 bytes each: transposed (the j-th
+  // spring of bead a at j T + a, so that threads summing neighbouring beads
+  // read neighbouring words) unless a long list makes that too large
+  int longest = 1;
+  for (int s = 0; s < ns; ++s)
+    if (!out.de_solo[s / tile]) longest = std::max(longest, out.start[s + 1] - out.start[s]);
+  out.de_step = 24L * longest * tile <= kMaxForceBytes ? tile : 1;
+  std::vector<int> ent(nsp, -1), order;
+  struct Entry {
+    int a, b, d, r;
+  };
+  std::vector<Entry> es;
+  for (int t = 0; t < ntiles; ++t) {
+    const int s0 = t * tile, s1 = s0 + tile, d0 = out.start[s0], d1 = out.start[s1];
+    const bool solo = out.de_solo[t] != 0;
+    std::vector<int> ext = answer[t];
+    for (int d = d0; d < d1; ++d)
+      if (out.so[d] < s0 || out.so[d] >= s1) ext.push_back(out.so[d]);
+    std::sort(ext.begin(), ext.end());
+    ext.erase(std::unique(ext.begin(), ext.end()), ext.end());
+    for (int d = d0; d < d1; ++d)
+      out.sl[d] = out.so[d] >= s0 && out.so[d] < s1
+                      ? out.so[d] - s0
+                      : tile + (int)(std::lower_bound(ext.begin(), ext.end(), out.so[d]) - ext.begin());
+    out.halo.insert(out.halo.end(), ext.begin(), ext.end());
+    out.hstart.push_back((int)out.halo.size());
+    out.hmax = std::max(out.hmax, (int)ext.size());
+    int words = d1 - d0;
+    if (out.de_step > 1) {
+      words = 0;
+      for (int s = s0; s < s1; ++s) words = std::max(words, (out.start[s + 1] - out.start[s]) * tile);
+    }
+    if (solo) words = 0;
+    if (words >= 0xffff) return "too many springs in a tile";
+    out.de_nslot.push_back(words);
+    out.de_ninc_max = std::max(out.de_ninc_max, words);
+    auto word_of = [&](int d, int bead) {  // spring d of local bead `bead`
+      return (uint32_t)(out.de_step > 1 ? (d - out.start[s0 + bead]) * tile + bead : d - d0);
+    };
+    // a spring and its exact reverse inside the tile form one entry
+    es.clear();
+    for (int s = s0; s < s1; ++s)
+      for (int d = out.start[s]; d < out.start[s + 1]; ++d) {
+        if (ent[d] >= 0) continue;
+        const int i = src[d], kind = in.sp_k[i];
+        if (kind < 0 || kind > 3) return "unknown spring kind";
+        Entry e{s - s0, out.sl[d], d, -1};
+        ent[d] = 1;
+        if (e.b < tile && e.b != e.a && !solo)
+          for (int r = out.start[out.so[d]]; r < out.start[out.so[d] + 1]; ++r) {
+            const int j = src[r];
+            if (ent[r] >= 0 || out.so[r] != s || in.sp_k[j] != kind || in.sp_kk[j] != in.sp_kk[i]) continue;
+            if (kind >= MPCD_SPRING_BOND ? in.sp_r[j] != in.sp_r[i] : in.sp_rest[j] != in.sp_rest[i]) continue;
+            ent[r] = 1;
+            e.r = r;
+            break;
+          }
+        es.push_back(e);
+      }
+    order.clear();
+    for (int k = 0; k < (int)es.size(); ++k)
+      if (es[k].b < tile) order.push_back(k);
+    out.de_local_end.push_back(out.de_start.back() + (int)order.size());
+    for (int k = 0; k < (int)es.size(); ++k)
+      if (es[k].b >= tile) order.push_back(k);
+    for (int k : order) {
+      const Entry& e = es[k];
+      const int i = src[e.d], kind = in.sp_k[i];
+      int lref = 0;
+      if (kind >= MPCD_SPRING_BOND) {
+        lref = in.sp_r[i] - out.df_b0[t];
+        if (lref < 0 || lref >= out.df_nb[t]) return "a bond spring refers to a bond outside its tile's cilia";
+      }
+      if (e.b >= 0x10000 || lref >= (1 << 29)) return "an MD tile is too large for packed entry codes";
+      const uint32_t ka = solo ? 0u : word_of(e.d, e.a), kb = e.r >= 0 ? word_of(e.r, e.b) : 0xffffu;
+      uint4 c;
+      c.x = (uint32_t)e.a | (kind == MPCD_SPRING_GUARDED ? 0x8000u : 0u) | ((uint32_t)e.b << 16);
+      c.y = ka | (kb << 16);
+      c.z = (uint32_t)kind | ((uint32_t)lref << 2);
+      c.w = 0u;
+      out.de_code.push_back(c);
+      out.de_rest.push_back(in.sp_rest[i]);
+      out.de_m2k.push_back(-2.0 * in.sp_kk[i]);
+    }
+    if (solo) {
+      // its threads read the halo through its entries only: a bead received
+      // just to answer a reader gets an entry without a force
+      if (out.de_local_end.back() != out.de_start.back()) return "a long list that reaches its own bead";
+      std::vector<char> has(ext.size(), 0);
+      for (const Entry& e : es) has[e.b - tile] = 1;
+      for (size_t k = 0; k < ext.size(); ++k)
+        if (!has[k]) {
+          uint4 c;
+          c.x = 0x8000u | ((uint32_t)(tile + (int)k) << 16);
+          c.y = 0xffff0000u;
+          c.z = c.w = 0u;
+          out.de_code.push_back(c);
+          out.de_rest.push_back(0.0);
+          out.de_m2k.push_back(0.0);
+        }
+    }
+    out.de_start.push_back((int)out.de_code.size());
+    out.de_nent_max = std::max(out.de_nent_max, out.de_start[t + 1] - out.de_start[t]);
+  }
+  out.de_ninc_max = std::max(out.de_ninc_max, 16);  // a solo tile's sums, one per warp
+  // cilia
+  out.tcil.assign(ntiles + 1, 0);
+  for (int c = 0; c < in.ncil; ++c) {
+    const mpcd_cilium& cl = in.cil[c];
+    CiliumDev d{};
+    d.stride = 1;
+    d.kind = cl.kind;
+    d.len = cl.rodlength;
+    d.num_anker = cl.num_anker;
+    d.slot0 = slot_of[cl.bead0];
+    d.bond_base = cl.bond_base;
+    d.beatstrength = cl.beatstrength;
+    d.bending = cl.bending;
+    d.max_bend = cl.max_bend;
+    d.m_speed = cl.m_speed;
+    d.power_dur = cl.power_stroke_duration;
+    d.recovery_dur = cl.recovery_stroke_duration;
+    d.start = cl.start;
+    out.cd.push_back(d);
+    out.mid.push_back(cl.midpnt);
+    out.ts.push_back(cl.tstroke);
+    out.tcil[cil_tile[c] + 1]++;
+  }
+  for (int t = 0; t < ntiles; ++t) out.tcil[t + 1] += out.tcil[t];
+  out.newlen.assign(in.newlen, in.newlen + in.nbond);
+  out.oldlen.assign(in.oldlen, in.oldlen + in.nbond);
+  out.diag.resize(in.nbond);
+  for (long k = 0; k < in.nbond; ++k) out.diag[k] = std::sqrt(0.5 * 0.5 + 0.5 * in.newlen[k]);
+  return "";
+}
+
+}  // namespace
+
+std::string plan_entries(const MDInput& in, int grid_f32cells, MDPlan& out, int min_tile) {
+  const long nb = in.nb, nsp = in.nsp;
+  std::vector<int> bstart(nb + 1, 0), blist(nsp);
+  for (long i = 0; i < nsp; ++i) {
+    if (in.sp_t[i] < 0 || in.sp_t[i] >= nb || in.sp_o[i] < 0 || in.sp_o[i] >= nb) return "spring bead index out of range";
+    bstart[in.sp_t[i] + 1]++;
+  }
+  for (long b = 0; b < nb; ++b) bstart[b + 1] += bstart[b];
+  {
+    std::vector<int> at(bstart.begin(), bstart.end() - 1);
+    for (long i = 0; i < nsp; ++i) blist[at[in.sp_t[i]]++] = (int)i;
+  }
+  std::vector<char> owned(nb, 0), solo(nb, 0);
+  int widest = 0;
+  for (int c = 0; c < in.ncil; ++c) {
+    widest = std::max(widest, 3 * in.cil[c].rodlength);
+    for (int k = 0; k < 3 * in.cil[c].rodlength; ++k) {
+      const long b = (long)in.cil[c].bead0 + k;
+      if (b < 0 || b >= nb || owned[b]) return "cilium beads out of range or shared";
+      owned[b] = 1;
+    }
+  }
+  int nsolo = 0;
+  std::vector<long> others;
+  for (long b = 0; b < nb; ++b) {
+    if (owned[b]) continue;
+    if (bstart[b + 1] - bstart[b] > kSoloSprings && nsolo < kMaxSolo) {
+      solo[b] = 1;
+      ++nsolo;
+    } else {
+      others.push_back(b);
+    }
+  }
+  const int sms = device_sms();
+  // narrow tiles first (more CTAs, more lanes per bead); the grid must be
+  // co-resident, one CTA per SM
+  std::vector<int> slot_of(nb), cil_tile(in.ncil);
+  std::vector<long> idx;
+  for (int tile = std::max(std::max(32, min_tile), (widest + 15) / 16 * 16); tile <= 256;
+       tile = tile < 64 ? tile + 16 : (tile + 32) / 32 * 32) {
+    int nt = 0, fill = tile;
+    for (int c = 0; c < in.ncil; ++c) {  // next fit, each cilium whole
+      const int w = 3 * in.cil[c].rodlength;
+      if (fill + w > tile) {
+        ++nt;
+        fill = 0;
+      }
+      cil_tile[c] = nt - 1;
+      for (int k = 0; k < w; ++k) slot_of[in.cil[c].bead0 + k] = (nt - 1) * tile + fill + k;
+      fill += w;
+    }
+    for (long b = 0; b < nb; ++b)
+      if (solo[b]) slot_of[b] = nt++ * tile;
+    if (!others.empty()) {
+      const int room = sms - nt;
+      if (room <= 0) continue;
+      const int patch = std::max(min_tile ? min_tile : kPatchBeads, (int)((others.size() + room - 1) / room));
+      if (patch > tile) continue;
+      idx = others;
+      bisect_beads(idx, in.bpos, patch, [&](size_t lo, size_t hi) {
+        for (size_t k = lo; k < hi; ++k) slot_of[idx[k]] = nt * tile + (int)(k - lo);
+        ++nt;
+      });
+    }
+    if (nt > sms) continue;
+    const std::string why = fill_entries(in, bstart, blist, cil_tile, solo, slot_of, tile, nt, out);
+    if (!why.empty()) return why;
+    MDState probe;
+    probe.tile = tile;
+    probe.ntiles = nt;
+    probe.df = probe.de = 1;
+    probe.hmax = out.hmax;
+    probe.de_nent_max = out.de_nent_max;
+    probe.de_ninc_max = out.de_ninc_max;
+    probe.df_nb_max = out.df_nb_max;
+    if (nt <= md_max_coresident_blocks(probe, grid_f32cells)) return "";
+  }
+  return "no entries layout fits the device";
+}
+
 }  // namespace mpcd

@@ -1,7 +1,8 @@
-"""The double-float grid MD kernel's exchange of positions between tiles
-(tagged packets, no grid barrier) on spring networks that the shipped objects
-do not make: one-sided lists (a tile that reads another without being read),
-beads with helper slots in short and long runs, and all tile widths.
+"""The double-float grid MD kernels (a thread per spring pair; lanes per bead
+slot) and their exchange of positions between tiles (tagged packets, no grid
+barrier) on spring networks that the shipped objects do not make: one-sided
+lists (a tile that reads another without being read), long lists (a tile of
+their own; helper slots in short and long runs), and all tile widths.
 
 Reference: the same velocity Verlet (src/libcilia/mdobject.cpp:36-72) in numpy
 float64.  Every bead is alone in its collision cell, so the collision leaves
@@ -62,7 +63,10 @@ def verlet(pos, vel, t, o, rest, k, nsub, dt):
 
 @pytest.mark.parametrize("min_tile", [0, 128, 256])
 @pytest.mark.parametrize("kind", ["oneway", "random", "hub"])
-def test_one_sided_networks_match_float64(kind, min_tile, monkeypatch):
+@pytest.mark.parametrize("slots", [False, True])
+def test_one_sided_networks_match_float64(kind, min_tile, slots, monkeypatch):
+    if slots:
+        monkeypatch.setenv("MPCD_MD_SLOTS", "1")
     if min_tile:
         monkeypatch.setenv("MPCD_MD_MIN_TILE", str(min_tile))
     rng = np.random.default_rng(5)
