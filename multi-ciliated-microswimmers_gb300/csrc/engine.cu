@@ -308,8 +308,11 @@ StepArgs step_args(mpcd_engine* h, const double* a_cur, const double* a_next, do
     s.a_next[q] = a_next[q];
     s.ta_cur[q] = 1.0 - a_cur[q];
     s.ta_next[q] = 1.0 - a_next[q];
+    s.xta_cur[q] = offset_threshold(s.ta_cur[q]);
+    s.xta_next[q] = offset_threshold(s.ta_next[q]);
   }
   s.h = h->p.tstep;
+  s.xh = fixed_step(h->p.tstep);
   s.gkick = h->p.gravity != 0.0 ? h->p.gravity * std::cos(t_move * h->p.omega) * h->p.tstep : 0.0;
   s.walls = h->p.walls;
   s.bead_mass = h->p.bead_mass;
@@ -1655,7 +1658,7 @@ int mpcd_snapshot(mpcd_engine* h, void* buf, long long bytes) {
   if (bytes < (long long)snapshot_bytes(h)) return fail(h, MPCD_EINVAL, "snapshot: buffer smaller than mpcd_snapshot_size");
   SnapHeader hd{};
   std::memcpy(hd.magic, kSnapMagic, 8);
-  hd.version = 1;
+  hd.version = h->p.precision == MPCD_FP64 ? 2 : 1;  // 2: float64 fluid offsets in units of 2^-60
   hd.precision = h->p.precision;
   for (int q = 0; q < 3; ++q) hd.sizes[q] = h->p.sizes[q];
   hd.nsph = h->nsph;
@@ -1691,7 +1694,7 @@ int mpcd_snapshot(mpcd_engine* h, void* buf, long long bytes) {
     const FluidF64& f = h->f64;
     CK(dev(f.id, 4 * n));
     CK(dev(f.cell, 4 * n));
-    for (double* a : {f.ox, f.oy, f.oz, f.vx, f.vy, f.vz}) CK(dev(a, 8 * n));
+    for (void* a : {(void*)f.ox, (void*)f.oy, (void*)f.oz, (void*)f.vx, (void*)f.vy, (void*)f.vz}) CK(dev(a, 8 * n));
   } else {
     CK(dev(h->f32.id, 4 * n));
     CK(dev(h->f32.pos, 16 * n));
@@ -1719,7 +1722,7 @@ int mpcd_restore(mpcd_engine* h, const void* buf, long long bytes) {
   SnapCursor c{const_cast<unsigned char*>(static_cast<const unsigned char*>(buf)), (size_t)bytes};
   SnapHeader hd;
   c.io(&hd, sizeof hd, false);
-  if (std::memcmp(hd.magic, kSnapMagic, 8) != 0 || hd.version != 1)
+  if (std::memcmp(hd.magic, kSnapMagic, 8) != 0 || (hd.version != 1 && hd.version != 2))
     return fail(h, MPCD_EINVAL, "restore: not a snapshot of this library");
   if (hd.precision != h->p.precision || hd.sizes[0] != h->p.sizes[0] || hd.sizes[1] != h->p.sizes[1] ||
       hd.sizes[2] != h->p.sizes[2] || hd.tstep != h->p.tstep || hd.ststep != h->p.ststep)
@@ -1744,7 +1747,9 @@ int mpcd_restore(mpcd_engine* h, const void* buf, long long bytes) {
     FluidF64& f = h->f64;
     CK(dev(f.id, 4 * n));
     CK(dev(f.cell, 4 * n));
-    for (double* a : {f.ox, f.oy, f.oz, f.vx, f.vy, f.vz}) CK(dev(a, 8 * n));
+    for (void* a : {(void*)f.ox, (void*)f.oy, (void*)f.oz, (void*)f.vx, (void*)f.vy, (void*)f.vz}) CK(dev(a, 8 * n));
+    if (hd.version == 1)  // float64 offsets
+      for (uint64_t* a : {f.ox, f.oy, f.oz}) h->launches += launch_convert_offsets((long)n, a, h->stream);
   } else {
     CK(dev(h->f32.id, 4 * n));
     CK(dev(h->f32.pos, 16 * n));

@@ -5,18 +5,19 @@
 
 #include <cuda_runtime.h>
 
+#include "fixed_offset.cuh"
 #include "mpcd_device.cuh"
 
 namespace mpcd {
 
 // ---------------------------------------------------------------- fluid ---
 // Plain (float64) fluid, structure of arrays.  Position = packed cell +
-// in-cell offset in [0,1) per axis.
+// in-cell offset in [0,1) per axis, in units of 2^-60 (fixed_offset.cuh).
 struct FluidF64 {
   long n = 0;
   uint32_t* id = nullptr;  // caller's index of each particle (permuted by the sort)
   uint32_t* cell = nullptr;
-  double *ox = nullptr, *oy = nullptr, *oz = nullptr;
+  uint64_t *ox = nullptr, *oy = nullptr, *oz = nullptr;
   double *vx = nullptr, *vy = nullptr, *vz = nullptr;
 };
 
@@ -69,6 +70,8 @@ struct StepArgs {
   double ta_next[3];  // 1 - a for the shift drawn after the MD loop
   double a_cur[3];
   double a_next[3];
+  uint64_t xta_cur[3], xta_next[3];  // ta_* as thresholds of fixed-point offsets
+  FixedStep xh;       // h for streaming fixed-point offsets
   double h;           // MPC time step
   double gkick;       // gravity * cos(omega t) * h, added to v_x after streaming
   int walls;          // MPCD_WALLS_*
@@ -309,6 +312,8 @@ int launch_load_fluid_f64(long n, const double* pos, const double* vel, const Bo
                           cudaStream_t s);
 int launch_load_fluid_f32(long n, const double* pos, const double* vel, const Box& box, const FluidF32& f,
                           cudaStream_t s);
+// an array of float64 offsets in [0, 1) into fixed-point ones, in place
+int launch_convert_offsets(long n, uint64_t* o, cudaStream_t s);
 int launch_store_fluid_f64(const FluidF64& f, double* pos, double* vel, unsigned* bad, cudaStream_t s);
 int launch_store_fluid_f32(const FluidF32& f, double* pos, double* vel, unsigned* bad, cudaStream_t s);
 // observables from the binned cell sums (float64 path; valid while the sums

@@ -54,66 +54,54 @@ inline int grid_for(long n, int threads = kThreads, int per_sm = 4) {
   return (int)(g < cap ? g : cap);
 }
 
-// Threshold 1 - a of one axis as the two 32-bit halves of its IEEE pattern.
-struct Thresh {
-  int hi;
-  uint32_t lo;
-};
-__device__ __forceinline__ Thresh thresh(double t) { return {__double2hiint(t), (uint32_t)__double2loint(t)}; }
-
 // shifted cell along one axis from the cell index and the in-cell offset:
-// floor(i + o + a) = i + (o >= 1 - a), compared on the IEEE bit patterns
-// (for a non-negative threshold, integer order of the patterns = numeric
-// order), high word signed then low word unsigned: 32-bit integer
-// instructions only (64-bit compares take GB300's small FP64 pipe)
-__device__ __forceinline__ int shifted(int i, double o, Thresh t, int L) {
-  const int hi = __double2hiint(o);
-  const bool ge = hi > t.hi || (hi == t.hi && (uint32_t)__double2loint(o) >= t.lo);
+// floor(i + o + a) = i + (o >= 1 - a), compared in fixed point, high word then
+// low word (32-bit integer instructions only)
+__device__ __forceinline__ int shifted(int i, uint64_t o, uint64_t t, int L) {
+  const uint32_t oh = (uint32_t)(o >> 32), th = (uint32_t)(t >> 32);
+  const bool ge = oh > th || (oh == th && (uint32_t)o >= (uint32_t)t);
   const int s = i + (ge ? 1 : 0);
   return s == L ? 0 : s;
 }
 
-// true unless 0 <= o < 1 (negative, -0, >= 1, NaN): one 32-bit compare of the
-// high word (0x3FF00000 = high word of 1.0; the sign bit makes a negative
-// pattern larger)
-__device__ __forceinline__ bool off_unit(double o) { return (uint32_t)__double2hiint(o) >= 0x3FF00000u; }
-
-// reduce an offset that left [0,1) back into the cell.  A streaming step
-// moves a particle by less than one cell almost always: 1 <= o < 2 and
-// -1 < o < 0 are told apart on the high word and corrected by one exact
-// float64 add (the same result as o - floor(o), without the FP64 floor and
-// compares); the general path takes the rest.
-__device__ __forceinline__ void rewrap(double& o, int& i, int L, unsigned& bad) {
-  const uint32_t hw = (uint32_t)__double2hiint(o);
-  if (hw < 0x3FF00000u) return;  // 0 <= o < 1
-  const bool up = hw < 0x40000000u;                       // 1 <= o < 2: o - 1 is exact
-  const bool down = hw >= 0x80000000u && hw < 0xBFF00000u;  // -1 < o < 0 (or -0)
-  if (up || down) {
-    o += up ? -1.0 : 1.0;  // one add for either case
-    if (up) {
-      i = i + 1 == L ? 0 : i + 1;
-    } else if (__double2hiint(o) == 0x3FF00000 && __double2loint(o) == 0) {
-      o = 0.0;  // rounded up to 1: the particle stays in its cell at offset 0
-    } else {
-      i = i == 0 ? L - 1 : i - 1;
-    }
-    return;
-  }
-  if (off_unit(o)) {
-    if (!(o > -1.0e9 && o < 1.0e9)) {  // non-finite: keep the particle in its cell and report
-      o = 0.5;
-      bad |= kErrCellRange;
-      return;
-    }
-    double fl = floor(o);
-    o -= fl;
-    i += (int)fl;
-    if (o >= 1.0) {  // o was a tiny negative number: o - floor(o) rounded to 1
-      o = 0.0;
-      i += 1;
-    }
+// cell index i back into [0, L)
+__device__ __forceinline__ void wrap_cell(int& i, int L) {
+  if ((unsigned)i < (unsigned)L) return;
+  i += i < 0 ? L : -L;
+  if ((unsigned)i >= (unsigned)L) {  // more than one box away
     i %= L;
     if (i < 0) i += L;
+  }
+}
+
+// an unwrapped coordinate (any finite value below about 1e9) as cell and offset
+__device__ __forceinline__ void split_coord(double x, int L, int& i, uint64_t& o, unsigned& bad) {
+  if (!(x > -1.0e9 && x < 1.0e9)) {  // non-finite: keep the particle in its cell and report
+    o = kOffOne / 2;
+    bad |= kErrCellRange;
+    return;
+  }
+  const double f = floor(x);
+  const double d = x - f;
+  i = (int)f;
+  o = 0;
+  if (d >= 1.0)
+    i += 1;  // x was a tiny negative number: x - floor(x) rounded to 1
+  else
+    o = offset_from_double(d);
+  i %= L;
+  if (i < 0) i += L;
+}
+
+// streams one coordinate by v h and wraps it into the box; the general form
+// takes displacements of four cells and more
+__device__ __forceinline__ void stream_coord(int& i, uint64_t& o, double v, const StepArgs& a, int L, unsigned& bad) {
+  int c;
+  if (stream_fixed(o, c, v, a.xh)) {
+    i += c;
+    wrap_cell(i, L);
+  } else {
+    split_coord((double)i + fma(v, a.h, offset_to_double(o)), L, i, o, bad);
   }
 }
 
@@ -321,70 +309,95 @@ __device__ __forceinline__ void wall_bounce(int walls, double ztop, double& x, d
   }
 }
 
+// kBoundary of the fluid pass: a periodic box; walls along z; rigid spheres
+// (with or without walls)
+constexpr int kPeriodic = 0, kWalled = 1, kSpheres = 2;
+
 // I: particle index type (32-bit whenever the particle count allows, so that
 // no 64-bit integer work competes with the float64 arithmetic).
-// kBoundary: walls or rigid spheres, streaming in unwrapped coordinates with
-// bounce-back; a separate instantiation, so that the common periodic pass
-// keeps the registers (about 60) that let its CTAs share the SMs with the MD
-// launch (the sphere bounce-back alone takes the kernel to over 100).
-template <typename I, bool kBoundary>
+// A particle's float64 operations are the collision map (9), its kinetic
+// energy (3) and nothing else: GB300 issues two per clock and SM, and with the
+// streaming, the wrap and the energy sum in float64 as well (26 with their
+// reductions) that pipe was 82 % busy at 134 us on 2.6 M particles.
+// Now 116 us there (float64 pipe still 70 % busy, issue 19 %); 36.5 to 33.9 us
+// a step on 32^3 x 10, 346 to 313 us on 80^3 x 10.
+// Walls and spheres are instantiations of their own, so that the common
+// periodic pass keeps the registers that let its CTAs share the SMs with the
+// MD launch (the sphere bounce-back alone takes the kernel to over 100).
+// Between walls only a particle that would leave the channel takes the
+// bounce-back's float64 path.
+template <typename I, int kBoundary>
 __global__ void __launch_bounds__(kThreads) k_fluid_step_f64(FluidF64 f, CellsF64 c, StepArgs a) {
   const int Lx = a.box.L[0], Ly = a.box.L[1], Lz = a.box.L[2];
-  const Thresh tcx = thresh(a.ta_cur[0]), tcy = thresh(a.ta_cur[1]), tcz = thresh(a.ta_cur[2]);
-  const Thresh tnx = thresh(a.ta_next[0]), tny = thresh(a.ta_next[1]), tnz = thresh(a.ta_next[2]);
   const double h = a.h, gk = a.gkick;
-  const bool kick = gk != 0.0, walls = kBoundary;
+  const bool kick = gk != 0.0;
   const I n = (I)f.n;
-  double ke_after = 0.0;
+  uint64_t ke_fixed = 0;  // sum of v'^2 in units of 2^-44 (flushed every 2^7 particles), and the rest
+  double ke_rest = 0.0;
+  int rounds = 0;
   unsigned bad = 0;
   for (I i = (I)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (I)gridDim.x * blockDim.x) {
     const uint32_t cp = f.cell[i];
     int ix = cell_x(cp), iy = cell_y(cp), iz = cell_z(cp);
-    double ox = f.ox[i], oy = f.oy[i], oz = f.oz[i];
+    uint64_t ox = f.ox[i], oy = f.oy[i], oz = f.oz[i];
     double vx = f.vx[i], vy = f.vy[i], vz = f.vz[i];
     // collision with the map of the shifted cell (box cells < 2^30: 32-bit index)
-    const uint32_t cid = (uint32_t)shifted(ix, ox, tcx, Lx) +
-                         (uint32_t)Lx * ((uint32_t)shifted(iy, oy, tcy, Ly) + (uint32_t)Ly * (uint32_t)shifted(iz, oz, tcz, Lz));
+    const uint32_t cid =
+        (uint32_t)shifted(ix, ox, a.xta_cur[0], Lx) +
+        (uint32_t)Lx * ((uint32_t)shifted(iy, oy, a.xta_cur[1], Ly) + (uint32_t)Ly * (uint32_t)shifted(iz, oz, a.xta_cur[2], Lz));
     apply_map_f64(c.par + 12 * (size_t)cid, vx, vy, vz);
-    const double k_post = vx * vx + vy * vy + vz * vz;
-    ke_after += k_post;
+    double K = vx * vx + vy * vy + vz * vz;
+    uint64_t q;
+    if (kinetic_fixed(K, q))
+      ke_fixed += q;
+    else
+      ke_rest += K;
+    if (++rounds == (1 << 7)) {
+      ke_rest += (double)ke_fixed * (1.0 / (double)(1ull << kKinBits));
+      ke_fixed = 0;
+      rounds = 0;
+    }
     // streaming
-    if (!walls) {
-      ox = fma(vx, h, ox);
-      oy = fma(vy, h, oy);
-      oz = fma(vz, h, oz);
-    } else {
-      double x = ix + ox, y = iy + oy, z = iz + oz;
-      double X[3] = {x, y, z}, V[3] = {vx, vy, vz};
-      if (a.sph.n && sphere_bounce(a.sph, a.box, h, X, V)) {
-        x = X[0];
-        y = X[1];
-        z = X[2];
+    bool turned = false;
+    if (kBoundary != kPeriodic) {
+      bool free_path = kBoundary == kWalled;
+      const int iz0 = iz;
+      const uint64_t oz0 = oz;
+      if (kBoundary == kWalled) {
+        // z stays in [0, Lz - 1]: no wrap, and the wall is at a cell's edge
+        int cz = 0;
+        free_path = stream_fixed(oz, cz, vz, a.xh);
+        iz += cz;
+        free_path = free_path && iz >= 0 && (iz < Lz - 1 || (iz == Lz - 1 && oz == 0));
+      }
+      if (!free_path) {
+        // bounce-back in unwrapped float64 coordinates
+        double X[3] = {ix + offset_to_double(ox), iy + offset_to_double(oy), iz0 + offset_to_double(oz0)};
+        double V[3] = {vx, vy, vz};
+        if (!(kBoundary == kSpheres && sphere_bounce(a.sph, a.box, h, X, V)))
+          for (int d = 0; d < 3; ++d) X[d] += V[d] * h;
+        if (a.walls) wall_bounce(a.walls, (double)(Lz - 1), X[0], X[1], X[2], V[0], V[1], V[2]);
         vx = V[0];
         vy = V[1];
         vz = V[2];
-      } else {
-        x += vx * h;
-        y += vy * h;
-        z += vz * h;
+        iz = iz0;
+        split_coord(X[0], Lx, ix, ox, bad);
+        split_coord(X[1], Ly, iy, oy, bad);
+        split_coord(X[2], Lz, iz, oz, bad);
+        turned = true;
       }
-      if (a.walls) wall_bounce(a.walls, (double)(Lz - 1), x, y, z, vx, vy, vz);
-      double fx = floor(x), fy = floor(y), fz = floor(z);
-      ox = x - fx;
-      oy = y - fy;
-      oz = z - fz;
-      ix = (((int)fx % Lx) + Lx) % Lx;
-      iy = (((int)fy % Ly) + Ly) % Ly;
-      iz = (((int)fz % Lz) + Lz) % Lz;
     }
-    rewrap(ox, ix, Lx, bad);
-    rewrap(oy, iy, Ly, bad);
-    rewrap(oz, iz, Lz, bad);
+    if (!turned) {
+      stream_coord(ix, ox, vx, a, Lx, bad);
+      stream_coord(iy, oy, vy, a, Ly, bad);
+      if (kBoundary == kPeriodic) stream_coord(iz, oz, vz, a, Lz, bad);
+    }
     if (kick) vx += gk;
     // bin with the next shift
-    const uint32_t cn = (uint32_t)shifted(ix, ox, tnx, Lx) +
-                        (uint32_t)Lx * ((uint32_t)shifted(iy, oy, tny, Ly) + (uint32_t)Ly * (uint32_t)shifted(iz, oz, tnz, Lz));
-    const double K = (kick || walls) ? vx * vx + vy * vy + vz * vz : k_post;
+    const uint32_t cn =
+        (uint32_t)shifted(ix, ox, a.xta_next[0], Lx) +
+        (uint32_t)Lx * ((uint32_t)shifted(iy, oy, a.xta_next[1], Ly) + (uint32_t)Ly * (uint32_t)shifted(iz, oz, a.xta_next[2], Lz));
+    if (kick || turned) K = vx * vx + vy * vy + vz * vz;
     double* sp = reinterpret_cast<double*>(c.sum + cn);
     atomicAdd(sp + 0, vx);
     atomicAdd(sp + 1, vy);
@@ -400,17 +413,30 @@ __global__ void __launch_bounds__(kThreads) k_fluid_step_f64(FluidF64 f, CellsF6
     f.vz[i] = vz;
   }
   if (bad) atomicOr(a.err, bad);
-  const double tot = block_sum_f64(ke_after);
-  if (threadIdx.x == 0 && tot != 0.0) atomicAdd(a.diss, -tot);
+  // the block's sum: integers up to the warp's, then one float64 per warp
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) ke_fixed += __shfl_xor_sync(0xffffffffu, ke_fixed, o);
+  __shared__ double s_ke[kThreads / 32];
+  __shared__ double s_rest;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  if (threadIdx.x == 0) s_rest = 0.0;
+  __syncthreads();
+  if (lane == 0) s_ke[wid] = (double)ke_fixed * (1.0 / (double)(1ull << kKinBits));
+  if (ke_rest != 0.0) atomicAdd(&s_rest, ke_rest);
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double tot = s_rest;
+    for (int w = 0; w < kThreads / 32; ++w) tot += s_ke[w];
+    if (tot != 0.0) atomicAdd(a.diss, -tot);
+  }
 }
 
 __global__ void k_bin_fluid_f64(FluidF64 f, CellsF64 c, StepArgs a) {
   const int Lx = a.box.L[0], Ly = a.box.L[1], Lz = a.box.L[2];
-  const Thresh tcx = thresh(a.ta_cur[0]), tcy = thresh(a.ta_cur[1]), tcz = thresh(a.ta_cur[2]);
   for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < f.n; i += (long)gridDim.x * blockDim.x) {
     const uint32_t cp = f.cell[i];
-    const long cid = shifted(cell_x(cp), f.ox[i], tcx, Lx) +
-                     (long)Lx * (shifted(cell_y(cp), f.oy[i], tcy, Ly) + (long)Ly * shifted(cell_z(cp), f.oz[i], tcz, Lz));
+    const long cid = shifted(cell_x(cp), f.ox[i], a.xta_cur[0], Lx) +
+                     (long)Lx * (shifted(cell_y(cp), f.oy[i], a.xta_cur[1], Ly) + (long)Ly * shifted(cell_z(cp), f.oz[i], a.xta_cur[2], Lz));
     const double vx = f.vx[i], vy = f.vy[i], vz = f.vz[i];
     double* sp = reinterpret_cast<double*>(c.sum + cid);
     atomicAdd(sp + 0, vx);
@@ -1056,9 +1082,9 @@ __global__ void k_load_fluid_f64(long n, const double* pos, const double* vel, B
     for (int q = 0; q < 3; ++q) wrap_coord_dev(pos[3 * i + q], box.L[q], c[q], o[q]);
     f.id[i] = (uint32_t)i;
     f.cell[i] = pack_cell(c[0], c[1], c[2]);
-    f.ox[i] = o[0];
-    f.oy[i] = o[1];
-    f.oz[i] = o[2];
+    f.ox[i] = offset_from_double(o[0]);
+    f.oy[i] = offset_from_double(o[1]);
+    f.oz[i] = offset_from_double(o[2]);
     f.vx[i] = vel[3 * i];
     f.vy[i] = vel[3 * i + 1];
     f.vz[i] = vel[3 * i + 2];
@@ -1086,6 +1112,15 @@ __global__ void k_load_fluid_f32(long n, const double* pos, const double* vel, B
   }
 }
 
+// float64 offsets (of an older snapshot) into fixed point, in place
+__global__ void k_convert_offsets(long n, uint64_t* o) {
+  for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
+    double d = __longlong_as_double((long long)o[i]);
+    if (!(d >= 0.0 && d < 1.0)) d = 0.5;
+    o[i] = offset_from_double(d);
+  }
+}
+
 // back to input order: particle k of the caller is the one with id k
 __global__ void k_store_fluid_f64(FluidF64 f, double* pos, double* vel, unsigned* bad) {
   for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < f.n; i += (long)gridDim.x * blockDim.x) {
@@ -1095,9 +1130,9 @@ __global__ void k_store_fluid_f64(FluidF64 f, double* pos, double* vel, unsigned
       continue;
     }
     const uint32_t cp = f.cell[i];
-    pos[3 * d] = __dadd_rn((double)cell_x(cp), f.ox[i]);
-    pos[3 * d + 1] = __dadd_rn((double)cell_y(cp), f.oy[i]);
-    pos[3 * d + 2] = __dadd_rn((double)cell_z(cp), f.oz[i]);
+    pos[3 * d] = __dadd_rn((double)cell_x(cp), offset_to_double(f.ox[i]));
+    pos[3 * d + 1] = __dadd_rn((double)cell_y(cp), offset_to_double(f.oy[i]));
+    pos[3 * d + 2] = __dadd_rn((double)cell_z(cp), offset_to_double(f.oz[i]));
     vel[3 * d] = f.vx[i];
     vel[3 * d + 1] = f.vy[i];
     vel[3 * d + 2] = f.vz[i];
@@ -1296,12 +1331,15 @@ int launch_fluid_step_f64(const FluidF64& f, const CellsF64& c, const StepArgs& 
   if (f.n == 0) return 0;
   const int grid = grid_for(f.n, kThreads, per_sm);
   const bool i32 = f.n + (long)grid * kThreads < (1L << 32);
-  if (a.walls != 0 || a.sph.n > 0)
-    i32 ? k_fluid_step_f64<uint32_t, true><<<grid, kThreads, 0, s>>>(f, c, a)
-        : k_fluid_step_f64<long, true><<<grid, kThreads, 0, s>>>(f, c, a);
+  if (a.sph.n > 0)
+    i32 ? k_fluid_step_f64<uint32_t, kSpheres><<<grid, kThreads, 0, s>>>(f, c, a)
+        : k_fluid_step_f64<long, kSpheres><<<grid, kThreads, 0, s>>>(f, c, a);
+  else if (a.walls != 0)
+    i32 ? k_fluid_step_f64<uint32_t, kWalled><<<grid, kThreads, 0, s>>>(f, c, a)
+        : k_fluid_step_f64<long, kWalled><<<grid, kThreads, 0, s>>>(f, c, a);
   else
-    i32 ? k_fluid_step_f64<uint32_t, false><<<grid, kThreads, 0, s>>>(f, c, a)
-        : k_fluid_step_f64<long, false><<<grid, kThreads, 0, s>>>(f, c, a);
+    i32 ? k_fluid_step_f64<uint32_t, kPeriodic><<<grid, kThreads, 0, s>>>(f, c, a)
+        : k_fluid_step_f64<long, kPeriodic><<<grid, kThreads, 0, s>>>(f, c, a);
   return 1;
 }
 int launch_bin_fluid_f64(const FluidF64& f, const CellsF64& c, const StepArgs& a, cudaStream_t s) {
@@ -1459,6 +1497,11 @@ int launch_load_fluid_f32(long n, const double* pos, const double* vel, const Bo
                           cudaStream_t s) {
   if (n == 0) return 0;
   k_load_fluid_f32<<<grid_for(n), kThreads, 0, s>>>(n, pos, vel, box, f);
+  return 1;
+}
+int launch_convert_offsets(long n, uint64_t* o, cudaStream_t s) {
+  if (n == 0) return 0;
+  k_convert_offsets<<<grid_for(n), kThreads, 0, s>>>(n, o);
   return 1;
 }
 int launch_store_fluid_f64(const FluidF64& f, double* pos, double* vel, unsigned* bad, cudaStream_t s) {
