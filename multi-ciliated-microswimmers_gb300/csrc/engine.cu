@@ -46,7 +46,7 @@ struct mpcd_engine {
   // launch shape of the fluid pass beside the MD launch: > 0 persistent with that
   // many CTAs per SM, <= 0 short-lived CTAs of -fluid_per_sm (at least 1)
   // particles per thread
-  int fluid_per_sm = -1;
+  int fluid_per_sm = 0;  // 0: 16 in float64 (CTAs of 128 threads), -1 in split precision
   std::string error;
   long long launches = 0;
 
@@ -314,6 +314,7 @@ StepArgs step_args(mpcd_engine* h, const double* a_cur, const double* a_next, do
   s.h = h->p.tstep;
   s.xh = fixed_step(h->p.tstep);
   s.gkick = h->p.gravity != 0.0 ? h->p.gravity * std::cos(t_move * h->p.omega) * h->p.tstep : 0.0;
+  s.xstep = stream_step(h->p.tstep, s.gkick, &s.xkick);
   s.walls = h->p.walls;
   s.bead_mass = h->p.bead_mass;
   s.seed = h->p.seed;
@@ -829,7 +830,7 @@ int mpcd_create(const mpcd_params* params, mpcd_engine** out) {
     if ((e = cudaEventCreateWithFlags(&h->ev_join, cudaEventDisableTiming)) != cudaSuccess) return bail(e, "event");
     const char* env = std::getenv("MPCD_MD_OVERLAP");  // 0: MD after the fluid pass on one stream
     h->overlap = !(env && std::atoi(env) == 0);
-    if (const char* f = std::getenv("MPCD_FLUID_PER_SM")) h->fluid_per_sm = std::max(-64, std::min(8, std::atoi(f)));
+    if (const char* f = std::getenv("MPCD_FLUID_PER_SM")) h->fluid_per_sm = std::max(-64, std::min(16, std::atoi(f)));
   }
   if ((e = dalloc(&h->d_err, 1)) != cudaSuccess) return bail(e, "alloc");
   if ((e = dalloc(&h->d_diss, 1)) != cudaSuccess) return bail(e, "alloc");
@@ -1297,13 +1298,15 @@ int mpcd_step(mpcd_engine* h, const mpcd_inject* inj) {
     h->launches += f64 ? launch_cell_params_f64(h->c64, s, h->stream) : launch_cell_params_f32(h->c32, s, h->stream);
   }
   {
-    // beside the MD launch the fluid pass runs as many short-lived CTAs (one
-    // round of particles per thread): as they retire, the higher-priority MD
-    // CTAs take their place, and the fluid CTAs fill what the MD leaves of
-    // every SM (swimmer64 float64: 0.336 ms per step against 0.405 with a
-    // persistent grid of 3 CTAs per SM)
+    // beside the MD launch the split-precision fluid pass runs as many
+    // short-lived CTAs (one round of particles per thread): as they retire, the
+    // higher-priority MD CTAs take their place, and the fluid CTAs fill what
+    // the MD leaves of every SM.  The float64 pass takes 16 CTAs of 128 threads
+    // per SM, two rounds of the eight that fit, alone and beside the MD
+    // (swimmer64: 228 us per step; one particle per thread 248, two 237; 8 per
+    // SM 250, 12 234)
     ProfScope ps(h, MPCD_K_FLUID);
-    const int per_sm = fork ? h->fluid_per_sm : 4;
+    const int per_sm = fork && h->fluid_per_sm ? h->fluid_per_sm : (f64 ? 16 : (fork ? -1 : 4));
     h->launches += f64 ? launch_fluid_step_f64(h->f64, h->c64, s, h->stream, per_sm)
                        : launch_fluid_step_f32(h->f32, h->c32, s, h->stream, per_sm);
   }

@@ -5,7 +5,7 @@
 
 #include <cuda_runtime.h>
 
-#include "fixed_offset.cuh"
+#include "fixed_collide.cuh"
 #include "mpcd_device.cuh"
 
 namespace mpcd {
@@ -31,7 +31,7 @@ struct FluidF32 {
 
 // Per-cell state.  sum: (P_x, P_y, P_z, K) mass-weighted; cnt: fluid count in
 // the low 16 bits, bead count in the high 16 bits.  par: collision map
-// v' = A v + b, stored as A (row-major 3x3) then b (12 values per cell).
+// v' = A v + b, twelve words per cell (fixed_collide.cuh).
 struct CellsF64 {
   long ncell = 0;
   double4* sum = nullptr;
@@ -71,7 +71,9 @@ struct StepArgs {
   double a_cur[3];
   double a_next[3];
   uint64_t xta_cur[3], xta_next[3];  // ta_* as thresholds of fixed-point offsets
-  FixedStep xh;       // h for streaming fixed-point offsets
+  FixedStep xh;       // h for streaming fixed-point offsets by a float64 velocity
+  StreamStep xstep;   // and by a fixed-point one
+  int64_t xkick;      // gkick in units of 2^-56; a larger one leaves no velocity that fits
   double h;           // MPC time step
   double gkick;       // gravity * cos(omega t) * h, added to v_x after streaming
   int walls;          // MPCD_WALLS_*

@@ -1,0 +1,207 @@
+// The SRD collision of the float64 fluid in 64-bit fixed point: the collision
+// map of a cell from its sums, and its application to a particle.
+//
+// GB300 issues about one float64 operation per clock and SM against 64 and
+// more 32-bit integer ones, so that a float64 multiply-add costs as much as
+// about fifty integer instructions: with the map, the kinetic energy and the
+// streaming in float64 the fluid pass and the cell maps were bound by that
+// pipe (73-82 % busy, everything else idle).  A 64 x 64 product takes three or
+// four 32 x 32 -> 64 multiply-adds here.
+//
+// All quantities are two's-complement integers times a power of two chosen so
+// that the thermal range has bits to spare: velocities and mean velocities in
+// units of 2^-58, new velocities 2^-56, map entries 2^-59, axis components and
+// the thermostat factor 2^-60.  A rounding is half a unit of these, against
+// 2^-54 for float64 numbers of one half and more, so results are at least as close to the exact ones as
+// the float64 form's wherever the terms of a sum are of order one.  What does
+// not fit (velocities of 16 thermal velocities and more, mean velocities of 8,
+// thermostat factors of 2, kinetic energies of a cell of 4096, momenta of 512,
+// non-finite values) takes the float64 form, about half as fast.
+//
+// Host and device code alike (tests run it on the CPU).
+#pragma once
+#include "fixed_offset.cuh"
+
+namespace mpcd {
+
+MPCD_HD double bits_f64(uint64_t u) {
+#ifdef __CUDA_ARCH__
+  return __longlong_as_double((long long)u);
+#else
+  double x;
+  std::memcpy(&x, &u, sizeof x);
+  return x;
+#endif
+}
+MPCD_HD int clz64(uint64_t x) {  // x != 0
+#ifdef __CUDA_ARCH__
+  return __clzll((long long)x);
+#else
+  return __builtin_clzll(x);
+#endif
+}
+
+// x in units of 2^-BITS, truncated towards zero; |x| < 2^EMAX, BITS + EMAX <= 62.
+// False (r unchanged) for larger values, infinities and NaN.
+template <int BITS, int EMAX>
+MPCD_HD bool to_fixed(double x, int64_t& r) {
+  static_assert(BITS + EMAX <= 62 && BITS + EMAX >= 53, "significand shifted left, sign kept");
+  const uint64_t b = f64_bits(x);
+  const uint32_t hi = (uint32_t)(b >> 32), lo = (uint32_t)b;
+  if ((hi & 0x7fffffffu) >= (uint32_t)(1023 + EMAX) << 20) return false;
+  const uint64_t m = ((uint64_t)((hi & 0xfffffu) | 0x100000u) << 32 | lo) << (BITS + EMAX - 53);
+  const int s = 1022 + EMAX - (int)((hi >> 20) & 0x7ffu);
+  const int64_t d = s < 64 ? (int64_t)(m >> s) : 0;
+  const int64_t sg = -(int64_t)(hi >> 31);
+  r = (d ^ sg) - sg;
+  return true;
+}
+
+// x 2^-bits to the nearest float64
+MPCD_HD double from_fixed(int64_t x, int bits) {
+  const uint64_t sg = (uint64_t)x >> 63;
+  const uint64_t m = sg ? 0ull - (uint64_t)x : (uint64_t)x;
+  if (m == 0) return 0.0;
+  const int lz = clz64(m);
+  const uint64_t n = m << lz;
+  const uint64_t mant = (n >> 11) + ((n >> 10) & 1u);  // 2^52 .. 2^53
+  return bits_f64((sg << 63) | (((uint64_t)(1023 + 63 - lz - bits - 1) << 52) + mant));
+}
+
+// h 2^32 + l with a signed low half: products of halves need no correction
+struct Limbs {
+  int32_t h, l;
+};
+MPCD_HD Limbs split_limbs(int64_t x) {
+  const int32_t l = (int32_t)(uint32_t)x;
+  return {(int32_t)((uint64_t)x >> 32) + (l < 0 ? 1 : 0), l};
+}
+MPCD_HD int64_t wide(int32_t a, int32_t b) { return (int64_t)a * b; }
+MPCD_HD uint64_t uwide(int32_t a, int32_t b) { return (uint64_t)((int64_t)a * b); }
+
+// a b 2^-S, rounded to within one unit; |a|, |b| <= 2^62 and the result within 2^62
+template <int S>
+MPCD_HD int64_t mul_sh(Limbs a, Limbs b) {
+  static_assert(S >= 34 && S <= 63, "shift");
+  const int64_t mid = wide(a.h, b.l) + wide(a.l, b.h) + (wide(a.l, b.l) >> 32) + (1ll << (S - 33));
+  return (int64_t)((uint64_t)wide(a.h, b.h) << (64 - S)) + (mid >> (S - 32));
+}
+
+// ------------------------------------------------------------ the map ---
+// Twelve words per cell: the matrix A (row-major, units of 2^-59, each word a
+// Limbs) and b (units of 2^-56) of v' = A v + b.  A cell whose numbers do not
+// fit holds kMapF64 in its first word instead, and the thermostat factor, the
+// rotation axis and the mean velocity as float64 in the next seven.
+constexpr int kVelBits = 58;         // velocities that go in, up to 16; mean velocities
+constexpr int kMapBits = 59;         // entries of A
+constexpr int kAxisBits = 60;        // axis components, thermostat factor
+constexpr int kOutBits = 56;         // velocities that come out: up to 92 with the limits below
+constexpr int64_t kMeanMax = 1ll << 61;  // 8, mean velocities
+constexpr uint64_t kMapF64 = 0x7fffffff00000000ull;
+
+MPCD_HD Limbs word_limbs(uint64_t w) { return {(int32_t)(w >> 32), (int32_t)(uint32_t)w}; }
+
+// a float in (-2, 2) in units of 2^-60
+MPCD_HD int64_t axis_fixed(float f) {
+#ifdef __CUDA_ARCH__
+  const uint32_t u = __float_as_uint(f);
+#else
+  uint32_t u;
+  std::memcpy(&u, &f, sizeof u);
+#endif
+  const int s = 127 - (int)((u >> 23) & 0xffu);
+  const int64_t d = s < 64 ? (int64_t)((uint64_t)((u & 0x7fffffu) | 0x800000u) << 37 >> s) : 0;
+  return (u >> 31) ? -d : d;
+}
+// r (units of 2^-60, |r|^2 = 1 + e with |e| < 2^-20) to unit length: r (1 - e/2 + 3 e^2/8)
+MPCD_HD void axis_normalise(int64_t* r) {
+  const Limbs x = split_limbs(r[0]), y = split_limbs(r[1]), z = split_limbs(r[2]);
+  const int64_t e = mul_sh<60>(x, x) + mul_sh<60>(y, y) + mul_sh<60>(z, z) - (1ll << 60);
+  const int32_t e8 = (int32_t)(e >> 12);
+  const int64_t e2 = wide(e8, e8) >> 36;  // e^2
+  const Limbs d = split_limbs((e >> 1) - ((3 * e2) >> 3));
+  r[0] -= mul_sh<60>(x, d);
+  r[1] -= mul_sh<60>(y, d);
+  r[2] -= mul_sh<60>(z, d);
+}
+
+// constants in units of 2^-60: cos and sin of the rotation angle as the
+// reference uses them (src/libcilia/mpcd.h:72-76)
+MPCD_HD int64_t unit60(double x) { return (int64_t)(x * 1152921504606846976.0); }
+
+// The map's words from the axis r and factor sc (units of 2^-60) and the mean
+// velocity u (2^-58): A = sc R, b = u - A u, R the rotation with the entries of
+// src/libcilia/mpcd.cpp:285-293 (R_ii = r_i^2 (1 - ca) + ca, R_ij = r_i r_j (1 -
+// ca) -+ r_k sa).
+MPCD_HD void map_words(const int64_t* r, int64_t sc, const int64_t* u, double cos_a, double sin_a, uint64_t* w) {
+  const Limbs x = split_limbs(r[0]), y = split_limbs(r[1]), z = split_limbs(r[2]);
+  const Limbs oc = split_limbs(unit60(1.0 - cos_a)), sa = split_limbs(unit60(sin_a)), f = split_limbs(sc);
+  const int64_t ca = unit60(cos_a);
+  const Limbs tx = split_limbs(mul_sh<60>(x, oc)), ty = split_limbs(mul_sh<60>(y, oc)), tz = split_limbs(mul_sh<60>(z, oc));
+  const int64_t sx = mul_sh<60>(x, sa), sy = mul_sh<60>(y, sa), sz = mul_sh<60>(z, sa);
+  const int64_t xy = mul_sh<60>(tx, y), xz = mul_sh<60>(tx, z), yz = mul_sh<60>(ty, z);
+  const int64_t R[9] = {mul_sh<60>(tx, x) + ca, xy - sz, xz + sy, xy + sz, mul_sh<60>(ty, y) + ca, yz - sx,
+                        xz - sy, yz + sx, mul_sh<60>(tz, z) + ca};
+  const Limbs ux = split_limbs(u[0]), uy = split_limbs(u[1]), uz = split_limbs(u[2]);
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    Limbs a[3];
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+      a[j] = split_limbs(mul_sh<61>(split_limbs(R[3 * i + j]), f));
+      w[3 * i + j] = (uint64_t)(uint32_t)a[j].h << 32 | (uint32_t)a[j].l;
+    }
+    const int64_t b = ((u[i] + 1) >> 1) - mul_sh<60>(a[0], ux) - mul_sh<60>(a[1], uy) - mul_sh<60>(a[2], uz);  // 2^-57
+    w[9 + i] = (uint64_t)((b + 1) >> 1);
+  }
+}
+
+// v' = A v + b in units of 2^-56 (|v_i| < 16, sc < 2 and |u_i| < 8 keep every sum
+// within 63 bits; anything else gives some number and no harm).  The products of low halves are left out
+// (up to two units each, 1.2 together in the mean square).
+MPCD_HD void apply_words(const uint64_t* w, const int64_t* v, int64_t* out) {
+  const Limbs x = split_limbs(v[0]), y = split_limbs(v[1]), z = split_limbs(v[2]);
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    const Limbs a = word_limbs(w[3 * i]), b = word_limbs(w[3 * i + 1]), c = word_limbs(w[3 * i + 2]);
+    const uint64_t top = uwide(a.h, x.h) + uwide(b.h, y.h) + uwide(c.h, z.h);
+    const uint64_t mid = uwide(a.h, x.l) + uwide(b.h, y.l) + uwide(c.h, z.l) + uwide(a.l, x.h) + uwide(b.l, y.h) + uwide(c.l, z.h);
+    out[i] = (int64_t)((top << 3) + (uint64_t)((int64_t)(mid + (1u << 28)) >> 29) + w[9 + i]);
+  }
+}
+
+// sum of v_i^2 in units of 2^-52, v_i in units of 2^-58 with |v_i| < 16
+constexpr int kSquareBits = 52;
+constexpr int kEnergyBits = 40;  // of the sums of kinetic energies
+MPCD_HD int64_t square_words(Limbs x, Limbs y, Limbs z) {
+  const int64_t top = wide(x.h, x.h) + wide(y.h, y.h) + wide(z.h, z.h);
+  const int64_t mid = wide(x.h, x.l) + wide(y.h, y.l) + wide(z.h, z.l);
+  return top + (mid >> 31);
+}
+
+// The time step for stream_words in units of 2^-61 (exact for 2^-9 <= h < 2),
+// and the high word of the velocity bound (units of 2^-56) below which |v| < 16
+// and |v| h < 4.  The bound is zero for larger steps: all in float64.
+struct StreamStep {
+  Limbs h = {0, 0};
+  int32_t vmax = 0;
+};
+// kick: a change of the velocity that is added after the bound was checked,
+// returned in units of 2^-56.
+inline StreamStep stream_step(double h, double kick, int64_t* xkick) {
+  StreamStep s;
+  *xkick = 0;
+  if (!(h >= 0 && h < 2 && std::fabs(kick) < 8)) return s;
+  s.h = split_limbs(std::llround(std::ldexp(h, 61)));
+  *xkick = std::llround(std::ldexp(kick, kOutBits));
+  s.vmax = (int32_t)std::floor(std::ldexp(std::fmin(16.0 - std::fabs(kick), 4.0 / h), kOutBits - 32));
+  return s;
+}
+// Streams an offset by v h, v in units of 2^-58.
+MPCD_HD void stream_words(uint64_t& k, int& cells, Limbs v, const StreamStep& s) {
+  const int64_t u = (int64_t)k + mul_sh<59>(v, s.h);
+  cells = (int)(u >> kOffBits);
+  k = (uint64_t)u & (kOffOne - 1);
+}
+
+}  // namespace mpcd

@@ -95,17 +95,4 @@ MPCD_HD bool stream_fixed(uint64_t& k, int& cells, double v, const FixedStep& h)
   return true;
 }
 
-// A non-negative float64 below 2^7 in units of 2^-44, rounded; false for
-// larger values (and infinities, NaN).  Up to 2^12 of them add up in 63 bits.
-constexpr int kKinBits = 44;
-MPCD_HD bool kinetic_fixed(double x, uint64_t& q) {
-  const uint64_t b = f64_bits(x);
-  const int e = (int)(b >> 52);  // the sign bit makes a negative value too large
-  if (e >= 1023 + 7) return false;
-  const uint64_t m = (b & 0xfffffffffffffull) | 0x10000000000000ull;
-  const int s = 1023 + 52 - kKinBits - e;  // x = m 2^(e - 1075)
-  q = s < 64 ? (m + (1ull << (s - 1))) >> s : 0ull;
-  return true;
-}
-
 }  // namespace mpcd

@@ -2,6 +2,7 @@
 // and the replica batch (batch_kernels.cu).
 #pragma once
 #include "engine_internal.h"
+#include "fixed_collide.cuh"
 
 namespace mpcd {
 
@@ -383,14 +384,53 @@ __device__ __forceinline__ void cell_map_f32(const float4 s0, const uint32_t w, 
   }
 }
 
-// v' = A v + b with the float64 map of one cell (A row-major, then b)
+// A and b of v' = A v + b from the thermostat factor, the axis and the mean
+// velocity in float64: A = sc R, R the rotation by alpha with the entries of
+// src/libcilia/mpcd.cpp:285-293 (R_ii = r_i^2 + (1 - r_i^2) ca,
+// R_ij = r_i r_j (1 - ca) -+ r_k sa), the factor sc folded in:
+// A_ii = (sc oc r_i) r_i + sc ca, A_ij = (sc oc r_i) r_j -+ sc sa r_k
+__device__ __forceinline__ void map_from_axis(double sc, double rx, double ry, double rz, double ux, double uy, double uz,
+                                              double* A, double* b) {
+  const double ca = kCosAlpha, sa = kSinAlpha, oc = 1.0 - kCosAlpha;
+  const double sco = sc * oc, scc = sc * ca, scs = sc * sa;
+  const double tx = sco * rx, ty = sco * ry, tz = sco * rz;
+  const double qx = scs * rx, qy = scs * ry, qz = scs * rz;
+  A[0] = fma(tx, rx, scc);
+  A[1] = fma(tx, ry, -qz);
+  A[2] = fma(tx, rz, qy);
+  A[3] = fma(tx, ry, qz);
+  A[4] = fma(ty, ry, scc);
+  A[5] = fma(ty, rz, -qx);
+  A[6] = fma(tx, rz, -qy);
+  A[7] = fma(ty, rz, qx);
+  A[8] = fma(tz, rz, scc);
+  b[0] = ux - (A[0] * ux + A[1] * uy + A[2] * uz);
+  b[1] = uy - (A[3] * ux + A[4] * uy + A[5] * uz);
+  b[2] = uz - (A[6] * ux + A[7] * uy + A[8] * uz);
+}
+
+// v' = A v + b in float64 with the map of one cell (fixed_collide.cuh: words
+// in fixed point, or factor, axis and mean velocity)
 __device__ __forceinline__ void apply_map_f64(const double* par, double& vx, double& vy, double& vz) {
-  const double2* p = reinterpret_cast<const double2*>(par);
-  const double2 p0 = __ldg(p + 0), p1 = __ldg(p + 1), p2 = __ldg(p + 2);
-  const double2 p3 = __ldg(p + 3), p4 = __ldg(p + 4), p5 = __ldg(p + 5);
-  const double nx = fma(p0.x, vx, fma(p0.y, vy, fma(p1.x, vz, p4.y)));
-  const double ny = fma(p1.y, vx, fma(p2.x, vy, fma(p2.y, vz, p5.x)));
-  const double nz = fma(p3.x, vx, fma(p3.y, vy, fma(p4.x, vz, p5.y)));
+  const uint64_t* w = reinterpret_cast<const uint64_t*>(par);
+  double A[9], b[3];
+  if (__ldg(w) == kMapF64) {
+    double d[7];
+#pragma unroll
+    for (int q = 0; q < 7; ++q) d[q] = __ldg(par + 1 + q);
+    map_from_axis(d[0], d[1], d[2], d[3], d[4], d[5], d[6], A, b);
+  } else {
+#pragma unroll
+    for (int q = 0; q < 9; ++q) {
+      const Limbs p = word_limbs(__ldg(w + q));
+      A[q] = from_fixed((int64_t)((uint64_t)(int64_t)p.h << 32) + p.l, kMapBits);
+    }
+#pragma unroll
+    for (int q = 0; q < 3; ++q) b[q] = from_fixed((int64_t)__ldg(w + 9 + q), kOutBits);
+  }
+  const double nx = fma(A[0], vx, fma(A[1], vy, fma(A[2], vz, b[0])));
+  const double ny = fma(A[3], vx, fma(A[4], vy, fma(A[5], vz, b[1])));
+  const double nz = fma(A[6], vx, fma(A[7], vy, fma(A[8], vz, b[2])));
   vx = nx;
   vy = ny;
   vz = nz;

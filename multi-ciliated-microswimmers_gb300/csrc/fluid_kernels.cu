@@ -105,15 +105,19 @@ __device__ __forceinline__ void stream_coord(int& i, uint64_t& o, double v, cons
   }
 }
 
-// 1/n for the particle counts of bead-free cells, rounded once as the IEEE
-// division rounds it (the same bits as 1.0 / n at run time), so that the
-// common cell needs no float64 division on GB300's small FP64 pipe
+// 1/n for the particle counts of bead-free cells: rounded once as the IEEE
+// division rounds it (the same bits as 1.0 / n at run time), and in units of
+// 2^-62 for the fixed-point form
 struct InvTable {
   double v[256];
+  int64_t x[256];
 };
 constexpr InvTable make_inv_table() {
   InvTable t{};
-  for (int i = 1; i < 256; ++i) t.v[i] = 1.0 / i;
+  for (int i = 1; i < 256; ++i) {
+    t.v[i] = 1.0 / i;
+    t.x[i] = (int64_t)(((1ull << 62) + (unsigned)i / 2) / (unsigned)i);
+  }
   return t;
 }
 __device__ const InvTable g_inv_n = make_inv_table();
@@ -143,68 +147,105 @@ __device__ __forceinline__ void draw_axis_f64(uint64_t seed, uint64_t step, uint
   rz *= y2;
 }
 
-__device__ __forceinline__ void collision_map(double4 s, uint32_t w, long cid, const StepArgs& a, double* A,
-                                              double* b, double& ldiss, unsigned& errbits, bool& gfail) {
-  const int nf = cnt_fluid(w), nb = cnt_beads(w);
-  int num = nf + nb;
-  double M = (double)nf + (double)nb * a.bead_mass;
-  const double preal[3] = {s.x, s.y, s.z}, mreal = M;  // the real particles' momentum and mass
-  int sk = -1;  // rigid sphere whose surface cuts the cell
-  double rel[3];
-  if (a.sph.n && num < 10 && !(a.walls && wall_layer_cell(a.box, cid))) {
+// the same direction in units of 2^-60
+__device__ __forceinline__ void draw_axis_fixed(uint64_t seed, uint64_t step, uint32_t cid, int64_t* r) {
+  const u32x4 q = draw4(seed, step, kStreamCell, cid, 0u);
+  const float ct = 2.0f * u01_flt(q.y) - 1.0f;
+  const float st = sqrtf(fmaxf(0.0f, 1.0f - ct * ct));
+  float sp, cp;
+  sincospif(2.0f * u01_flt(q.x), &sp, &cp);
+  r[0] = axis_fixed(st * cp);
+  r[1] = axis_fixed(st * sp);
+  r[2] = axis_fixed(ct);
+  axis_normalise(r);
+}
+
+// The thermostat factor sqrt(g / (erel / 2)) = 2g / sqrt(2g erel): one
+// reciprocal square root in place of a float64 division and square root;
+// outside the float range the direct form.
+__device__ __forceinline__ double thermostat_factor(double g, double erel) {
+  const double q = 2.0 * g, x = q * erel;
+  return (x > 1e-30 && x < 1e30) ? q * rsqrt_f64(x) : sqrt(g / (erel * 0.5));
+}
+// the same for a float g > 0: the seed's conversions and the range check on
+// the bit patterns (they are float64 instructions otherwise)
+__device__ __forceinline__ double thermostat_factor(float g, double erel) {
+  const uint32_t gb = __float_as_uint(g);
+  const double q = __hiloint2double((int)((gb >> 3) + (897u << 20)), (int)(gb << 29));  // 2 g
+  const double x = q * erel;
+  const uint32_t hi = (uint32_t)__double2hiint(x);
+  if (hi - (923u << 20) >= (200u << 20)) return sqrt((double)g / (erel * 0.5));  // x outside 2^-100 .. 2^100
+  const float y0 = rsqrtf(__uint_as_float(((hi - (896u << 20)) << 3) | ((uint32_t)__double2loint(x) >> 29)));
+  const uint32_t yb = __float_as_uint(y0);
+  const double y = __hiloint2double((int)((yb >> 3) + (896u << 20)), (int)(yb << 29));
+  const double r = fma(-x * y, y, 1.0);
+  return q * fma(y * r, fma(0.375, r, 0.5), y);
+}
+
+// A cell on its way to the map: its sums (virtual particles included), the
+// real particles' momentum and mass, and the sphere that cuts it.
+struct CellSums {
+  double4 s;
+  double M;
+  int num;
+  int sk;  // rigid sphere whose surface cuts the cell, or -1
+  double rel[3], preal[3], mreal;
+};
+
+// Virtual particles up to rho = 10 in cells cut by a sphere's surface (moving
+// with it) or in the wall layers.  Not inlined, like the float64 map below:
+// the common path fits the instruction cache better without them.
+__device__ __noinline__ void add_virtual(CellSums& t, long cid, const StepArgs& a) {
+  const bool wall = a.walls && wall_layer_cell(a.box, cid);
+  if (a.sph.n && !wall) {
     const int L0 = a.box.L[0], L1 = a.box.L[1];
-    sk = sphere_cut_cell(a.sph, a.box, a.a_cur, (int)(cid % L0), (int)((cid / L0) % L1), (int)(cid / ((long)L0 * L1)),
-                         rel);
-    if (sk >= 0) {  // virtual particles up to rho = 10, moving with the surface
-      const int dm = 10 - num;
-      double pv[3];
-      sphere_virtual(a.sph.s[sk], rel, dm, a.seed, a.step, (uint32_t)cid, a.inj_virt, pv);
-      s.x += pv[0];
-      s.y += pv[1];
-      s.z += pv[2];
-      s.w += (pv[0] * pv[0] + pv[1] * pv[1] + pv[2] * pv[2]) / dm;
-      M += dm;
-      num += dm;
-    }
+    t.sk = sphere_cut_cell(a.sph, a.box, a.a_cur, (int)(cid % L0), (int)((cid / L0) % L1), (int)(cid / ((long)L0 * L1)),
+                           t.rel);
   }
-  if (a.walls && num < 10 && wall_layer_cell(a.box, cid)) {  // virtual particles up to rho = 10
-    const int dm = 10 - num;
-    double pv[3];
-    if (a.inj_virt) {
-      pv[0] = a.inj_virt[3 * cid];
-      pv[1] = a.inj_virt[3 * cid + 1];
-      pv[2] = a.inj_virt[3 * cid + 2];
-    } else {
-      virtual_momentum(a.seed, a.step, (uint32_t)cid, dm, pv);
-    }
-    s.x += pv[0];
-    s.y += pv[1];
-    s.z += pv[2];
-    s.w += (pv[0] * pv[0] + pv[1] * pv[1] + pv[2] * pv[2]) / dm;
-    M += dm;
-    num += dm;
+  if (t.sk < 0 && !wall) return;
+  const int dm = 10 - t.num;
+  double pv[3];
+  if (t.sk >= 0) {
+    t.preal[0] = t.s.x;
+    t.preal[1] = t.s.y;
+    t.preal[2] = t.s.z;
+    t.mreal = t.M;
+    sphere_virtual(a.sph.s[t.sk], t.rel, dm, a.seed, a.step, (uint32_t)cid, a.inj_virt, pv);
+  } else if (a.inj_virt) {
+    pv[0] = a.inj_virt[3 * cid];
+    pv[1] = a.inj_virt[3 * cid + 1];
+    pv[2] = a.inj_virt[3 * cid + 2];
+  } else {
+    virtual_momentum(a.seed, a.step, (uint32_t)cid, dm, pv);
   }
-  const double inv = (nb == 0 && num < 256) ? __ldg(g_inv_n.v + num) : 1.0 / M;  // M = num without beads
-  const double ux = s.x * inv, uy = s.y * inv, uz = s.z * inv;
+  t.s.x += pv[0];
+  t.s.y += pv[1];
+  t.s.z += pv[2];
+  t.s.w += (pv[0] * pv[0] + pv[1] * pv[1] + pv[2] * pv[2]) / dm;
+  t.M += dm;
+  t.num += dm;
+}
+
+// the Gamma draw of a cell of num > 1 particles, injected or generated
+__device__ __forceinline__ double injected_gamma(const StepArgs& a, long cid, unsigned& errbits) {
+  const double g = a.inj_gamma[cid];
+  if (g < 0) {
+    errbits |= kErrGammaMissing;
+    return 0.0;
+  }
+  return g;
+}
+
+// The map in float64, for cells whose numbers do not fit the fixed-point form
+// and for cells cut by a sphere, whose impulse follows from it.
+__device__ __noinline__ unsigned map_f64(const CellSums& t, long cid, float gf, uint64_t* out, const StepArgs& a) {
+  unsigned errbits = 0;
+  const double4 s = t.s;
+  const double dinv = 1.0 / t.M;
+  const double ux = s.x * dinv, uy = s.y * dinv, uz = s.z * dinv;
   const double erel = s.w - (ux * s.x + uy * s.y + uz * s.z);  // K - M u^2
   double sc = 1.0;
-  if (erel > 0 && num > 1) {
-    double g;
-    if (a.inj_gamma) {
-      g = a.inj_gamma[cid];
-      if (g < 0) {
-        errbits |= kErrGammaMissing;
-        g = 0.0;
-      }
-    } else {
-      g = (double)gamma_mt(num, a.seed, a.step, (uint32_t)cid, &gfail);
-    }
-    // sqrt(g / (erel / 2)) = 2g / sqrt(2g erel): one reciprocal square root in
-    // place of a float64 division and square root (the cell pass is bound
-    // by the float64 pipe); outside the float range the direct form
-    const double q = 2.0 * g, x = q * erel;
-    sc = (x > 1e-30 && x < 1e30) ? q * rsqrt_f64(x) : sqrt(g / (erel * 0.5));
-  }
+  if (erel > 0 && t.num > 1) sc = thermostat_factor(a.inj_gamma ? injected_gamma(a, cid, errbits) : (double)gf, erel);
   double rx, ry, rz;
   if (a.inj_axis) {
     rx = a.inj_axis[3 * cid + 0];
@@ -213,70 +254,180 @@ __device__ __forceinline__ void collision_map(double4 s, uint32_t w, long cid, c
   } else {
     draw_axis_f64(a.seed, a.step, (uint32_t)cid, rx, ry, rz);
   }
-  const double ca = kCosAlpha, sa = kSinAlpha, oc = 1.0 - kCosAlpha;
-  // A = sc R, R the rotation about (rx, ry, rz) by alpha with the entries of
-  // src/libcilia/mpcd.cpp:285-293 (R_ii = r_i^2 + (1 - r_i^2) ca,
-  // R_ij = r_i r_j (1 - ca) -+ r_k sa), the factor sc folded in:
-  // A_ii = (sc oc r_i) r_i + sc ca, A_ij = (sc oc r_i) r_j -+ sc sa r_k
-  const double sco = sc * oc, scc = sc * ca, scs = sc * sa;
-  const double tx = sco * rx, ty = sco * ry, tz = sco * rz;
-  const double qx = scs * rx, qy = scs * ry, qz = scs * rz;
-  A[0] = fma(tx, rx, scc);
-  A[1] = fma(tx, ry, -qz);
-  A[2] = fma(tx, rz, qy);
-  A[3] = fma(tx, ry, qz);
-  A[4] = fma(ty, ry, scc);
-  A[5] = fma(ty, rz, -qx);
-  A[6] = fma(tx, rz, -qy);
-  A[7] = fma(ty, rz, qx);
-  A[8] = fma(tz, rz, scc);
-  b[0] = ux - (A[0] * ux + A[1] * uy + A[2] * uz);
-  b[1] = uy - (A[3] * ux + A[4] * uy + A[5] * uz);
-  b[2] = uz - (A[6] * ux + A[7] * uy + A[8] * uz);
-  if (sk >= 0) {
+  if (t.sk >= 0) {
     // the real particles' momentum after the collision is A P + M b; what
     // they gained came from the virtual particles, i.e. from the sphere
-    double J[3];
-#pragma unroll
+    double A[9], b[3], J[3];
+    map_from_axis(sc, rx, ry, rz, ux, uy, uz, A, b);
     for (int q = 0; q < 3; ++q)
-      J[q] = preal[q] - (A[3 * q] * preal[0] + A[3 * q + 1] * preal[1] + A[3 * q + 2] * preal[2] + mreal * b[q]);
-    add_impulse(a.sph.acc + 6 * sk, rel, J);
+      J[q] = t.preal[q] -
+             (A[3 * q] * t.preal[0] + A[3 * q + 1] * t.preal[1] + A[3 * q + 2] * t.preal[2] + t.mreal * b[q]);
+    add_impulse(a.sph.acc + 6 * t.sk, t.rel, J);
+  }
+  const double d[7] = {sc, rx, ry, rz, ux, uy, uz};
+  out[0] = kMapF64;
+  for (int q = 0; q < 7; ++q) out[1 + q] = f64_bits(d[q]);
+  for (int q = 8; q < 12; ++q) out[q] = 0;
+  return errbits;
+}
+
+// The collision map of one cell (MPCD::next_tstep, src/libcilia/mpcd.cpp:
+// 140-247) as twelve words (fixed_collide.cuh): in fixed point when the
+// cell's numbers fit, else as float64 factor, axis and mean velocity.  The
+// cell's sum m v^2 before the collision goes to the sums of ke (units of
+// 2^-40) or ke_rest.
+__device__ __forceinline__ void collision_map(double4 s, uint32_t w, long cid, const StepArgs& a, double* par,
+                                              uint64_t& ke, double& ke_rest, unsigned& errbits, bool& gfail) {
+  const int nf = cnt_fluid(w), nb = cnt_beads(w);
+  int num = nf + nb, sk = -1;
+  double M = (double)num;
+  if (nb) M = (double)nf + (double)nb * a.bead_mass;
+  CellSums t;
+  if ((a.sph.n || a.walls) && num < 10) {
+    t.s = s;
+    t.M = M;
+    t.num = num;
+    t.sk = -1;
+    add_virtual(t, cid, a);
+    s = t.s;
+    M = t.M;
+    num = t.num;
+    sk = t.sk;
+  }
+  // the random part first: it needs the count alone, and the sums are still on
+  // their way
+  float gf = 0.f;
+  if (num > 1 && !a.inj_gamma) gf = gamma_mt(num, a.seed, a.step, (uint32_t)cid, &gfail);
+  int64_t r[3];
+  bool fit = sk < 0;
+  if (a.inj_axis) {
+#pragma unroll
+    for (int q = 0; q < 3; ++q) fit = to_fixed<60, 1>(a.inj_axis[3 * cid + q], r[q]) && fit;
+  } else {
+    draw_axis_fixed(a.seed, a.step, (uint32_t)cid, r);
   }
   // dissipated energy (src/libcilia/mpcd.cpp:166-168, 232-234, 243-246): every
   // cell adds sum m v^2 before the collision here, and every particle
   // subtracts its m v'^2 after it (fluid_step, bead_collide), so the total
   // matches the reference's bookkeeping including the rounding of its
   // rotation constants
-  ldiss += s.w;
+  int64_t kin = 0;
+  if (to_fixed<50, 12>(s.w, kin)) {
+    ke += (uint64_t)((kin + 512) >> 10);
+  } else {
+    ke_rest += s.w;
+    fit = false;
+  }
+  int64_t p[3], inv = 0, sc = 1ll << kAxisBits;
+  fit = fit && to_fixed<52, 9>(s.x, p[0]) && to_fixed<52, 9>(s.y, p[1]) && to_fixed<52, 9>(s.z, p[2]);
+  if (nb == 0 && num < 256)
+    inv = __ldg(g_inv_n.x + num);  // M = num without beads
+  else
+    fit = to_fixed<62, 0>(1.0 / M, inv) && fit;
+  uint64_t out[12];
+  if (fit) {
+    const Limbs iv = split_limbs(inv);
+    int64_t u[3];
+    uint64_t rel = (uint64_t)kin;
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+      const Limbs pq = split_limbs(p[q]);
+      u[q] = mul_sh<56>(pq, iv);
+      fit = fit && u[q] < kMeanMax && u[q] > -kMeanMax;
+      rel -= (uint64_t)mul_sh<60>(split_limbs(u[q]), pq);  // K - M u^2
+    }
+    const int64_t erel = (int64_t)rel;
+    if (fit && erel > 0 && num > 1) {
+      const double e = from_fixed(erel, 50);
+      const double f = a.inj_gamma ? thermostat_factor(injected_gamma(a, cid, errbits), e) : thermostat_factor(gf, e);
+      fit = to_fixed<60, 1>(f, sc);
+    }
+    if (fit) map_words(r, sc, u, kCosAlpha, kSinAlpha, out);
+  }
+  if (!fit) {
+    t.s = s;
+    t.M = M;
+    t.num = num;
+    t.sk = sk;
+    uint64_t o[12];
+    errbits |= map_f64(t, cid, gf, o, a);
+#pragma unroll
+    for (int q = 0; q < 12; ++q) out[q] = o[q];
+  }
+  ulonglong2* pm = reinterpret_cast<ulonglong2*>(par);
+#pragma unroll
+  for (int q = 0; q < 6; ++q) pm[q] = make_ulonglong2(out[2 * q], out[2 * q + 1]);
+}
+
+// The block's sum of fixed-point energies (units of 2^-40, each thread's below
+// 2^58) and a float64 rest, added to *dst with the given sign by the warp that
+// comes last: no barrier at the end of a block, whose other warps would wait
+// there for the slowest (0.8 to 1.1 of 12 cycles per instruction before).
+struct BlockEnergy {
+  double sum;
+  unsigned warps;
+};
+__device__ __forceinline__ void energy_begin(BlockEnergy& b) {
+  if (threadIdx.x == 0) {
+    b.sum = 0.0;
+    b.warps = 0;
+  }
+  __syncthreads();
+}
+__device__ __forceinline__ void energy_end(BlockEnergy& b, uint64_t ke, double rest, double sign, double* dst) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) ke += __shfl_xor_sync(0xffffffffu, ke, o);
+  if (rest != 0.0) atomicAdd(&b.sum, rest);
+  __syncwarp();
+  if ((threadIdx.x & 31) == 0) {
+    atomicAdd(&b.sum, (double)ke * (1.0 / (double)(1ull << kEnergyBits)));
+    __threadfence_block();
+    if (atomicAdd(&b.warps, 1u) == (blockDim.x >> 5) - 1) {
+      __threadfence_block();
+      const double tot = *reinterpret_cast<volatile double*>(&b.sum);
+      if (tot != 0.0) atomicAdd(dst, sign * tot);
+    }
+  }
+}
+// before a thread's fixed-point sum can outgrow energy_end
+__device__ __forceinline__ void flush_ke(uint64_t& ke, double& rest) {
+  rest += (double)ke * (1.0 / (double)(1ull << kEnergyBits));
+  ke = 0;
 }
 
 // ============================================================== float64 ===
 
-__global__ void k_cell_params_f64(CellsF64 c, StepArgs a) {
-  double ldiss = 0.0;
+// Bound by latency: the generator's Gamma loop and the map are one long chain
+// per cell (1890 instructions, 12 cycles each at six warps per scheduler); the
+// float64 form kept that pipe 73 % busy.  64-thread blocks fill the SMs in the
+// finest steps (24 warps with 80 registers; five blocks of 128: 36 us, eight
+// with 64 registers: 43).  64^3 cells 48 to 34 us, 80^3 96 to 61, with walls
+// (24 x 21 x 37) 24.6 to 18.8; 8^3 cells take 11.4 us as before.
+constexpr int kCellThreads = 64;
+__global__ void __launch_bounds__(kCellThreads, 12) k_cell_params_f64(CellsF64 c, StepArgs a) {
+  __shared__ BlockEnergy s_e;
+  energy_begin(s_e);
+  uint64_t ke = 0;
+  double ke_rest = 0.0;
+  int rounds = 0;
   unsigned errbits = 0;
   bool gfail = false;
   for (long cid = (long)blockIdx.x * blockDim.x + threadIdx.x; cid < c.ncell; cid += (long)gridDim.x * blockDim.x) {
     const uint32_t w = c.cnt[cid];
-    if (w == 0) continue;
     const double4 s = c.sum[cid];
+    if (w == 0) continue;
     c.sum[cid] = make_double4(0.0, 0.0, 0.0, 0.0);
     c.cnt[cid] = 0u;
     if (a.premapped && cnt_beads(w) > 0) continue;  // mapped by k_bead_maps_f64
-    double A[9], b[3];
-    collision_map(s, w, cid, a, A, b, ldiss, errbits, gfail);
-    double2* p = reinterpret_cast<double2*>(c.par + 12 * cid);
-    p[0] = make_double2(A[0], A[1]);
-    p[1] = make_double2(A[2], A[3]);
-    p[2] = make_double2(A[4], A[5]);
-    p[3] = make_double2(A[6], A[7]);
-    p[4] = make_double2(A[8], b[0]);
-    p[5] = make_double2(b[1], b[2]);
+    collision_map(s, w, cid, a, c.par + 12 * cid, ke, ke_rest, errbits, gfail);
+    if (++rounds == (1 << 6)) {  // a cell's energy is below 2^52 units
+      flush_ke(ke, ke_rest);
+      rounds = 0;
+    }
   }
   if (gfail) errbits |= kErrGammaLoop;
   if (errbits) atomicOr(a.err, errbits);
-  double tot = block_sum_f64(ldiss);
-  if (threadIdx.x == 0 && tot != 0.0) atomicAdd(a.diss, tot);
+  energy_end(s_e, ke, ke_rest, 1.0, a.diss);
 }
 
 // Walls along z (NOSLIP / SLIP, src/libcilia/mpcd.cpp:346-376): the channel is
@@ -313,26 +464,92 @@ __device__ __forceinline__ void wall_bounce(int walls, double ztop, double& x, d
 // (with or without walls)
 constexpr int kPeriodic = 0, kWalled = 1, kSpheres = 2;
 
-// I: particle index type (32-bit whenever the particle count allows, so that
-// no 64-bit integer work competes with the float64 arithmetic).
-// A particle's float64 operations are the collision map (9), its kinetic
-// energy (3) and nothing else: GB300 issues two per clock and SM, and with the
-// streaming, the wrap and the energy sum in float64 as well (26 with their
-// reductions) that pipe was 82 % busy at 134 us on 2.6 M particles.
-// Now 116 us there (float64 pipe still 70 % busy, issue 19 %); 36.5 to 33.9 us
-// a step on 32^3 x 10, 346 to 313 us on 80^3 x 10.
-// Walls and spheres are instantiations of their own, so that the common
-// periodic pass keeps the registers that let its CTAs share the SMs with the
-// MD launch (the sphere bounce-back alone takes the kernel to over 100).
-// Between walls only a particle that would leave the channel takes the
-// bounce-back's float64 path.
+// A particle whose numbers do not fit the fixed-point form: collision, energy
+// (returned), streaming and kick in float64 (no inlining: it would hold
+// registers of the common path).
+struct SlowParticle {
+  double v[3], K;
+  int i[3];
+  uint64_t o[3];
+  unsigned bad;
+};
+__device__ __forceinline__ double square_f64(const double* v) { return v[0] * v[0] + v[1] * v[1] + v[2] * v[2]; }
+// the kick of a body force, and the energy that is binned
+__device__ __forceinline__ void kick_f64(SlowParticle& t, const StepArgs& a) {
+  if (a.gkick != 0.0) t.v[0] += a.gkick;
+  t.K = square_f64(t.v);
+}
+__device__ __noinline__ double slow_particle(SlowParticle& t, const double* par, const StepArgs& a) {
+  apply_map_f64(par, t.v[0], t.v[1], t.v[2]);
+  const double k = square_f64(t.v);
+  t.bad = 0;
+  for (int d = 0; d < 3; ++d) stream_coord(t.i[d], t.o[d], t.v[d], a, a.box.L[d], t.bad);
+  kick_f64(t, a);
+  return k;
+}
+// The same with walls or rigid spheres: bounce-back in unwrapped float64
+// coordinates; par is null if the collision is done.
+__device__ __noinline__ double bounced_particle(SlowParticle& t, const double* par, const StepArgs& a) {
+  double k = 0.0;
+  if (par) {
+    apply_map_f64(par, t.v[0], t.v[1], t.v[2]);
+    k = square_f64(t.v);
+  }
+  double X[3];
+  for (int d = 0; d < 3; ++d) X[d] = t.i[d] + offset_to_double(t.o[d]);
+  if (!(a.sph.n > 0 && sphere_bounce(a.sph, a.box, a.h, X, t.v)))
+    for (int d = 0; d < 3; ++d) X[d] += t.v[d] * a.h;
+  if (a.walls) wall_bounce(a.walls, (double)(a.box.L[2] - 1), X[0], X[1], X[2], t.v[0], t.v[1], t.v[2]);
+  t.bad = 0;
+  for (int d = 0; d < 3; ++d) split_coord(X[d], a.box.L[d], t.i[d], t.o[d], t.bad);
+  kick_f64(t, a);
+  return k;
+}
+
+// Adds the four values of a particle to its cell's sums.  The lanes of a quad
+// exchange their values first (a 4 x 4 transpose) so that each instruction adds
+// the 32 contiguous bytes of eight cells instead of one word of up to 32: the
+// L2 takes a quarter of the requests (80^3 x 10: 206 to 173 us).
+__device__ __forceinline__ void add_to_cell(double* sum, uint32_t cell, double v0, double v1, double v2, double v3, bool whole) {
+  if (!whole) {
+    double* p = sum + 4 * (size_t)cell;
+    atomicAdd(p + 0, v0);
+    atomicAdd(p + 1, v1);
+    atomicAdd(p + 2, v2);
+    atomicAdd(p + 3, v3);
+    return;
+  }
+  const int q = threadIdx.x & 3;
+  const bool q0 = q & 1, q1 = q & 2;
+  const double a0 = __shfl_xor_sync(0xffffffffu, q0 ? v0 : v1, 1), a1 = __shfl_xor_sync(0xffffffffu, q0 ? v2 : v3, 1);
+  const double w0 = q0 ? a0 : v0, w1 = q0 ? v1 : a0, w2 = q0 ? a1 : v2, w3 = q0 ? v3 : a1;
+  const double b0 = __shfl_xor_sync(0xffffffffu, q1 ? w0 : w2, 2), b1 = __shfl_xor_sync(0xffffffffu, q1 ? w1 : w3, 2);
+  // component q of the quad's particles 0 to 3
+  const double x[4] = {q1 ? b0 : w0, q1 ? b1 : w1, q1 ? w2 : b0, q1 ? w3 : b1};
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+    atomicAdd(sum + 4 * (size_t)__shfl_sync(0xffffffffu, cell, j, 4) + q, x[j]);
+}
+
+// I: particle index type (32-bit whenever the particle count allows).
+// Collision, kinetic energy, streaming, wrap and the comparison with the grid
+// shift run in 64-bit fixed point (fixed_collide.cuh, fixed_offset.cuh); float64
+// appears only as the stored velocity and in the atomic sums, which the L2
+// adds.  Nothing is saturated now (issue 52 %, the L1 data path 59 %, crossbar
+// 50 %); 32 warps of 64 registers per SM did best (24 of 80: 107 us), and
+// fetching the next particle ahead brought nothing.  64^3 x 10: 116 us with the
+// collision in float64 to 98; 80^3 x 10: 234 to 177; 32^3 x 10: 21.
+// Walls and spheres are instantiations of their own; between walls only a
+// particle that would leave the channel takes the bounce-back.
+constexpr int kFluidThreads = 128;
 template <typename I, int kBoundary>
-__global__ void __launch_bounds__(kThreads) k_fluid_step_f64(FluidF64 f, CellsF64 c, StepArgs a) {
+__global__ void __launch_bounds__(kFluidThreads, 8) k_fluid_step_f64(FluidF64 f, CellsF64 c, StepArgs a) {
   const int Lx = a.box.L[0], Ly = a.box.L[1], Lz = a.box.L[2];
-  const double h = a.h, gk = a.gkick;
-  const bool kick = gk != 0.0;
+  const bool kick = a.xkick != 0;  // what does not fit is in vmax
   const I n = (I)f.n;
-  uint64_t ke_fixed = 0;  // sum of v'^2 in units of 2^-44 (flushed every 2^7 particles), and the rest
+  __shared__ BlockEnergy s_e;
+  energy_begin(s_e);
+  uint64_t ke = 0;  // sum of v'^2 in units of 2^-40, and the rest
   double ke_rest = 0.0;
   int rounds = 0;
   unsigned bad = 0;
@@ -345,64 +562,100 @@ __global__ void __launch_bounds__(kThreads) k_fluid_step_f64(FluidF64 f, CellsF6
     const uint32_t cid =
         (uint32_t)shifted(ix, ox, a.xta_cur[0], Lx) +
         (uint32_t)Lx * ((uint32_t)shifted(iy, oy, a.xta_cur[1], Ly) + (uint32_t)Ly * (uint32_t)shifted(iz, oz, a.xta_cur[2], Lz));
-    apply_map_f64(c.par + 12 * (size_t)cid, vx, vy, vz);
-    double K = vx * vx + vy * vy + vz * vz;
-    uint64_t q;
-    if (kinetic_fixed(K, q))
-      ke_fixed += q;
-    else
-      ke_rest += K;
-    if (++rounds == (1 << 7)) {
-      ke_rest += (double)ke_fixed * (1.0 / (double)(1ull << kKinBits));
-      ke_fixed = 0;
+    const double* par = c.par + 12 * (size_t)cid;
+    uint64_t m[12];
+    {
+      const ulonglong2* p = reinterpret_cast<const ulonglong2*>(par);
+#pragma unroll
+      for (int q = 0; q < 6; ++q) {
+        const ulonglong2 t = __ldg(p + q);
+        m[2 * q] = t.x;
+        m[2 * q + 1] = t.y;
+      }
+    }
+    int64_t x[3] = {0, 0, 0}, y[3];
+    bool fit = to_fixed<58, 4>(vx, x[0]) && to_fixed<58, 4>(vy, x[1]) && to_fixed<58, 4>(vz, x[2]) &&
+               (uint32_t)(m[0] >> 32) != (uint32_t)(kMapF64 >> 32);
+    apply_words(m, x, y);
+    const uint32_t lim = (uint32_t)a.xstep.vmax;
+#pragma unroll
+    for (int q = 0; q < 3; ++q) fit = fit && (uint32_t)(y[q] >> 32) + lim < 2 * lim;
+    double K;
+    if (fit) {
+      const Limbs wx = split_limbs(y[0] << 2), wy = split_limbs(y[1] << 2), wz = split_limbs(y[2] << 2);
+      const int64_t k2 = square_words(wx, wy, wz);
+      ke += (uint64_t)((k2 + 2048) >> 12);
+      if (kick) {
+        const int64_t yk = y[0] + a.xkick;
+        K = from_fixed(square_words(split_limbs(yk << 2), wy, wz), kSquareBits);
+        vx = from_fixed(yk, kOutBits);
+      } else {
+        K = from_fixed(k2, kSquareBits);
+        vx = from_fixed(y[0], kOutBits);
+      }
+      vy = from_fixed(y[1], kOutBits);
+      vz = from_fixed(y[2], kOutBits);
+      bool free_path = kBoundary != kSpheres;
+      if (kBoundary != kSpheres) {
+        int cx, cy, cz;
+        uint64_t nx = ox, ny = oy, nz = oz;
+        stream_words(nx, cx, wx, a.xstep);
+        stream_words(ny, cy, wy, a.xstep);
+        stream_words(nz, cz, wz, a.xstep);
+        // between walls z stays in [0, Lz - 1], whose upper end is a cell's edge
+        if (kBoundary == kWalled) free_path = iz + cz >= 0 && (iz + cz < Lz - 1 || (iz + cz == Lz - 1 && nz == 0));
+        if (free_path) {
+          ox = nx;
+          oy = ny;
+          oz = nz;
+          ix += cx;
+          iy += cy;
+          iz += cz;
+          wrap_cell(ix, Lx);
+          wrap_cell(iy, Ly);
+          if (kBoundary == kPeriodic) wrap_cell(iz, Lz);
+        }
+      }
+      if (kBoundary != kPeriodic && !free_path) {
+        SlowParticle t{{kick ? from_fixed(y[0], kOutBits) : vx, vy, vz}, 0.0, {ix, iy, iz}, {ox, oy, oz}, 0u};
+        bounced_particle(t, nullptr, a);
+        K = t.K;
+        vx = t.v[0];
+        vy = t.v[1];
+        vz = t.v[2];
+        ix = t.i[0];
+        iy = t.i[1];
+        iz = t.i[2];
+        ox = t.o[0];
+        oy = t.o[1];
+        oz = t.o[2];
+        bad |= t.bad;
+      }
+    } else {
+      SlowParticle t{{vx, vy, vz}, 0.0, {ix, iy, iz}, {ox, oy, oz}, 0u};
+      ke_rest += kBoundary == kPeriodic ? slow_particle(t, par, a) : bounced_particle(t, par, a);
+      K = t.K;
+      vx = t.v[0];
+      vy = t.v[1];
+      vz = t.v[2];
+      ix = t.i[0];
+      iy = t.i[1];
+      iz = t.i[2];
+      ox = t.o[0];
+      oy = t.o[1];
+      oz = t.o[2];
+      bad |= t.bad;
+    }
+    if (++rounds == (1 << 8)) {  // a particle's energy is below 2^50 units
+      flush_ke(ke, ke_rest);
       rounds = 0;
     }
-    // streaming
-    bool turned = false;
-    if (kBoundary != kPeriodic) {
-      bool free_path = kBoundary == kWalled;
-      const int iz0 = iz;
-      const uint64_t oz0 = oz;
-      if (kBoundary == kWalled) {
-        // z stays in [0, Lz - 1]: no wrap, and the wall is at a cell's edge
-        int cz = 0;
-        free_path = stream_fixed(oz, cz, vz, a.xh);
-        iz += cz;
-        free_path = free_path && iz >= 0 && (iz < Lz - 1 || (iz == Lz - 1 && oz == 0));
-      }
-      if (!free_path) {
-        // bounce-back in unwrapped float64 coordinates
-        double X[3] = {ix + offset_to_double(ox), iy + offset_to_double(oy), iz0 + offset_to_double(oz0)};
-        double V[3] = {vx, vy, vz};
-        if (!(kBoundary == kSpheres && sphere_bounce(a.sph, a.box, h, X, V)))
-          for (int d = 0; d < 3; ++d) X[d] += V[d] * h;
-        if (a.walls) wall_bounce(a.walls, (double)(Lz - 1), X[0], X[1], X[2], V[0], V[1], V[2]);
-        vx = V[0];
-        vy = V[1];
-        vz = V[2];
-        iz = iz0;
-        split_coord(X[0], Lx, ix, ox, bad);
-        split_coord(X[1], Ly, iy, oy, bad);
-        split_coord(X[2], Lz, iz, oz, bad);
-        turned = true;
-      }
-    }
-    if (!turned) {
-      stream_coord(ix, ox, vx, a, Lx, bad);
-      stream_coord(iy, oy, vy, a, Ly, bad);
-      if (kBoundary == kPeriodic) stream_coord(iz, oz, vz, a, Lz, bad);
-    }
-    if (kick) vx += gk;
     // bin with the next shift
     const uint32_t cn =
         (uint32_t)shifted(ix, ox, a.xta_next[0], Lx) +
         (uint32_t)Lx * ((uint32_t)shifted(iy, oy, a.xta_next[1], Ly) + (uint32_t)Ly * (uint32_t)shifted(iz, oz, a.xta_next[2], Lz));
-    if (kick || turned) K = vx * vx + vy * vy + vz * vz;
-    double* sp = reinterpret_cast<double*>(c.sum + cn);
-    atomicAdd(sp + 0, vx);
-    atomicAdd(sp + 1, vy);
-    atomicAdd(sp + 2, vz);
-    atomicAdd(sp + 3, K);
+    const bool whole = (threadIdx.x & ~31u) + 31u - threadIdx.x + i < n;  // all lanes of the warp are here
+    add_to_cell(reinterpret_cast<double*>(c.sum), cn, vx, vy, vz, K, whole);
     atomicAdd(c.cnt + cn, 1u);
     f.cell[i] = pack_cell(ix, iy, iz);
     f.ox[i] = ox;
@@ -413,22 +666,7 @@ __global__ void __launch_bounds__(kThreads) k_fluid_step_f64(FluidF64 f, CellsF6
     f.vz[i] = vz;
   }
   if (bad) atomicOr(a.err, bad);
-  // the block's sum: integers up to the warp's, then one float64 per warp
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) ke_fixed += __shfl_xor_sync(0xffffffffu, ke_fixed, o);
-  __shared__ double s_ke[kThreads / 32];
-  __shared__ double s_rest;
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  if (threadIdx.x == 0) s_rest = 0.0;
-  __syncthreads();
-  if (lane == 0) s_ke[wid] = (double)ke_fixed * (1.0 / (double)(1ull << kKinBits));
-  if (ke_rest != 0.0) atomicAdd(&s_rest, ke_rest);
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double tot = s_rest;
-    for (int w = 0; w < kThreads / 32; ++w) tot += s_ke[w];
-    if (tot != 0.0) atomicAdd(a.diss, -tot);
-  }
+  energy_end(s_e, ke, ke_rest, -1.0, a.diss);
 }
 
 __global__ void k_bin_fluid_f64(FluidF64 f, CellsF64 c, StepArgs a) {
@@ -1163,7 +1401,10 @@ __global__ void k_store_fluid_f32(FluidF32 f, double* pos, double* vel, unsigned
 // word with this step's tag makes it.  The sums are left for the cell-map
 // kernel to clear.
 __global__ void k_bead_maps_f64(MDState m, CellsF64 c, StepArgs a, uint32_t* claim, uint32_t tag) {
-  double ldiss = 0.0;
+  __shared__ BlockEnergy s_e;
+  energy_begin(s_e);
+  uint64_t ke = 0;
+  double ke_rest = 0.0;
   unsigned errbits = 0;
   bool gfail = false;
   for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < m.nslots; s += gridDim.x * blockDim.x) {
@@ -1176,20 +1417,12 @@ __global__ void k_bead_maps_f64(MDState m, CellsF64 c, StepArgs a, uint32_t* cla
     if (atomicExch(claim + cid, tag) == tag) continue;  // another bead of the cell makes it
     const uint32_t w = c.cnt[cid];
     if (w == 0) continue;
-    double A[9], b[3];
-    collision_map(c.sum[cid], w, cid, a, A, b, ldiss, errbits, gfail);
-    double2* p = reinterpret_cast<double2*>(c.par + 12 * cid);
-    p[0] = make_double2(A[0], A[1]);
-    p[1] = make_double2(A[2], A[3]);
-    p[2] = make_double2(A[4], A[5]);
-    p[3] = make_double2(A[6], A[7]);
-    p[4] = make_double2(A[8], b[0]);
-    p[5] = make_double2(b[1], b[2]);
+    collision_map(c.sum[cid], w, cid, a, c.par + 12 * cid, ke, ke_rest, errbits, gfail);
+    flush_ke(ke, ke_rest);
   }
   if (gfail) errbits |= kErrGammaLoop;
   if (errbits) atomicOr(a.err, errbits);
-  const double tot = block_sum_f64(ldiss);
-  if (threadIdx.x == 0 && tot != 0.0) atomicAdd(a.diss, tot);
+  energy_end(s_e, ke, ke_rest, 1.0, a.diss);
 }
 
 __global__ void k_bead_maps_f32(MDState m, CellsF32 c, StepArgs a, uint32_t* claim, uint32_t tag) {
@@ -1324,22 +1557,22 @@ int launch_collision_draws(int nc, uint64_t seed, uint64_t step, long n, double*
 }
 
 int launch_cell_params_f64(const CellsF64& c, const StepArgs& a, cudaStream_t s) {
-  k_cell_params_f64<<<grid_for(c.ncell), kThreads, 0, s>>>(c, a);
+  k_cell_params_f64<<<grid_for(c.ncell, kCellThreads, -1), kCellThreads, 0, s>>>(c, a);
   return 1;
 }
 int launch_fluid_step_f64(const FluidF64& f, const CellsF64& c, const StepArgs& a, cudaStream_t s, int per_sm) {
   if (f.n == 0) return 0;
-  const int grid = grid_for(f.n, kThreads, per_sm);
+  const int grid = grid_for(f.n, kFluidThreads, per_sm);
   const bool i32 = f.n + (long)grid * kThreads < (1L << 32);
   if (a.sph.n > 0)
-    i32 ? k_fluid_step_f64<uint32_t, kSpheres><<<grid, kThreads, 0, s>>>(f, c, a)
-        : k_fluid_step_f64<long, kSpheres><<<grid, kThreads, 0, s>>>(f, c, a);
+    i32 ? k_fluid_step_f64<uint32_t, kSpheres><<<grid, kFluidThreads, 0, s>>>(f, c, a)
+        : k_fluid_step_f64<long, kSpheres><<<grid, kFluidThreads, 0, s>>>(f, c, a);
   else if (a.walls != 0)
-    i32 ? k_fluid_step_f64<uint32_t, kWalled><<<grid, kThreads, 0, s>>>(f, c, a)
-        : k_fluid_step_f64<long, kWalled><<<grid, kThreads, 0, s>>>(f, c, a);
+    i32 ? k_fluid_step_f64<uint32_t, kWalled><<<grid, kFluidThreads, 0, s>>>(f, c, a)
+        : k_fluid_step_f64<long, kWalled><<<grid, kFluidThreads, 0, s>>>(f, c, a);
   else
-    i32 ? k_fluid_step_f64<uint32_t, kPeriodic><<<grid, kThreads, 0, s>>>(f, c, a)
-        : k_fluid_step_f64<long, kPeriodic><<<grid, kThreads, 0, s>>>(f, c, a);
+    i32 ? k_fluid_step_f64<uint32_t, kPeriodic><<<grid, kFluidThreads, 0, s>>>(f, c, a)
+        : k_fluid_step_f64<long, kPeriodic><<<grid, kFluidThreads, 0, s>>>(f, c, a);
   return 1;
 }
 int launch_bin_fluid_f64(const FluidF64& f, const CellsF64& c, const StepArgs& a, cudaStream_t s) {

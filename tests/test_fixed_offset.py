@@ -1,6 +1,6 @@
 """Fixed-point offsets of the float64 fluid (csrc/fixed_offset.cuh), compiled for
 the CPU and compared with exact rational arithmetic: streaming o += v h with
-the cells moved, conversions, thresholds, and the fixed-point kinetic energy.
+the cells moved, conversions, thresholds.
 
 Bounds from the method: the displacement is the exact product of the two
 significands truncated twice (the 128-bit product's high half, then the shift
@@ -29,7 +29,6 @@ int stream(unsigned long long* k, int* cells, double v, double h) {
 unsigned long long from_double(double o) { return offset_from_double(o); }
 double to_double(unsigned long long k) { return offset_to_double(k); }
 unsigned long long threshold(double t) { return offset_threshold(t); }
-int kinetic(double x, unsigned long long* q) { uint64_t r = 0; const bool ok = kinetic_fixed(x, r); *q = r; return ok; }
 }
 """
 
@@ -47,7 +46,6 @@ def lib(tmp_path_factory):
     L.from_double.argtypes, L.from_double.restype = [d64], u
     L.to_double.argtypes, L.to_double.restype = [u], d64
     L.threshold.argtypes, L.threshold.restype = [d64], u
-    L.kinetic.argtypes = [d64, ctypes.POINTER(u)]
     return L
 
 
@@ -97,13 +95,3 @@ def test_conversions_and_thresholds(lib):
             if 0 <= k < ONE:
                 assert (k >= th) == (Fraction(k, ONE) >= Fraction(t))
     assert lib.threshold(1.0) == ONE  # no offset reaches it
-
-
-def test_kinetic_energy_in_fixed_point(lib):
-    rng = np.random.default_rng(5)
-    q = ctypes.c_ulonglong()
-    for x in map(float, np.concatenate([rng.chisquare(3, 500), [0.0, 5e-324, 127.99999, 1e-30, 2.0 ** -45, 2.0 ** -46]])):
-        assert lib.kinetic(x, ctypes.byref(q))
-        assert abs(Fraction(q.value, 1 << 44) - Fraction(x)) <= Fraction(1, 1 << 45), x
-    for x in (128.0, 1e300, math.inf, math.nan, -1.0):
-        assert not lib.kinetic(x, ctypes.byref(q))
