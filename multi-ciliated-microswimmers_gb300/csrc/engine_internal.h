@@ -316,8 +316,14 @@ int launch_load_fluid_f32(long n, const double* pos, const double* vel, const Bo
                           cudaStream_t s);
 // an array of float64 offsets in [0, 1) into fixed-point ones, in place
 int launch_convert_offsets(long n, uint64_t* o, cudaStream_t s);
-int launch_store_fluid_f64(const FluidF64& f, double* pos, double* vel, unsigned* bad, cudaStream_t s);
-int launch_store_fluid_f32(const FluidF32& f, double* pos, double* vel, unsigned* bad, cudaStream_t s);
+// read-back into the caller's order (status: {bad id, error word} in host memory)
+template <typename F>
+int launch_store_fluid(const F& f, double* pos, double* vel, unsigned* status, const unsigned* err, cudaStream_t s);
+template <typename F>
+int launch_find_particles(const F& f, uint32_t* at, unsigned* status, const unsigned* err, cudaStream_t s);
+template <typename F>
+int launch_gather_fluid(const F& f, const uint32_t* at, long d0, long d1, bool velocity, double* out, unsigned* status,
+                        cudaStream_t s);
 // observables from the binned cell sums (float64 path; valid while the sums
 // are those of the last binning): out[10], part[7 * kObsBlocks], counter zeroed once
 constexpr int kObsBlocks = 512;

@@ -1359,39 +1359,75 @@ __global__ void k_convert_offsets(long n, uint64_t* o) {
   }
 }
 
-// back to input order: particle k of the caller is the one with id k
-__global__ void k_store_fluid_f64(FluidF64 f, double* pos, double* vel, unsigned* bad) {
+// Back to input order: particle k of the caller is the one with id k.
+// status: {an id is out of range, the engine's error word}, in host memory.
+__device__ __forceinline__ void report_error(unsigned* status, const unsigned* err) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) status[1] = *err;
+}
+__device__ __forceinline__ void store_pos(const FluidF64& f, long i, double* p) {
+  const uint32_t cp = f.cell[i];
+  const uint64_t ox = f.ox[i], oy = f.oy[i], oz = f.oz[i];
+  p[0] = __dadd_rn((double)cell_x(cp), offset_to_double(ox));
+  p[1] = __dadd_rn((double)cell_y(cp), offset_to_double(oy));
+  p[2] = __dadd_rn((double)cell_z(cp), offset_to_double(oz));
+}
+__device__ __forceinline__ void store_vel(const FluidF64& f, long i, double* v) {
+  const double vx = f.vx[i], vy = f.vy[i], vz = f.vz[i];
+  v[0] = vx;
+  v[1] = vy;
+  v[2] = vz;
+}
+__device__ __forceinline__ void store_pos(const FluidF32& f, long i, double* q) {
+  const float4 p = f.pos[i];
+  const uint32_t cp = __float_as_uint(p.w);
+  q[0] = __dadd_rn((double)cell_x(cp), (double)p.x);
+  q[1] = __dadd_rn((double)cell_y(cp), (double)p.y);
+  q[2] = __dadd_rn((double)cell_z(cp), (double)p.z);
+}
+__device__ __forceinline__ void store_vel(const FluidF32& f, long i, double* q) {
+  const float4 v = f.vel[i];
+  q[0] = v.x;
+  q[1] = v.y;
+  q[2] = v.z;
+}
+// the whole fluid in one launch
+template <typename F>
+__global__ void k_store_fluid(F f, double* pos, double* vel, unsigned* status, const unsigned* err) {
+  report_error(status, err);
   for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < f.n; i += (long)gridDim.x * blockDim.x) {
     const long d = f.id[i];
     if (d >= f.n) {
-      atomicOr(bad, 1u);
+      status[0] = 1u;
       continue;
     }
-    const uint32_t cp = f.cell[i];
-    pos[3 * d] = __dadd_rn((double)cell_x(cp), offset_to_double(f.ox[i]));
-    pos[3 * d + 1] = __dadd_rn((double)cell_y(cp), offset_to_double(f.oy[i]));
-    pos[3 * d + 2] = __dadd_rn((double)cell_z(cp), offset_to_double(f.oz[i]));
-    vel[3 * d] = f.vx[i];
-    vel[3 * d + 1] = f.vy[i];
-    vel[3 * d + 2] = f.vz[i];
+    store_pos(f, i, pos + 3 * d);
+    store_vel(f, i, vel + 3 * d);
   }
 }
-
-__global__ void k_store_fluid_f32(FluidF32 f, double* pos, double* vel, unsigned* bad) {
+// In parts of the caller's order, so that a part is copied to the host while
+// the next is gathered: where each particle is kept, then positions or
+// velocities of the particles d0 .. d1.
+template <typename F>
+__global__ void k_find_particles(F f, uint32_t* at, unsigned* status, const unsigned* err) {
+  report_error(status, err);
   for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < f.n; i += (long)gridDim.x * blockDim.x) {
     const long d = f.id[i];
-    if (d >= f.n) {
-      atomicOr(bad, 1u);
-      continue;
-    }
-    const float4 p = f.pos[i], v = f.vel[i];
-    const uint32_t cp = __float_as_uint(p.w);
-    pos[3 * d] = __dadd_rn((double)cell_x(cp), (double)p.x);
-    pos[3 * d + 1] = __dadd_rn((double)cell_y(cp), (double)p.y);
-    pos[3 * d + 2] = __dadd_rn((double)cell_z(cp), (double)p.z);
-    vel[3 * d] = v.x;
-    vel[3 * d + 1] = v.y;
-    vel[3 * d + 2] = v.z;
+    if (d < f.n)
+      at[d] = (uint32_t)i;
+    else
+      status[0] = 1u;
+  }
+}
+template <typename F>
+__global__ void k_gather_fluid(F f, const uint32_t* at, long d0, long d1, bool velocity, double* out, unsigned* status) {
+  for (long d = d0 + (long)blockIdx.x * blockDim.x + threadIdx.x; d < d1; d += (long)gridDim.x * blockDim.x) {
+    const long i = at[d];
+    if (i >= f.n)
+      status[0] = 1u;
+    else if (velocity)
+      store_vel(f, i, out + 3 * d);
+    else
+      store_pos(f, i, out + 3 * d);
   }
 }
 
@@ -1737,15 +1773,30 @@ int launch_convert_offsets(long n, uint64_t* o, cudaStream_t s) {
   k_convert_offsets<<<grid_for(n), kThreads, 0, s>>>(n, o);
   return 1;
 }
-int launch_store_fluid_f64(const FluidF64& f, double* pos, double* vel, unsigned* bad, cudaStream_t s) {
+template <typename F>
+int launch_store_fluid(const F& f, double* pos, double* vel, unsigned* status, const unsigned* err, cudaStream_t s) {
   if (f.n == 0) return 0;
-  k_store_fluid_f64<<<grid_for(f.n), kThreads, 0, s>>>(f, pos, vel, bad);
+  k_store_fluid<<<grid_for(f.n), kThreads, 0, s>>>(f, pos, vel, status, err);
   return 1;
 }
-int launch_store_fluid_f32(const FluidF32& f, double* pos, double* vel, unsigned* bad, cudaStream_t s) {
-  if (f.n == 0) return 0;
-  k_store_fluid_f32<<<grid_for(f.n), kThreads, 0, s>>>(f, pos, vel, bad);
+template <typename F>
+int launch_find_particles(const F& f, uint32_t* at, unsigned* status, const unsigned* err, cudaStream_t s) {
+  k_find_particles<<<grid_for(f.n, kThreads, 8), kThreads, 0, s>>>(f, at, status, err);
   return 1;
 }
+template <typename F>
+int launch_gather_fluid(const F& f, const uint32_t* at, long d0, long d1, bool velocity, double* out, unsigned* status,
+                        cudaStream_t s) {
+  if (d1 <= d0) return 0;
+  k_gather_fluid<<<grid_for(d1 - d0, kThreads, 8), kThreads, 0, s>>>(f, at, d0, d1, velocity, out, status);
+  return 1;
+}
+#define MPCD_READ_BACK(F)                                                                                        \
+  template int launch_store_fluid(const F&, double*, double*, unsigned*, const unsigned*, cudaStream_t);         \
+  template int launch_find_particles(const F&, uint32_t*, unsigned*, const unsigned*, cudaStream_t);             \
+  template int launch_gather_fluid(const F&, const uint32_t*, long, long, bool, double*, unsigned*, cudaStream_t)
+MPCD_READ_BACK(FluidF64);
+MPCD_READ_BACK(FluidF32);
+#undef MPCD_READ_BACK
 
 }  // namespace mpcd
