@@ -144,6 +144,8 @@ struct mpcd_batch {
   cudaEvent_t ev_fork = nullptr, ev_join[kMaxClusterTiles] = {};
   int T = 512, lanes = 2;
   long part_cap = 0, cell_cap = 0, tile_cap = 0;
+  double* d_beads = nullptr;  // read-back of a replica's beads
+  long beads_cap = 0;
   long slot_cap = 0, tile_arr_cap = 0;  // MD slots; entries of the per-tile arrays (any layout)
   long npart_pages = 0, ncell_pages = 0;
   // device tables
@@ -255,6 +257,8 @@ void free_all(mpcd_batch* b) {
   cudaFree(m.vy);
   cudaFree(m.vz);
   cudaFree(m.moves);
+  cudaFree(m.bead);
+  cudaFree(b->d_beads);
   cudaFree(m.prim);
   cudaFree(m.nhelp);
   cudaFree(m.tile_help);
@@ -515,6 +519,7 @@ int upload_md(mpcd_batch* b, int r, Replica& R) {
     if ((rc = put_range(b, m.vy, sb, pl.VY.data(), ns))) return rc;
     if ((rc = put_range(b, m.vz, sb, pl.VZ.data(), ns))) return rc;
     if ((rc = put_range(b, m.moves, sb, pl.mv.data(), ns))) return rc;
+    if ((rc = put_range(b, m.bead, sb, pl.bead_of().data(), ns))) return rc;
     std::vector<int> v(ns + 1);
     for (long k = 0; k < ns; ++k) v[k] = pl.prim[k] + (int)sb;
     if ((rc = put_range(b, m.prim, sb, v.data(), ns))) return rc;
@@ -718,6 +723,7 @@ int mpcd_batch_create(const mpcd_batch_params* params, mpcd_batch** out) {
   if ((e = dalloc(&m.vy, nslots)) != cudaSuccess) return bail(e, "alloc MD");
   if ((e = dalloc(&m.vz, nslots)) != cudaSuccess) return bail(e, "alloc MD");
   if ((e = dalloc(&m.moves, nslots)) != cudaSuccess) return bail(e, "alloc MD");
+  if ((e = dalloc(&m.bead, nslots)) != cudaSuccess) return bail(e, "alloc MD");
   if ((e = dalloc(&m.prim, nslots)) != cudaSuccess) return bail(e, "alloc MD");
   if ((e = dalloc(&m.nhelp, nslots)) != cudaSuccess) return bail(e, "alloc MD");
   if ((e = dalloc(&m.sp_start, nslots + 1)) != cudaSuccess) return bail(e, "alloc MD");
@@ -1229,10 +1235,28 @@ int mpcd_batch_get_beads(mpcd_batch* b, int r, long nb, double* pos, double* vel
   Replica* R = get_rep(b, r);
   if (!R || !R->admitted || nb != R->nb) return fail(b, MPCD_EINVAL, "get_beads: bad replica or size");
   if (nb == 0) return MPCD_OK;
-  int rc = pull_md_state(b, *R);
-  if (rc) return rc;
-  if (pos) std::memcpy(pos, R->bpos.data(), 3 * nb * sizeof(double));
-  if (vel) std::memcpy(vel, R->bvel.data(), 3 * nb * sizeof(double));
+  if (R->plan.ntiles == 0) {
+    if (pos) std::memcpy(pos, R->bpos.data(), 3 * nb * sizeof(double));
+    if (vel) std::memcpy(vel, R->bvel.data(), 3 * nb * sizeof(double));
+    return MPCD_OK;
+  }
+  // one gather into bead order and a copy per array, as mpcd_get_beads
+  if (b->beads_cap < nb) {
+    cudaFree(b->d_beads);
+    b->d_beads = nullptr;
+    b->beads_cap = 0;
+    BK(cudaMalloc((void**)&b->d_beads, 6 * (size_t)nb * sizeof(double)));
+    b->beads_cap = nb;
+  }
+  double *dpos = b->d_beads, *dvel = dpos + 3 * (size_t)nb;
+  const size_t bytes = 3 * (size_t)nb * sizeof(double);
+  b->launches_total += launch_store_beads(b->md, R->tile0 * (long)b->T, R->plan.nslots, nb, dpos, dvel, nullptr, nullptr,
+                                          b->s0);
+  touch_pages(pos, bytes);
+  touch_pages(vel, bytes);
+  if (pos) BK(cudaMemcpyAsync(pos, dpos, bytes, cudaMemcpyDeviceToHost, b->s0));
+  if (vel) BK(cudaMemcpyAsync(vel, dvel, bytes, cudaMemcpyDeviceToHost, b->s0));
+  BK(cudaStreamSynchronize(b->s0));
   return MPCD_OK;
 }
 

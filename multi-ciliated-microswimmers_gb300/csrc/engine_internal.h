@@ -138,6 +138,7 @@ struct MDState {
   double* z[2] = {nullptr, nullptr};
   double *vx = nullptr, *vy = nullptr, *vz = nullptr;
   int* moves = nullptr;  // 1 integrated + binned, 0 fixed, 2 helper, -1 empty slot
+  int* bead = nullptr;   // primary slot -> its bead, other slots -1 (read-back)
   int* prim = nullptr;   // helper slot -> primary slot of its bead; primary -> itself
   int* nhelp = nullptr;  // primary slot -> number of helper slots following it
   int* tile_help = nullptr;  // per tile: 1 if it holds helper slots
@@ -316,6 +317,19 @@ int launch_load_fluid_f32(long n, const double* pos, const double* vel, const Bo
                           cudaStream_t s);
 // an array of float64 offsets in [0, 1) into fixed-point ones, in place
 int launch_convert_offsets(long n, uint64_t* o, cudaStream_t s);
+// Writes to every page of a small host buffer that a copy from the device is
+// about to fill: a page that was never touched costs the copy engine about 40
+// us, the host a few.
+inline void touch_pages(void* p, size_t bytes) {
+  volatile char* c = static_cast<char*>(p);
+  if (!c) return;
+  for (size_t i = 0; i < bytes; i += 4096) c[i] = 0;
+  if (bytes) c[bytes - 1] = 0;
+}
+// positions and velocities of the beads in the slots s0 .. s0 + ns, in bead
+// order; status may be null
+int launch_store_beads(const MDState& m, long s0, long ns, long nb, double* pos, double* vel, unsigned* status,
+                       const unsigned* err, cudaStream_t s);
 // read-back into the caller's order (status: {bad id, error word} in host memory)
 template <typename F>
 int launch_store_fluid(const F& f, double* pos, double* vel, unsigned* status, const unsigned* err, cudaStream_t s);

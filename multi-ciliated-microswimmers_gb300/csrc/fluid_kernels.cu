@@ -1404,6 +1404,20 @@ __global__ void k_store_fluid(F f, double* pos, double* vel, unsigned* status, c
     store_vel(f, i, vel + 3 * d);
   }
 }
+__global__ void k_store_beads(MDState m, int s0, int ns, int nb, double* pos, double* vel, unsigned* status,
+                              const unsigned* err) {
+  if (status) report_error(status, err);
+  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < ns; k += gridDim.x * blockDim.x) {
+    const int s = s0 + k, d = m.bead[s];
+    if ((unsigned)d >= (unsigned)nb) continue;
+    pos[3 * d] = m.x[0][s];
+    pos[3 * d + 1] = m.y[0][s];
+    pos[3 * d + 2] = m.z[0][s];
+    vel[3 * d] = m.vx[s];
+    vel[3 * d + 1] = m.vy[s];
+    vel[3 * d + 2] = m.vz[s];
+  }
+}
 // In parts of the caller's order, so that a part is copied to the host while
 // the next is gathered: where each particle is kept, then positions or
 // velocities of the particles d0 .. d1.
@@ -1771,6 +1785,11 @@ int launch_load_fluid_f32(long n, const double* pos, const double* vel, const Bo
 int launch_convert_offsets(long n, uint64_t* o, cudaStream_t s) {
   if (n == 0) return 0;
   k_convert_offsets<<<grid_for(n), kThreads, 0, s>>>(n, o);
+  return 1;
+}
+int launch_store_beads(const MDState& m, long s0, long ns, long nb, double* pos, double* vel, unsigned* status,
+                       const unsigned* err, cudaStream_t s) {
+  k_store_beads<<<grid_for(ns, 128), 128, 0, s>>>(m, (int)s0, (int)ns, (int)nb, pos, vel, status, err);
   return 1;
 }
 template <typename F>

@@ -9,6 +9,7 @@ import numpy as np
 import pytest
 
 import cilia_gpu as cg
+import simcfg
 
 pytestmark = pytest.mark.gpu
 
@@ -38,4 +39,26 @@ def test_read_back_order(n, precision):
         args = [None, None]
         args[q] = buf.ctypes.data_as(dp)
         assert cg.lib().mpcd_get_fluid(e._h, n, *args) == 0
+        assert np.array_equal(buf, want)
+
+
+@pytest.mark.parametrize("precision, arith", [(cg.MPCD_FP64, cg.MD_AUTO), (cg.MPCD_FP64, cg.MD_PAIR), (cg.MPCD_FP32, cg.MD_AUTO)])
+@pytest.mark.parametrize("cilia", [0, 1, 10])
+def test_beads_come_back_in_their_order(cilia, precision, arith):
+    """Right after the upload the beads are those of the configuration, bit for bit."""
+    s = cg.Sim(simcfg.dumps(simcfg.swimmer_config(16, radius=4.0, n_cilia=cilia, rodlength=8, seed=3, ststep=0.002)),
+               precision=precision, seed=3, ststep=0.002, create_fluid=False, md_arith=arith)
+    before = s.beads()  # the host's description: not uploaded yet
+    s.engine.prepare()
+    after = s.beads()
+    again = s.beads()
+    for a, b, c in zip(before, after, again):
+        assert a.shape == (s.nbeads, 3)
+        assert np.array_equal(a, b) and np.array_equal(b, c)
+    dp = ctypes.POINTER(ctypes.c_double)
+    for q, want in enumerate(after):
+        buf = np.full((s.nbeads, 3), np.nan)
+        args = [None, None]
+        args[q] = buf.ctypes.data_as(dp)
+        assert cg.lib().mpcd_get_beads(s.engine._h, s.nbeads, *args) == 0
         assert np.array_equal(buf, want)
