@@ -73,6 +73,7 @@ struct StepArgs {
   uint64_t xta_cur[3], xta_next[3];  // ta_* as thresholds of fixed-point offsets
   FixedStep xh;       // h for streaming fixed-point offsets by a float64 velocity
   StreamStep xstep;   // and by a fixed-point one
+  const unsigned* skip = nullptr;  // a word that stops the pass (launch_last_fluid_step_f32)
   int64_t xkick;      // gkick in units of 2^-56; a larger one leaves no velocity that fits
   double h;           // MPC time step
   double gkick;       // gravity * cos(omega t) * h, added to v_x after streaming
@@ -344,6 +345,9 @@ constexpr int kObsBlocks = 512;
 int launch_observables_cells_f64(const CellsF64& c, const MDState& m, double bead_mass, const double* diss,
                                  const unsigned* err, double* part, unsigned* counter, double* out, cudaStream_t s);
 int launch_fluid_step_f32(const FluidF32& f, const CellsF32& c, const StepArgs& a, cudaStream_t s, int per_sm = 4);
+// the same for a plain fluid whose next cell sums are not wanted; does nothing
+// when *a.skip is set
+int launch_last_fluid_step_f32(const FluidF32& f, const CellsF32& c, const StepArgs& a, cudaStream_t s);
 int launch_bin_fluid_f32(const FluidF32& f, const CellsF32& c, const StepArgs& a, cudaStream_t s);
 int launch_bead_collide_f32(const MDState& m, const CellsF32& c, const StepArgs& a, cudaStream_t s);
 int launch_bin_beads_f32(const MDState& m, const CellsF32& c, const StepArgs& a, cudaStream_t s);

@@ -1068,8 +1068,11 @@ constexpr int kFluidOpt = 3;
 //   kOptAggregate the warp's particles binned into the same next cell are
 //                 summed in registers (peer_sum) and added by one vector
 //                 reduction and one count add per cell and warp
+//   kOptLast      a step whose cell sums nobody will read: nothing is binned,
+//                 and nothing happens at all if *a.skip is set
 constexpr int kOptPrefetch = 1;
 constexpr int kOptAggregate = 2;
+constexpr int kOptLast = 4;
 
 // kWalls: the bounce-back path (its float64 temporaries would otherwise
 // crowd the registers of the batched loads).
@@ -1082,6 +1085,7 @@ __global__ void __launch_bounds__(kThreads, FluidMinBlocks<U>::value)
   const float h = a.fh, gk = a.fgkick;
   float ke_after = 0.0f;
   unsigned bad = 0;
+  if ((kOpt & kOptLast) && *a.skip) return;
   const I n = (I)f.n;
   const I lane = (I)(threadIdx.x & 31);
   // each block takes U x blockDim consecutive particles per round; the loop
@@ -1172,7 +1176,8 @@ __global__ void __launch_bounds__(kThreads, FluidMinBlocks<U>::value)
       const uint32_t cn = (uint32_t)shifted_f(ix, ox, tnx, Lx) +
                           (uint32_t)Lx * ((uint32_t)shifted_f(iy, oy, tny, Ly) + (uint32_t)Ly * (uint32_t)shifted_f(iz, oz, tnz, Lz));
       const float4 contrib = make_float4(vx, vy, vz, vx * vx + vy * vy + vz * vz);
-      if (kOpt & kOptAggregate) {
+      if (kOpt & kOptLast) {
+      } else if (kOpt & kOptAggregate) {
         const uint32_t key = valid ? cn : 0xffffffffu;
         const unsigned peers = __match_any_sync(0xffffffffu, key);
         const float4 tot = peer_sum(peers, valid ? contrib : make_float4(0.f, 0.f, 0.f, 0.f));
@@ -1729,6 +1734,10 @@ int launch_fluid_step_f32(const FluidF32& f, const CellsF32& c, const StepArgs& 
     case 10: launch_fluid_f32_opt<2, 2>(f, c, a, s, per_sm); break;
     default: launch_fluid_f32_opt<2, 3>(f, c, a, s, per_sm); break;
   }
+  return 1;
+}
+int launch_last_fluid_step_f32(const FluidF32& f, const CellsF32& c, const StepArgs& a, cudaStream_t s) {
+  launch_fluid_f32_opt<kFluidBatch, kOptPrefetch | kOptLast>(f, c, a, s, 4);
   return 1;
 }
 int launch_bin_fluid_f32(const FluidF32& f, const CellsF32& c, const StepArgs& a, cudaStream_t s) {
