@@ -283,67 +283,65 @@ __device__ __forceinline__ void sphere_virtual(const RigidSphereDev& S, const do
 // random axis, written as three float4 rows (A row, b) of v' = A v + b.  The
 // cell's sum m v^2 before the collision goes into ldiss.  `cid` keys the
 // generator (the cell's index within its own box).
+// The virtual particles of a cell on a sphere's surface or in a wall layer, up
+// to rho = 10 (src/libcilia/mpcd.cpp:175-198); returns the sphere or -1.  Not
+// inlined: the common path fits the instruction cache better without it.
+static __device__ __noinline__ int add_virtual_f32(float4& s, float& M, int& num, double* rel, uint32_t cid, bool wall_cell,
+                                            const StepArgs& a) {
+  int sk = -1;
+  if (a.sph.n && !wall_cell) {
+    const int L0 = a.box.L[0], L1 = a.box.L[1];
+    sk = sphere_cut_cell(a.sph, a.box, a.a_cur, (int)(cid % L0), (int)((cid / L0) % L1),
+                         (int)(cid / ((uint32_t)L0 * L1)), rel);
+  }
+  if (sk < 0 && !wall_cell) return -1;
+  const int dm = 10 - num;
+  double pv[3];
+  if (sk >= 0) {  // moving with the surface
+    sphere_virtual(a.sph.s[sk], rel, dm, a.seed, a.step, cid, a.inj_virt, pv);
+  } else if (a.inj_virt) {
+    pv[0] = a.inj_virt[3 * cid];
+    pv[1] = a.inj_virt[3 * cid + 1];
+    pv[2] = a.inj_virt[3 * cid + 2];
+  } else {
+    virtual_momentum(a.seed, a.step, cid, dm, pv);
+  }
+  s.x += (float)pv[0];
+  s.y += (float)pv[1];
+  s.z += (float)pv[2];
+  s.w += (float)((pv[0] * pv[0] + pv[1] * pv[1] + pv[2] * pv[2]) / dm);
+  M += (float)dm;
+  num += dm;
+  return sk;
+}
+
 __device__ __forceinline__ void cell_map_f32(const float4 s0, const uint32_t w, const uint32_t cid, const uint64_t seed,
                                              const uint64_t step, const float mb, const double* inj_gamma,
                                              const double* inj_axis, float4* par_out, float& ldiss, unsigned& errbits,
-                                             bool& gfail, const bool wall_cell = false,
-                                             const double* inj_virt = nullptr, const StepArgs* sa = nullptr) {
+                                             bool& gfail, const StepArgs* sa = nullptr) {
   const int nf = cnt_fluid(w), nb = cnt_beads(w);
   int num = nf + nb;
   float M = (float)nf + (float)nb * mb;
   float4 s = s0;
   int sk = -1;  // rigid sphere whose surface cuts the cell
   double rel[3];
-  if (sa && sa->sph.n && num < 10 && !wall_cell) {
-    const int L0 = sa->box.L[0], L1 = sa->box.L[1];
-    sk = sphere_cut_cell(sa->sph, sa->box, sa->a_cur, (int)(cid % L0), (int)((cid / L0) % L1),
-                         (int)(cid / ((uint32_t)L0 * L1)), rel);
-    if (sk >= 0) {  // virtual particles up to rho = 10, moving with the surface
-      const int dm = 10 - num;
-      double pv[3];
-      sphere_virtual(sa->sph.s[sk], rel, dm, seed, step, cid, inj_virt, pv);
-      s.x += (float)pv[0];
-      s.y += (float)pv[1];
-      s.z += (float)pv[2];
-      s.w += (float)((pv[0] * pv[0] + pv[1] * pv[1] + pv[2] * pv[2]) / dm);
-      M += (float)dm;
-      num += dm;
-    }
+  if (sa && (sa->sph.n || sa->walls) && num < 10) {
+    float4 ts = s;  // copies: what a call takes by reference lives in memory
+    float tM = M;
+    int tn = num;
+    double tr[3] = {0.0, 0.0, 0.0};
+    sk = add_virtual_f32(ts, tM, tn, tr, cid, sa->walls != 0 && wall_layer_cell(sa->box, cid), *sa);
+    s = ts;
+    M = tM;
+    num = tn;
+    rel[0] = tr[0];
+    rel[1] = tr[1];
+    rel[2] = tr[2];
   }
-  if (wall_cell && num < 10) {  // virtual particles up to rho = 10 (src/libcilia/mpcd.cpp:175-198)
-    const int dm = 10 - num;
-    double pv[3];
-    if (inj_virt) {
-      pv[0] = inj_virt[3 * cid];
-      pv[1] = inj_virt[3 * cid + 1];
-      pv[2] = inj_virt[3 * cid + 2];
-    } else {
-      virtual_momentum(seed, step, cid, dm, pv);
-    }
-    s.x += (float)pv[0];
-    s.y += (float)pv[1];
-    s.z += (float)pv[2];
-    s.w += (float)((pv[0] * pv[0] + pv[1] * pv[1] + pv[2] * pv[2]) / dm);
-    M += (float)dm;
-    num += dm;
-  }
-  const float inv = 1.0f / M;
-  const float ux = s.x * inv, uy = s.y * inv, uz = s.z * inv;
-  const float erel = s.w - (ux * s.x + uy * s.y + uz * s.z);
-  float sc = 1.0f;
-  if (erel > 0.f && num > 1) {
-    float g;
-    if (inj_gamma) {
-      g = (float)inj_gamma[cid];
-      if (g < 0.f) {
-        errbits |= kErrGammaMissing;
-        g = 0.f;
-      }
-    } else {
-      g = gamma_mt(num, seed, step, cid, &gfail);
-    }
-    sc = sqrtf(2.0f * g / erel);
-  }
+  // the random part first: it needs the count alone, and the sums are still on
+  // their way
+  float g = 0.f;
+  if (num > 1 && !inj_gamma) g = gamma_mt(num, seed, step, cid, &gfail);
   float rx, ry, rz;
   if (inj_axis) {
     rx = (float)inj_axis[3 * cid + 0];
@@ -358,6 +356,20 @@ __device__ __forceinline__ void cell_map_f32(const float4 s0, const uint32_t w, 
     rx = st * cp;
     ry = st * sp;
     rz = ct;
+  }
+  const float inv = 1.0f / M;
+  const float ux = s.x * inv, uy = s.y * inv, uz = s.z * inv;
+  const float erel = s.w - (ux * s.x + uy * s.y + uz * s.z);
+  float sc = 1.0f;
+  if (erel > 0.f && num > 1) {
+    if (inj_gamma) {
+      g = (float)inj_gamma[cid];
+      if (g < 0.f) {
+        errbits |= kErrGammaMissing;
+        g = 0.f;
+      }
+    }
+    sc = sqrtf(2.0f * g / erel);
   }
   // v' = u + sc R (v - u), R the rotation about (rx, ry, rz) with the
   // reference's matrix entries (src/libcilia/mpcd.cpp:285-293), applied as

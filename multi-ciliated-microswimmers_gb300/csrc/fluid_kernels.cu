@@ -401,8 +401,8 @@ __device__ __forceinline__ void flush_ke(uint64_t& ke, double& rest) {
 // per cell (1890 instructions, 12 cycles each at six warps per scheduler); the
 // float64 form kept that pipe 73 % busy.  64-thread blocks fill the SMs in the
 // finest steps (24 warps with 80 registers; five blocks of 128: 36 us, eight
-// with 64 registers: 43).  64^3 cells 48 to 34 us, 80^3 96 to 61, with walls
-// (24 x 21 x 37) 24.6 to 18.8; 8^3 cells take 11.4 us as before.
+// with 64 registers: 43).  64^3 cells 48 to 31 us, 80^3 96 to 51, with walls
+// (24 x 21 x 37) 24.6 to 18.5; 8^3 cells take 11.5 us as before.
 constexpr int kCellThreads = 64;
 __global__ void __launch_bounds__(kCellThreads, 12) k_cell_params_f64(CellsF64 c, StepArgs a) {
   __shared__ BlockEnergy s_e;
@@ -412,17 +412,34 @@ __global__ void __launch_bounds__(kCellThreads, 12) k_cell_params_f64(CellsF64 c
   int rounds = 0;
   unsigned errbits = 0;
   bool gfail = false;
-  for (long cid = (long)blockIdx.x * blockDim.x + threadIdx.x; cid < c.ncell; cid += (long)gridDim.x * blockDim.x) {
-    const uint32_t w = c.cnt[cid];
-    const double4 s = c.sum[cid];
-    if (w == 0) continue;
-    c.sum[cid] = make_double4(0.0, 0.0, 0.0, 0.0);
-    c.cnt[cid] = 0u;
-    if (a.premapped && cnt_beads(w) > 0) continue;  // mapped by k_bead_maps_f64
-    collision_map(s, w, cid, a, c.par + 12 * cid, ke, ke_rest, errbits, gfail);
-    if (++rounds == (1 << 6)) {  // a cell's energy is below 2^52 units
-      flush_ke(ke, ke_rest);
-      rounds = 0;
+  constexpr int kU = 2;
+  const long stride = (long)gridDim.x * blockDim.x;
+  for (long cb = (long)blockIdx.x * blockDim.x + threadIdx.x; cb < c.ncell; cb += kU * stride) {
+    uint32_t w[kU];
+    double4 sm[kU];
+#pragma unroll
+    for (int u = 0; u < kU; ++u) {
+      const long cid = cb + u * stride;
+      w[u] = cid < c.ncell ? __ldcg(c.cnt + cid) : 0u;
+      sm[u] = make_double4(0.0, 0.0, 0.0, 0.0);
+      if (cid < c.ncell) {
+        const double2* p = reinterpret_cast<const double2*>(c.sum + cid);
+        const double2 lo = __ldcg(p), hi = __ldcg(p + 1);
+        sm[u] = make_double4(lo.x, lo.y, hi.x, hi.y);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < kU; ++u) {
+      if (!w[u]) continue;
+      const long cid = cb + u * stride;
+      c.sum[cid] = make_double4(0.0, 0.0, 0.0, 0.0);
+      c.cnt[cid] = 0u;
+      if (a.premapped && cnt_beads(w[u]) > 0) continue;  // mapped by k_bead_maps_f64
+      collision_map(sm[u], w[u], cid, a, c.par + 12 * cid, ke, ke_rest, errbits, gfail);
+      if (++rounds == (1 << 6)) {  // a cell's energy is below 2^52 units
+        flush_ke(ke, ke_rest);
+        rounds = 0;
+      }
     }
   }
   if (gfail) errbits |= kErrGammaLoop;
@@ -1005,14 +1022,33 @@ int scan_counts(const uint32_t* count, long ncell, uint32_t* start, uint32_t* bl
 // per-cell sums and collision maps float32.  The thermostat factor and the
 // rotation are computed per cell in float64 and rounded once.
 
+// Adds a block's sum to *dst by the warp that comes last, as energy_end.
+__device__ __forceinline__ void energy_end_f32(BlockEnergy& b, float v, double* dst) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  if ((threadIdx.x & 31) == 0) {
+    atomicAdd(&b.sum, (double)v);
+    __threadfence_block();
+    if (atomicAdd(&b.warps, 1u) == (blockDim.x >> 5) - 1) {
+      __threadfence_block();
+      const double tot = *reinterpret_cast<volatile double*>(&b.sum);
+      if (tot != 0.0) atomicAdd(dst, tot);
+    }
+  }
+}
 // Split-precision collision map: everything per cell in float (the sums
 // are float); the dissipated-energy bookkeeping accumulates in float64.
-__global__ void k_cell_params_f32(CellsF32 c, StepArgs a) {
+// Small blocks, loads of two cells issued together before any generator runs
+// (one cell's alone: 158 us, four with persistent blocks of 256 as before 59,
+// at 128^3 cells); the draws come before the sums are needed.  128^3 cells 91
+// to 50 us, 64^3 16.4 to 14.8.
+__global__ void __launch_bounds__(kCellThreads) k_cell_params_f32(CellsF32 c, StepArgs a) {
+  __shared__ BlockEnergy s_e;
+  energy_begin(s_e);
   float ldiss = 0.0f;
   unsigned errbits = 0;
   bool gfail = false;
-  // four cells per thread at a time, their loads issued together
-  constexpr int kU = 4;
+  constexpr int kU = 2;
   const long stride = (long)gridDim.x * blockDim.x;
   for (long cb = (long)blockIdx.x * blockDim.x + threadIdx.x; cb < c.ncell; cb += kU * stride) {
     uint32_t w[kU];
@@ -1021,9 +1057,8 @@ __global__ void k_cell_params_f32(CellsF32 c, StepArgs a) {
     for (int u = 0; u < kU; ++u) {
       const long cid = cb + u * stride;
       w[u] = cid < c.ncell ? __ldcg(c.cnt + cid) : 0u;
+      sm[u] = cid < c.ncell ? __ldcg(c.sum + cid) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
-#pragma unroll
-    for (int u = 0; u < kU; ++u) sm[u] = w[u] ? __ldcg(c.sum + cb + u * stride) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
     for (int u = 0; u < kU; ++u) {
       if (!w[u]) continue;
@@ -1031,14 +1066,13 @@ __global__ void k_cell_params_f32(CellsF32 c, StepArgs a) {
       c.sum[cid] = make_float4(0.f, 0.f, 0.f, 0.f);
       c.cnt[cid] = 0u;
       if (a.premapped && cnt_beads(w[u]) > 0) continue;  // mapped by k_bead_maps_f32
-      cell_map_f32(sm[u], w[u], (uint32_t)cid, a.seed, a.step, a.fbead_mass, a.inj_gamma, a.inj_axis, c.par + 2 * cid,
-                   ldiss, errbits, gfail, a.walls != 0 && wall_layer_cell(a.box, cid), a.inj_virt, &a);
+      cell_map_f32(sm[u], w[u], (uint32_t)cid, a.seed, a.step, a.fbead_mass, a.inj_gamma, a.inj_axis, c.par + 2 * cid, ldiss,
+                 errbits, gfail, &a);
     }
   }
   if (gfail) errbits |= kErrGammaLoop;
   if (errbits) atomicOr(a.err, errbits);
-  const double tot = block_sum_f32(ldiss);
-  if (threadIdx.x == 0 && tot != 0.0) atomicAdd(a.diss, tot);
+  energy_end_f32(s_e, ldiss, a.diss);
 }
 
 // Particles per thread whose loads (state, then collision map) are issued
@@ -1495,7 +1529,7 @@ __global__ void k_bead_maps_f32(MDState m, CellsF32 c, StepArgs a, uint32_t* cla
     const uint32_t w = c.cnt[cid];
     if (w == 0) continue;
     cell_map_f32(c.sum[cid], w, (uint32_t)cid, a.seed, a.step, a.fbead_mass, a.inj_gamma, a.inj_axis, c.par + 2 * cid,
-                 ldiss, errbits, gfail, a.walls != 0 && wall_layer_cell(a.box, cid), a.inj_virt, &a);
+                 ldiss, errbits, gfail, &a);
   }
   if (gfail) errbits |= kErrGammaLoop;
   if (errbits) atomicOr(a.err, errbits);
@@ -1677,7 +1711,7 @@ int scan_counts_ext(const uint32_t* count, long ncell, uint32_t* start, uint32_t
 }
 
 int launch_cell_params_f32(const CellsF32& c, const StepArgs& a, cudaStream_t s) {
-  k_cell_params_f32<<<grid_for(c.ncell), kThreads, 0, s>>>(c, a);
+  k_cell_params_f32<<<grid_for(c.ncell, kCellThreads, -1), kCellThreads, 0, s>>>(c, a);
   return 1;
 }
 template <int U, int kOpt>
