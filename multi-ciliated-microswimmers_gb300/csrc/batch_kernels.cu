@@ -24,16 +24,44 @@ namespace mpcd {
 
 namespace {
 
+// One warp per replica.  The chain of time additions is serial (its roundings
+// are the reference's); the remainders that decide the refreshes, some hundred
+// instructions each, are taken by one lane per force evaluation (one thread
+// for all of them: 64 us with the cell maps of twelve boxes; this 25).
 __global__ void k_batch_prologue(BatchTables t) {
-  const int r = blockIdx.x * blockDim.x + threadIdx.x;
+  const int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
   if (r >= t.nrep) return;
   const BatchRep& R = t.rep[r];
   BatchStep& S = t.step[r];
   BatchState& st = t.state[r];
   if (!R.resident || st.steps_left <= 0) {
-    S.active = 0;
+    if (lane == 0) S.active = 0;
     return;
   }
+  // simulation time as the reference accumulates it (n additions of ststep),
+  // and the rest-length refresh of force evaluation e (src/cilia.cpp:206-215):
+  // evaluations 0 and 1 at t0, evaluation k+1 after k additions of ststep
+  MDStepArgs& m = S.md;
+  const double t0 = st.globalt, ststep = R.ststep;
+  const int nsub = R.nsub;
+  double te = t0;
+  for (int e0 = 0; e0 < 512; e0 += 32) {
+    bool due = false;
+    if (e0 <= nsub) {
+      double mine = te;
+      const int end = min(32, nsub + 1 - e0);
+      for (int i = 0; i < end; ++i) {
+        if (e0 + i >= 2) te += ststep;
+        if (i == lane) mine = te;
+      }
+      due = lane < end && fmod(mine + ststep / 10., 0.01) < ststep;
+    }
+    const unsigned mask = __ballot_sync(0xffffffffu, due);
+    if (lane == 0) reinterpret_cast<uint32_t*>(m.refresh)[e0 >> 5] = mask;
+  }
+  if (lane != 0) return;
+  const double t_move = nsub >= 1 ? te + ststep : t0;
   S.active = 1;
   const uint64_t step = st.steps + 1;
   S.step = step;
@@ -48,24 +76,11 @@ __global__ void k_batch_prologue(BatchTables t) {
     an[1] = u01_dbl(q.y);
     an[2] = u01_dbl(q.z);
   }
-  // simulation time as the reference accumulates it (n additions of ststep)
-  const double t0 = st.globalt;
-  double t_move = t0;
-  for (int k = 0; k < R.nsub; ++k) t_move += R.ststep;
-  MDStepArgs& m = S.md;
   m.t0 = t0;
   m.dt = R.ststep;
   m.tstep = R.h;
   m.n = R.nsub;
   m.t_end = t_move;
-  // rest-length refresh of force evaluation e (src/cilia.cpp:206-215):
-  // evaluations 0 and 1 at t0, evaluation k+1 after k additions of ststep
-  for (int w = 0; w < 8; ++w) m.refresh[w] = 0ull;
-  double te = t0;
-  for (int e = 0; e <= R.nsub && e < 512; ++e) {
-    if (e >= 2) te += R.ststep;
-    if (fmod(te + R.ststep / 10., 0.01) < R.ststep) m.refresh[e >> 6] |= 1ull << (e & 63);
-  }
   m.box.L[0] = R.L[0];
   m.box.L[1] = R.L[1];
   m.box.L[2] = R.L[2];
@@ -508,7 +523,7 @@ inline int page_grid(long pages, int per_sm = 8) {
 }  // namespace
 
 int launch_batch_prologue(const BatchTables& t, cudaStream_t s) {
-  k_batch_prologue<<<(t.nrep + 127) / 128, 128, 0, s>>>(t);
+  k_batch_prologue<<<(t.nrep + 3) / 4, 128, 0, s>>>(t);
   return 1;
 }
 
