@@ -46,7 +46,7 @@ struct mpcd_engine {
   // launch shape of the fluid pass beside the MD launch: > 0 persistent with that
   // many CTAs per SM, <= 0 short-lived CTAs of -fluid_per_sm (at least 1)
   // particles per thread
-  int fluid_per_sm = 0;  // 0: 16 in float64 (CTAs of 128 threads), -1 in split precision
+  int fluid_per_sm = 0;  // 0: chosen with the step
   std::string error;
   long long launches = 0;
 
@@ -1376,15 +1376,20 @@ int mpcd_step(mpcd_engine* h, const mpcd_inject* inj) {
     h->launches += f64 ? launch_cell_params_f64(h->c64, s, h->stream) : launch_cell_params_f32(h->c32, s, h->stream);
   }
   {
-    // beside the MD launch the split-precision fluid pass runs as many
-    // short-lived CTAs (one round of particles per thread): as they retire, the
+    // Beside the MD launch the fluid pass runs as many short-lived CTAs (one
+    // round of particles per thread, two in float64): as they retire, the
     // higher-priority MD CTAs take their place, and the fluid CTAs fill what
-    // the MD leaves of every SM.  The float64 pass takes 16 CTAs of 128 threads
-    // per SM, two rounds of the eight that fit, alone and beside the MD
-    // (swimmer64: 228 us per step; one particle per thread 248, two 237; 8 per
-    // SM 250, 12 234)
+    // the MD leaves of every SM.  Per step, short-lived CTAs against a
+    // persistent grid: swimmer64 223 us against 224 (float64; 268 with half
+    // the grid), 489 against 522 (float64, IEEE springs), 145 against 153
+    // (split precision).  MD CTAs of 512 threads leave registers for one fluid
+    // CTA: the pass runs after them, best on its persistent grid (20 k beads
+    // in 128^3: 581 against 628).  Alone: persistent, in float64 two rounds of
+    // the CTAs that fit.
     ProfScope ps(h, MPCD_K_FLUID);
-    const int per_sm = fork && h->fluid_per_sm ? h->fluid_per_sm : (f64 ? 16 : (fork ? -1 : 4));
+    const bool wide = h->md.de && md_entries_threads(h->md.tile) > 384;
+    const int alone = f64 ? 16 : 4, beside = wide ? alone : (f64 ? -2 : -1);
+    const int per_sm = !fork ? alone : (h->fluid_per_sm ? h->fluid_per_sm : beside);
     h->launches += f64 ? launch_fluid_step_f64(h->f64, h->c64, s, h->stream, per_sm)
                        : launch_fluid_step_f32(h->f32, h->c32, s, h->stream, per_sm);
   }
