@@ -1323,6 +1323,7 @@ int mpcd_step(mpcd_engine* h, const mpcd_inject* inj) {
   // beside it (the beads' binning is deferred to a kernel after the join).
   // Otherwise every map is made before the fork.
   const bool first = folded && h->bead_first;
+  s.chained = !md && !h->profiling;
   if (first) {
     s.premapped = 1;
     ma.deferred = 1;

@@ -73,6 +73,7 @@ struct StepArgs {
   uint64_t xta_cur[3], xta_next[3];  // ta_* as thresholds of fixed-point offsets
   FixedStep xh;       // h for streaming fixed-point offsets by a float64 velocity
   StreamStep xstep;   // and by a fixed-point one
+  bool chained = false;  // launch as a programmatic dependent of the stream's last kernel
   const unsigned* skip = nullptr;  // a word that stops the pass (launch_last_fluid_step_f32)
   int64_t xkick;      // gkick in units of 2^-56; a larger one leaves no velocity that fits
   double h;           // MPC time step

@@ -421,24 +421,34 @@ __device__ __forceinline__ void map_from_axis(double sc, double rx, double ry, d
   b[2] = uz - (A[6] * ux + A[7] * uy + A[8] * uz);
 }
 
+// Programmatic dependent launch: a kernel launched so may start while its
+// predecessor on the stream drains; chain_begin waits until that one's results
+// are there, and lets the next kernel be scheduled in turn.  What the
+// predecessor wrote is not read through the read-only path.  No effect in a
+// kernel launched the ordinary way.
+__device__ __forceinline__ void chain_begin() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // v' = A v + b in float64 with the map of one cell (fixed_collide.cuh: words
 // in fixed point, or factor, axis and mean velocity)
 __device__ __forceinline__ void apply_map_f64(const double* par, double& vx, double& vy, double& vz) {
   const uint64_t* w = reinterpret_cast<const uint64_t*>(par);
   double A[9], b[3];
-  if (__ldg(w) == kMapF64) {
+  if (w[0] == kMapF64) {
     double d[7];
 #pragma unroll
-    for (int q = 0; q < 7; ++q) d[q] = __ldg(par + 1 + q);
+    for (int q = 0; q < 7; ++q) d[q] = par[1 + q];
     map_from_axis(d[0], d[1], d[2], d[3], d[4], d[5], d[6], A, b);
   } else {
 #pragma unroll
     for (int q = 0; q < 9; ++q) {
-      const Limbs p = word_limbs(__ldg(w + q));
+      const Limbs p = word_limbs(w[q]);
       A[q] = from_fixed((int64_t)((uint64_t)(int64_t)p.h << 32) + p.l, kMapBits);
     }
 #pragma unroll
-    for (int q = 0; q < 3; ++q) b[q] = from_fixed((int64_t)__ldg(w + 9 + q), kOutBits);
+    for (int q = 0; q < 3; ++q) b[q] = from_fixed((int64_t)w[9 + q], kOutBits);
   }
   const double nx = fma(A[0], vx, fma(A[1], vy, fma(A[2], vz, b[0])));
   const double ny = fma(A[3], vx, fma(A[4], vy, fma(A[5], vz, b[1])));

@@ -407,6 +407,7 @@ constexpr int kCellThreads = 64;
 __global__ void __launch_bounds__(kCellThreads, 12) k_cell_params_f64(CellsF64 c, StepArgs a) {
   __shared__ BlockEnergy s_e;
   energy_begin(s_e);
+  chain_begin();
   uint64_t ke = 0;
   double ke_rest = 0.0;
   int rounds = 0;
@@ -566,6 +567,7 @@ __global__ void __launch_bounds__(kFluidThreads, 8) k_fluid_step_f64(FluidF64 f,
   const I n = (I)f.n;
   __shared__ BlockEnergy s_e;
   energy_begin(s_e);
+  chain_begin();
   uint64_t ke = 0;  // sum of v'^2 in units of 2^-40, and the rest
   double ke_rest = 0.0;
   int rounds = 0;
@@ -585,7 +587,7 @@ __global__ void __launch_bounds__(kFluidThreads, 8) k_fluid_step_f64(FluidF64 f,
       const ulonglong2* p = reinterpret_cast<const ulonglong2*>(par);
 #pragma unroll
       for (int q = 0; q < 6; ++q) {
-        const ulonglong2 t = __ldg(p + q);
+        const ulonglong2 t = p[q];
         m[2 * q] = t.x;
         m[2 * q + 1] = t.y;
       }
@@ -1045,6 +1047,7 @@ __device__ __forceinline__ void energy_end_f32(BlockEnergy& b, float v, double* 
 __global__ void __launch_bounds__(kCellThreads) k_cell_params_f32(CellsF32 c, StepArgs a) {
   __shared__ BlockEnergy s_e;
   energy_begin(s_e);
+  chain_begin();
   float ldiss = 0.0f;
   unsigned errbits = 0;
   bool gfail = false;
@@ -1119,6 +1122,7 @@ __global__ void __launch_bounds__(kThreads, FluidMinBlocks<U>::value)
   const float h = a.fh, gk = a.fgkick;
   float ke_after = 0.0f;
   unsigned bad = 0;
+  chain_begin();
   if ((kOpt & kOptLast) && *a.skip) return;
   const I n = (I)f.n;
   const I lane = (I)(threadIdx.x & 31);
@@ -1152,8 +1156,8 @@ __global__ void __launch_bounds__(kThreads, FluidMinBlocks<U>::value)
                              (uint32_t)Lx * ((uint32_t)shifted_f(cell_y(cp), p[q].y, tcy, Ly) +
                                              (uint32_t)Ly * (uint32_t)shifted_f(cell_z(cp), p[q].z, tcz, Lz));
         const float4* m = c.par + 2 * (size_t)cid;
-        mk[q] = __ldg(m);
-        mu[q] = __ldg(m + 1);
+        mk[q] = m[0];
+        mu[q] = m[1];
       }
     }
 #pragma unroll
@@ -1432,6 +1436,7 @@ __device__ __forceinline__ void store_vel(const FluidF32& f, long i, double* q) 
 // the whole fluid in one launch
 template <typename F>
 __global__ void k_store_fluid(F f, double* pos, double* vel, unsigned* status, const unsigned* err) {
+  chain_begin();
   report_error(status, err);
   for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < f.n; i += (long)gridDim.x * blockDim.x) {
     const long d = f.id[i];
@@ -1462,6 +1467,7 @@ __global__ void k_store_beads(MDState m, int s0, int ns, int nb, double* pos, do
 // velocities of the particles d0 .. d1.
 template <typename F>
 __global__ void k_find_particles(F f, uint32_t* at, unsigned* status, const unsigned* err) {
+  chain_begin();
   report_error(status, err);
   for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < f.n; i += (long)gridDim.x * blockDim.x) {
     const long d = f.id[i];
@@ -1638,6 +1644,25 @@ int launch_spheres_update(RigidSphereDev* sph, int n, double* acc, double* fsum,
   return 1;
 }
 
+// Launches a kernel that begins with chain_begin(), in a chain as a
+// programmatic dependent: its CTAs are placed while the predecessor drains.
+// Per step of two kernels: 8^3 cells 18.4 to 13.2 us, 32^3 30.2 to 27.2, the
+// channel 37.7 to 36.0, 80^3 232 to 227.  Not beside an MD launch, where an
+// event lies between the two.
+template <typename... P, typename... A>
+void launch_in_chain(void (*kernel)(P...), int grid, int threads, cudaStream_t s, bool chained, const A&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(threads);
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = chained ? 1 : 0;
+  cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
 int launch_collision_draws(int nc, uint64_t seed, uint64_t step, long n, double* gamma, double* axis, unsigned* err,
                            cudaStream_t s) {
   if (n == 0) return 0;
@@ -1646,22 +1671,20 @@ int launch_collision_draws(int nc, uint64_t seed, uint64_t step, long n, double*
 }
 
 int launch_cell_params_f64(const CellsF64& c, const StepArgs& a, cudaStream_t s) {
-  k_cell_params_f64<<<grid_for(c.ncell, kCellThreads, -1), kCellThreads, 0, s>>>(c, a);
+  launch_in_chain(k_cell_params_f64, grid_for(c.ncell, kCellThreads, -1), kCellThreads, s, a.chained, c, a);
   return 1;
 }
 int launch_fluid_step_f64(const FluidF64& f, const CellsF64& c, const StepArgs& a, cudaStream_t s, int per_sm) {
   if (f.n == 0) return 0;
   const int grid = grid_for(f.n, kFluidThreads, per_sm);
   const bool i32 = f.n + (long)grid * kThreads < (1L << 32);
+  auto launch = [&](auto kernel) { launch_in_chain(kernel, grid, kFluidThreads, s, a.chained, f, c, a); };
   if (a.sph.n > 0)
-    i32 ? k_fluid_step_f64<uint32_t, kSpheres><<<grid, kFluidThreads, 0, s>>>(f, c, a)
-        : k_fluid_step_f64<long, kSpheres><<<grid, kFluidThreads, 0, s>>>(f, c, a);
+    i32 ? launch(k_fluid_step_f64<uint32_t, kSpheres>) : launch(k_fluid_step_f64<long, kSpheres>);
   else if (a.walls != 0)
-    i32 ? k_fluid_step_f64<uint32_t, kWalled><<<grid, kFluidThreads, 0, s>>>(f, c, a)
-        : k_fluid_step_f64<long, kWalled><<<grid, kFluidThreads, 0, s>>>(f, c, a);
+    i32 ? launch(k_fluid_step_f64<uint32_t, kWalled>) : launch(k_fluid_step_f64<long, kWalled>);
   else
-    i32 ? k_fluid_step_f64<uint32_t, kPeriodic><<<grid, kFluidThreads, 0, s>>>(f, c, a)
-        : k_fluid_step_f64<long, kPeriodic><<<grid, kFluidThreads, 0, s>>>(f, c, a);
+    i32 ? launch(k_fluid_step_f64<uint32_t, kPeriodic>) : launch(k_fluid_step_f64<long, kPeriodic>);
   return 1;
 }
 int launch_bin_fluid_f64(const FluidF64& f, const CellsF64& c, const StepArgs& a, cudaStream_t s) {
@@ -1711,7 +1734,7 @@ int scan_counts_ext(const uint32_t* count, long ncell, uint32_t* start, uint32_t
 }
 
 int launch_cell_params_f32(const CellsF32& c, const StepArgs& a, cudaStream_t s) {
-  k_cell_params_f32<<<grid_for(c.ncell, kCellThreads, -1), kCellThreads, 0, s>>>(c, a);
+  launch_in_chain(k_cell_params_f32, grid_for(c.ncell, kCellThreads, -1), kCellThreads, s, a.chained, c, a);
   return 1;
 }
 template <int U, int kOpt>
@@ -1732,9 +1755,9 @@ void launch_fluid_f32_opt(const FluidF32& f, const CellsF32& c, const StepArgs& 
     pf = (long)std::min(gb, resident) * U * kThreads;
   }
   if (i32)
-    k_fluid_step_f32<U, false, uint32_t, kOpt><<<gb, kThreads, 0, s>>>(f, c, a, pf);
+    launch_in_chain(k_fluid_step_f32<U, false, uint32_t, kOpt>, gb, kThreads, s, a.chained, f, c, a, pf);
   else
-    k_fluid_step_f32<U, false, long, kOpt><<<gb, kThreads, 0, s>>>(f, c, a, pf);
+    launch_in_chain(k_fluid_step_f32<U, false, long, kOpt>, gb, kThreads, s, a.chained, f, c, a, pf);
 }
 
 int launch_fluid_step_f32(const FluidF32& f, const CellsF32& c, const StepArgs& a, cudaStream_t s, int per_sm) {
@@ -1838,12 +1861,12 @@ int launch_store_beads(const MDState& m, long s0, long ns, long nb, double* pos,
 template <typename F>
 int launch_store_fluid(const F& f, double* pos, double* vel, unsigned* status, const unsigned* err, cudaStream_t s) {
   if (f.n == 0) return 0;
-  k_store_fluid<<<grid_for(f.n), kThreads, 0, s>>>(f, pos, vel, status, err);
+  launch_in_chain(k_store_fluid<F>, grid_for(f.n), kThreads, s, true, f, pos, vel, status, err);
   return 1;
 }
 template <typename F>
 int launch_find_particles(const F& f, uint32_t* at, unsigned* status, const unsigned* err, cudaStream_t s) {
-  k_find_particles<<<grid_for(f.n, kThreads, 8), kThreads, 0, s>>>(f, at, status, err);
+  launch_in_chain(k_find_particles<F>, grid_for(f.n, kThreads, 8), kThreads, s, true, f, at, status, err);
   return 1;
 }
 template <typename F>

@@ -146,6 +146,7 @@ extern "C" int mpcd_fluid_step_noalloc(const int* sizes, long n, void* pos, void
   a.err = &d_out->err;
   a.diss = &d_out->diss;
   a.skip = &d_out->rejected;
+  a.chained = true;
   if (n > 0) {
     const long g = std::min<long>((n + 255) / 256, 4096);
     k_check_bin_f32<<<(int)g, 256, 0, s>>>(f, cells, a, &d_out->rejected);
