@@ -167,19 +167,14 @@ __device__ __forceinline__ double thermostat_factor(double g, double erel) {
   const double q = 2.0 * g, x = q * erel;
   return (x > 1e-30 && x < 1e30) ? q * rsqrt_f64(x) : sqrt(g / (erel * 0.5));
 }
-// the same for a float g > 0: the seed's conversions and the range check on
-// the bit patterns (they are float64 instructions otherwise)
+// the same for a float g > 0, its conversion and the range check on the bit
+// patterns (they are float64 instructions otherwise)
 __device__ __forceinline__ double thermostat_factor(float g, double erel) {
   const uint32_t gb = __float_as_uint(g);
   const double q = __hiloint2double((int)((gb >> 3) + (897u << 20)), (int)(gb << 29));  // 2 g
   const double x = q * erel;
-  const uint32_t hi = (uint32_t)__double2hiint(x);
-  if (hi - (923u << 20) >= (200u << 20)) return sqrt((double)g / (erel * 0.5));  // x outside 2^-100 .. 2^100
-  const float y0 = rsqrtf(__uint_as_float(((hi - (896u << 20)) << 3) | ((uint32_t)__double2loint(x) >> 29)));
-  const uint32_t yb = __float_as_uint(y0);
-  const double y = __hiloint2double((int)((yb >> 3) + (896u << 20)), (int)(yb << 29));
-  const double r = fma(-x * y, y, 1.0);
-  return q * fma(y * r, fma(0.375, r, 0.5), y);
+  if ((uint32_t)__double2hiint(x) - (923u << 20) >= (200u << 20)) return sqrt((double)g / (erel * 0.5));  // x outside 2^-100 .. 2^100
+  return q * rsqrt_f64(x);
 }
 
 // A cell on its way to the map: its sums (virtual particles included), the

@@ -203,7 +203,16 @@ __device__ __forceinline__ bool grid_sync(const GridBarrier& b, unsigned target,
 // float64 operations, where GB300's float64 division and square root cost
 // several times more
 __device__ __forceinline__ double rsqrt_f64(double x) {
-  const double y = (double)rsqrtf((float)x);
+  // the seed's conversions on the bit patterns (they are float64 instructions
+  // otherwise) where x and the seed are normal floats
+  const uint32_t hi = (uint32_t)__double2hiint(x);
+  double y;
+  if (hi - (923u << 20) < (200u << 20)) {  // 2^-100 .. 2^100
+    const uint32_t b = __float_as_uint(rsqrtf(__uint_as_float(((hi - (896u << 20)) << 3) | ((uint32_t)__double2loint(x) >> 29))));
+    y = __hiloint2double((int)((b >> 3) + (896u << 20)), (int)(b << 29));
+  } else {
+    y = (double)rsqrtf((float)x);
+  }
   const double r = fma(-x * y, y, 1.0);
   return fma(y * r, fma(0.375, r, 0.5), y);
 }
