@@ -20,9 +20,12 @@
 // summed by warps: lane-strided, then a xor tree.
 //
 // Positions are exchanged between tiles through two global buffers of four
-// float64 per slot after a bounded grid barrier, the halo arriving by bulk
-// asynchronous copies (TMA) and cp.async while the entries between the tile's
-// own beads are evaluated.  The cilia's rest lengths: the beat's target of
+// float64 per slot and a bounded grid barrier whose arrival and wait are apart:
+// one warp waits for the other tiles and fetches the halo (bulk asynchronous
+// copies and cp.async) while the rest evaluate the entries between the tile's
+// own beads, which need nobody (64^3 swimmer: 347 to 327 us per launch, a step
+// beside the fluid pass 473 to 443; a substep was 13 k cycles, 5.1 k of them in
+// the barrier and 2.5 to 3 k in those entries).  The cilia's rest lengths: the beat's target of
 // every bond is fixed during one MPC step's substeps and computed once per
 // launch; the bending-rate limit runs at every refresh (every 0.01 time units).
 //
@@ -375,6 +378,20 @@ __device__ void md_pair_body(const MDState& m, const MDStepArgs& a, Bin bin) {
   int eval = 0;
   bool refreshed = false;
 
+  // one warp's wait for every tile's arrival; on a timeout the CTA leaves
+  // after the evaluation
+  __shared__ int s_lost;
+  if (tid == 0) s_lost = 0;  // read after the barriers of an evaluation
+  auto warp_waits = [&]() {
+    int ok = 1;
+    if (lane == 0) {
+      ok = grid_wait(m.bar, barriers * nblocks, a.err);
+      if (!ok) s_lost = 1;
+    }
+    ok = __shfl_sync(0xffffffffu, ok, 0);
+    __syncwarp();
+    return ok != 0;
+  };
   // own beads into shared memory and the global buffer b
   auto publish = [&](int b) {
     if (oprim && !ohub) {
@@ -525,6 +542,7 @@ __device__ void md_pair_body(const MDState& m, const MDStepArgs& a, Bin bin) {
   auto hub_update = [&](int e) {
     const int j = nwarps - 1 - warp;
     if (j < 0 || j >= nth) return;
+    if (!warp_waits()) return;
     const HubRef r = s_href[j];
     W f[3];
     hub_force(j, e - 1, f);
@@ -557,24 +575,31 @@ __device__ void md_pair_body(const MDState& m, const MDStepArgs& a, Bin bin) {
   auto evaluate = [&](int b) {
     const int ev = eval;
     // from the second evaluation on, the last nth warps advance the hubs'
-    // copies (hub_update) while the others (ethr threads) copy the halo and
-    // evaluate the entries that do not reach a hub
+    // copies (hub_update) while the others (ethr threads) evaluate the entries
+    // that do not reach a hub; the last of these warps waits for the other
+    // tiles and fetches the halo while the rest evaluate the entries between
+    // the tile's own beads
     const bool hubs_due = ev >= 1 && nth > 0;
     const int ethr = hubs_due ? nthr - 32 * nth : nthr;
-    if (hn > 0 && tid < ethr) {
+    const int cwarp = ethr / 32 - 1;
+    const int lthr = cwarp > 0 ? 32 * cwarp : 32;  // one warp alone does both
+    auto fetch_halo = [&]() {
+      if (!warp_waits() || hn == 0) return;
       // the other tiles wrote the buffer through the generic proxy; order
       // those writes (acquired at the barrier) before this thread's bulk reads
-      if (tid < nrun) asm volatile("fence.proxy.async.global;" ::: "memory");
-      for (int r = tid; r < nrun; r += ethr) {
+      if (lane < nrun) asm volatile("fence.proxy.async.global;" ::: "memory");
+      for (int r = lane; r < nrun; r += 32) {
         const int4 run = s_runs[r];
         bulk_load(st + 2 * (T + run.y), q[b] + 2 * (size_t)run.x, (uint32_t)sizeof(Pos4) * (uint32_t)run.z, hbar);
       }
-      for (int i = tid; i < nsingle; i += ethr) {
+      for (int i = lane; i < nsingle; i += 32) {
         const int2 e = s_single[i];
         cp_async16_p(st + 2 * (T + e.y), q[b] + 2 * (size_t)e.x);
         cp_async16_p(st + 2 * (T + e.y) + 1, q[b] + 2 * (size_t)e.x + 1);
       }
-    }
+      if (long_bytes && !mbar_wait(hbar, hphase & 1u, kPairHaloWait)) atomicOr(a.err, kErrBarrier);
+      cp_async_wait_all_p();
+    };
     if (c1 > c0 && refresh_due(a, eval)) {
       // Cilia::length (src/cilia.cpp:79-121) for every refreshed bond
       refreshed = true;
@@ -616,13 +641,11 @@ __device__ void md_pair_body(const MDState& m, const MDStepArgs& a, Bin bin) {
     ++eval;
     if (tid < ethr) {
       // the entries between the tile's own beads, then the halo's
-      for (int i = tid; i < nloc; i += ethr) entry(i);
+      if (warp == cwarp) fetch_halo();
+      if (tid < lthr)
+        for (int i = tid; i < nloc; i += lthr) entry(i);
+      ++hphase;
       if (hn > 0) {
-        if (long_bytes) {
-          if (!mbar_wait(hbar, hphase & 1u, kPairHaloWait)) atomicOr(a.err, kErrBarrier);
-          ++hphase;
-        }
-        cp_async_wait_all_p();
         if (hubs_due)
           asm volatile("bar.sync 1, %0;" ::"r"(ethr) : "memory");  // these warps only
         else
@@ -707,11 +730,13 @@ __device__ void md_pair_body(const MDState& m, const MDStepArgs& a, Bin bin) {
       }
     }
   };
-  // the grid barrier before every evaluation; the halo's mbarrier is armed
-  // with the next copies' bytes before any of them can be issued
-  auto barrier = [&]() {
+  // the arrival at the grid barrier before every evaluation (warp_waits is
+  // the other half); the halo's mbarrier is armed with the next copies' bytes
+  // before any of them can be issued
+  auto arrive = [&]() {
     if (tid == 0 && long_bytes) mbar_arrive_expect_tx(hbar, long_bytes);
-    return grid_sync(m.bar, ++barriers * nblocks, a.err);
+    grid_arrive(m.bar);
+    ++barriers;
   };
   // v += F c (c = dt or dt/2), and x += v dt when `drift`
   const bool kicks = omoves && !ohub;  // a hub moves by its copies (hub_update)
@@ -742,21 +767,24 @@ __device__ void md_pair_body(const MDState& m, const MDStepArgs& a, Bin bin) {
 
   // md_loop_start: forces at t0, v += F dt/2, x += v dt
   publish(0);
-  if (!barrier()) return;
+  arrive();
   evaluate(0);
+  if (s_lost) return;
   int cur = 0;
   verlet(true, true);
   publish(cur ^ 1);
-  if (!barrier()) return;
+  arrive();
   cur ^= 1;
   evaluate(cur);
+  if (s_lost) return;
   // md_loop: v += F dt, x += v dt, forces
   for (int k = 1; k < a.n; ++k) {
     verlet(false, true);
     publish(cur ^ 1);
-    if (!barrier()) return;
+    arrive();
     cur ^= 1;
     evaluate(cur);
+    if (s_lost) return;
   }
   // md_loop_stop: v += F dt/2, then bin with the next shift
   verlet(true, false);

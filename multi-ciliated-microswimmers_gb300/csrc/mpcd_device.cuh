@@ -176,6 +176,22 @@ __device__ __forceinline__ unsigned ld_acquire(const unsigned* p) {
   return v;
 }
 
+// Its two halves: the CTA's arrival (every thread calls; one thread releases
+// what the CTA has written), and one thread's wait, bounded.
+__device__ __forceinline__ void grid_arrive(const GridBarrier& b) {
+  __syncthreads();
+  if (threadIdx.x == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(b.count) : "memory");
+}
+__device__ __forceinline__ bool grid_wait(const GridBarrier& b, unsigned target, unsigned* err) {
+  unsigned long long spins = 0;
+  while (ld_acquire(b.count) < target) {
+    if (++spins > (1ull << 23)) {  // each poll is an L2 round trip: a few seconds
+      atomicOr(err, kErrBarrier);
+      return false;
+    }
+  }
+  return true;
+}
 __device__ __forceinline__ bool grid_sync(const GridBarrier& b, unsigned target, unsigned* err) {
   __shared__ int ok;
   __syncthreads();
