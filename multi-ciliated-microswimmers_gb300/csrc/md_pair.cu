@@ -25,9 +25,10 @@
 // copies and cp.async) while the rest evaluate the entries between the tile's
 // own beads, which need nobody (64^3 swimmer: 347 to 327 us per launch, a step
 // beside the fluid pass 473 to 443; a substep was 13 k cycles, 5.1 k of them in
-// the barrier and 2.5 to 3 k in those entries).  The cilia's rest lengths: the beat's target of
-// every bond is fixed during one MPC step's substeps and computed once per
-// launch; the bending-rate limit runs at every refresh (every 0.01 time units).
+// the barrier and 2.5 to 3 k in those entries).  The cilia's rest lengths: the
+// beat's target of every bond is fixed during one MPC step's substeps and
+// computed once per launch; the bending-rate limit runs at every refresh (every
+// 0.01 time units).
 //
 // The double-float instance keeps every bead as an integer cell plus a float
 // pair offset (md_df_coord.cuh) and the velocities, forces and sums as float

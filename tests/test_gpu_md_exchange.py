@@ -1,5 +1,5 @@
-"""The double-float grid MD kernels (a thread per spring pair; lanes per bead
-slot) and their exchange of positions between tiles (tagged packets, no grid
+"""The grid MD kernels (double-float: a thread per spring pair, lanes per bead
+slot; the pair kernels) and their exchange of positions between tiles (tagged packets, no grid
 barrier) on spring networks that the shipped objects do not make: one-sided
 lists (a tile that reads another without being read), long lists (a tile of
 their own; helper slots in short and long runs), and all tile widths.
@@ -61,14 +61,7 @@ def verlet(pos, vel, t, o, rest, k, nsub, dt):
     return x, v + f * dt / 2
 
 
-@pytest.mark.parametrize("min_tile", [0, 128, 256])
-@pytest.mark.parametrize("kind", ["oneway", "random", "hub"])
-@pytest.mark.parametrize("slots", [False, True])
-def test_one_sided_networks_match_float64(kind, min_tile, slots, monkeypatch):
-    if slots:
-        monkeypatch.setenv("MPCD_MD_SLOTS", "1")
-    if min_tile:
-        monkeypatch.setenv("MPCD_MD_MIN_TILE", str(min_tile))
+def run_network(kind, arith, min_tile):
     rng = np.random.default_rng(5)
     pos = lattice() + rng.uniform(-0.3, 0.3, (343, 3))
     vel = rng.normal(0, 0.2, (343, 3))
@@ -77,7 +70,7 @@ def test_one_sided_networks_match_float64(kind, min_tile, slots, monkeypatch):
     t, o = t[keep].astype(np.int32), o[keep].astype(np.int32)
     d = np.sqrt(((pos[t] - pos[o]) ** 2).sum(axis=1))
     rest, k = d * rng.uniform(0.97, 1.03, len(t)), rng.uniform(0.5, 3.0, len(t))
-    e = cg.Engine(L, tstep=TSTEP, ststep=SUB, precision=cg.MPCD_FP64, md_split=cg.MD_DF)
+    e = cg.Engine(L, tstep=TSTEP, ststep=SUB, precision=cg.MPCD_FP64, md_split=arith)
     e.set_fluid(np.array([[1.5, 1.5, 1.5]]), np.zeros((1, 3)))
     e.set_beads(pos, vel)
     ip, dp = ctypes.POINTER(ctypes.c_int), ctypes.POINTER(ctypes.c_double)
@@ -86,10 +79,32 @@ def test_one_sided_networks_match_float64(kind, min_tile, slots, monkeypatch):
                                    z.ctypes.data_as(ip), rest.ctypes.data_as(dp), k.ctypes.data_as(dp))
     assert rc == 0
     lay = e.md_layout()
-    assert lay["arith"] == cg.MD_DF and lay["ntiles"] > 1 and lay["tile"] >= min_tile
+    assert lay["arith"] == arith and lay["ntiles"] > 1 and lay["tile"] >= min_tile
     for _ in range(2):
         e.run(1)
         pos, vel = verlet(pos, vel, t, o, rest, k, 50, SUB)
     x, v = e.beads(343)
     assert np.abs(x - pos).max() < 1e-10
     assert np.abs(v - vel).max() < 1e-8
+
+
+@pytest.mark.parametrize("min_tile", [0, 128, 256])
+@pytest.mark.parametrize("kind", ["oneway", "random", "hub"])
+@pytest.mark.parametrize("slots", [False, True])
+def test_one_sided_networks_match_float64(kind, min_tile, slots, monkeypatch):
+    if slots:
+        monkeypatch.setenv("MPCD_MD_SLOTS", "1")
+    if min_tile:
+        monkeypatch.setenv("MPCD_MD_MIN_TILE", str(min_tile))
+    run_network(kind, cg.MD_DF, min_tile)
+
+
+@pytest.mark.parametrize("min_tile", [0, 128, 256])
+@pytest.mark.parametrize("kind", ["oneway", "random", "hub"])
+@pytest.mark.parametrize("arith", [cg.MD_PAIR, cg.MD_PAIR_DF])
+def test_pair_kernel_on_one_sided_networks(kind, min_tile, arith, monkeypatch):
+    """One warp waits for the other tiles while the rest evaluate: tiles that
+    reach no other tile, many, or a hub."""
+    if min_tile:
+        monkeypatch.setenv("MPCD_MD_MIN_TILE", str(min_tile))
+    run_network(kind, arith, min_tile)
