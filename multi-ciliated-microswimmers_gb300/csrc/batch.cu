@@ -145,6 +145,7 @@ struct mpcd_batch {
   int T = 512, lanes = 2;
   long part_cap = 0, cell_cap = 0, tile_cap = 0;
   double* d_beads = nullptr;  // read-back of a replica's beads
+  double* h_beads = nullptr;  // pinned, for small swimmers
   long beads_cap = 0;
   long slot_cap = 0, tile_arr_cap = 0;  // MD slots; entries of the per-tile arrays (any layout)
   long npart_pages = 0, ncell_pages = 0;
@@ -257,7 +258,8 @@ void free_all(mpcd_batch* b) {
   cudaFree(m.vy);
   cudaFree(m.vz);
   cudaFree(m.moves);
-  cudaFree(m.bead);
+  cudaFree(m.slot_of);
+  cudaFreeHost(b->h_beads);
   cudaFree(b->d_beads);
   cudaFree(m.prim);
   cudaFree(m.nhelp);
@@ -519,7 +521,7 @@ int upload_md(mpcd_batch* b, int r, Replica& R) {
     if ((rc = put_range(b, m.vy, sb, pl.VY.data(), ns))) return rc;
     if ((rc = put_range(b, m.vz, sb, pl.VZ.data(), ns))) return rc;
     if ((rc = put_range(b, m.moves, sb, pl.mv.data(), ns))) return rc;
-    if ((rc = put_range(b, m.bead, sb, pl.bead_of().data(), ns))) return rc;
+    if ((rc = put_range(b, m.slot_of, sb, pl.slot_of.data(), (long)pl.slot_of.size()))) return rc;
     std::vector<int> v(ns + 1);
     for (long k = 0; k < ns; ++k) v[k] = pl.prim[k] + (int)sb;
     if ((rc = put_range(b, m.prim, sb, v.data(), ns))) return rc;
@@ -723,7 +725,7 @@ int mpcd_batch_create(const mpcd_batch_params* params, mpcd_batch** out) {
   if ((e = dalloc(&m.vy, nslots)) != cudaSuccess) return bail(e, "alloc MD");
   if ((e = dalloc(&m.vz, nslots)) != cudaSuccess) return bail(e, "alloc MD");
   if ((e = dalloc(&m.moves, nslots)) != cudaSuccess) return bail(e, "alloc MD");
-  if ((e = dalloc(&m.bead, nslots)) != cudaSuccess) return bail(e, "alloc MD");
+  if ((e = dalloc(&m.slot_of, nslots)) != cudaSuccess) return bail(e, "alloc MD");
   if ((e = dalloc(&m.prim, nslots)) != cudaSuccess) return bail(e, "alloc MD");
   if ((e = dalloc(&m.nhelp, nslots)) != cudaSuccess) return bail(e, "alloc MD");
   if ((e = dalloc(&m.sp_start, nslots + 1)) != cudaSuccess) return bail(e, "alloc MD");
@@ -1240,7 +1242,20 @@ int mpcd_batch_get_beads(mpcd_batch* b, int r, long nb, double* pos, double* vel
     if (vel) std::memcpy(vel, R->bvel.data(), 3 * nb * sizeof(double));
     return MPCD_OK;
   }
-  // one gather into bead order and a copy per array, as mpcd_get_beads
+  // as mpcd_get_beads
+  const size_t bytes = 3 * (size_t)nb * sizeof(double);
+  const long s0 = R->tile0 * (long)b->T;
+  if (nb <= kPinnedBeads) {
+    if (!b->h_beads)
+      BK(cudaHostAlloc((void**)&b->h_beads, 6 * kPinnedBeads * sizeof(double), cudaHostAllocMapped | cudaHostAllocPortable));
+    double* d = nullptr;
+    BK(cudaHostGetDevicePointer((void**)&d, b->h_beads, 0));
+    b->launches_total += launch_store_beads(b->md, s0, nb, d, d + 3 * nb, nullptr, nullptr, b->s0);
+    BK(cudaStreamSynchronize(b->s0));
+    if (pos) std::memcpy(pos, b->h_beads, bytes);
+    if (vel) std::memcpy(vel, b->h_beads + 3 * nb, bytes);
+    return MPCD_OK;
+  }
   if (b->beads_cap < nb) {
     cudaFree(b->d_beads);
     b->d_beads = nullptr;
@@ -1249,9 +1264,7 @@ int mpcd_batch_get_beads(mpcd_batch* b, int r, long nb, double* pos, double* vel
     b->beads_cap = nb;
   }
   double *dpos = b->d_beads, *dvel = dpos + 3 * (size_t)nb;
-  const size_t bytes = 3 * (size_t)nb * sizeof(double);
-  b->launches_total += launch_store_beads(b->md, R->tile0 * (long)b->T, R->plan.nslots, nb, dpos, dvel, nullptr, nullptr,
-                                          b->s0);
+  b->launches_total += launch_store_beads(b->md, s0, nb, dpos, dvel, nullptr, nullptr, b->s0);
   touch_pages(pos, bytes);
   touch_pages(vel, bytes);
   if (pos) BK(cudaMemcpyAsync(pos, dpos, bytes, cudaMemcpyDeviceToHost, b->s0));

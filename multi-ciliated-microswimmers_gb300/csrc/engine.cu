@@ -77,6 +77,7 @@ struct mpcd_engine {
   // read-back: {bad id, error word} written by the device into host memory, a
   // stream for copies and an event per part
   volatile unsigned* h_status = nullptr;
+  double* h_beads = nullptr;  // pinned, for small swimmers
   unsigned* d_status = nullptr;
   cudaStream_t scopy = nullptr;
   cudaEvent_t ev_part[3] = {};
@@ -205,7 +206,7 @@ void free_md(MDState& m) {
   cudaFree(m.vy);
   cudaFree(m.vz);
   cudaFree(m.moves);
-  cudaFree(m.bead);
+  cudaFree(m.slot_of);
   cudaFree(m.prim);
   cudaFree(m.nhelp);
   cudaFree(m.tile_help);
@@ -440,7 +441,7 @@ int build_md(mpcd_engine* h) {
   CK(dalloc(&m.vy, ns));
   CK(dalloc(&m.vz, ns));
   CK(dalloc(&m.moves, ns));
-  CK(dalloc(&m.bead, ns));
+  CK(dalloc(&m.slot_of, ns));
   CK(dalloc(&m.prim, ns));
   CK(dalloc(&m.nhelp, ns));
   CK(dalloc(&m.tile_help, m.ntiles));
@@ -466,7 +467,7 @@ int build_md(mpcd_engine* h) {
   CK(up(m.vy, pl.VY.data(), ns * 8));
   CK(up(m.vz, pl.VZ.data(), ns * 8));
   CK(up(m.moves, pl.mv.data(), ns * 4));
-  CK(up(m.bead, pl.bead_of().data(), ns * 4));
+  CK(up(m.slot_of, pl.slot_of.data(), pl.slot_of.size() * 4));
   CK(up(m.prim, pl.prim.data(), ns * 4));
   CK(up(m.nhelp, pl.nhelp.data(), ns * 4));
   CK(up(m.tile_help, pl.thelp.data(), m.ntiles * 4));
@@ -916,6 +917,7 @@ int mpcd_destroy(mpcd_engine* h) {
   cudaFree(h->d_diss);
   cudaFree(h->d_obs);
   cudaFreeHost(h->h_ring);
+  cudaFreeHost(h->h_beads);
   cudaFree(h->d_stage);
   cudaFree(h->d_stage_flag);
   for (cudaEvent_t ev : h->ring_ev)
@@ -1143,11 +1145,22 @@ int mpcd_get_beads(mpcd_engine* h, long nb, double* pos, double* vel) {
   // one gather into bead order and a copy per array (5 k beads: six copies of
   // slot arrays, four of the beat's state, three waits and the host's gather
   // took 155 us, this 44)
-  if (int rc = stage_buffer(h, nb)) return rc;
-  double *dpos = h->d_stage, *dvel = dpos + 3 * (size_t)nb;
   const size_t bytes = 3 * (size_t)nb * sizeof(double);
   h->h_status[0] = h->h_status[1] = 0u;
-  h->launches += launch_store_beads(h->md, 0, h->md.nslots, nb, dpos, dvel, h->d_status, h->d_err, h->stream);
+  if (nb <= kPinnedBeads) {
+    if (!h->h_beads)
+      CK(cudaHostAlloc((void**)&h->h_beads, 6 * kPinnedBeads * sizeof(double), cudaHostAllocMapped | cudaHostAllocPortable));
+    double* d = nullptr;
+    CK(cudaHostGetDevicePointer((void**)&d, h->h_beads, 0));
+    h->launches += launch_store_beads(h->md, 0, nb, d, d + 3 * nb, h->d_status, h->d_err, h->stream);
+    CK(cudaStreamSynchronize(h->stream));
+    if (pos) std::memcpy(pos, h->h_beads, bytes);
+    if (vel) std::memcpy(vel, h->h_beads + 3 * nb, bytes);
+    return report_error(h, h->h_status[1]);
+  }
+  if (int rc = stage_buffer(h, nb)) return rc;
+  double *dpos = h->d_stage, *dvel = dpos + 3 * (size_t)nb;
+  h->launches += launch_store_beads(h->md, 0, nb, dpos, dvel, h->d_status, h->d_err, h->stream);
   touch_pages(pos, bytes);
   touch_pages(vel, bytes);
   if (pos) CK(cudaMemcpyAsync(pos, dpos, bytes, cudaMemcpyDeviceToHost, h->stream));

@@ -140,7 +140,7 @@ struct MDState {
   double* z[2] = {nullptr, nullptr};
   double *vx = nullptr, *vy = nullptr, *vz = nullptr;
   int* moves = nullptr;  // 1 integrated + binned, 0 fixed, 2 helper, -1 empty slot
-  int* bead = nullptr;   // primary slot -> its bead, other slots -1 (read-back)
+  int* slot_of = nullptr;  // bead -> primary slot, both counted from the swimmer's first (read-back)
   int* prim = nullptr;   // helper slot -> primary slot of its bead; primary -> itself
   int* nhelp = nullptr;  // primary slot -> number of helper slots following it
   int* tile_help = nullptr;  // per tile: 1 if it holds helper slots
@@ -328,10 +328,15 @@ inline void touch_pages(void* p, size_t bytes) {
   for (size_t i = 0; i < bytes; i += 4096) c[i] = 0;
   if (bytes) c[bytes - 1] = 0;
 }
-// positions and velocities of the beads in the slots s0 .. s0 + ns, in bead
+// positions and velocities of the nb beads whose slots begin at s0, in bead
 // order; status may be null
-int launch_store_beads(const MDState& m, long s0, long ns, long nb, double* pos, double* vel, unsigned* status,
+int launch_store_beads(const MDState& m, long s0, long nb, double* pos, double* vel, unsigned* status,
                        const unsigned* err, cudaStream_t s);
+// Swimmers of up to this many beads are read through pinned host memory that
+// the kernel writes and the host copies from, larger ones by two copies of the
+// copy engine (2 x 24 KB: 12 us against 19; 2 x 123 KB: 24 against 20, the
+// host reads what the device has just written at 14 GB/s)
+constexpr long kPinnedBeads = 3072;
 // read-back into the caller's order (status: {bad id, error word} in host memory)
 template <typename F>
 int launch_store_fluid(const F& f, double* pos, double* vel, unsigned* status, const unsigned* err, cudaStream_t s);

@@ -1443,18 +1443,15 @@ __global__ void k_store_fluid(F f, double* pos, double* vel, unsigned* status, c
     store_vel(f, i, vel + 3 * d);
   }
 }
-__global__ void k_store_beads(MDState m, int s0, int ns, int nb, double* pos, double* vel, unsigned* status,
+// a thread per bead and axis: whole rows go out, also to host memory
+__global__ void k_store_beads(MDState m, long s0, int nb, double* pos, double* vel, unsigned* status,
                               const unsigned* err) {
   if (status) report_error(status, err);
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < ns; k += gridDim.x * blockDim.x) {
-    const int s = s0 + k, d = m.bead[s];
-    if ((unsigned)d >= (unsigned)nb) continue;
-    pos[3 * d] = m.x[0][s];
-    pos[3 * d + 1] = m.y[0][s];
-    pos[3 * d + 2] = m.z[0][s];
-    vel[3 * d] = m.vx[s];
-    vel[3 * d + 1] = m.vy[s];
-    vel[3 * d + 2] = m.vz[s];
+  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < 3 * nb; k += gridDim.x * blockDim.x) {
+    const int d = k / 3, ax = k - 3 * d;
+    const long s = s0 + m.slot_of[s0 + d];
+    pos[k] = ax == 0 ? m.x[0][s] : (ax == 1 ? m.y[0][s] : m.z[0][s]);
+    vel[k] = ax == 0 ? m.vx[s] : (ax == 1 ? m.vy[s] : m.vz[s]);
   }
 }
 // In parts of the caller's order, so that a part is copied to the host while
@@ -1848,9 +1845,9 @@ int launch_convert_offsets(long n, uint64_t* o, cudaStream_t s) {
   k_convert_offsets<<<grid_for(n), kThreads, 0, s>>>(n, o);
   return 1;
 }
-int launch_store_beads(const MDState& m, long s0, long ns, long nb, double* pos, double* vel, unsigned* status,
+int launch_store_beads(const MDState& m, long s0, long nb, double* pos, double* vel, unsigned* status,
                        const unsigned* err, cudaStream_t s) {
-  k_store_beads<<<grid_for(ns, 128), 128, 0, s>>>(m, (int)s0, (int)ns, (int)nb, pos, vel, status, err);
+  k_store_beads<<<grid_for(3 * nb, 128), 128, 0, s>>>(m, s0, (int)nb, pos, vel, status, err);
   return 1;
 }
 template <typename F>

@@ -49,11 +49,6 @@ struct MDPlan {
   std::vector<double> mid, ts, newlen, oldlen, diag;
   std::vector<int> tcil;
   std::vector<int> slot_of;  // bead -> primary slot
-  std::vector<int> bead_of() const {  // its inverse, -1 in other slots
-    std::vector<int> v(nslots, -1);
-    for (size_t k = 0; k < slot_of.size(); ++k) v[slot_of[k]] = (int)k;
-    return v;
-  }
   // double-float grid kernel (md_df.cu)
   std::vector<int> df_split, df_b0, df_nb;
   std::vector<uint32_t> df_code;
