@@ -1016,7 +1016,7 @@ int mpcd_set_fluid(mpcd_engine* h, long n, const double* pos, const double* vel)
 }  // extern "C"
 namespace {
 // Fluids of at least this many particles are read in parts, each copied while
-// the next is gathered (64^3 x 10: 0.92 to 0.78 ms, 80^3 x 10: 1.86 to 1.49 of
+// the next is gathered (64^3 x 10: 0.92 to 0.78 ms, 80 x 71 x 89 x 10: 1.86 to 1.49 of
 // which 1.3 are the link; 32^3 x 10 0.136 instead of 0.130: one launch below)
 constexpr long kPartsMin = 1l << 20;
 

@@ -1,8 +1,8 @@
 // In-cell offsets of the float64 fluid as 64-bit fixed point, and the few
 // operations on them that the fluid pass needs, in integer arithmetic.
 //
-// An offset o in [0, 1) is the integer k = o 2^60.  GB300 issues about two
-// float64 operations per clock and SM against 64 integer ones, and the fluid
+// An offset o in [0, 1) is the integer k = o 2^60.  GB300 completes about one
+// float64 operation per clock and SM against 64 integer ones, and the fluid
 // pass is bound by its float64 pipe; streaming (x += v h), the wrap into the
 // next cell and the comparison with the grid shift need none of it this way.
 // The displacement v h is the truncated high part of the exact product of the

@@ -105,19 +105,13 @@ __device__ __forceinline__ void stream_coord(int& i, uint64_t& o, double v, cons
   }
 }
 
-// 1/n for the particle counts of bead-free cells: rounded once as the IEEE
-// division rounds it (the same bits as 1.0 / n at run time), and in units of
-// 2^-62 for the fixed-point form
+// 1/n for the particle counts of bead-free cells, in units of 2^-62
 struct InvTable {
-  double v[256];
   int64_t x[256];
 };
 constexpr InvTable make_inv_table() {
   InvTable t{};
-  for (int i = 1; i < 256; ++i) {
-    t.v[i] = 1.0 / i;
-    t.x[i] = (int64_t)(((1ull << 62) + (unsigned)i / 2) / (unsigned)i);
-  }
+  for (int i = 1; i < 256; ++i) t.x[i] = (int64_t)(((1ull << 62) + (unsigned)i / 2) / (unsigned)i);
   return t;
 }
 __device__ const InvTable g_inv_n = make_inv_table();
@@ -173,7 +167,7 @@ __device__ __forceinline__ double thermostat_factor(float g, double erel) {
   const uint32_t gb = __float_as_uint(g);
   const double q = __hiloint2double((int)((gb >> 3) + (897u << 20)), (int)(gb << 29));  // 2 g
   const double x = q * erel;
-  if ((uint32_t)__double2hiint(x) - (923u << 20) >= (200u << 20)) return sqrt((double)g / (erel * 0.5));  // x outside 2^-100 .. 2^100
+  if ((uint32_t)__double2hiint(x) - (923u << 20) >= (200u << 20)) return sqrt((double)g / (erel * 0.5));
   return q * rsqrt_f64(x);
 }
 
@@ -396,7 +390,7 @@ __device__ __forceinline__ void flush_ke(uint64_t& ke, double& rest) {
 // per cell (1890 instructions, 12 cycles each at six warps per scheduler); the
 // float64 form kept that pipe 73 % busy.  64-thread blocks fill the SMs in the
 // finest steps (24 warps with 80 registers; five blocks of 128: 36 us, eight
-// with 64 registers: 43).  64^3 cells 48 to 31 us, 80^3 96 to 51, with walls
+// with 64 registers: 43).  64^3 cells 48 to 31 us, 80 x 71 x 89 96 to 51, with walls
 // (24 x 21 x 37) 24.6 to 18.5; 8^3 cells take 11.5 us as before.
 constexpr int kCellThreads = 64;
 __global__ void __launch_bounds__(kCellThreads, 12) k_cell_params_f64(CellsF64 c, StepArgs a) {
@@ -522,7 +516,7 @@ __device__ __noinline__ double bounced_particle(SlowParticle& t, const double* p
 // Adds the four values of a particle to its cell's sums.  The lanes of a quad
 // exchange their values first (a 4 x 4 transpose) so that each instruction adds
 // the 32 contiguous bytes of eight cells instead of one word of up to 32: the
-// L2 takes a quarter of the requests (80^3 x 10: 206 to 173 us).
+// L2 takes a quarter of the requests (80 x 71 x 89 x 10: 206 to 173 us).
 __device__ __forceinline__ void add_to_cell(double* sum, uint32_t cell, double v0, double v1, double v2, double v3, bool whole) {
   if (!whole) {
     double* p = sum + 4 * (size_t)cell;
@@ -551,7 +545,7 @@ __device__ __forceinline__ void add_to_cell(double* sum, uint32_t cell, double v
 // adds.  Nothing is saturated now (issue 52 %, the L1 data path 59 %, crossbar
 // 50 %); 32 warps of 64 registers per SM did best (24 of 80: 107 us), and
 // fetching the next particle ahead brought nothing.  64^3 x 10: 116 us with the
-// collision in float64 to 98; 80^3 x 10: 234 to 177; 32^3 x 10: 21.
+// collision in float64 to 98; 80 x 71 x 89 x 10: 234 to 177; 32^3 x 10: 21.
 // Walls and spheres are instantiations of their own; between walls only a
 // particle that would leave the channel takes the bounce-back.
 constexpr int kFluidThreads = 128;
@@ -1639,7 +1633,7 @@ int launch_spheres_update(RigidSphereDev* sph, int n, double* acc, double* fsum,
 // Launches a kernel that begins with chain_begin(), in a chain as a
 // programmatic dependent: its CTAs are placed while the predecessor drains.
 // Per step of two kernels: 8^3 cells 18.4 to 13.2 us, 32^3 30.2 to 27.2, the
-// channel 37.7 to 36.0, 80^3 232 to 227.  Not beside an MD launch, where an
+// channel 37.7 to 36.0, 80 x 71 x 89 232 to 227.  Not beside an MD launch, where an
 // event lies between the two.
 template <typename... P, typename... A>
 void launch_in_chain(void (*kernel)(P...), int grid, int threads, cudaStream_t s, bool chained, const A&... args) {
