@@ -88,8 +88,8 @@ MPCD_HD int64_t mul_sh(Limbs a, Limbs b) {
 }
 
 // ------------------------------------------------------------ the map ---
-// Twelve words per cell: the matrix A (row-major, units of 2^-59, each word a
-// Limbs) and b (units of 2^-56) of v' = A v + b.  A cell whose numbers do not
+// Twelve words per cell, four per row i: A_i0, A_i1, A_i2 (units of 2^-59, each a
+// Limbs) and b_i (units of 2^-56) of v' = A v + b.  A cell whose numbers do not
 // fit holds kMapF64 in its first word instead, and the thermostat factor, the
 // rotation axis and the mean velocity as float64 in the next seven.
 constexpr int kVelBits = 58;         // velocities that go in, up to 16; mean velocities
@@ -129,31 +129,44 @@ MPCD_HD void axis_normalise(int64_t* r) {
 // reference uses them (src/libcilia/mpcd.h:72-76)
 MPCD_HD int64_t unit60(double x) { return (int64_t)(x * 1152921504606846976.0); }
 
-// The map's words from the axis r and factor sc (units of 2^-60) and the mean
-// velocity u (2^-58): A = sc R, b = u - A u, R the rotation with the entries of
+// The rotation (units of 2^-60) about the axis r (2^-60), with the entries of
 // src/libcilia/mpcd.cpp:285-293 (R_ii = r_i^2 (1 - ca) + ca, R_ij = r_i r_j (1 -
 // ca) -+ r_k sa).
-MPCD_HD void map_words(const int64_t* r, int64_t sc, const int64_t* u, double cos_a, double sin_a, uint64_t* w) {
+MPCD_HD void rotation_fixed(const int64_t* r, double cos_a, double sin_a, int64_t* R) {
   const Limbs x = split_limbs(r[0]), y = split_limbs(r[1]), z = split_limbs(r[2]);
-  const Limbs oc = split_limbs(unit60(1.0 - cos_a)), sa = split_limbs(unit60(sin_a)), f = split_limbs(sc);
+  const Limbs oc = split_limbs(unit60(1.0 - cos_a)), sa = split_limbs(unit60(sin_a));
   const int64_t ca = unit60(cos_a);
   const Limbs tx = split_limbs(mul_sh<60>(x, oc)), ty = split_limbs(mul_sh<60>(y, oc)), tz = split_limbs(mul_sh<60>(z, oc));
   const int64_t sx = mul_sh<60>(x, sa), sy = mul_sh<60>(y, sa), sz = mul_sh<60>(z, sa);
   const int64_t xy = mul_sh<60>(tx, y), xz = mul_sh<60>(tx, z), yz = mul_sh<60>(ty, z);
-  const int64_t R[9] = {mul_sh<60>(tx, x) + ca, xy - sz, xz + sy, xy + sz, mul_sh<60>(ty, y) + ca, yz - sx,
-                        xz - sy, yz + sx, mul_sh<60>(tz, z) + ca};
-  const Limbs ux = split_limbs(u[0]), uy = split_limbs(u[1]), uz = split_limbs(u[2]);
+  R[0] = mul_sh<60>(tx, x) + ca;
+  R[1] = xy - sz;
+  R[2] = xz + sy;
+  R[3] = xy + sz;
+  R[4] = mul_sh<60>(ty, y) + ca;
+  R[5] = yz - sx;
+  R[6] = xz - sy;
+  R[7] = yz + sx;
+  R[8] = mul_sh<60>(tz, z) + ca;
+}
+// Row i of the map's words from that row of R, the factor sc (2^-60) and the
+// mean velocity u (2^-58): A = sc R, b = u - A u.
+MPCD_HD void map_row(int i, const int64_t* row, int64_t sc, const int64_t* u, uint64_t* w) {
+  const Limbs f = split_limbs(sc);
+  int64_t b = (u[i] + 1) >> 1;  // 2^-57
 #pragma unroll
-  for (int i = 0; i < 3; ++i) {
-    Limbs a[3];
-#pragma unroll
-    for (int j = 0; j < 3; ++j) {
-      a[j] = split_limbs(mul_sh<61>(split_limbs(R[3 * i + j]), f));
-      w[3 * i + j] = (uint64_t)(uint32_t)a[j].h << 32 | (uint32_t)a[j].l;
-    }
-    const int64_t b = ((u[i] + 1) >> 1) - mul_sh<60>(a[0], ux) - mul_sh<60>(a[1], uy) - mul_sh<60>(a[2], uz);  // 2^-57
-    w[9 + i] = (uint64_t)((b + 1) >> 1);
+  for (int j = 0; j < 3; ++j) {
+    const Limbs a = split_limbs(mul_sh<61>(split_limbs(row[j]), f));
+    w[j] = (uint64_t)(uint32_t)a.h << 32 | (uint32_t)a.l;
+    b -= mul_sh<60>(a, split_limbs(u[j]));
   }
+  w[3] = (uint64_t)((b + 1) >> 1);
+}
+MPCD_HD void map_words(const int64_t* r, int64_t sc, const int64_t* u, double cos_a, double sin_a, uint64_t* w) {
+  int64_t R[9];
+  rotation_fixed(r, cos_a, sin_a, R);
+#pragma unroll
+  for (int i = 0; i < 3; ++i) map_row(i, R + 3 * i, sc, u, w + 4 * i);
 }
 
 // v' = A v + b in units of 2^-56 (|v_i| < 16, sc < 2 and |u_i| < 8 keep every sum
@@ -163,10 +176,10 @@ MPCD_HD void apply_words(const uint64_t* w, const int64_t* v, int64_t* out) {
   const Limbs x = split_limbs(v[0]), y = split_limbs(v[1]), z = split_limbs(v[2]);
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
-    const Limbs a = word_limbs(w[3 * i]), b = word_limbs(w[3 * i + 1]), c = word_limbs(w[3 * i + 2]);
+    const Limbs a = word_limbs(w[4 * i]), b = word_limbs(w[4 * i + 1]), c = word_limbs(w[4 * i + 2]);
     const uint64_t top = uwide(a.h, x.h) + uwide(b.h, y.h) + uwide(c.h, z.h);
     const uint64_t mid = uwide(a.h, x.l) + uwide(b.h, y.l) + uwide(c.h, z.l) + uwide(a.l, x.h) + uwide(b.l, y.h) + uwide(c.l, z.h);
-    out[i] = (int64_t)((top << 3) + (uint64_t)((int64_t)(mid + (1u << 28)) >> 29) + w[9 + i]);
+    out[i] = (int64_t)((top << 3) + (uint64_t)((int64_t)(mid + (1u << 28)) >> 29) + w[4 * i + 3]);
   }
 }
 

@@ -444,11 +444,11 @@ __device__ __forceinline__ void apply_map_f64(const double* par, double& vx, dou
   } else {
 #pragma unroll
     for (int q = 0; q < 9; ++q) {
-      const Limbs p = word_limbs(w[q]);
+      const Limbs p = word_limbs(w[q + q / 3]);
       A[q] = from_fixed((int64_t)((uint64_t)(int64_t)p.h << 32) + p.l, kMapBits);
     }
 #pragma unroll
-    for (int q = 0; q < 3; ++q) b[q] = from_fixed((int64_t)w[9 + q], kOutBits);
+    for (int q = 0; q < 3; ++q) b[q] = from_fixed((int64_t)w[4 * q + 3], kOutBits);
   }
   const double nx = fma(A[0], vx, fma(A[1], vy, fma(A[2], vz, b[0])));
   const double ny = fma(A[3], vx, fma(A[4], vy, fma(A[5], vz, b[1])));

@@ -262,11 +262,14 @@ __device__ __noinline__ unsigned map_f64(const CellSums& t, long cid, float gf, 
 
 // The collision map of one cell (MPCD::next_tstep, src/libcilia/mpcd.cpp:
 // 140-247) as twelve words (fixed_collide.cuh): in fixed point when the
-// cell's numbers fit, else as float64 factor, axis and mean velocity.  The
-// cell's sum m v^2 before the collision goes to the sums of ke (units of
-// 2^-40) or ke_rest.
-__device__ __forceinline__ void collision_map(double4 s, uint32_t w, long cid, const StepArgs& a, double* par,
-                                              uint64_t& ke, double& ke_rest, unsigned& errbits, bool& gfail) {
+// cell's numbers fit, else as float64 factor, axis and mean velocity, in two
+// parts that need nothing of each other.  The cell's sum m v^2 before the
+// collision goes to the sums of ke (units of 2^-40) or ke_rest.
+//
+// The sums' part: factor and mean velocity.  False if the cell takes the
+// float64 form, whose words it has written to par.
+__device__ __forceinline__ bool cell_factor(double4 s, uint32_t w, long cid, const StepArgs& a, double* par, int64_t& sc,
+                                            int64_t* u, uint64_t& ke, double& ke_rest, unsigned& errbits, bool& gfail) {
   const int nf = cnt_fluid(w), nb = cnt_beads(w);
   int num = nf + nb, sk = -1;
   double M = (double)num;
@@ -287,13 +290,11 @@ __device__ __forceinline__ void collision_map(double4 s, uint32_t w, long cid, c
   // their way
   float gf = 0.f;
   if (num > 1 && !a.inj_gamma) gf = gamma_mt(num, a.seed, a.step, (uint32_t)cid, &gfail);
-  int64_t r[3];
   bool fit = sk < 0;
   if (a.inj_axis) {
+    int64_t r;
 #pragma unroll
-    for (int q = 0; q < 3; ++q) fit = to_fixed<60, 1>(a.inj_axis[3 * cid + q], r[q]) && fit;
-  } else {
-    draw_axis_fixed(a.seed, a.step, (uint32_t)cid, r);
+    for (int q = 0; q < 3; ++q) fit = to_fixed<60, 1>(a.inj_axis[3 * cid + q], r) && fit;
   }
   // dissipated energy (src/libcilia/mpcd.cpp:166-168, 232-234, 243-246): every
   // cell adds sum m v^2 before the collision here, and every particle
@@ -307,16 +308,15 @@ __device__ __forceinline__ void collision_map(double4 s, uint32_t w, long cid, c
     ke_rest += s.w;
     fit = false;
   }
-  int64_t p[3], inv = 0, sc = 1ll << kAxisBits;
+  int64_t p[3], inv = 0;
+  sc = 1ll << kAxisBits;
   fit = fit && to_fixed<52, 9>(s.x, p[0]) && to_fixed<52, 9>(s.y, p[1]) && to_fixed<52, 9>(s.z, p[2]);
   if (nb == 0 && num < 256)
     inv = __ldg(g_inv_n.x + num);  // M = num without beads
   else
     fit = to_fixed<62, 0>(1.0 / M, inv) && fit;
-  uint64_t out[12];
   if (fit) {
     const Limbs iv = split_limbs(inv);
-    int64_t u[3];
     uint64_t rel = (uint64_t)kin;
 #pragma unroll
     for (int q = 0; q < 3; ++q) {
@@ -331,7 +331,6 @@ __device__ __forceinline__ void collision_map(double4 s, uint32_t w, long cid, c
       const double f = a.inj_gamma ? thermostat_factor(injected_gamma(a, cid, errbits), e) : thermostat_factor(gf, e);
       fit = to_fixed<60, 1>(f, sc);
     }
-    if (fit) map_words(r, sc, u, kCosAlpha, kSinAlpha, out);
   }
   if (!fit) {
     t.s = s;
@@ -340,12 +339,39 @@ __device__ __forceinline__ void collision_map(double4 s, uint32_t w, long cid, c
     t.sk = sk;
     uint64_t o[12];
     errbits |= map_f64(t, cid, gf, o, a);
+    ulonglong2* pm = reinterpret_cast<ulonglong2*>(par);
 #pragma unroll
-    for (int q = 0; q < 12; ++q) out[q] = o[q];
+    for (int q = 0; q < 6; ++q) pm[q] = make_ulonglong2(o[2 * q], o[2 * q + 1]);
   }
-  ulonglong2* pm = reinterpret_cast<ulonglong2*>(par);
+  return fit;
+}
+// The axis' part: the rotation.
+__device__ __forceinline__ void cell_rotation(long cid, const StepArgs& a, int64_t* R) {
+  int64_t r[3] = {0, 0, 0};
+  if (a.inj_axis) {
 #pragma unroll
-  for (int q = 0; q < 6; ++q) pm[q] = make_ulonglong2(out[2 * q], out[2 * q + 1]);
+    for (int q = 0; q < 3; ++q) (void)to_fixed<60, 1>(a.inj_axis[3 * cid + q], r[q]);  // cell_factor minds the rest
+  } else {
+    draw_axis_fixed(a.seed, a.step, (uint32_t)cid, r);
+  }
+  rotation_fixed(r, kCosAlpha, kSinAlpha, R);
+}
+__device__ __forceinline__ void store_row(double* par, int i, const int64_t* row, int64_t sc, const int64_t* u) {
+  uint64_t w[4];
+  map_row(i, row, sc, u, w);
+  ulonglong2* p = reinterpret_cast<ulonglong2*>(par + 4 * i);
+  p[0] = make_ulonglong2(w[0], w[1]);
+  p[1] = make_ulonglong2(w[2], w[3]);
+}
+
+// The whole map by one thread.
+__device__ __forceinline__ void collision_map(double4 s, uint32_t w, long cid, const StepArgs& a, double* par, uint64_t& ke,
+                                              double& ke_rest, unsigned& errbits, bool& gfail) {
+  int64_t R[9], u[3], sc;
+  if (!cell_factor(s, w, cid, a, par, sc, u, ke, ke_rest, errbits, gfail)) return;
+  cell_rotation(cid, a, R);
+#pragma unroll
+  for (int i = 0; i < 3; ++i) store_row(par, i, R + 3 * i, sc, u);
 }
 
 // The block's sum of fixed-point energies (units of 2^-40, each thread's below
@@ -390,8 +416,8 @@ __device__ __forceinline__ void flush_ke(uint64_t& ke, double& rest) {
 // per cell (1890 instructions, 12 cycles each at six warps per scheduler); the
 // float64 form kept that pipe 73 % busy.  64-thread blocks fill the SMs in the
 // finest steps (24 warps with 80 registers; five blocks of 128: 36 us, eight
-// with 64 registers: 43).  64^3 cells 48 to 31 us, 80 x 71 x 89 96 to 51, with walls
-// (24 x 21 x 37) 24.6 to 18.5; 8^3 cells take 11.5 us as before.
+// with 64 registers: 43).  64^3 cells 48 to 31 us, 80 x 71 x 89 96 to 51.  For
+// boxes beyond one wave of the pair form below.
 constexpr int kCellThreads = 64;
 __global__ void __launch_bounds__(kCellThreads, 12) k_cell_params_f64(CellsF64 c, StepArgs a) {
   __shared__ BlockEnergy s_e;
@@ -430,6 +456,77 @@ __global__ void __launch_bounds__(kCellThreads, 12) k_cell_params_f64(CellsF64 c
         flush_ke(ke, ke_rest);
         rounds = 0;
       }
+    }
+  }
+  if (gfail) errbits |= kErrGammaLoop;
+  if (errbits) atomicOr(a.err, errbits);
+  energy_end(s_e, ke, ke_rest, 1.0, a.diss);
+}
+
+// The same by pairs of warps, 32 cells a CTA: one warp makes count, sums, Gamma
+// draw and thermostat factor, the other axis and rotation, and both the rows of
+// the map: half the chain, for twice the warps.  That pays while all pairs are
+// on the SMs at once (10 CTAs of 92 registers each): per step 36^3 cells 30.8
+// us against 31.9, 32^3 26.1 / 27.5, the channel (24 x 21 x 37) 33.0 / 36.0, 8^3
+// 12.4 / 13.2; beyond, the one-thread form does: 40^3 39.0 against 41.3, 64^3
+// cells 31 us against 41.
+constexpr int kPairCTAs = 10;  // per SM
+__global__ void __launch_bounds__(kCellThreads, kPairCTAs) k_cell_pairs_f64(CellsF64 c, StepArgs a) {
+  __shared__ BlockEnergy s_e;
+  __shared__ int64_t s_R[2][3][32], s_u[2][3][32], s_sc[2][32];
+  __shared__ int s_fits[2][32];
+  energy_begin(s_e);
+  chain_begin();
+  const int lane = threadIdx.x & 31;
+  const bool sums = threadIdx.x < 32;  // the warp of the sums; the other makes the rotations
+  uint64_t ke = 0;
+  double ke_rest = 0.0;
+  int rounds = 0;
+  unsigned errbits = 0;
+  bool gfail = false;
+  int b = 0;  // two sets of words: one barrier per round
+  for (long c0 = 32l * blockIdx.x; c0 < c.ncell; c0 += 32l * gridDim.x, b ^= 1) {
+    const long cid = c0 + lane;
+    double* par = c.par + 12 * cid;
+    int64_t R[9], u[3] = {0, 0, 0}, sc = 0;
+    if (sums) {
+      int fits = 0;
+      if (cid < c.ncell) {
+        const uint32_t w = __ldcg(c.cnt + cid);
+        const double2* p = reinterpret_cast<const double2*>(c.sum + cid);
+        const double2 lo = __ldcg(p), hi = __ldcg(p + 1);
+        if (w) {
+          c.sum[cid] = make_double4(0.0, 0.0, 0.0, 0.0);
+          c.cnt[cid] = 0u;
+          if (!(a.premapped && cnt_beads(w) > 0))  // else mapped by k_bead_maps_f64
+            fits = cell_factor(make_double4(lo.x, lo.y, hi.x, hi.y), w, cid, a, par, sc, u, ke, ke_rest, errbits, gfail);
+        }
+      }
+      s_fits[b][lane] = fits;
+      s_sc[b][lane] = sc;
+#pragma unroll
+      for (int q = 0; q < 3; ++q) s_u[b][q][lane] = u[q];
+      if (++rounds == (1 << 6)) {  // a cell's energy is below 2^52 units
+        flush_ke(ke, ke_rest);
+        rounds = 0;
+      }
+    } else if (cid < c.ncell) {
+      cell_rotation(cid, a, R);
+#pragma unroll
+      for (int q = 0; q < 3; ++q) s_R[b][q][lane] = R[q];  // the first row goes to the other warp
+    }
+    __syncthreads();
+    if (!s_fits[b][lane]) continue;
+    if (sums) {
+#pragma unroll
+      for (int q = 0; q < 3; ++q) R[q] = s_R[b][q][lane];
+      store_row(par, 0, R, sc, u);
+    } else {
+      sc = s_sc[b][lane];
+#pragma unroll
+      for (int q = 0; q < 3; ++q) u[q] = s_u[b][q][lane];
+      store_row(par, 1, R + 3, sc, u);
+      store_row(par, 2, R + 6, sc, u);
     }
   }
   if (gfail) errbits |= kErrGammaLoop;
@@ -1657,7 +1754,11 @@ int launch_collision_draws(int nc, uint64_t seed, uint64_t step, long n, double*
 }
 
 int launch_cell_params_f64(const CellsF64& c, const StepArgs& a, cudaStream_t s) {
-  launch_in_chain(k_cell_params_f64, grid_for(c.ncell, kCellThreads, -1), kCellThreads, s, a.chained, c, a);
+  // by warp pairs as long as all of them are on the SMs at once (figures there)
+  if (c.ncell <= 32l * kPairCTAs * sm_count())
+    launch_in_chain(k_cell_pairs_f64, (int)((c.ncell + 31) / 32), kCellThreads, s, a.chained, c, a);
+  else
+    launch_in_chain(k_cell_params_f64, grid_for(c.ncell, kCellThreads, -1), kCellThreads, s, a.chained, c, a);
   return 1;
 }
 int launch_fluid_step_f64(const FluidF64& f, const CellsF64& c, const StepArgs& a, cudaStream_t s, int per_sm) {

@@ -40,8 +40,8 @@ void map(const ll* r, ll sc, const ll* u, double ca, double sa, ll* A, ll* b, co
   for (int i = 0; i < 3; ++i) { R[i] = r[i]; U[i] = u[i]; V[i] = v[i]; }
   uint64_t w[12];
   map_words(R, sc, U, ca, sa, w);
-  for (int i = 0; i < 9; ++i) { const Limbs l = word_limbs(w[i]); A[i] = (ll)((uint64_t)(int64_t)l.h << 32) + l.l; }
-  for (int i = 0; i < 3; ++i) b[i] = (ll)w[9 + i];
+  for (int i = 0; i < 9; ++i) { const Limbs l = word_limbs(w[i + i / 3]); A[i] = (ll)((uint64_t)(int64_t)l.h << 32) + l.l; }
+  for (int i = 0; i < 3; ++i) b[i] = (ll)w[4 * i + 3];
   apply_words(w, V, o);
   for (int i = 0; i < 3; ++i) out[i] = o[i];
   if (K) *K = square_words(split_limbs((int64_t)((uint64_t)o[0] << 2)), split_limbs((int64_t)((uint64_t)o[1] << 2)),
