@@ -1848,8 +1848,8 @@ int mpcd_restore(mpcd_engine* h, const void* buf, long long bytes) {
     CK(dev(f.id, 4 * n));
     CK(dev(f.cell, 4 * n));
     for (void* a : {(void*)f.ox, (void*)f.oy, (void*)f.oz, (void*)f.vx, (void*)f.vy, (void*)f.vz}) CK(dev(a, 8 * n));
-    if (hd.version == 1)  // float64 offsets
-      for (uint64_t* a : {f.ox, f.oy, f.oz}) h->launches += launch_convert_offsets((long)n, a, h->stream);
+    for (uint64_t* a : {f.ox, f.oy, f.oz})  // version 1: float64 offsets
+      h->launches += launch_convert_offsets((long)n, a, hd.version == 2, h->stream);
   } else {
     CK(dev(h->f32.id, 4 * n));
     CK(dev(h->f32.pos, 16 * n));

@@ -318,7 +318,7 @@ int launch_load_fluid_f64(long n, const double* pos, const double* vel, const Bo
 int launch_load_fluid_f32(long n, const double* pos, const double* vel, const Box& box, const FluidF32& f,
                           cudaStream_t s);
 // an array of float64 offsets in [0, 1) into fixed-point ones, in place
-int launch_convert_offsets(long n, uint64_t* o, cudaStream_t s);
+int launch_convert_offsets(long n, uint64_t* o, bool integers, cudaStream_t s);
 // Writes to every page of a small host buffer that a copy from the device is
 // about to fill: a page that was never touched costs the copy engine about 40
 // us, the host a few.

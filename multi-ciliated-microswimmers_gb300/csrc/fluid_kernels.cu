@@ -1479,9 +1479,14 @@ __global__ void k_load_fluid_f32(long n, const double* pos, const double* vel, B
   }
 }
 
-// float64 offsets (of an older snapshot) into fixed point, in place
-__global__ void k_convert_offsets(long n, uint64_t* o) {
+// a snapshot's offsets in place: float64 ones (of an older version) into fixed
+// point, integers into their range
+__global__ void k_convert_offsets(long n, uint64_t* o, bool integers) {
   for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
+    if (integers) {  // whatever the bytes were, an offset
+      o[i] &= kOffOne - 1;
+      continue;
+    }
     double d = __longlong_as_double((long long)o[i]);
     if (!(d >= 0.0 && d < 1.0)) d = 0.5;
     o[i] = offset_from_double(d);
@@ -1935,9 +1940,9 @@ int launch_load_fluid_f32(long n, const double* pos, const double* vel, const Bo
   k_load_fluid_f32<<<grid_for(n), kThreads, 0, s>>>(n, pos, vel, box, f);
   return 1;
 }
-int launch_convert_offsets(long n, uint64_t* o, cudaStream_t s) {
+int launch_convert_offsets(long n, uint64_t* o, bool integers, cudaStream_t s) {
   if (n == 0) return 0;
-  k_convert_offsets<<<grid_for(n), kThreads, 0, s>>>(n, o);
+  k_convert_offsets<<<grid_for(n), kThreads, 0, s>>>(n, o, integers);
   return 1;
 }
 int launch_store_beads(const MDState& m, long s0, long nb, double* pos, double* vel, unsigned* status,
