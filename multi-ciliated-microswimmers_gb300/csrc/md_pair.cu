@@ -920,8 +920,12 @@ int launch_pair(const MDState& m, const typename Bin::Cells& c, const MDStepArgs
 
 }  // namespace
 
-// enough threads for a thread per owned bead and axis in the force sums
-int md_pair_threads(int tile) { return tile <= 64 ? 256 : (tile <= 128 ? 384 : 512); }
+// Enough threads for a thread per owned bead and axis in the force sums, and so
+// many that an SM's registers hold one CTA: two of 256 threads fit, and beside
+// the fluid pass pairs of tiles shared an SM while others had none (a step of
+// the 64^3 swimmer 446 us; 288 threads 404, 320 404, 384 409; alone 326 / 329 /
+// 330 / 335 per launch, 192 threads 342)
+int md_pair_threads(int tile) { return tile <= 64 ? 288 : (tile <= 128 ? 384 : 512); }
 
 int launch_md_pair_f64cells(const MDState& m, const CellsF64& c, const MDStepArgs& a, cudaStream_t s,
                             cudaError_t* st) {
