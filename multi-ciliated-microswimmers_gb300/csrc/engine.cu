@@ -245,6 +245,9 @@ void free_md(MDState& m) {
   cudaFree(m.de_local_end);
   cudaFree(m.de_solo);
   cudaFree(m.de_nslot);
+  cudaFree(m.de_slots);
+  cudaFree(m.de_at);
+  cudaFree(m.de_shape);
   cudaFree(m.de_code);
   cudaFree(m.de_rk);
   cudaFree(m.pr_start);
@@ -395,14 +398,16 @@ int build_md(mpcd_engine* h) {
   const char* mt = std::getenv("MPCD_MD_MIN_TILE");
   const int min_tile = mt ? std::max(0, std::min(256, std::atoi(mt))) : 0;
   const int f32cells = h->p.precision == MPCD_FP32 ? 1 : 0;
-  // double-float arithmetic: the entries layout (md_entries.cu) where the bead
-  // set fits it, else the slot layouts of plan_md.  MPCD_MD_SLOTS=1 keeps the
-  // slot layout (tests of that kernel)
-  const char* slots = std::getenv("MPCD_MD_SLOTS");
-  const bool entries = in.df && !in.pair && !(slots && std::atoi(slots) != 0) &&
-                       plan_entries(in, f32cells, pl, min_tile).empty();
-  const std::string why = entries ? "" : plan_md(in, MDForce{}, allow_cluster, false, f32cells, pl, min_tile);
+  const std::string why = plan_md(in, MDForce{}, allow_cluster, false, f32cells, pl, min_tile);
   if (!why.empty()) return fail(h, MPCD_EINVAL, why);
+  // double-float arithmetic: the entries layout (md_entries.cu) where the bead
+  // set fits it, with the same results.  MPCD_MD_SLOTS=1 keeps the slot layout
+  // (tests of that kernel)
+  const char* slots = std::getenv("MPCD_MD_SLOTS");
+  if (in.df && !in.pair && !(slots && std::atoi(slots) != 0)) {
+    MDPlan de;
+    if (plan_entries(in, f32cells, pl, de, min_tile).empty()) pl = std::move(de);
+  }
   if (const char* ps = std::getenv("MPCD_MD_PLAN_STATS"); ps && std::atoi(ps) && pl.pair) {
     // the pair layout's per-tile sizes: force entries (of them reaching only
     // the tile), halo, incidences, hubs reached
@@ -549,7 +554,7 @@ int build_md(mpcd_engine* h) {
   if (m.df || m.pair) {
     m.df_nb_max = pl.df_nb_max;
     for (int b = 0; b < 2; ++b) {
-      if (m.pair) {
+      if (!m.de) {
         CK(dalloc(&m.q[b], 2 * (size_t)ns));
       } else {  // tag 0: no evaluation's packet
         CK(dalloc(&m.qp[b], 3 * (size_t)ns));
@@ -573,11 +578,18 @@ int build_md(mpcd_engine* h) {
     m.de_nent_max = pl.de_nent_max;
     m.de_ninc_max = pl.de_ninc_max;
     m.de_step = pl.de_step;
+    m.de_lanes = pl.de_lanes;
     CK(dalloc(&m.de_start, m.ntiles + 1));
     CK(dalloc(&m.de_local_end, m.ntiles));
     CK(dalloc(&m.de_solo, m.ntiles));
     CK(dalloc(&m.de_nslot, m.ntiles));
     CK(up(m.de_nslot, pl.de_nslot.data(), m.ntiles * sizeof(int)));
+    CK(dalloc(&m.de_slots, m.ntiles));
+    CK(dalloc(&m.de_at, ns));
+    CK(dalloc(&m.de_shape, ns));
+    CK(up(m.de_slots, pl.de_slots.data(), m.ntiles * sizeof(int)));
+    CK(up(m.de_at, pl.de_at.data(), ns * sizeof(int)));
+    CK(up(m.de_shape, pl.de_shape.data(), ns * sizeof(uint32_t)));
     CK(dalloc(&m.de_code, ne));
     CK(dalloc(&m.de_rk, ne));
     CK(up(m.de_start, pl.de_start.data(), (m.ntiles + 1) * sizeof(int)));

@@ -182,21 +182,29 @@ struct MDState {
   int* halo_run_start = nullptr;   // ntiles + 1
   int2* halo_single = nullptr;     // per tile: halo entries outside long runs {slot, rank}
   int* halo_single_start = nullptr;
-  float4* q[2] = {nullptr, nullptr};  // pair kernel: two buffers of positions, 32 bytes per slot
-  // double-float kernels: two buffers of position packets, one per coordinate
+  float4* q[2] = {nullptr, nullptr};  // two buffers of positions, 32 bytes per slot (md_df.cu, md_pair.cu)
+  // entries kernel: two buffers of position packets, one per coordinate
   // and slot (coordinate-major: offset pair, cell, tag of the force evaluation)
   uint4* qp[2] = {nullptr, nullptr};
   // entries kernel (md_entries.cu; de = 1), one slot per bead: per tile its
   // force entries, those between its own beads first (codes as the kernel
-  // stages them, {rest length, -2k} as float pairs); a bead's incidences are
-  // its springs (sp_start).  de_solo: the tile holds one bead with a long list
+  // stages them, {rest length, -2k} as float pairs).  The forces on a bead lie
+  // in words, in the order in which the slots and lanes of md_df.cu (de_lanes per
+  // slot) add them: from de_at on, a nibble of de_shape per slot, its rows of
+  // de_lanes words.  de_solo: the tile holds one bead with a long list; its
+  // de_shape is the number of slots, its de_at the lane whose side of the last
+  // tree counts, the tile's de_slots the rows of every slot
   int de = 0;
   int de_nent_max = 0, de_ninc_max = 0;
   int* de_start = nullptr;      // ntiles + 1
   int* de_local_end = nullptr;  // ntiles
   int* de_solo = nullptr;       // ntiles
-  int* de_nslot = nullptr;      // ntiles: incidence words of the tile
-  int de_step = 1;  // words between a bead's incidences: 1 (bead after bead) or the tile width (transposed)
+  int* de_nslot = nullptr;      // ntiles: force words of the tile
+  int* de_slots = nullptr;      // ntiles: most slots of one of its beads
+  int* de_at = nullptr;         // per slot
+  uint32_t* de_shape = nullptr;
+  int de_lanes = 8;
+  int de_step = 1;  // between a bead's words: 1 (bead after bead) or the tile width (transposed)
   uint4* de_code = nullptr;
   float4* de_rk = nullptr;
   // pair kernel (md_pair.cu), on the layout above with one slot per bead:

@@ -1,10 +1,6 @@
 // MD substeps of one MPC step for the float64 path, in double-float
 // arithmetic on the FP32 pipes.
 //
-// The general form of the double-float MD: every bead set whose layout fits the
-// device runs here; those that fit the layout of md_entries.cu (a thread per
-// spring pair, less than half the time on large swimmers) run there.
-//
 // Same integrator and forces as md_kernels.cu (velocity Verlet of
 // src/libcilia/mdobject.cpp:36-72 inside the loop of src/simulation.cpp:217-265;
 // springs of src/cilia.cpp:127-239, src/sphere.cpp:87-119, src/clami.cpp:188-198)
@@ -21,24 +17,14 @@
 // spring constants come as float pairs prepared on the host.
 //
 // Each CTA keeps its tile's spring and bond tables in shared memory for the
-// whole launch.  Positions are exchanged between tiles as tagged packets: a
-// coordinate of a bead is one 16-byte packet {offset high, offset low, cell,
-// tag} written by one 128-bit store into one of two global buffers, the tag
-// naming the force evaluation it belongs to; a tile that needs the bead polls
-// the packet itself until the tag is the one it waits for.  No barrier and no
-// second read: data and flag arrive together, one way through L2.  The chain
-// of a substep is what bounds the launch (a few thousand beads, 51 dependent
-// evaluations; every pipe and DRAM are idle), so it is kept short: the lanes
-// that sum a bead's force own its state (lane k its coordinate k), the lanes'
-// partial forces are combined by a transposing exchange that leaves each
-// coordinate with its owner, and a tile without helper slots needs two CTA
-// barriers per substep.  Measured alone on swimmer64 (116 tiles, 51
-// evaluations), against a grid barrier followed by copies of the halo: 168
-// against 217 us in double-float, 148 against 203 with float springs; the
-// 19 tiles of a 700-bead swimmer 158 against 192.
-// The partial forces of a bead's helper slots are added in a fixed order: by
-// one warp (lane-strided, then by a transposing tree) for long runs, in slot
-// order for short ones.
+// whole launch.  Positions are exchanged between tiles through two global
+// buffers of pairs (two float4 per bead) after a bounded grid barrier: the
+// halo arrives by bulk asynchronous copies (TMA, one per run of consecutive
+// slots, completing on an mbarrier) while the lanes work on the springs
+// between beads of their own tile, and is waited for (bounded) before the
+// springs that reach it.  The partial forces of a bead's helper slots are
+// added in a fixed order: by one warp (lane-strided, then a xor tree) for
+// long runs, by the primary in slot order for short ones.
 //
 // The cilia's rest lengths: the beat's target length of every bond is fixed
 // during one MPC step's substeps (the midpoint moves after them), so it is
@@ -50,11 +36,19 @@
 #include "df32.cuh"
 #include "md_common.cuh"
 #include "md_df_coord.cuh"
-#include "md_packets.cuh"
+#include "tma.cuh"
 
 namespace mpcd {
 
 namespace {
+
+constexpr uint32_t kHaloWait = 1u << 22;  // polls of the halo's mbarrier before giving up
+
+// 16-byte asynchronous global -> shared copy through L2 (cp.async.cg)
+__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 // Tile-resident spring and bond tables in shared memory.
 struct Tables {
@@ -114,24 +108,10 @@ __device__ __forceinline__ void springs_df(const Tables& tb, const float4* st, c
 }
 
 
-// Coordinate k of a staged entry (two float4, md_df_coord.cuh): its words are
-// the offset's high part k, low part 3 + k, and the cell (x and y as 16-bit
-// halves of word 6, z as a float in word 7).
-__device__ __forceinline__ void stage_coord(float4* e, int k, float h, float l, int c) {
-  float* w = reinterpret_cast<float*>(e);
-  w[k] = h;
-  w[3 + k] = l;
-  if (k < 2)
-    reinterpret_cast<unsigned short*>(w + 6)[k] = (unsigned short)c;
-  else
-    w[7] = (float)c;
-}
-
-// shared-memory layout of one tile: two buffers of its own beads, its halo,
-// the halo's slots and the tables
+// shared-memory layout of one tile
 struct DfSmem {
-  size_t st, halo, hslot, flag, code, rest, m2k, nl, ol, dg, tg, bd, part, total;
-  __host__ __device__ DfSmem(int T, int hmax, int nsp, int nb) {
+  size_t st, bar, flag, runs, single, code, rest, m2k, nl, ol, dg, tg, bd, part, total;
+  __host__ __device__ DfSmem(int T, int hmax, int nsp, int nb, int nrun, int nsingle) {
     size_t o = 0;
     auto take = [&](size_t bytes, size_t align) {
       o = (o + align - 1) / align * align;
@@ -139,10 +119,11 @@ struct DfSmem {
       o += bytes;
       return r;
     };
-    st = take(64 * (size_t)T, 16);
-    halo = take(32 * (size_t)hmax, 16);
-    hslot = take(4 * (size_t)hmax, 4);
+    st = take(32 * (size_t)(T + hmax), 16);
+    bar = take(8, 8);
     flag = take(4, 4);
+    runs = take(16 * (size_t)nrun, 16);
+    single = take(8 * (size_t)nsingle, 8);
     rest = take(8 * (size_t)nsp, 8);
     m2k = take(8 * (size_t)nsp, 8);
     nl = take(8 * (size_t)nb, 8);
@@ -151,7 +132,7 @@ struct DfSmem {
     tg = take(8 * (size_t)nb, 8);
     bd = take(8 * (size_t)nb, 8);
     code = take(4 * (size_t)nsp, 4);
-    part = take(24 * (size_t)T, 8);
+    part = take(24 * (size_t)T, 4);
     total = o;
   }
 };
@@ -160,11 +141,8 @@ template <int LANES, bool kFloat, typename Bin>
 __device__ void md_df_body(const MDState& m, const MDStepArgs& a, Bin bin) {
   extern __shared__ __align__(16) unsigned char smem[];
   const int T = m.tile;
-  const DfSmem L(T, m.hmax, m.df_nsp_max, m.df_nb_max);
-  float4* own0 = reinterpret_cast<float4*>(smem + L.st);  // buffer b at own0 + 2 T b
-  float4* halo = reinterpret_cast<float4*>(smem + L.halo);
-  int* s_hslot = reinterpret_cast<int*>(smem + L.hslot);
-  int* s_fail = reinterpret_cast<int*>(smem + L.flag);  // 1: a packet never came
+  const DfSmem L(T, m.hmax, m.df_nsp_max, m.df_nb_max, m.df_nrun_max, m.df_nsingle_max);
+  float4* st = reinterpret_cast<float4*>(smem + L.st);
   uint32_t* s_code = reinterpret_cast<uint32_t*>(smem + L.code);
   float2* s_rest = reinterpret_cast<float2*>(smem + L.rest);
   float2* s_m2k = reinterpret_cast<float2*>(smem + L.m2k);
@@ -173,8 +151,13 @@ __device__ void md_df_body(const MDState& m, const MDStepArgs& a, Bin bin) {
   float2* s_dg = reinterpret_cast<float2*>(smem + L.dg);
   float2* s_tg = reinterpret_cast<float2*>(smem + L.tg);
   float2* s_bd = reinterpret_cast<float2*>(smem + L.bd);
-  float2* part = reinterpret_cast<float2*>(smem + L.part);  // per slot: its lanes' force (three pairs)
+  float* part = reinterpret_cast<float*>(smem + L.part);  // per slot: its lanes' force (6 floats)
+  uint64_t* hbar = reinterpret_cast<uint64_t*>(smem + L.bar);  // halo copies' completion
+  int* hflag = reinterpret_cast<int*>(smem + L.flag);           // 1: the halo runs are valid
+  int4* s_runs = reinterpret_cast<int4*>(smem + L.runs);         // this tile's long halo runs
+  int2* s_single = reinterpret_cast<int2*>(smem + L.single);     // and its other halo entries
   const Tables tb{s_code, s_rest, s_m2k, s_nl, s_dg};
+  const StageDF sv{st};
 
   const int tile = blockIdx.x;
   const int base = tile * T;
@@ -187,35 +170,54 @@ __device__ void md_df_body(const MDState& m, const MDStepArgs& a, Bin bin) {
   const int mv = m.moves[slot];
   const int me = mv >= 0 ? m.prim[slot] - base : 0;
   const int s0 = m.sp_start[slot] - S0, sm = m.sp_split[slot] - S0, s1 = m.sp_start[slot + 1] - S0;
-  // the lanes of a primary slot own its bead: coordinate k belongs to lane
-  // k mod LANES (with two lanes, x and z to lane 0)
-  constexpr int NC = (3 + LANES - 1) / LANES;
-  const bool prim = mv == 0 || mv == 1, moves = mv == 1;
+  // bead owners: thread tid < T owns slot base + tid
+  const int oslot = base + tid;
+  const int omv = tid < T ? m.moves[oslot] : -1;
+  const bool oprim = omv == 0 || omv == 1, omoves = omv == 1;
   const bool helpers = m.tile_help[tile] != 0;
   // a primary with helpers and its helper slots form a run of 1 + nh slots;
-  // runs longer than kTreeRun are summed by the primary's warp, shorter ones
-  // by the owners
+  // runs longer than kTreeRun are summed by a warp, shorter ones by the primary
   constexpr int kTreeRun = 8;
-  const int nh = prim ? m.nhelp[slot] : 0;
+  const int onh = oprim ? m.nhelp[oslot] : 0;
+  const int owarps = (T + 31) / 32;  // warps holding the owner threads
   const int h0 = m.halo_start[tile], hn0 = m.halo_start[tile + 1] - h0;
   const int c0 = m.tile_cil[tile], c1 = m.tile_cil[tile + 1];
   const int b0 = m.tile_b0[tile], nb = m.tile_nb[tile];
   const int nsp = m.sp_start[base + T] - S0;
-  const dfloat dt{a.dt_pair.x, a.dt_pair.y}, dt2{a.dt2_pair.x, a.dt2_pair.y};
+  const dfloat dt = df_from_double(a.dt), dt2 = df_from_double(a.dt / 2.0);
 
-  // the halo's slots; every one must lie in the packet buffers
-  if (tid == 0) *s_fail = hn0 > m.hmax;
-  __syncthreads();
-  for (int i = tid; i < hn0 && hn0 <= m.hmax; i += nthr) {
-    const int g = m.halo[h0 + i];
-    s_hslot[i] = g;
-    if (g < 0 || g >= m.nslots) *s_fail = 1;
+  // halo copies: long runs of consecutive slots by bulk copies (TMA) that
+  // complete on an mbarrier, the other entries by per-thread cp.async
+  const int r0 = m.halo_run_start[tile], nrun = m.halo_run_start[tile + 1] - r0;
+  const int e0 = m.halo_single_start[tile], nsingle = m.halo_single_start[tile + 1] - e0;
+  for (int r = tid; r < nrun && nrun <= m.df_nrun_max; r += nthr) s_runs[r] = m.halo_run[r0 + r];
+  for (int i = tid; i < nsingle && nsingle <= m.df_nsingle_max; i += nthr) s_single[i] = m.halo_single[e0 + i];
+  if (tid == 0) {
+    // every copy must stay inside the staged halo and the position buffers,
+    // and the copies must cover the halo exactly
+    int ok = 1, tot = nsingle;
+    for (int r = 0; r < nrun; ++r) {
+      const int4 run = m.halo_run[r0 + r];
+      ok &= run.z > 0 && run.y >= 0 && run.y + run.z <= m.hmax && run.x >= 0 && run.x + run.z <= m.nslots;
+      tot += run.z;
+    }
+    for (int i = 0; i < nsingle; ++i) {
+      const int2 e = m.halo_single[e0 + i];
+      ok &= e.y >= 0 && e.y < m.hmax && e.x >= 0 && e.x < m.nslots;
+    }
+    ok &= tot == hn0 && nrun <= m.df_nrun_max && nsingle <= m.df_nsingle_max;
+    if (!ok) atomicOr(a.err, kErrLayout);
+    *hflag = ok;
+    mbar_init(hbar, 1);
+    fence_mbar_init();
   }
   __syncthreads();
-  const int hn = *s_fail ? 0 : hn0;  // no halo (and an error) for an inconsistent plan
-  if (*s_fail && tid == 0) atomicOr(a.err, kErrLayout);
-  __syncthreads();
-  if (tid == 0) *s_fail = 0;
+  const bool halo_ok = *hflag != 0;  // no halo copies (and an error) for an inconsistent plan
+  const int hn = halo_ok ? hn0 : 0;
+  uint32_t long_bytes = 0;
+  if (halo_ok)
+    for (int r = 0; r < nrun; ++r) long_bytes += 32u * (uint32_t)s_runs[r].z;
+  uint32_t hphase = 0;
   // tile-resident tables
   for (int i = tid; i < nsp; i += nthr) {
     s_code[i] = __ldg(m.sp_code + S0 + i);
@@ -247,69 +249,61 @@ __device__ void md_df_body(const MDState& m, const MDStepArgs& a, Bin bin) {
       off += nbnd;
     }
   }
-  // the owned coordinates
-  BeadCoord x[NC];
-  dfloat v[NC], f[NC];
+  BeadCoord x{0, {0.f, 0.f}}, y{0, {0.f, 0.f}}, z{0, {0.f, 0.f}};
+  dfloat vx{0.f, 0.f}, vy{0.f, 0.f}, vz{0.f, 0.f};
+  dfloat fx{0.f, 0.f}, fy{0.f, 0.f}, fz{0.f, 0.f};
   double ke_coll = 0.0;
-  {
-    double X[3] = {0.0, 0.0, 0.0}, V[3] = {0.0, 0.0, 0.0};
-    if (prim) {
-      X[0] = m.x[0][slot];
-      X[1] = m.y[0][slot];
-      X[2] = m.z[0][slot];
-      V[0] = m.vx[slot];
-      V[1] = m.vy[slot];
-      V[2] = m.vz[slot];
-      if (a.collide && moves) {  // the beads' collision, folded in (every lane of the slot the same)
-        const double ke = bin.collide(X[0], X[1], X[2], V[0], V[1], V[2]);
-        if (lane == 0) ke_coll = ke;
-      }
-    }
-#pragma unroll
-    for (int j = 0; j < NC; ++j) {
-      const int k = lane + j * LANES;
-      x[j] = coord_from_double(k == 0 ? X[0] : (k == 1 ? X[1] : X[2]));
-      v[j] = df_from_double(k == 0 ? V[0] : (k == 1 ? V[1] : V[2]));
-      f[j] = {0.f, 0.f};
-    }
+  if (oprim) {
+    const double X = m.x[0][oslot], Y = m.y[0][oslot], Z = m.z[0][oslot];
+    double VX = m.vx[oslot], VY = m.vy[oslot], VZ = m.vz[oslot];
+    if (a.collide && omoves) ke_coll = bin.collide(X, Y, Z, VX, VY, VZ);  // the beads' collision, folded in
+    x = coord_from_double(X);
+    y = coord_from_double(Y);
+    z = coord_from_double(Z);
+    vx = df_from_double(VX);
+    vy = df_from_double(VY);
+    vz = df_from_double(VZ);
   }
   if (a.collide) {  // the dissipated-energy bookkeeping of the collided beads
     const double tot = block_sum_f64(ke_coll);
     if (tid == 0 && tot != 0.0) atomicAdd(a.diss, -tot);
   }
+  const unsigned nblocks = gridDim.x;
+  unsigned barriers = 0;
+  int eval = 0;
   bool refreshed = false;
 
-  // own beads of evaluation e: into shared memory (buffer e & 1) and, as
-  // packets, into global buffer e & 1
-  auto publish = [&](int e) {
-    if (prim) {
-#pragma unroll
-      for (int j = 0; j < NC; ++j) {
-        const int k = lane + j * LANES;
-        if (k < 3) {
-          const Packet pk{__float_as_uint(x[j].o.h), __float_as_uint(x[j].o.l), (uint32_t)x[j].c, a.tag0 + (uint32_t)e};
-          packet_store(m.qp[e & 1] + (size_t)k * m.nslots + slot, pk);
-          stage_coord(own0 + 2 * ((size_t)T * (e & 1) + q), k, x[j].o.h, x[j].o.l, x[j].c);
-        }
-      }
+  // own beads into shared memory and the global pair buffer b
+  auto publish = [&](int b) {
+    if (oprim) {
+      float4 p0, p1;
+      pack_coords(x, y, z, p0, p1);
+      st[2 * tid] = p0;
+      st[2 * tid + 1] = p1;
+      m.q[b][2 * oslot] = p0;
+      m.q[b][2 * oslot + 1] = p1;
     }
   };
-  // the halo of evaluation e into shared memory.  A tile writes a buffer again
-  // two evaluations later, for which it has to have received the next
-  // evaluation's packets of every tile that reads it (the planner makes the
-  // halo relation symmetric), and those are published after this read.
-  auto receive = [&](int e) {
-    receive_packets(m.qp[e & 1], m.nslots, a.tag0 + (uint32_t)e, hn, s_hslot, tid, nthr, a.err, s_fail,
-                    [&](int p, int k, const Packet& d) {
-                      stage_coord(halo + 2 * p, k, __uint_as_float(d.h), __uint_as_float(d.l), (int)d.c);
-                    });
-  };
-  // forces on the owned beads at evaluation e; false when a packet never came
-  auto evaluate = [&](int e) -> bool {
-    const float4* own = own0 + 2 * (size_t)T * (e & 1);
-    __syncthreads();  // the tile's own positions are staged
-    if (*s_fail) return false;
-    if (c1 > c0 && refresh_due(a, e)) {
+  // forces on the owned beads; buffer b holds the other tiles' beads
+  auto evaluate = [&](int b) {
+    // other tiles' beads: one bulk asynchronous copy (TMA) per run of
+    // consecutive slots, completing on the mbarrier; waited for before the
+    // halo springs
+    if (hn > 0) {
+      // the other tiles wrote the buffer through the generic proxy; order
+      // those writes (acquired at the barrier) before this thread's bulk reads
+      if (tid < nrun) asm volatile("fence.proxy.async.global;" ::: "memory");
+      for (int r = tid; r < nrun; r += nthr) {
+        const int4 run = s_runs[r];
+        bulk_load(st + 2 * (T + run.y), m.q[b] + 2 * (size_t)run.x, 32u * (uint32_t)run.z, hbar);
+      }
+      for (int i = tid; i < nsingle; i += nthr) {
+        const int2 e = s_single[i];
+        cp_async16(st + 2 * (T + e.y), m.q[b] + 2 * (size_t)e.x);
+        cp_async16(st + 2 * (T + e.y) + 1, m.q[b] + 2 * (size_t)e.x + 1);
+      }
+    }
+    if (c1 > c0 && refresh_due(a, eval)) {
       // Cilia::length (src/cilia.cpp:79-121) for every refreshed bond, in pairs
       refreshed = true;
       int off = 0;
@@ -322,7 +316,7 @@ __device__ void md_df_body(const MDState& m, const MDStepArgs& a, Bin bin) {
           const int k = cl.bond_base + i - b0;
           const int l0 = cl.slot0 - base;
           const int ia = l0 + cl.stride * i, ib = l0 + cl.stride * (i + 1);
-          const DfDiff d = df_diff(own[2 * ia], own[2 * ia + 1], own[2 * ib], own[2 * ib + 1]);
+          const DfDiff d = df_diff(st[2 * ia], st[2 * ia + 1], st[2 * ib], st[2 * ib + 1]);
           const dfloat tl = df_mul(d.d2, df_rsqrt(d.d2));
           const dfloat tg{s_tg[k].x, s_tg[k].y}, bd{s_bd[k].x, s_bd[k].y}, ol{s_ol[k].x, s_ol[k].y};
           dfloat l = tg;
@@ -339,141 +333,157 @@ __device__ void md_df_body(const MDState& m, const MDStepArgs& a, Bin bin) {
       }
       __syncthreads();
     }
+    ++eval;
     float axh = 0.f, axl = 0.f, ayh = 0.f, ayl = 0.f, azh = 0.f, azl = 0.f;
     float4 m0 = make_float4(0.f, 0.f, 0.f, 0.f), m1 = m0;
     if (mv >= 0) {
-      m0 = own[2 * me];
-      m1 = own[2 * me + 1];
-      springs_df<LANES, kFloat>(tb, own, m0, m1, s0 + lane, sm, axh, axl, ayh, ayl, azh, azl);
+      m0 = st[2 * me];
+      m1 = st[2 * me + 1];
+      springs_df<LANES, kFloat>(tb, st, m0, m1, s0 + lane, sm, axh, axl, ayh, ayl, azh, azl);
     }
     if (hn > 0) {
-      receive(e);
-      __syncthreads();
-      if (mv >= 0)
-        springs_df<LANES, kFloat>(tb, halo - 2 * T, m0, m1, sm + lane, s1, axh, axl, ayh, ayl, azh, azl);
-    }
-    // the lanes' partial forces, each coordinate to its owner
-    float fh[NC], fl[NC];
-    if constexpr (LANES == 2) {
-      fh[0] = lane ? ayh : axh;
-      fl[0] = lane ? ayl : axl;
-      exchange_add(fh[0], fl[0], lane ? axh : ayh, lane ? axl : ayl, 1);
-      fh[1] = azh;
-      fl[1] = azl;
-      exchange_add(fh[1], fl[1], azh, azl, 1);
-    } else {
-      // quarters of the group: with eight lanes, lanes 2k and 2k + 1 hold
-      // component k; lane k of the slot takes it from there
-      group_sum_xyz<LANES>(lane, axh, axl, ayh, ayl, azh, azl, fh[0], fl[0]);
-      if constexpr (LANES == 8) {
-        const int src = (tid & 31 & ~7) | (2 * lane & 7);
-        fh[0] = __shfl_sync(0xffffffffu, fh[0], src);
-        fl[0] = __shfl_sync(0xffffffffu, fl[0], src);
+      if (long_bytes) {
+        if (!mbar_wait(hbar, hphase & 1u, kHaloWait)) atomicOr(a.err, kErrBarrier);
+        ++hphase;
       }
-    }
-    if (helpers) {
-#pragma unroll
-      for (int j = 0; j < NC; ++j)
-        if (lane + j * LANES < 3) part[3 * q + lane + j * LANES] = make_float2(fh[j], fl[j]);
+      cp_async_wait_all();
       __syncthreads();
-      // long runs: the warp holding the primary's lanes adds the run's slot
-      // sums, lane-strided and then by a tree -- a fixed order
+    }
+    if (mv >= 0) springs_df<LANES, kFloat>(tb, st, m0, m1, sm + lane, s1, axh, axl, ayh, ayl, azh, azl);
+    // the halo region is refilled by the async proxy next substep
+    fence_proxy_async_smem();
+    // fixed-order combination of the four lanes
+#pragma unroll
+    for (int o = 1; o < LANES; o <<= 1) {
+      const float bxh = __shfl_xor_sync(0xffffffffu, axh, o), bxl = __shfl_xor_sync(0xffffffffu, axl, o);
+      const float byh = __shfl_xor_sync(0xffffffffu, ayh, o), byl = __shfl_xor_sync(0xffffffffu, ayl, o);
+      const float bzh = __shfl_xor_sync(0xffffffffu, azh, o), bzl = __shfl_xor_sync(0xffffffffu, azl, o);
+      df_acc(axh, axl, bxh, bxl);
+      df_acc(ayh, ayl, byh, byl);
+      df_acc(azh, azl, bzh, bzl);
+    }
+    if (lane == 0) {
+      float* pp = part + 6 * q;
+      pp[0] = axh;
+      pp[1] = axl;
+      pp[2] = ayh;
+      pp[3] = ayl;
+      pp[4] = azh;
+      pp[5] = azl;
+    }
+    __syncthreads();
+    if (helpers && tid < 32 * owarps) {
+      // long runs: the warp holding the primary's owner thread adds the run's
+      // slot sums, lane-strided and then by a xor tree -- a fixed order
       const int lane32 = tid & 31;
-      unsigned runs = __ballot_sync(0xffffffffu, lane == 0 && nh + 1 > kTreeRun);
+      unsigned runs = __ballot_sync(0xffffffffu, onh + 1 > kTreeRun);
       while (runs) {
-        const int src = __ffs(runs) - 1;  // the primary's lane 0
+        const int src = __ffs(runs) - 1;
         runs &= runs - 1;
-        const int p = ((tid & ~31) + src) / LANES;
-        const int len = 1 + __shfl_sync(0xffffffffu, nh, src);
+        const int p = (tid & ~31) + src;
+        const int len = 1 + __shfl_sync(0xffffffffu, onh, src);
         float gxh = 0.f, gxl = 0.f, gyh = 0.f, gyl = 0.f, gzh = 0.f, gzl = 0.f;
         for (int k = lane32; k < len; k += 32) {
-          const float2* ph = part + 3 * (p + k);
-          df_acc(gxh, gxl, ph[0].x, ph[0].y);
-          df_acc(gyh, gyl, ph[1].x, ph[1].y);
-          df_acc(gzh, gzl, ph[2].x, ph[2].y);
+          const float* ph = part + 6 * (p + k);
+          df_acc(gxh, gxl, ph[0], ph[1]);
+          df_acc(gyh, gyl, ph[2], ph[3]);
+          df_acc(gzh, gzl, ph[4], ph[5]);
         }
-        float h, l;
-        group_sum_xyz<32>(lane32, gxh, gxl, gyh, gyl, gzh, gzl, h, l);
 #pragma unroll
-        for (int j = 0; j < NC; ++j) {
-          const int k = lane + j * LANES;  // component k lies in lanes 8 k ..
-          const float oh = __shfl_sync(0xffffffffu, h, 8 * k & 31), ol = __shfl_sync(0xffffffffu, l, 8 * k & 31);
-          if ((lane32 & ~(LANES - 1)) == src) {
-            fh[j] = oh;
-            fl[j] = ol;
-          }
+        for (int o = 16; o > 0; o >>= 1) {
+          const float bxh = __shfl_xor_sync(0xffffffffu, gxh, o), bxl = __shfl_xor_sync(0xffffffffu, gxl, o);
+          const float byh = __shfl_xor_sync(0xffffffffu, gyh, o), byl = __shfl_xor_sync(0xffffffffu, gyl, o);
+          const float bzh = __shfl_xor_sync(0xffffffffu, gzh, o), bzl = __shfl_xor_sync(0xffffffffu, gzl, o);
+          df_acc(gxh, gxl, bxh, bxl);
+          df_acc(gyh, gyl, byh, byl);
+          df_acc(gzh, gzl, bzh, bzl);
         }
-      }
-      if (nh > 0 && nh + 1 <= kTreeRun) {  // short runs, in slot order
-#pragma unroll
-        for (int j = 0; j < NC; ++j) {
-          const int k = lane + j * LANES;
-          if (k < 3)
-            for (int r = 1; r <= nh; ++r) {
-              const float2 ph = part[3 * (q + r) + k];
-              df_acc(fh[j], fl[j], ph.x, ph.y);
-            }
+        if (lane32 == src) {
+          fx = df_norm(gxh, gxl);
+          fy = df_norm(gyh, gyl);
+          fz = df_norm(gzh, gzl);
         }
       }
     }
-#pragma unroll
-    for (int j = 0; j < NC; ++j) f[j] = df_norm(fh[j], fl[j]);
-    return true;
+    if (oprim && onh > 0 && onh + 1 <= kTreeRun) {  // short runs, in slot order
+      const float* pp = part + 6 * tid;
+      float gxh = pp[0], gxl = pp[1], gyh = pp[2], gyl = pp[3], gzh = pp[4], gzl = pp[5];
+      for (int k = 1; k <= onh; ++k) {
+        const float* ph = pp + 6 * k;
+        df_acc(gxh, gxl, ph[0], ph[1]);
+        df_acc(gyh, gyl, ph[2], ph[3]);
+        df_acc(gzh, gzl, ph[4], ph[5]);
+      }
+      fx = df_norm(gxh, gxl);
+      fy = df_norm(gyh, gyl);
+      fz = df_norm(gzh, gzl);
+    }
+    if (oprim && onh == 0) {
+      const float* pp = part + 6 * tid;
+      fx = df_norm(pp[0], pp[1]);
+      fy = df_norm(pp[2], pp[3]);
+      fz = df_norm(pp[4], pp[5]);
+    }
   };
-  auto kick_all = [&](dfloat c) {
-#pragma unroll
-    for (int j = 0; j < NC; ++j) kick(v[j], f[j], c);
-  };
-  auto drift_all = [&]() {
-#pragma unroll
-    for (int j = 0; j < NC; ++j) coord_kick(x[j], v[j], dt);
+  // the grid barrier before every evaluation; the halo's mbarrier is armed
+  // with the next copies' bytes before any of them can be issued
+  auto barrier = [&]() {
+    if (tid == 0 && long_bytes) mbar_arrive_expect_tx(hbar, long_bytes);
+    return grid_sync(m.bar, ++barriers * nblocks, a.err);
   };
 
   // md_loop_start: forces at t0, v += F dt/2, x += v dt
   publish(0);
-  if (!evaluate(0)) return;
-  if (moves) {
-    kick_all(dt2);
-    drift_all();
+  if (!barrier()) return;
+  evaluate(0);
+  int cur = 0;
+  if (omoves) {
+    kick(vx, fx, dt2);
+    kick(vy, fy, dt2);
+    kick(vz, fz, dt2);
+    coord_kick(x, vx, dt);
+    coord_kick(y, vy, dt);
+    coord_kick(z, vz, dt);
   }
-  publish(1);
-  if (!evaluate(1)) return;
+  publish(cur ^ 1);
+  if (!barrier()) return;
+  cur ^= 1;
+  evaluate(cur);
   // md_loop: v += F dt, x += v dt, forces
   for (int k = 1; k < a.n; ++k) {
-    if (moves) {
-      kick_all(dt);
-      drift_all();
+    if (omoves) {
+      kick(vx, fx, dt);
+      kick(vy, fy, dt);
+      kick(vz, fz, dt);
+      coord_kick(x, vx, dt);
+      coord_kick(y, vy, dt);
+      coord_kick(z, vz, dt);
     }
-    publish(k + 1);
-    if (!evaluate(k + 1)) return;
+    publish(cur ^ 1);
+    if (!barrier()) return;
+    cur ^= 1;
+    evaluate(cur);
   }
-  __syncthreads();
-  if (*s_fail) return;  // the last evaluation's packets never came
   // md_loop_stop: v += F dt/2, then bin with the next shift
-  if (moves) kick_all(dt2);
-  {
-    double X[3], V[3];
-    const int g0 = (tid & 31) - lane;  // the slot's lane 0 within the warp
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      constexpr int kL = LANES;
-      const int j = k / kL;
-      X[k] = __shfl_sync(0xffffffffu, coord_to_double(x[j < NC ? j : 0]), g0 + k % kL);
-      V[k] = __shfl_sync(0xffffffffu, df_to_double(v[j < NC ? j : 0]), g0 + k % kL);
-    }
-    if (prim && lane == 0) {
-      m.x[0][slot] = X[0];
-      m.y[0][slot] = X[1];
-      m.z[0][slot] = X[2];
-      m.vx[slot] = V[0];
-      m.vy[slot] = V[1];
-      m.vz[slot] = V[2];
-      if (moves) {
-        if (a.deferred)
-          bin.defer(slot, X[0], X[1], X[2], V[0], V[1], V[2]);
-        else
-          bin(X[0], X[1], X[2], V[0], V[1], V[2]);
-      }
+  if (omoves) {
+    kick(vx, fx, dt2);
+    kick(vy, fy, dt2);
+    kick(vz, fz, dt2);
+  }
+  if (oprim) {
+    const double X = coord_to_double(x), Y = coord_to_double(y), Z = coord_to_double(z);
+    const double VX = df_to_double(vx), VY = df_to_double(vy), VZ = df_to_double(vz);
+    m.x[0][oslot] = X;
+    m.y[0][oslot] = Y;
+    m.z[0][oslot] = Z;
+    m.vx[oslot] = VX;
+    m.vy[oslot] = VY;
+    m.vz[oslot] = VZ;
+    if (omoves) {
+      if (a.deferred)
+        bin.defer(oslot, X, Y, Z, VX, VY, VZ);
+      else
+        bin(X, Y, Z, VX, VY, VZ);
     }
   }
   // refreshed bonds back to float64
@@ -494,8 +504,9 @@ __device__ void md_df_body(const MDState& m, const MDStepArgs& a, Bin bin) {
     }
   }
   // switch_logic for the cilia of this tile (the staged positions are the final ones)
-  const StageDF sv{own0 + 2 * (size_t)T * (a.n & 1)};
   for (int c = c0 + tid; c < c1; c += nthr) cilium_switch(m, a, c, a.t_end, base, sv);
+  __syncthreads();
+  if (tid == 0) mbar_inval(hbar);
 }
 
 template <int LANES, bool kFloat, typename Bin>
@@ -529,16 +540,16 @@ int md_df_lanes(int tile) {
 namespace {
 
 size_t md_df_smem(const MDState& m) {
-  return DfSmem(m.tile, m.hmax, m.df_nsp_max, m.df_nb_max).total;
+  return DfSmem(m.tile, m.hmax, m.df_nsp_max, m.df_nb_max, m.df_nrun_max, m.df_nsingle_max).total;
 }
 
 template <typename Bin>
 int launch_df(const MDState& m, const typename Bin::Cells& c, const MDStepArgs& a, cudaStream_t s, cudaError_t* st) {
   if (m.nslots == 0 || m.ntiles == 0) return 0;
+  cudaMemsetAsync(m.bar.count, 0, 2 * sizeof(unsigned), s);  // count and gen are adjacent
   MDState mm = m;
   typename Bin::Cells cc = c;
   MDStepArgs aa = a;
-  md_set_dt_pairs(aa);
   void* args[] = {&mm, &cc, &aa};
   const size_t smem = md_df_smem(m);
   const int lanes = md_df_lanes(m.tile);

@@ -75,8 +75,11 @@ __device__ __forceinline__ dfloat coord_diff(float dc, float ha, float hb, float
 struct DfDiff {
   dfloat dx, dy, dz, d2;
 };
-// the squared length of r's components, as a normalised pair
-__device__ __forceinline__ void df_square(DfDiff& r) {
+__device__ __forceinline__ DfDiff df_diff(const float4 a0, const float4 a1, const float4 b0, const float4 b1) {
+  DfDiff r;
+  r.dx = coord_diff((float)(cell_x(a1) - cell_x(b1)), a0.x, b0.x, a0.w, b0.w);
+  r.dy = coord_diff((float)(cell_y(a1) - cell_y(b1)), a0.y, b0.y, a1.x, b1.x);
+  r.dz = coord_diff(__fsub_rn(a1.w, b1.w), a0.z, b0.z, a1.y, b1.y);
   const dfloat px = df_two_prod(r.dx.h, r.dx.h), py = df_two_prod(r.dy.h, r.dy.h), pz = df_two_prod(r.dz.h, r.dz.h);
   const dfloat q1 = df_two_sum(px.h, py.h);
   const dfloat q2 = df_two_sum(q1.h, pz.h);
@@ -84,13 +87,6 @@ __device__ __forceinline__ void df_square(DfDiff& r) {
   low += 2.0f * (r.dx.h * r.dx.l + r.dy.h * r.dy.l + r.dz.h * r.dz.l);
   low += r.dx.l * r.dx.l + r.dy.l * r.dy.l + r.dz.l * r.dz.l;
   r.d2 = df_fast_two_sum(q2.h, low);
-}
-__device__ __forceinline__ DfDiff df_diff(const float4 a0, const float4 a1, const float4 b0, const float4 b1) {
-  DfDiff r;
-  r.dx = coord_diff((float)(cell_x(a1) - cell_x(b1)), a0.x, b0.x, a0.w, b0.w);
-  r.dy = coord_diff((float)(cell_y(a1) - cell_y(b1)), a0.y, b0.y, a1.x, b1.x);
-  r.dz = coord_diff(__fsub_rn(a1.w, b1.w), a0.z, b0.z, a1.y, b1.y);
-  df_square(r);
   return r;
 }
 

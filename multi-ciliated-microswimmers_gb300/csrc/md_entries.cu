@@ -11,27 +11,31 @@
 // behind the other, although every CTA has threads to spare.  Here a spring
 // and its exact reverse inside the tile form one entry (the reference makes
 // cilium and sphere springs from both ends; the two forces are negations of
-// each other bit for bit), the threads take one entry each, and a bead's lanes
-// then add the forces of its entries.  The planner cuts the beads into many
+// each other bit for bit), the threads take one entry each, and every bead's
+// forces are then added in the order in which md_df.cu's lanes and slots add
+// them: the two kernels give the same results bit for bit (a sum in another
+// order grows, in stiff springs, to 1e-9 of a small swimmer's velocities within
+// five steps).  The planner cuts the beads into many
 // small tiles, up to the number of SMs: cilia as they are, the other beads in
 // compact patches, and a bead with a very long list (a sphere's centre) in a
-// tile of its own, whose threads keep running sums.
+// tile of its own.
 //
 // The chain of one substep: packets arrive -> one entry -> a bead's sum ->
 // Verlet -> packets leave.  The entries between the tile's own beads are
 // evaluated by the first warps while the last warps poll.  The launch is
-// latency bound (51 dependent evaluations of about 2.2 us; issue slots, pipes
+// latency bound (51 dependent evaluations of about 2.7 us; issue slots, pipes
 // and DRAM mostly idle): a packet takes 250-600 ns from one SM to another,
-// an entry about 0.4 us, a bead's sum and Verlet step 0.3 us, and the round of
+// an entry about 0.4 us, a bead's sum and Verlet step 0.4 us, and the round of
 // the sphere centre's tile (its 642 beads' packets, written elsewhere since the
-// last read, take about 0.9 us to fetch) alternates with the patches' rounds.
+// last read, take about 0.9 us to fetch, its sum's last tree 0.12) alternates
+// with the patches' rounds.
 //
-// MD per launch timed alone, this kernel / md_df.cu with packets / with a grid
-// barrier: swimmer64 123 / 168 / 217 us in double-float, 115 / 148 / 203 with
-// float springs; a 700-bead swimmer 120 / 158 / 192; swimmer128 with float
-// springs 211 / 432 / 430 (there a tile of 256 slots has two lanes per slot, and
-// its springs follow one another; here 152 tiles of three cilia or 151 sphere
-// beads).
+// MD per launch timed alone, this kernel / md_df.cu: swimmer64 146 / 217 us in
+// double-float, 134 / 196 with float springs; a 700-bead swimmer 135 / 187;
+// swimmer128 with float springs 227 / 431 (there a tile of 256 slots has two
+// lanes per slot, and its springs follow one another; here 152 tiles of three
+// cilia or 151 sphere beads).  Running sums of the entries in any order took
+// 122, 114, 117 and 213 us.
 #include <algorithm>
 
 #include "../../include/mpcd_gpu.h"
@@ -44,59 +48,8 @@ namespace mpcd {
 
 namespace {
 
-// A bead coordinate is c / 2 + (h - 1/2) + l: an integer count of half cells,
-// h in [1/2, 1) and the low part l, |l| <= 2^-25.  All floats of [1/2, 1) lie
-// on the grid of multiples of 2^-24, so that adding a small displacement to h
-// rounds onto the grid by itself (md_df_coord.cuh's coordinate of offsets in
-// [0, 1) has the same resolution but needs a rounding and a floor at every
-// substep), and the difference of two h is exact.
-struct HalfCoord {
-  int c;
-  float h, l;
-};
-__device__ __forceinline__ HalfCoord half_from_double(double x) {
-  const double c = floor(2.0 * x);
-  const double o = x - 0.5 * c;                                // exact, [0, 1/2)
-  const double g = rint(o * 16777216.0) * (1.0 / 16777216.0);  // exact, on the grid
-  const bool up = g >= 0.5;                                    // rounded up to the next half cell
-  return {(int)c + (up ? 1 : 0), (float)(up ? g : g + 0.5), (float)(o - g)};
-}
-__device__ __forceinline__ double half_to_double(const HalfCoord& q) {
-  return 0.5 * (double)(q.c - 1) + ((double)q.h + (double)q.l);
-}
-// The product f c as a float and the rest of it (f, c pairs; f.l may exceed
-// half an ulp of f.h).
-__device__ __forceinline__ dfloat pair_times(dfloat f, dfloat c) {
-  const float p = __fmul_rn(f.h, c.h);
-  return {p, fmaf(f.l, c.h, fmaf(f.h, c.l, fmaf(f.h, c.h, -p)))};
-}
-// v += f c
-__device__ __forceinline__ void pair_kick(dfloat& v, dfloat f, dfloat c) {
-  const dfloat g = pair_times(f, c);
-  const dfloat s = df_two_sum(v.h, g.h);
-  v = df_fast_two_sum(s.h, __fadd_rn(v.l, __fadd_rn(s.l, g.l)));
-}
-// x += v c
-__device__ __forceinline__ void half_drift(HalfCoord& x, dfloat v, dfloat c) {
-  const dfloat g = pair_times(v, c);
-  const dfloat s = df_two_sum(x.h, g.h);
-  dfloat r = df_fast_two_sum(s.h, __fadd_rn(x.l, __fadd_rn(s.l, g.l)));
-  if (!(r.h >= 0.5f && r.h < 1.0f)) {  // into another half cell
-    const float k = floorf(2.0f * r.h) - 1.0f;
-    const dfloat t = df_two_sum(r.h, -0.5f * k);
-    r = df_fast_two_sum(t.h, __fadd_rn(t.l, r.l));
-    x.c += (int)k;
-    if (r.h >= 1.0f) {  // rounded up to the edge
-      r.h -= 0.5f;
-      x.c += 1;
-    }
-  }
-  x.h = r.h;
-  x.l = r.l;
-}
-
-// A staged position: {h of x, y, z, half cells of x as a cell coordinate},
-// {l of x, y, z, the same of y}, the same of z (exact as floats below 2^22).
+// A staged position: {h of x, y, z, the cell of x}, {l of x, y, z, the cell of
+// y}, the cell of z (exact as floats below 2^24).
 struct Staged {
   float4* a;
   float4* b;
@@ -104,7 +57,7 @@ struct Staged {
   __device__ void put(int i, int k, float h, float l, int cell) const {
     reinterpret_cast<float*>(a + i)[k] = h;
     reinterpret_cast<float*>(b + i)[k] = l;
-    const float f = 0.5f * (float)cell;
+    const float f = (float)cell;
     if (k == 0)
       reinterpret_cast<float*>(a + i)[3] = f;
     else if (k == 1)
@@ -122,6 +75,12 @@ struct Staged {
   }
 };
 
+// a b + c d + e f with the roundings that the compiler gives df_diff's sums (it
+// may fuse either product of the first two): both kernels' springs are the same
+// bit for bit
+__device__ __forceinline__ float dot3(float a, float b, float c, float d, float e, float f) {
+  return fmaf(e, f, fmaf(c, d, __fmul_rn(a, b)));
+}
 // x_i - x_j of two staged positions as pairs, and its squared length as a
 // normalised pair (as df_diff)
 __device__ __forceinline__ DfDiff staged_diff(const float4 a0, const float4 a1, float az, const float4 b0,
@@ -130,13 +89,33 @@ __device__ __forceinline__ DfDiff staged_diff(const float4 a0, const float4 a1, 
   r.dx = coord_diff(__fsub_rn(a0.w, b0.w), a0.x, b0.x, a1.x, b1.x);
   r.dy = coord_diff(__fsub_rn(a1.w, b1.w), a0.y, b0.y, a1.y, b1.y);
   r.dz = coord_diff(__fsub_rn(az, bz), a0.z, b0.z, a1.z, b1.z);
-  df_square(r);
+  const dfloat px = df_two_prod(r.dx.h, r.dx.h), py = df_two_prod(r.dy.h, r.dy.h), pz = df_two_prod(r.dz.h, r.dz.h);
+  const dfloat q1 = df_two_sum(px.h, py.h);
+  const dfloat q2 = df_two_sum(q1.h, pz.h);
+  float low = __fadd_rn(__fadd_rn(q1.l, q2.l), __fadd_rn(__fadd_rn(px.l, py.l), pz.l));
+  low = fmaf(2.0f, dot3(r.dx.h, r.dx.l, r.dy.h, r.dy.l, r.dz.h, r.dz.l), low);
+  low = __fadd_rn(low, dot3(r.dx.l, r.dx.l, r.dy.l, r.dy.l, r.dz.l, r.dz.l));
+  r.d2 = df_fast_two_sum(q2.h, low);
   return r;
 }
 
+// The three components of a force: pairs (high part, unnormalised low part)
+// or, with float springs, the factors {fac, d} of a product that the sum rounds
+// once (fused multiply-add).
 struct Force {
-  float2 x, y, z;  // pairs (high part, unnormalised low part)
+  float2 x, y, z;
 };
+template <bool kFloat>
+__device__ __forceinline__ float2 opposite(float2 p) {
+  return kFloat ? make_float2(p.x, -p.y) : make_float2(-p.x, -p.y);
+}
+template <bool kFloat>
+__device__ __forceinline__ void force_acc(float& h, float& l, float2 p) {
+  if constexpr (kFloat)
+    h = fmaf(p.x, p.y, h);
+  else
+    df_acc(h, l, p.x, p.y);
+}
 // F = -2k (1 - b / |d|) d on the first bead, d its position less the other's,
 // rk = {b, -2k} as pairs; guarded: no force at zero distance (the vector-form
 // spring).  kFloat: d formed exactly as pairs and rounded to float, the rest in
@@ -150,18 +129,18 @@ __device__ __forceinline__ Force spring_force(const float4 a0, const float4 a1, 
     const dfloat ey = coord_diff(__fsub_rn(a1.w, b1.w), a0.y, b0.y, a1.y, b1.y);
     const dfloat ez = coord_diff(__fsub_rn(az, bz), a0.z, b0.z, a1.z, b1.z);
     const float dx = ex.h + ex.l, dy = ey.h + ey.l, dz = ez.h + ez.l;
-    const float d2 = dx * dx + dy * dy + dz * dz;
+    const float d2 = dot3(dx, dx, dy, dy, dz, dz);
     float fac = rk.z * (1.0f - rk.x * rsqrtf(d2));
     if (guarded && d2 == 0.0f) fac = 0.0f;
-    F.x = make_float2(fac * dx, 0.f);
-    F.y = make_float2(fac * dy, 0.f);
-    F.z = make_float2(fac * dz, 0.f);
+    F.x = make_float2(fac, dx);
+    F.y = make_float2(fac, dy);
+    F.z = make_float2(fac, dz);
   } else {
     const DfDiff d = staged_diff(a0, a1, az, b0, b1, bz);
     const dfloat r = df_rsqrt(d.d2);
-    // w = 1 - b r (the sum exact for b r < 2, else to about 2^-48 b r)
+    // w = 1 - b r
     const dfloat u = df_two_prod(rk.x, r.h);
-    const dfloat w = df_fast_two_sum(1.0f, -u.h);
+    const dfloat w = df_two_sum(1.0f, -u.h);
     const float wl = ((w.l - u.l) - rk.x * r.l) - rk.y * r.h;
     // fac = -2k w
     dfloat f = df_two_prod(rk.z, w.h);
@@ -180,11 +159,85 @@ template <bool kFloat>
 __device__ __forceinline__ Force packet_force(const float4 a0, const float4 a1, float az, const Packet* d,
                                               const float4 rk, bool guarded) {
   const float4 b0 = make_float4(__uint_as_float(d[0].h), __uint_as_float(d[1].h), __uint_as_float(d[2].h),
-                                0.5f * (float)(int)d[0].c);
+                                (float)(int)d[0].c);
   const float4 b1 = make_float4(__uint_as_float(d[0].l), __uint_as_float(d[1].l), __uint_as_float(d[2].l),
-                                0.5f * (float)(int)d[1].c);
-  return spring_force<kFloat>(a0, a1, az, b0, b1, 0.5f * (float)(int)d[2].c, rk, guarded);
+                                (float)(int)d[1].c);
+  return spring_force<kFloat>(a0, a1, az, b0, b1, (float)(int)d[2].c, rk, guarded);
 }
+
+// A slot's sum as md_df.cu's lanes make it: LN running sums over the rows of
+// the slot's words (a row: one word per lane, `step` apart), combined by the
+// lanes' tree as its lane 0 sees it.  A lane without a spring in a row holds zero,
+// which changes nothing.
+template <int LN, bool kFloat>
+__device__ __forceinline__ void lane_sums(const float2* F, int step, int row, int rows, float& h, float& l) {
+  float sh[LN], sl[LN];
+#pragma unroll
+  for (int q = 0; q < LN; ++q) {
+    const float2 p = F[q * step];
+    sh[q] = kFloat ? __fmul_rn(p.x, p.y) : p.x;
+    sl[q] = kFloat ? 0.f : p.y;
+  }
+  constexpr int kAhead = LN >= 4 ? 1 : 4;  // rows whose loads go out together; past the last one zero
+#pragma unroll 1
+  for (int r = 1; r < rows; r += kAhead) {
+    float2 p[kAhead][LN];
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) {
+      F += row;
+#pragma unroll
+      for (int q = 0; q < LN; ++q) p[u][q] = r + u < rows ? F[q * step] : make_float2(0.f, 0.f);
+    }
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u)
+#pragma unroll
+      for (int q = 0; q < LN; ++q) force_acc<kFloat>(sh[q], sl[q], p[u][q]);
+  }
+#pragma unroll
+  for (int o = 1; o < LN; o <<= 1)
+#pragma unroll
+    for (int q = 0; q + o < LN; q += 2 * o) df_acc(sh[q], sl[q], sh[q + o], sl[q + o]);
+  h = sh[0];
+  l = sl[0];
+}
+template <int HALVES, bool kFloat>
+__device__ __forceinline__ void slot_sum(int lanes, const float2* F, int step, int rows, float& h, float& l) {
+  if (lanes == 8)
+    lane_sums<8 / HALVES, kFloat>(F, step, lanes * step, rows, h, l);
+  else if (lanes == 4)
+    lane_sums<4 / HALVES, kFloat>(F, step, lanes * step, rows, h, l);
+  else
+    lane_sums<2 / HALVES, kFloat>(F, step, lanes * step, rows, h, l);
+}
+// The sums of three components over a warp by md_df.cu's xor tree (16 first, every lane
+// adding its partner's value to its own) as lane `src` ends with them.  Only the
+// lanes on src's side of a level count for the next one: the others take a
+// component over, added from src's side.  x ends in lane src, y in src ^ 8, z in
+// src ^ 16.
+__device__ __forceinline__ void shfl_acc(float& h, float& l, float gh, float gl, bool first, int o) {
+  const float bh = __shfl_xor_sync(0xffffffffu, gh, o), bl = __shfl_xor_sync(0xffffffffu, gl, o);
+  float al = first ? l : bl;
+  df_acc(h, al, bh, first ? bl : l);  // the high parts' sum and its error do not depend on the order
+  l = al;
+}
+__device__ __forceinline__ void warp_tree(const float (&s)[6], int lane, int src, float& h, float& l) {
+  const bool a = ((lane ^ src) & 16) == 0, b = ((lane ^ src) & 8) == 0;
+  // src's half adds x and y, the other z
+  float xh = a ? s[0] : s[4], xl = a ? s[1] : s[5], yh = s[2], yl = s[3];
+  shfl_acc(xh, xl, a ? s[4] : s[0], a ? s[5] : s[1], a, 16);
+  shfl_acc(yh, yl, s[2], s[3], true, 16);
+  // src's quarter goes on with x, its neighbour with y
+  const bool y = a && !b;
+  h = y ? yh : xh;
+  l = y ? yl : xl;
+  shfl_acc(h, l, !a ? xh : (y ? xh : yh), !a ? xl : (y ? xl : yl), !y, 8);
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) shfl_acc(h, l, h, l, true, o);
+}
+
+// md_df.cu adds the slots of a bead with more than this many by a warp's tree,
+// fewer in order
+constexpr int kTreeRun = 8;
 
 // Makes x opaque to the compiler from here on: what a substep uses stays in
 // its register instead of being computed again (integer divisions, float64
@@ -237,7 +290,7 @@ __device__ void md_entries_body(const MDState& m, const MDStepArgs& a, Bin bin) 
   int* s_hslot = reinterpret_cast<int*>(smem + L.hslot);
   int* s_fail = reinterpret_cast<int*>(smem + L.flag);  // 1: a packet never came
   // entries: {bead a | guarded << 15 | bead b << 16, incidence of a | of b << 16 (0xffff: none)},
-  // {rest length, -2k} as pairs, {kind | bond << 2}
+  // {rest length, -2k} as pairs, {kind | bond << 2} (a solo tile: the rows of its i-th slot)
   uint2* s_code = reinterpret_cast<uint2*>(smem + L.code);
   float4* s_rk = reinterpret_cast<float4*>(smem + L.rk);
   uint32_t* s_meta = reinterpret_cast<uint32_t*>(smem + L.meta);
@@ -253,8 +306,9 @@ __device__ void md_entries_body(const MDState& m, const MDStepArgs& a, Bin bin) 
   const int tile = blockIdx.x;
   const int base = tile * T;
   const int tid = threadIdx.x, nthr = blockDim.x, back = nthr - 1 - tid;
-  const int lane32 = tid & 31, warp = tid >> 5, nwarps = nthr >> 5;
+  const int lane32 = tid & 31, warp = tid >> 5;
   const bool solo = m.de_solo[tile] != 0;
+  const int lanes = m.de_lanes;
   // owned coordinates: number c = tid / HALVES + j nthr below 3 T is coordinate
   // c / T of bead c mod T, so that few warps run the sums and the Verlet step
   // (a warp's instructions count once, however many lanes take part); with
@@ -272,25 +326,28 @@ __device__ void md_entries_body(const MDState& m, const MDStepArgs& a, Bin bin) 
   const int c0 = m.tile_cil[tile], c1 = m.tile_cil[tile + 1];
   const int b0 = m.tile_b0[tile], nb = m.tile_nb[tile];
   const int e0 = m.de_start[tile], nent0 = m.de_start[tile + 1] - e0, nloc0 = m.de_local_end[tile] - e0;
-  const int i0 = m.sp_start[base];
-  // a bead's incidences: fn words from f0 on, fstep apart; in a solo tile the
-  // warps' partial sums take their place
-  const int ninc = solo ? nwarps : m.de_nslot[tile];
-  const int fstep = solo ? 1 : m.de_step;
-  int f0[NC], fn[NC];
+  // a bead's force words: from f0 on, fstep apart, a nibble of fshape per slot:
+  // its rows of one word per lane
+  const int ninc = m.de_nslot[tile];
+  const int fstep = m.de_step;
+  int f0[NC];
+  uint32_t fshape[NC];
 #pragma unroll
   for (int j = 0; j < NC; ++j) {
     const int s = base + cq[j];
-    const bool has = cmv[j] >= 0;
-    f0[j] = has && !solo ? (fstep == 1 ? m.sp_start[s] - i0 : cq[j]) : 0;
-    fn[j] = has ? (solo ? nwarps : m.sp_start[s + 1] - m.sp_start[s]) : 0;
+    f0[j] = cmv[j] >= 0 && !solo ? m.de_at[s] : 0;
+    fshape[j] = cmv[j] == 1 && !solo ? m.de_shape[s] : 0u;  // a fixed bead needs no force
   }
+  const int wmax = m.de_slots[tile];  // most slots of one of its beads
+  // a solo tile's words: as many rows for every slot, then the slots' sums
+  const int solo_src = solo ? m.de_at[base] : 0, solo_slots0 = solo ? (int)m.de_shape[base] : 0;
   const dfloat dt{a.dt_pair.x, a.dt_pair.y}, dt2{a.dt2_pair.x, a.dt2_pair.y};
 
   // the plan must fit the tables and the halo's slots the packet buffers
   if (tid == 0)
     *s_fail = hn0 < 0 || hn0 > m.hmax || nent0 < 0 || nent0 > m.de_nent_max || nloc0 < 0 || nloc0 > nent0 || ninc < 0 ||
-              ninc > m.de_ninc_max || nb > m.df_nb_max;
+              ninc > m.de_ninc_max || nb > m.df_nb_max ||
+              (solo && (solo_slots0 < 1 || solo_slots0 > nent0 || wmax < 0 || solo_slots0 * (wmax * lanes + 1) > ninc));
   __syncthreads();
   const bool fits = *s_fail == 0;
   __syncthreads();
@@ -303,11 +360,11 @@ __device__ void md_entries_body(const MDState& m, const MDStepArgs& a, Bin bin) 
     const uint4 c = __ldg(m.de_code + e0 + i);
     const int ea = (int)(c.x & 0x7fffu), eb = (int)(c.x >> 16), ka = (int)(c.y & 0xffffu), kb = (int)(c.y >> 16);
     const int kind = (int)(c.z & 3u), lref = (int)(c.z >> 2);
-    if (ea >= T || eb >= T + hn0 || (eb >= T) != (i >= nloc0) || (!solo && ka >= ninc) || (kb != 0xffff && kb >= ninc) ||
-        (kind >= MPCD_SPRING_BOND && lref >= nb))
+    if (ea >= T || eb >= T + hn0 || (eb >= T) != (i >= nloc0) || ka >= ninc || (kb != 0xffff && kb >= ninc) ||
+        (kind >= MPCD_SPRING_BOND && lref >= nb) || (solo && (int)c.w > wmax))
       *s_fail = 1;
     s_code[i] = make_uint2(c.x, c.y);
-    s_meta[i] = c.z;
+    s_meta[i] = solo ? c.w : c.z;
     float4 rk = __ldg(m.de_rk + e0 + i);
     if (kind >= MPCD_SPRING_BOND && lref < nb) {
       const dfloat r = df_from_double((kind == MPCD_SPRING_BOND ? m.newlen : m.diag)[b0 + lref]);
@@ -315,6 +372,13 @@ __device__ void md_entries_body(const MDState& m, const MDStepArgs& a, Bin bin) 
       rk.y = r.l;
     }
     s_rk[i] = rk;
+  }
+  for (int i = tid; i < 3 * fw && fits; i += nthr) s_fx[i] = make_float2(0.f, 0.f);  // words without a spring stay zero
+#pragma unroll
+  for (int j = 0; j < NC && fits; ++j) {  // every owned bead's words lie in the table
+    int words = 0;
+    for (uint32_t t = fshape[j]; t; t >>= 4) words += (int)(t & 15u) * lanes;
+    if (f0[j] < 0 || (words > 0 && f0[j] + (words - 1) * fstep >= ninc)) *s_fail = 1;
   }
   __syncthreads();
   const bool plan_ok = *s_fail == 0;  // an inconsistent plan: no halo, no entries (and an error)
@@ -324,7 +388,7 @@ __device__ void md_entries_body(const MDState& m, const MDStepArgs& a, Bin bin) 
     *s_fail = 0;
   }
   const int hn = plan_ok ? hn0 : 0, nent = plan_ok ? nent0 : 0, nloc = plan_ok ? nloc0 : 0;
-  const int nbt = plan_ok ? nb : 0;
+  const int nbt = plan_ok ? nb : 0, solo_slots = plan_ok ? solo_slots0 : 0;
   for (int i = tid; i < nbt; i += nthr) {
     const dfloat n = df_from_double(m.newlen[b0 + i]), o = df_from_double(m.oldlen[b0 + i]);
     const dfloat g = df_from_double(m.diag[b0 + i]);
@@ -354,7 +418,7 @@ __device__ void md_entries_body(const MDState& m, const MDStepArgs& a, Bin bin) 
     s_bd[k] = make_float2(bd.h, bd.l);
   });
   // the owned coordinates
-  HalfCoord x[NC];
+  BeadCoord x[NC];
   dfloat v[NC];
   double ke_coll = 0.0;
 #pragma unroll
@@ -372,9 +436,9 @@ __device__ void md_entries_body(const MDState& m, const MDStepArgs& a, Bin bin) 
         const double ke = bin.collide(X[0], X[1], X[2], V[0], V[1], V[2]);
         if (ck[j] == 0 && half == 0) ke_coll += ke;
       }
-      if (!plan_ok) fn[j] = 0;
+      if (!plan_ok) fshape[j] = 0u;
     }
-    x[j] = half_from_double(ck[j] == 0 ? X[0] : (ck[j] == 1 ? X[1] : X[2]));
+    x[j] = coord_from_double(ck[j] == 0 ? X[0] : (ck[j] == 1 ? X[1] : X[2]));
     v[j] = df_from_double(ck[j] == 0 ? V[0] : (ck[j] == 1 ? V[1] : V[2]));
   }
   if (a.collide) {  // the dissipated-energy bookkeeping of the collided beads
@@ -384,15 +448,23 @@ __device__ void md_entries_body(const MDState& m, const MDStepArgs& a, Bin bin) 
   int my_k = (back >= hn) + (back >= 2 * hn), my_p = back - my_k * hn;  // this thread's halo packet
   int my_src = back < 3 * hn ? my_k * m.nslots + s_hslot[my_p] : 0;
   int si = tid - 32, si2 = si + nthr - 32 < nent ? si + nthr - 32 : si;  // a solo tile's first two entries
+  // the place of number p of a solo tile's sums: slot (-1: none), first word
+  // (word j of slot k at j solo_slots + k), and where the sum goes
+  auto solo_place = [&](int p, int& k, int& at, int& to) {
+    const int ax = (p >> 1) / max(1, solo_slots);
+    k = ax < 3 && solo ? (p >> 1) - ax * solo_slots : -1;
+    at = ax * fw + (p & 1) * (lanes / 2) * solo_slots + k;
+    to = ax * fw + lanes * wmax * solo_slots + k;
+  };
+  int sk, sat, sout;
+  solo_place(tid, sk, sat, sout);
   int pub[NC], fat[NC];  // packet of each owned coordinate (-1: not this thread's), and its first incidence
 #pragma unroll
   for (int j = 0; j < NC; ++j) {
     pub[j] = cmv[j] < 0 || half ? -1 : ck[j] * m.nslots + base + cq[j];
-    fat[j] = ck[j] * fw + f0[j] + half * fstep;
-    fn[j] -= half;
+    fat[j] = ck[j] * fw + f0[j] + half * (lanes / HALVES) * fstep;
     keep(pub[j]);
     keep(fat[j]);
-    keep(fn[j]);
     keep(cq[j]);
     keep(ck[j]);
     keep(cmv[j]);
@@ -402,6 +474,12 @@ __device__ void md_entries_body(const MDState& m, const MDStepArgs& a, Bin bin) 
   keep(my_src);
   keep(si);
   keep(si2);
+  keep(sk);
+  keep(sat);
+  keep(sout);
+  int wslots[NC];  // most slots of a bead of this warp
+#pragma unroll
+  for (int j = 0; j < NC; ++j) wslots[j] = (int)__reduce_max_sync(0xffffffffu, (35u - __clz((int)fshape[j])) >> 2);
   bool refreshed = false;
 
   // md_loop_start, n x md_loop, md_loop_stop: evaluation e of the forces at
@@ -413,21 +491,26 @@ __device__ void md_entries_body(const MDState& m, const MDStepArgs& a, Bin bin) 
     for (int j = 0; j < NC; ++j)
       if (pub[j] >= 0) {
         packet_store(m.qp[e & 1] + pub[j],
-                     Packet{__float_as_uint(x[j].h), __float_as_uint(x[j].l), (uint32_t)x[j].c, a.tag0 + (uint32_t)e});
-        own.put(cq[j], ck[j], x[j].h, x[j].l, x[j].c);
+                     Packet{__float_as_uint(x[j].o.h), __float_as_uint(x[j].o.l), (uint32_t)x[j].c, a.tag0 + (uint32_t)e});
+        own.put(cq[j], ck[j], x[j].o.h, x[j].o.l, x[j].c);
       }
     // a solo tile's other warps ask for the next positions of their entries'
     // beads while the first one sums and moves the tile's bead
     Packet d[6];
-    uint32_t sc1 = 0, sc2 = 0;
+    uint2 sc1 = make_uint2(0, 0), sc2 = sc1;
     if (solo && tid >= 32 && si < nent) {
-      sc1 = s_code[si].x;
-      sc2 = s_code[si2].x;
-      receive_two(m.qp[e & 1], m.nslots, a.tag0 + (uint32_t)e, s_hslot[(int)(sc1 >> 16) - T],
-                  s_hslot[(int)(sc2 >> 16) - T], d, a.err, s_fail);
+      sc1 = s_code[si];
+      sc2 = s_code[si2];
+      receive_two(m.qp[e & 1], m.nslots, a.tag0 + (uint32_t)e, s_hslot[(int)(sc1.x >> 16) - T],
+                  s_hslot[(int)(sc2.x >> 16) - T], d, a.err, s_fail);
     }
-    __syncthreads();  // the tile's own positions are staged, the last evaluation's forces read
-    if ((e & 7) == 7 && *s_fail) return;
+    // the tile's own positions are staged, the last evaluation's forces read;
+    // now and then the CTA looks, as one, whether a packet never came
+    if ((e & 7) == 7) {
+      if (__syncthreads_or(*(volatile int*)s_fail)) return;
+    } else {
+      __syncthreads();
+    }
     const bool due = c1 > c0 && refresh_due(a, e);
     if (due) {
       // Cilia::length (src/cilia.cpp:79-121) for every refreshed bond, in pairs
@@ -452,36 +535,42 @@ __device__ void md_entries_body(const MDState& m, const MDStepArgs& a, Bin bin) 
     }
     if (solo) {
       // one bead with a long list: a thread takes its entries' other beads
-      // straight from their packets, two at a time, and keeps running sums
+      // straight from their packets, two at a time; the lanes of the bead's slots
+      // then add their words
       const float4 ca = own.a[0], cb = own.b[0];
       const float cc = own.c[0];
-      float sum[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
       if (tid >= 32) {
+        auto put = [&](uint32_t k, const Force& g) {
+          s_fx[k] = g.x;
+          s_fx[k + fw] = g.y;
+          s_fx[k + 2 * fw] = g.z;
+        };
 #pragma unroll 1
         for (int i = si, i2 = si2; i < nent;) {
-          const Force g1 = packet_force<kFloat>(ca, cb, cc, d, s_rk[i], (sc1 & 0x8000u) != 0);
-          const Force g2 = packet_force<kFloat>(ca, cb, cc, d + 3, s_rk[i2], (sc2 & 0x8000u) != 0);
-          df_acc(sum[0], sum[1], g1.x.x, g1.x.y);
-          df_acc(sum[2], sum[3], g1.y.x, g1.y.y);
-          df_acc(sum[4], sum[5], g1.z.x, g1.z.y);
-          if (i2 != i) {
-            df_acc(sum[0], sum[1], g2.x.x, g2.x.y);
-            df_acc(sum[2], sum[3], g2.y.x, g2.y.y);
-            df_acc(sum[4], sum[5], g2.z.x, g2.z.y);
-          }
+          put(sc1.y & 0xffffu, packet_force<kFloat>(ca, cb, cc, d, s_rk[i], (sc1.x & 0x8000u) != 0));
+          if (i2 != i) put(sc2.y & 0xffffu, packet_force<kFloat>(ca, cb, cc, d + 3, s_rk[i2], (sc2.x & 0x8000u) != 0));
           i += 2 * (nthr - 32);
           if (i >= nent) break;
           i2 = i + nthr - 32 < nent ? i + nthr - 32 : i;
-          sc1 = s_code[i].x;
-          sc2 = s_code[i2].x;
-          receive_two(m.qp[e & 1], m.nslots, a.tag0 + (uint32_t)e, s_hslot[(int)(sc1 >> 16) - T],
-                      s_hslot[(int)(sc2 >> 16) - T], d, a.err, s_fail);
+          sc1 = s_code[i];
+          sc2 = s_code[i2];
+          receive_two(m.qp[e & 1], m.nslots, a.tag0 + (uint32_t)e, s_hslot[(int)(sc1.x >> 16) - T],
+                      s_hslot[(int)(sc2.x >> 16) - T], d, a.err, s_fail);
         }
       }
-      // the warps' sums, in a fixed order
-      float h, l;
-      group_sum_xyz<32>(lane32, sum[0], sum[1], sum[2], sum[3], sum[4], sum[5], h, l);
-      if ((lane32 & 7) == 0 && lane32 < 24) s_fx[(lane32 >> 3) * fw + warp] = make_float2(h, l);
+      __syncthreads();
+      // a thread per slot, half of its lanes and coordinate (sk, its words at
+      // sat, its sum to sout): the first round's place is kept
+#pragma unroll 1
+      for (int p = tid, k = sk, at = sat, to = sout; p - lane32 < 6 * solo_slots;) {  // whole warps
+        float h = 0.f, l = 0.f;
+        if (k >= 0) slot_sum<2, kFloat>(lanes, s_fx + at, solo_slots, (int)s_meta[k], h, l);
+        const float oh = __shfl_xor_sync(0xffffffffu, h, 1), ol = __shfl_xor_sync(0xffffffffu, l, 1);
+        df_acc(h, l, oh, ol);
+        if (k >= 0 && !(tid & 1)) s_fx[to] = make_float2(h, l);
+        p += nthr;
+        if (p - lane32 < 6 * solo_slots) solo_place(p, k, at, to);
+      }
     } else {
       // phase 0: the entries between own beads, from the first thread up;
       // phase 1: the halo arrives and its entries, from the last thread down
@@ -535,39 +624,71 @@ __device__ void md_entries_body(const MDState& m, const MDStepArgs& a, Bin bin) 
           s_fx[ka + fw] = g.y;
           s_fx[ka + 2 * fw] = g.z;
           if (kb != 0xffff) {
-            s_fx[kb] = make_float2(-g.x.x, -g.x.y);
-            s_fx[kb + fw] = make_float2(-g.y.x, -g.y.y);
-            s_fx[kb + 2 * fw] = make_float2(-g.z.x, -g.z.y);
+            s_fx[kb] = opposite<kFloat>(g.x);
+            s_fx[kb + fw] = opposite<kFloat>(g.y);
+            s_fx[kb + 2 * fw] = opposite<kFloat>(g.z);
           }
         }
       }
     }
     __syncthreads();
-    // every owned coordinate of the force: the bead's incidences in its spring
-    // order, dealt to two running sums per thread (a fixed order), then the
-    // Verlet step
+    // every owned coordinate of the force, summed as md_df.cu's lanes, helper
+    // slots and warps sum it, then the Verlet step
     const bool last = e == a.n;
     const dfloat c = e == 0 || last ? dt2 : dt;
+    float ssum[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    if (solo && warp == 0) {
+      const bool tree = solo_slots > kTreeRun;
+      const int k0 = tree ? lane32 : 0, kstep = tree ? 32 : 1;
+      for (int k = k0; k < solo_slots; k += kstep) {
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+          const float2 p = s_fx[q * fw + solo_slots * lanes * wmax + k];
+          df_acc(ssum[2 * q], ssum[2 * q + 1], p.x, p.y);
+        }
+      }
+      __syncwarp();
+      if (tree) {
+        float h, l;
+        warp_tree(ssum, lane32, solo_src, h, l);
+        // the owner of a coordinate fetches it
+        const int from = ck[0] < 3 ? solo_src ^ (8 * ck[0]) : lane32;  // x, y, z: src, src ^ 8, src ^ 16
+        ssum[0] = ssum[2] = ssum[4] = __shfl_sync(0xffffffffu, h, from);
+        ssum[1] = ssum[3] = ssum[5] = __shfl_sync(0xffffffffu, l, from);
+      }
+    }
 #pragma unroll
     for (int j = 0; j < NC; ++j) {
-      float sh = 0.f, sl = 0.f, th = 0.f, tl = 0.f;
-      const float2* F = s_fx + fat[j];
-      int n = fn[j];
+      float th = 0.f, tl = 0.f;
+      if (solo) {
+        th = ck[j] == 0 ? ssum[0] : (ck[j] == 1 ? ssum[2] : ssum[4]);
+        tl = ck[j] == 0 ? ssum[1] : (ck[j] == 1 ? ssum[3] : ssum[5]);
+      } else {
+        const float2* F = s_fx + fat[j];
+        uint32_t shape = fshape[j];
 #pragma unroll 1
-      for (; n > HALVES; n -= 2 * HALVES, F += 2 * HALVES * fstep) {
-        const float2 p = F[0], r = F[HALVES * fstep];
-        df_acc(sh, sl, p.x, p.y);
-        df_acc(th, tl, r.x, r.y);
-      }
-      if (n > 0) df_acc(sh, sl, F[0].x, F[0].y);
-      df_acc(sh, sl, th, tl);
-      if constexpr (HALVES == 2) {
-        const float oh = __shfl_xor_sync(0xffffffffu, sh, 1), ol = __shfl_xor_sync(0xffffffffu, sl, 1);
-        df_acc(sh, sl, oh, ol);
+        for (int k = 0; k < wslots[j]; ++k, shape >>= 4) {  // slot after slot
+          const int rows = (int)(shape & 15u);
+          float h = 0.f, l = 0.f;
+          if (rows > 0) {
+            slot_sum<HALVES, kFloat>(lanes, F, fstep, rows, h, l);
+            F += rows * lanes * fstep;
+          }
+          if constexpr (HALVES == 2) {
+            const float oh = __shfl_xor_sync(0xffffffffu, h, 1), ol = __shfl_xor_sync(0xffffffffu, l, 1);
+            df_acc(h, l, oh, ol);
+          }
+          if (k == 0) {
+            th = h;
+            tl = l;
+          } else {
+            df_acc(th, tl, h, l);
+          }
+        }
       }
       if (cmv[j] == 1) {
-        pair_kick(v[j], dfloat{sh, sl}, c);
-        if (!last) half_drift(x[j], v[j], dt);
+        kick(v[j], df_norm(th, tl), c);
+        if (!last) coord_kick(x[j], v[j], dt);
       }
     }
     if (last) break;
@@ -579,7 +700,7 @@ __device__ void md_entries_body(const MDState& m, const MDStepArgs& a, Bin bin) 
 #pragma unroll
   for (int j = 0; j < NC; ++j)
     if (pub[j] >= 0) {
-      const double X = half_to_double(x[j]), V = df_to_double(v[j]);
+      const double X = coord_to_double(x[j]), V = df_to_double(v[j]);
       const int s = base + cq[j];
       (ck[j] == 0 ? m.x[0] : (ck[j] == 1 ? m.y[0] : m.z[0]))[s] = X;
       (ck[j] == 0 ? m.vx : (ck[j] == 1 ? m.vy : m.vz))[s] = V;
@@ -650,7 +771,7 @@ int launch_entries(const MDState& m, const typename Bin::Cells& c, const MDStepA
 }  // namespace
 
 // entries, polls and a solo tile's list are dealt to all threads of the CTA
-// (swimmer64 MD 123 us at 384 threads, 137 at 320 or 512)
+// (swimmer64 MD at 384 threads against 320 or 512, sums in any order: 123 us against 137)
 int md_entries_threads(int tile) { return tile <= 64 ? 384 : 512; }
 
 int launch_md_entries_f64cells(const MDState& m, const CellsF64& c, const MDStepArgs& a, cudaStream_t s,

@@ -1,6 +1,5 @@
-// Exchange of bead positions between the tiles of the double-float grid MD
-// kernels (md_df.cu, md_entries.cu) as tagged packets through L2, and the
-// transposing sums that leave each coordinate of a force with one lane.
+// Exchange of bead positions between the tiles of the entries kernel
+// (md_entries.cu) as tagged packets through L2.
 #pragma once
 #include <cstdint>
 
@@ -114,33 +113,6 @@ __device__ __forceinline__ void receive_packets(const uint4* src, int nslots, ui
       if (p < np) put(p - k * hn, k, d[u]);
     }
   }
-}
-
-// a pair-wise exchange step: keeps `mine`, sends `give` to the lane `o` away,
-// and adds what comes back
-__device__ __forceinline__ void exchange_add(float& mh, float& ml, float gh, float gl, int o) {
-  const float bh = __shfl_xor_sync(0xffffffffu, gh, o), bl = __shfl_xor_sync(0xffffffffu, gl, o);
-  df_acc(mh, ml, bh, bl);
-}
-
-// The sum over groups of G lanes (G = 4, 8 or 32) of (x, y, z): the two top
-// levels trade components instead of summing all three in every lane, so that
-// the quarter of the group with index k ends with component k, summed over
-// the group (quarter 3 holds nothing).  A fixed order.
-template <int G>
-__device__ __forceinline__ void group_sum_xyz(int lane, float fxh, float fxl, float fyh, float fyl, float fzh, float fzl,
-                                              float& h, float& l) {
-  const bool up = (lane & (G / 2)) != 0, odd = (lane & (G / 4)) != 0;
-  // lower half keeps x and y, the upper half z
-  float ah = up ? fzh : fxh, al = up ? fzl : fxl, bh = up ? 0.0f : fyh, bl = up ? 0.0f : fyl;
-  exchange_add(ah, al, up ? fxh : fzh, up ? fxl : fzl, G / 2);
-  exchange_add(bh, bl, up ? fyh : 0.0f, up ? fyl : 0.0f, G / 2);
-  // the even quarter keeps the first, the odd one the second
-  h = odd ? bh : ah;
-  l = odd ? bl : al;
-  exchange_add(h, l, odd ? ah : bh, odd ? al : bl, G / 4);
-#pragma unroll
-  for (int o = G / 8; o > 0; o >>= 1) exchange_add(h, l, h, l, o);
 }
 
 }  // namespace

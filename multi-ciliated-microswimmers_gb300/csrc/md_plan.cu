@@ -9,6 +9,7 @@
 #include <climits>
 #include <cmath>
 #include <cstdlib>
+#include <map>
 #include <utility>
 
 #include "md_plan.h"
@@ -227,7 +228,7 @@ std::string plan_md(const MDInput& in, const MDForce& force, bool allow_cluster,
     for (long i = 0; i < nsp; ++i) blist[fillp[in.sp_t[i]]++] = (int)i;
   }
   std::vector<char> hub(nb, 0), react(nsp, 0), dropped(nsp, 0);
-  if (!no_react) {
+  if (!no_react && (forced || (in.split && allow_cluster))) {  // the grid layouts have no such hubs
     for (long b = 0; b < nb; ++b) {
       if (owner[b] >= 0 || nspr[b] <= kChunk) continue;
       std::vector<int> partners;
@@ -667,33 +668,9 @@ std::string plan_md(const MDInput& in, const MDForce& force, bool allow_cluster,
   out.df_single.clear();
   out.df_single_start.assign(1, 0);
   int hmax = 0;
-  // The double-float grid kernel has no grid barrier: a tile may overwrite a
-  // position buffer once it has received the next evaluation from every tile
-  // that reads it, so every tile must read something of each of its readers.
-  // Spring networks made in both directions (every reference object) are so by
-  // themselves; for one-sided lists each missing direction gets one bead.
-  std::vector<std::vector<int>> answer(out.ntiles);  // per tile: its readers' beads to receive as well
-  if (out.df && !in.pair && !out.cluster) {
-    std::vector<std::vector<std::pair<int, int>>> reads(out.ntiles);  // (tile read, a primary slot of the reader)
-    std::vector<int> stamp(out.ntiles, -1);
-    for (int t = 0; t < out.ntiles; ++t)
-      for (int s2 = t * tile; s2 < (t + 1) * tile; ++s2)
-        for (int d = start[s2]; d < start[s2 + 1]; ++d) {
-          const int u = out.so[d] / tile;
-          if (u == t || stamp[u] == t) continue;
-          stamp[u] = t;
-          reads[t].push_back({u, out.prim[s2]});
-        }
-    for (int t = 0; t < out.ntiles; ++t)
-      for (const auto& r : reads[t]) {
-        bool back = false;
-        for (const auto& w : reads[r.first]) back = back || w.first == t;
-        if (!back) answer[r.first].push_back(r.second);
-      }
-  }
   for (int t = 0; t < out.ntiles; ++t) {
     const int b0 = t * tile, b1 = b0 + tile;
-    std::vector<int> ext = answer[t];
+    std::vector<int> ext;
     for (int s2 = start[b0]; s2 < start[b1]; ++s2)
       if (out.so[s2] < b0 || out.so[s2] >= b1) ext.push_back(out.so[s2]);
     std::sort(ext.begin(), ext.end());
@@ -756,6 +733,8 @@ std::string plan_md(const MDInput& in, const MDForce& force, bool allow_cluster,
       out.df_nsp_max = std::max(out.df_nsp_max, start[(t + 1) * tile] - start[t * tile]);
     }
     std::vector<long> idx;
+    std::vector<int> so, sk, sr, slv;
+    std::vector<double> srest, sm2k;
     for (int sl_ = 0; sl_ < ns; ++sl_) {
       const int a0 = start[sl_], a1 = start[sl_ + 1];
       idx.clear();
@@ -764,8 +743,8 @@ std::string plan_md(const MDInput& in, const MDForce& force, bool allow_cluster,
       out.df_split[sl_] = a0 + (int)idx.size();
       for (int k = a0; k < a1; ++k)
         if (out.sl[k] >= tile) idx.push_back(k);
-      std::vector<int> so(a1 - a0), sk(a1 - a0), sr(a1 - a0), slv(a1 - a0);
-      std::vector<double> srest(a1 - a0), sm2k(a1 - a0);
+      for (std::vector<int>* v : {&so, &sk, &sr, &slv}) v->resize(a1 - a0);
+      for (std::vector<double>* v : {&srest, &sm2k}) v->resize(a1 - a0);
       for (int k = 0; k < a1 - a0; ++k) {
         so[k] = out.so[idx[k]];
         sk[k] = out.sk[idx[k]];
@@ -877,6 +856,7 @@ std::string plan_md(const MDInput& in, const MDForce& force, bool allow_cluster,
   out.diag.resize(in.nbond);
   for (long k = 0; k < in.nbond; ++k) out.diag[k] = std::sqrt(0.5 * 0.5 + 0.5 * in.newlen[k]);
   out.slot_of = slot_of;
+  out.chunk = cl_chunk;
   return "";
 }
 
@@ -939,7 +919,7 @@ void bisect_beads(std::vector<long>& idx, const double* pos, int cap, Leaf&& lea
 // the tables of a chosen tiling (tile of every bead's slot in slot_of)
 std::string fill_entries(const MDInput& in, const std::vector<int>& bstart, const std::vector<int>& blist,
                          const std::vector<int>& cil_tile, const std::vector<char>& solo_bead,
-                         const std::vector<int>& slot_of, int tile, int ntiles, MDPlan& out) {
+                         const std::vector<int>& slot_of, int tile, int ntiles, const MDPlan& slots, MDPlan& out) {
   const long nb = in.nb;
   const int ns = ntiles * tile;
   out = MDPlan{};
@@ -970,7 +950,8 @@ std::string fill_entries(const MDInput& in, const std::vector<int>& bstart, cons
     if (solo_bead[b]) out.de_solo[s / tile] = 1;
   }
   // springs by slot, every bead's in its input order: the incidences
-  out.start.assign(ns + 1, 0);
+  std::vector<int>& start = out.start;
+  start.assign(ns + 1, 0);
   for (int s = 0; s < ns; ++s)
     out.start[s + 1] = out.start[s] + (bead_at[s] >= 0 ? bstart[bead_at[s] + 1] - bstart[bead_at[s]] : 0);
   const int nsp = out.start[ns];
@@ -999,8 +980,11 @@ std::string fill_entries(const MDInput& in, const std::vector<int>& bstart, cons
       out.df_nb_max = std::max(out.df_nb_max, out.df_nb[t]);
     }
   }
-  // every tile has to read something of each of its readers (the position
-  // buffers are reused without a grid barrier; see plan_md)
+  // every tile has to read something of each of its readers: the position
+  // buffers are reused without a grid barrier, a tile overwriting one once it
+  // has received the next evaluation from every tile that reads it.  Spring
+  // networks made in both directions (every reference object) are so by
+  // themselves; for one-sided lists each missing direction gets one bead.
   std::vector<std::vector<int>> reads(ntiles), answer(ntiles);
   {
     std::vector<int> stamp(ntiles, -1);
@@ -1022,13 +1006,67 @@ std::string fill_entries(const MDInput& in, const std::vector<int>& bstart, cons
   }
   out.hstart.assign(1, 0);
   out.de_start.assign(1, 0);
-  // the forces of a tile's incidences, 24 bytes each: transposed (the j-th
-  // spring of bead a at j T + a, so that threads summing neighbouring beads
-  // read neighbouring words) unless a long list makes that too large
-  int longest = 1;
-  for (int s = 0; s < ns; ++s)
-    if (!out.de_solo[s / tile]) longest = std::max(longest, out.start[s + 1] - out.start[s]);
-  out.de_step = 24L * longest * tile <= kMaxForceBytes ? tile : 1;
+  // The force words of every bead, as the slot layout adds its springs: slot by
+  // slot (a chunk of the list each), a slot's springs inside the slot layout's
+  // tile dealt to the lanes in turn, then the others likewise.  A lane's k-th
+  // spring is in row k of the slot.
+  const int lanes = out.de_lanes = md_df_lanes(slots.tile);
+  out.de_at.assign(ns, 0);
+  out.de_shape.assign(ns, 0u);
+  out.de_slots.assign(ntiles, 0);
+  std::vector<int> word(nsp, 0);      // of each spring (by slot), within its bead
+  std::vector<int> words(ns, 0);      // of each bead
+  std::map<int, std::vector<int>> solo_slot_rows;  // by tile
+  int most = 1;
+  for (int s = 0; s < ns; ++s) {
+    if (bead_at[s] < 0) continue;
+    const long b = bead_at[s];
+    const int ref = slots.slot_of[b], rtile = ref / slots.tile, nslot = slots.nhelp[ref] + 1;
+    const int n = start[s + 1] - start[s], chunk = nslot > 1 ? slots.chunk : std::max(1, n);
+    const bool solo = solo_bead[b] != 0;
+    if (!solo && nslot > 8) return "a bead with too many helper slots";
+    std::vector<int> slot_rows;
+    int row0 = 0, solo_rows = 1;
+    std::vector<int> place;  // of a solo bead's springs: {spring, slot, lane, row}
+    for (int k = 0; k < nslot && k * chunk < n; ++k) {
+      int count[8] = {};  // springs of each lane
+      for (int pass = 0; pass < 2; ++pass)
+        for (int j = k * chunk, at = 0; j < std::min(n, (k + 1) * chunk); ++j) {
+          const int d = start[s] + j;
+          const bool inside = slots.slot_of[in.sp_o[src[d]]] / slots.tile == rtile;
+          if (inside != (pass == 0)) continue;
+          const int lane = at++ % lanes, row = count[lane]++;
+          word[d] = (row0 + row) * lanes + lane;
+          if (solo) place.insert(place.end(), {d, k, lane, row});
+        }
+      const int rows = *std::max_element(count, count + lanes);
+      solo_rows = std::max(solo_rows, rows);
+      if (solo) {
+        slot_rows.push_back(rows);
+        continue;
+      }
+      if (rows > 15) return "too many springs in a slot";
+      out.de_shape[s] |= (uint32_t)rows << (4 * k);
+      row0 += rows;
+      words[s] = row0 * lanes;
+      out.de_slots[s / tile] = std::max(out.de_slots[s / tile], k + 1);
+    }
+    if (solo) {  // room for as many rows in every slot, then a word per slot for its sum and a spare one
+      for (size_t q = 0; q < place.size(); q += 4)
+        word[place[q]] = (place[q + 3] * lanes + place[q + 2]) * nslot + place[q + 1];
+      solo_slot_rows[s / tile] = slot_rows;
+      out.de_slots[s / tile] = solo_rows;
+      out.de_shape[s] = (uint32_t)nslot;
+      out.de_at[s] = (ref % slots.tile) & 31;
+      words[s] = nslot * (solo_rows * lanes + 1) + 1;
+      continue;
+    }
+    most = std::max(most, words[s]);
+  }
+  // the words, 24 bytes each: transposed (word j of bead a at j T + a, so that
+  // threads summing neighbouring beads read neighbouring words) unless a long
+  // list makes that too large
+  out.de_step = 24L * most * tile <= kMaxForceBytes ? tile : 1;
   std::vector<int> ent(nsp, -1), order;
   struct Entry {
     int a, b, d, r;
@@ -1049,17 +1087,16 @@ std::string fill_entries(const MDInput& in, const std::vector<int>& bstart, cons
     out.halo.insert(out.halo.end(), ext.begin(), ext.end());
     out.hstart.push_back((int)out.halo.size());
     out.hmax = std::max(out.hmax, (int)ext.size());
-    int words = d1 - d0;
-    if (out.de_step > 1) {
-      words = 0;
-      for (int s = s0; s < s1; ++s) words = std::max(words, (out.start[s + 1] - out.start[s]) * tile);
+    int nword = solo ? words[s0] : 0;
+    for (int s = s0; s < s1 && !solo; ++s) {
+      out.de_at[s] = out.de_step > 1 ? s - s0 : nword;
+      nword = out.de_step > 1 ? std::max(nword, words[s] * tile) : nword + words[s];
     }
-    if (solo) words = 0;
-    if (words >= 0xffff) return "too many springs in a tile";
-    out.de_nslot.push_back(words);
-    out.de_ninc_max = std::max(out.de_ninc_max, words);
+    if (nword >= 0xffff) return "too many springs in a tile";
+    out.de_nslot.push_back(nword);
+    out.de_ninc_max = std::max(out.de_ninc_max, nword);
     auto word_of = [&](int d, int bead) {  // spring d of local bead `bead`
-      return (uint32_t)(out.de_step > 1 ? (d - out.start[s0 + bead]) * tile + bead : d - d0);
+      return solo ? (uint32_t)word[d] : (uint32_t)(out.de_at[s0 + bead] + word[d] * out.de_step);
     };
     // a spring and its exact reverse inside the tile form one entry
     es.clear();
@@ -1072,8 +1109,9 @@ std::string fill_entries(const MDInput& in, const std::vector<int>& bstart, cons
         ent[d] = 1;
         if (e.b < tile && e.b != e.a && !solo)
           for (int r = out.start[out.so[d]]; r < out.start[out.so[d] + 1]; ++r) {
+            if (out.so[r] != s || ent[r] >= 0) continue;
             const int j = src[r];
-            if (ent[r] >= 0 || out.so[r] != s || in.sp_k[j] != kind || in.sp_kk[j] != in.sp_kk[i]) continue;
+            if (in.sp_k[j] != kind || in.sp_kk[j] != in.sp_kk[i]) continue;
             if (kind >= MPCD_SPRING_BOND ? in.sp_r[j] != in.sp_r[i] : in.sp_rest[j] != in.sp_rest[i]) continue;
             ent[r] = 1;
             e.r = r;
@@ -1096,7 +1134,7 @@ std::string fill_entries(const MDInput& in, const std::vector<int>& bstart, cons
         if (lref < 0 || lref >= out.df_nb[t]) return "a bond spring refers to a bond outside its tile's cilia";
       }
       if (e.b >= 0x10000 || lref >= (1 << 29)) return "an MD tile is too large for packed entry codes";
-      const uint32_t ka = solo ? 0u : word_of(e.d, e.a), kb = e.r >= 0 ? word_of(e.r, e.b) : 0xffffu;
+      const uint32_t ka = word_of(e.d, e.a), kb = e.r >= 0 ? word_of(e.r, e.b) : 0xffffu;
       uint4 c;
       c.x = (uint32_t)e.a | (kind == MPCD_SPRING_GUARDED ? 0x8000u : 0u) | ((uint32_t)e.b << 16);
       c.y = ka | (kb << 16);
@@ -1114,19 +1152,18 @@ std::string fill_entries(const MDInput& in, const std::vector<int>& bstart, cons
       for (const Entry& e : es) has[e.b - tile] = 1;
       for (size_t k = 0; k < ext.size(); ++k)
         if (!has[k]) {
-          uint4 c;
-          c.x = 0x8000u | ((uint32_t)(tile + (int)k) << 16);
-          c.y = 0xffff0000u;
-          c.z = c.w = 0u;
-          out.de_code.push_back(c);
+          out.de_code.push_back(
+              make_uint4(0x8000u | ((uint32_t)(tile + (int)k) << 16), 0xffff0000u | (uint32_t)(nword - 1), 0u, 0u));
           out.de_rest.push_back(0.0);
           out.de_m2k.push_back(0.0);
         }
     }
+    if (solo)
+      for (size_t k = 0; k < solo_slot_rows[t].size(); ++k) out.de_code[out.de_start.back() + k].w = (uint32_t)solo_slot_rows[t][k];
     out.de_start.push_back((int)out.de_code.size());
     out.de_nent_max = std::max(out.de_nent_max, out.de_start[t + 1] - out.de_start[t]);
   }
-  out.de_ninc_max = std::max(out.de_ninc_max, 16);  // a solo tile's sums, one per warp
+  out.de_ninc_max = std::max(out.de_ninc_max, 1);
   // cilia
   out.tcil.assign(ntiles + 1, 0);
   for (int c = 0; c < in.ncil; ++c) {
@@ -1160,7 +1197,7 @@ std::string fill_entries(const MDInput& in, const std::vector<int>& bstart, cons
 
 }  // namespace
 
-std::string plan_entries(const MDInput& in, int grid_f32cells, MDPlan& out, int min_tile) {
+std::string plan_entries(const MDInput& in, int grid_f32cells, const MDPlan& slots, MDPlan& out, int min_tile) {
   const long nb = in.nb, nsp = in.nsp;
   std::vector<int> bstart(nb + 1, 0), blist(nsp);
   for (long i = 0; i < nsp; ++i) {
@@ -1225,7 +1262,7 @@ std::string plan_entries(const MDInput& in, int grid_f32cells, MDPlan& out, int 
       });
     }
     if (nt > sms) continue;
-    const std::string why = fill_entries(in, bstart, blist, cil_tile, solo, slot_of, tile, nt, out);
+    const std::string why = fill_entries(in, bstart, blist, cil_tile, solo, slot_of, tile, nt, slots, out);
     if (!why.empty()) return why;
     MDState probe;
     probe.tile = tile;

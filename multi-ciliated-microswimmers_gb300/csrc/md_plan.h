@@ -56,10 +56,12 @@ struct MDPlan {
   std::vector<int> df_run_start;  // ntiles + 1
   std::vector<int2> df_single;     // other halo entries {slot, staged rank}
   std::vector<int> df_single_start;
+  int chunk = 0;  // springs per slot of a bead with helper slots
   int df_nsp_max = 0, df_nb_max = 0, df_nrun_max = 0, df_nsingle_max = 0;
   // entries kernel (md_entries.cu)
-  int de = 0, de_nent_max = 0, de_ninc_max = 0, de_step = 1;
-  std::vector<int> de_start, de_local_end, de_solo, de_nslot;
+  int de = 0, de_nent_max = 0, de_ninc_max = 0, de_step = 1, de_lanes = 8;
+  std::vector<int> de_start, de_local_end, de_solo, de_nslot, de_slots, de_at;
+  std::vector<uint32_t> de_shape;
   std::vector<uint4> de_code;             // {a | guarded << 15 | b << 16, ka | kb << 16, kind | bond << 2, 0}
   std::vector<double> de_rest, de_m2k;
   // pair kernel (md_pair.cu): per tile its force entries (a spring and its
@@ -88,11 +90,11 @@ struct MDPlan {
   long nsp_kept() const { return (long)so.size(); }
 };
 
-// Plans the layout of the entries kernel (md_entries.cu) for double-float
-// arithmetic.  Returns an empty string on success; any other answer means
-// that plan_md's layouts are to be used (a bead set the entries layout has no
-// room for, or an input that plan_md rejects).
-std::string plan_entries(const MDInput& in, int grid_f32cells, MDPlan& out, int min_tile = 0);
+// Plans the layout of the entries kernel (md_entries.cu) for a bead set that
+// plan_md has given the slot layout `slots` of md_df.cu, in whose order every
+// bead's forces are added.  Returns an empty string on success; any other
+// answer means that the slot layout is to be used.
+std::string plan_entries(const MDInput& in, int grid_f32cells, const MDPlan& slots, MDPlan& out, int min_tile = 0);
 
 // Plans the layout.  Returns an empty string on success, else the reason.
 // `grid_f32cells` selects the co-resident limit checked for the grid layout.
