@@ -101,6 +101,39 @@ constexpr uint64_t kMapF64 = 0x7fffffff00000000ull;
 
 MPCD_HD Limbs word_limbs(uint64_t w) { return {(int32_t)(w >> 32), (int32_t)(uint32_t)w}; }
 
+// The mean velocity u (units of 2^-58) and the kinetic energy K - M u^2 relative
+// to it (units of 2^-50) of a cell with momentum p, kinetic energy kin (units of
+// 2^-50, below 4096) and mass M, inv = 1 / M in units of 2^-62.  top: 8 M in units of
+// 2^-52, or anything above 512 in them: a larger momentum is refused before the product
+// can wrap.  False if the numbers do not fit.
+constexpr int kMomentumBits = 52;
+MPCD_HD bool cell_mean(const double* p, int64_t kin, int64_t inv, int64_t top, int64_t* u, int64_t& erel) {
+  int64_t q[3];
+  if (!(to_fixed<kMomentumBits, 9>(p[0], q[0]) && to_fixed<kMomentumBits, 9>(p[1], q[1]) &&
+        to_fixed<kMomentumBits, 9>(p[2], q[2])))
+    return false;
+  bool fit = true;
+#pragma unroll
+  for (int i = 0; i < 3; ++i) fit = fit && q[i] < top && q[i] > -top;
+  if (!fit) return false;
+  const Limbs iv = split_limbs(inv);
+  uint64_t rel = (uint64_t)kin;
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    const Limbs l = split_limbs(q[i]);
+    u[i] = mul_sh<56>(l, iv);
+    fit = fit && u[i] < kMeanMax && u[i] > -kMeanMax;
+    rel -= (uint64_t)mul_sh<60>(split_limbs(u[i]), l);
+  }
+  erel = (int64_t)rel;
+  return fit;
+}
+// 8 M in the units of cell_mean: whole numbers of particles, and any mass
+MPCD_HD int64_t mean_limit(int num) { return (int64_t)(num < 64 ? num : 64) << (kMomentumBits + 3); }
+MPCD_HD int64_t mean_limit(double mass) {
+  return (int64_t)((mass < 64.0 ? mass : 64.0) * (double)(1ll << (kMomentumBits + 3)));
+}
+
 // a float in (-2, 2) in units of 2^-60
 MPCD_HD int64_t axis_fixed(float f) {
 #ifdef __CUDA_ARCH__

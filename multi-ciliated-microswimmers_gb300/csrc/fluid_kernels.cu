@@ -308,24 +308,18 @@ __device__ __forceinline__ bool cell_factor(double4 s, uint32_t w, long cid, con
     ke_rest += s.w;
     fit = false;
   }
-  int64_t p[3], inv = 0;
+  int64_t inv = 0, top = 0, erel = 0;
   sc = 1ll << kAxisBits;
-  fit = fit && to_fixed<52, 9>(s.x, p[0]) && to_fixed<52, 9>(s.y, p[1]) && to_fixed<52, 9>(s.z, p[2]);
-  if (nb == 0 && num < 256)
+  if (nb == 0 && num < 256) {
     inv = __ldg(g_inv_n.x + num);  // M = num without beads
-  else
+    top = mean_limit(num);
+  } else {
     fit = to_fixed<62, 0>(1.0 / M, inv) && fit;
+    top = mean_limit(M);
+  }
   if (fit) {
-    const Limbs iv = split_limbs(inv);
-    uint64_t rel = (uint64_t)kin;
-#pragma unroll
-    for (int q = 0; q < 3; ++q) {
-      const Limbs pq = split_limbs(p[q]);
-      u[q] = mul_sh<56>(pq, iv);
-      fit = fit && u[q] < kMeanMax && u[q] > -kMeanMax;
-      rel -= (uint64_t)mul_sh<60>(split_limbs(u[q]), pq);  // K - M u^2
-    }
-    const int64_t erel = (int64_t)rel;
+    const double p[3] = {s.x, s.y, s.z};
+    fit = cell_mean(p, kin, inv, top, u, erel);
     if (fit && erel > 0 && num > 1) {
       const double e = from_fixed(erel, 50);
       const double f = a.inj_gamma ? thermostat_factor(injected_gamma(a, cid, errbits), e) : thermostat_factor(gf, e);
