@@ -16,7 +16,8 @@
 // the float64 form's wherever the terms of a sum are of order one.  What does
 // not fit (velocities of 16 thermal velocities and more, mean velocities of 8,
 // thermostat factors of 2, kinetic energies of a cell of 4096, momenta of 512,
-// non-finite values) takes the float64 form, about half as fast.
+// cells colder than 1/16, non-finite values) takes the float64 form, about half
+// as fast.
 //
 // Host and device code alike (tests run it on the CPU).
 #pragma once
@@ -101,17 +102,28 @@ constexpr uint64_t kMapF64 = 0x7fffffff00000000ull;
 
 MPCD_HD Limbs word_limbs(uint64_t w) { return {(int32_t)(w >> 32), (int32_t)(uint32_t)w}; }
 
-// The mean velocity u (units of 2^-58) and the kinetic energy K - M u^2 relative
-// to it (units of 2^-50) of a cell with momentum p, kinetic energy kin (units of
-// 2^-50, below 4096) and mass M, inv = 1 / M in units of 2^-62.  top: 8 M in units of
-// 2^-52, or anything above 512 in them: a larger momentum is refused before the product
-// can wrap.  False if the numbers do not fit.
+// 8 M in units of 2^-PB, for whole numbers of particles and for any mass, as far
+// as it matters to momenta in 62 bits.
 constexpr int kMomentumBits = 52;
+template <int PB = kMomentumBits>
+MPCD_HD int64_t mean_limit(int num) {
+  constexpr int most = 1 << (59 - PB);
+  return (int64_t)(num < most ? num : most) << (PB + 3);
+}
+template <int PB = kMomentumBits>
+MPCD_HD int64_t mean_limit(double mass) {
+  constexpr double most = 1 << (59 - PB);
+  return (int64_t)((mass < most ? mass : most) * (double)(1ll << (PB + 3)));
+}
+// The mean velocity u (units of 2^-58) and the kinetic energy K - M u^2 relative
+// to it (units of 2^-KB) of a cell with momentum p (each below 2^PE), kinetic energy kin
+// (units of 2^-KB, below 2^62) and mass M, inv = 1 / M in units of 2^-62.  top: 8 M in
+// units of 2^-PB; a momentum that reaches it is refused before the product can
+// wrap.  False if the numbers do not fit.
+template <int PB = kMomentumBits, int PE = 9, int KB = 50>
 MPCD_HD bool cell_mean(const double* p, int64_t kin, int64_t inv, int64_t top, int64_t* u, int64_t& erel) {
   int64_t q[3];
-  if (!(to_fixed<kMomentumBits, 9>(p[0], q[0]) && to_fixed<kMomentumBits, 9>(p[1], q[1]) &&
-        to_fixed<kMomentumBits, 9>(p[2], q[2])))
-    return false;
+  if (!(to_fixed<PB, PE>(p[0], q[0]) && to_fixed<PB, PE>(p[1], q[1]) && to_fixed<PB, PE>(p[2], q[2]))) return false;
   bool fit = true;
 #pragma unroll
   for (int i = 0; i < 3; ++i) fit = fit && q[i] < top && q[i] > -top;
@@ -121,17 +133,27 @@ MPCD_HD bool cell_mean(const double* p, int64_t kin, int64_t inv, int64_t top, i
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
     const Limbs l = split_limbs(q[i]);
-    u[i] = mul_sh<56>(l, iv);
+    u[i] = mul_sh<PB + 4>(l, iv);
     fit = fit && u[i] < kMeanMax && u[i] > -kMeanMax;
-    rel -= (uint64_t)mul_sh<60>(split_limbs(u[i]), l);
+    rel -= (uint64_t)mul_sh<58 + PB - KB>(split_limbs(u[i]), l);
   }
   erel = (int64_t)rel;
   return fit;
 }
-// 8 M in the units of cell_mean: whole numbers of particles, and any mass
-MPCD_HD int64_t mean_limit(int num) { return (int64_t)(num < 64 ? num : 64) << (kMomentumBits + 3); }
-MPCD_HD int64_t mean_limit(double mass) {
-  return (int64_t)((mass < 64.0 ? mass : 64.0) * (double)(1ll << (kMomentumBits + 3)));
+// A cell's kinetic energy in units of 2^-55 below 128 (ten thermal particles hold
+// 30), else of 2^-50; 0 if it does not fit.
+MPCD_HD int kinetic_fixed(double K, int64_t& kin) { return to_fixed<55, 7>(K, kin) ? 55 : (to_fixed<50, 12>(K, kin) ? 50 : 0); }
+// 8 M in the units of the momenta that go with it
+template <typename M>
+MPCD_HD int64_t mean_top(int bits, M mass) { return bits == 55 ? mean_limit<55>(mass) : mean_limit(mass); }
+// cell_mean in the units of kinetic_fixed.  A cell whose particles differ by too
+// little from each other (a single one: from rest) is refused: below an energy of
+// 1/16 the units are coarser than float64, and below one unit nothing would be left
+// for the thermostat to scale.
+MPCD_HD bool cell_energy(const double* p, int64_t kin, int bits, int64_t inv, int64_t top, bool single, int64_t* u,
+                         int64_t& erel) {
+  const bool fit = bits == 55 ? cell_mean<55, 7, 55>(p, kin, inv, top, u, erel) : cell_mean(p, kin, inv, top, u, erel);
+  return fit && (single ? kin : erel) >= 1ll << (bits - 4);
 }
 
 // a float in (-2, 2) in units of 2^-60

@@ -302,8 +302,9 @@ __device__ __forceinline__ bool cell_factor(double4 s, uint32_t w, long cid, con
   // matches the reference's bookkeeping including the rounding of its
   // rotation constants
   int64_t kin = 0;
-  if (to_fixed<50, 12>(s.w, kin)) {
-    ke += (uint64_t)((kin + 512) >> 10);
+  const int ebits = kinetic_fixed(s.w, kin);
+  if (ebits) {
+    ke += (uint64_t)((kin + (1ll << (ebits - kEnergyBits - 1))) >> (ebits - kEnergyBits));
   } else {
     ke_rest += s.w;
     fit = false;
@@ -312,16 +313,16 @@ __device__ __forceinline__ bool cell_factor(double4 s, uint32_t w, long cid, con
   sc = 1ll << kAxisBits;
   if (nb == 0 && num < 256) {
     inv = __ldg(g_inv_n.x + num);  // M = num without beads
-    top = mean_limit(num);
+    top = mean_top(ebits, num);
   } else {
     fit = to_fixed<62, 0>(1.0 / M, inv) && fit;
-    top = mean_limit(M);
+    top = mean_top(ebits, M);
   }
   if (fit) {
     const double p[3] = {s.x, s.y, s.z};
-    fit = cell_mean(p, kin, inv, top, u, erel);
-    if (fit && erel > 0 && num > 1) {
-      const double e = from_fixed(erel, 50);
+    fit = cell_energy(p, kin, ebits, inv, top, num == 1, u, erel);
+    if (fit && num > 1) {
+      const double e = from_fixed(erel, ebits);
       const double f = a.inj_gamma ? thermostat_factor(injected_gamma(a, cid, errbits), e) : thermostat_factor(gf, e);
       fit = to_fixed<60, 1>(f, sc);
     }

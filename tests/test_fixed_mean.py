@@ -103,3 +103,56 @@ def test_masses_that_do_not_fit(mean, mass):
 def test_numbers_that_are_not_finite(mean):
     for bad in (float("inf"), -float("inf"), float("nan"), 1e300, 512.0):
         assert not mean([bad, 0.0, 0.0], 1.0, 10)[0] and not mean([0.0, 0.0, bad], 1.0, 10)[0]
+
+
+ENERGY = r"""
+#include "fixed_collide.cuh"
+using namespace mpcd;
+extern "C" int energy(const double* p, double K, int num, double* u, double* erel) {
+  int64_t kin = 0, v[3] = {0, 0, 0}, e = 0;
+  const int bits = kinetic_fixed(K, kin);
+  if (!bits) return 0;
+  const int64_t inv = (int64_t)(((1ull << 62) + (unsigned)num / 2) / (unsigned)num);
+  const bool fit = cell_energy(p, kin, bits, inv, mean_top(bits, num), num == 1, v, e);
+  for (int i = 0; i < 3; ++i) u[i] = from_fixed(v[i], kVelBits);
+  *erel = from_fixed(e, bits);
+  return fit;
+}
+"""
+
+
+@pytest.mark.parametrize("num", [2, 3, 10, 40])
+@pytest.mark.parametrize("drift", [0.0, 0.3, 5.0])
+def test_relative_energy_is_as_close_as_in_float64(tmp_path, num, drift):
+    """Cells at thermal speeds from 1 down: what is refused is cold, and what is
+    kept has an energy no further from the exact one than float64's in the mean;
+    at worst by the roundings of its units beside the half unit of float64 that
+    both end with (three products of one unit each, and the mean's rounding)."""
+    src, so = tmp_path / "e.cpp", tmp_path / "e.so"
+    src.write_text(ENERGY)
+    subprocess.run(["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-Wall", "-I", os.path.join(PKG, "csrc"), str(src), "-o",
+                    str(so)], check=True)
+    f = ctypes.CDLL(str(so)).energy
+    dp = ctypes.POINTER(ctypes.c_double)
+    f.argtypes = [dp, ctypes.c_double, ctypes.c_int, dp, dp]
+    rng = np.random.default_rng(11)
+    ours, theirs = [], []
+    for speed in (1.0, 0.5, 0.2, 0.05, 1e-3, 1e-6, 1e-9):
+        for _ in range(150):
+            v = rng.normal(size=(num, 3)) * speed + drift
+            p, K = v.sum(axis=0), float((v * v).sum())
+            u, e = (ctypes.c_double * 3)(), ctypes.c_double()
+            fit = f((ctypes.c_double * 3)(*p), K, num, u, ctypes.byref(e))
+            exact = Fraction(K) - sum(Fraction(q) ** 2 for q in p) / num
+            if exact < Fraction(1, 17):
+                assert not fit
+            if not fit:
+                assert exact < Fraction(1, 15) or np.abs(p).max() / num > 7.9 or K > 4000
+                continue
+            inv = 1.0 / num
+            w = p * inv
+            e64 = K - (w[0] * p[0] + w[1] * p[1] + w[2] * p[2])
+            ours.append(abs(float(Fraction(e.value) - exact)))
+            theirs.append(abs(float(Fraction(e64) - exact)))
+    assert len(ours) > 100
+    assert np.mean(ours) <= np.mean(theirs) and max(ours) <= max(theirs) + 4 * 2.0 ** -50
