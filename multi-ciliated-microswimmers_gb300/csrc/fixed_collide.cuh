@@ -15,9 +15,13 @@
 // 2^-54 for float64 numbers of one half and more, so results are at least as close to the exact ones as
 // the float64 form's wherever the terms of a sum are of order one.  What does
 // not fit (velocities of 16 thermal velocities and more, mean velocities of 8,
-// thermostat factors of 2, kinetic energies of a cell of 4096, momenta of 512,
+// thermostat factors of 8 (of 2 where the mean velocity is 2), kinetic energies of a cell of 4096, momenta of 512,
 // cells colder than 1/16, non-finite values) takes the float64 form, about half
-// as fast.
+// as fast; a warp with one such particle makes both.  The factor's limit is what
+// counts at low densities: with 2 in place of 8, 4 % of the particles of a box with
+// three per cell were beyond it, in half of the warps, and 0.1 % with ten per cell
+// (64^3 cells, us per step, limit 2 / limit 8 / all in float64: two per cell 92 / 58 / 77,
+// three 109 / 66 / 90, ten 125 / 120 / 182, twenty 201 / 207 / 313).
 //
 // Host and device code alike (tests run it on the CPU).
 #pragma once
@@ -98,9 +102,18 @@ constexpr int kMapBits = 59;         // entries of A
 constexpr int kAxisBits = 60;        // axis components, thermostat factor
 constexpr int kOutBits = 56;         // velocities that come out: up to 92 with the limits below
 constexpr int64_t kMeanMax = 1ll << 61;  // 8, mean velocities
+constexpr int64_t kMeanMaxHot = 1ll << 59;  // 2, where the thermostat factor is 2 or more
+constexpr float kGammaMax = 4096.f;         // and the Gamma variate there
 constexpr uint64_t kMapF64 = 0x7fffffff00000000ull;
 
 MPCD_HD Limbs word_limbs(uint64_t w) { return {(int32_t)(w >> 32), (int32_t)(uint32_t)w}; }
+// The first word of a map: an entry of A is below 2 (29 bits and a sign in its
+// high limb), so that bit 62 differs from the sign only where it was flipped to say
+// that A is held divided by four.  kMapF64 is neither.
+MPCD_HD int word_scale(uint64_t w) { return (int)((w ^ (w << 1)) >> 62) & 2; }
+MPCD_HD Limbs first_limbs(uint64_t w) {
+  return {(int32_t)((uint32_t)(w >> 32) << 2) >> 2, (int32_t)(uint32_t)w};
+}
 
 // 8 M in units of 2^-PB, for whole numbers of particles and for any mass, as far
 // as it matters to momenta in 62 bits.
@@ -205,36 +218,43 @@ MPCD_HD void rotation_fixed(const int64_t* r, double cos_a, double sin_a, int64_
   R[8] = mul_sh<60>(tz, z) + ca;
 }
 // Row i of the map's words from that row of R, the factor sc (2^-60) and the
-// mean velocity u (2^-58): A = sc R, b = u - A u.
-MPCD_HD void map_row(int i, const int64_t* row, int64_t sc, const int64_t* u, uint64_t* w) {
+// mean velocity u (2^-58): A = sc R, b = u - A u.  With s = 2 the factor is 4 sc: A is
+// held divided by four (word_scale).
+MPCD_HD void map_row(int i, const int64_t* row, int64_t sc, const int64_t* u, uint64_t* w, int s = 0) {
   const Limbs f = split_limbs(sc);
   int64_t b = (u[i] + 1) >> 1;  // 2^-57
 #pragma unroll
   for (int j = 0; j < 3; ++j) {
     const Limbs a = split_limbs(mul_sh<61>(split_limbs(row[j]), f));
     w[j] = (uint64_t)(uint32_t)a.h << 32 | (uint32_t)a.l;
-    b -= mul_sh<60>(a, split_limbs(u[j]));
+    b -= (int64_t)((uint64_t)mul_sh<60>(a, split_limbs(u[j])) << s);
   }
   w[3] = (uint64_t)((b + 1) >> 1);
+  if (i == 0 && s) w[0] ^= 1ull << 62;
 }
-MPCD_HD void map_words(const int64_t* r, int64_t sc, const int64_t* u, double cos_a, double sin_a, uint64_t* w) {
+MPCD_HD void map_words(const int64_t* r, int64_t sc, const int64_t* u, double cos_a, double sin_a, uint64_t* w, int s = 0) {
   int64_t R[9];
   rotation_fixed(r, cos_a, sin_a, R);
 #pragma unroll
-  for (int i = 0; i < 3; ++i) map_row(i, R + 3 * i, sc, u, w + 4 * i);
+  for (int i = 0; i < 3; ++i) map_row(i, R + 3 * i, sc, u, w + 4 * i, s);
 }
 
-// v' = A v + b in units of 2^-56 (|v_i| < 16, sc < 2 and |u_i| < 8 keep every sum
-// within 63 bits; anything else gives some number and no harm).  The products of low halves are left out
-// (up to two units each, 1.2 together in the mean square).
+// v' = A v + b in units of 2^-56, for |v_i| < 16 of a particle that is in the cell.
+// The sums are taken modulo 2^64; the result, |u| + sc |v - u|, is below 2^7: with sc < 2
+// and |u_i| < 8 by these limits, with sc < 8 because sc |v - u| is at most the root of sc^2
+// E_rel = 2 g, g < kGammaMax.  The products of low halves are left out (up to two units
+// each, 1.2 together in the mean square; four times that where A is held divided
+// by four, whose float64 form rounds as much more coarsely).
 MPCD_HD void apply_words(const uint64_t* w, const int64_t* v, int64_t* out) {
   const Limbs x = split_limbs(v[0]), y = split_limbs(v[1]), z = split_limbs(v[2]);
+  const int s = word_scale(w[0]);
+  const uint32_t half = 1u << (28 - s);
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
-    const Limbs a = word_limbs(w[4 * i]), b = word_limbs(w[4 * i + 1]), c = word_limbs(w[4 * i + 2]);
+    const Limbs a = i ? word_limbs(w[4 * i]) : first_limbs(w[0]), b = word_limbs(w[4 * i + 1]), c = word_limbs(w[4 * i + 2]);
     const uint64_t top = uwide(a.h, x.h) + uwide(b.h, y.h) + uwide(c.h, z.h);
     const uint64_t mid = uwide(a.h, x.l) + uwide(b.h, y.l) + uwide(c.h, z.l) + uwide(a.l, x.h) + uwide(b.l, y.h) + uwide(c.l, z.h);
-    out[i] = (int64_t)((top << 3) + (uint64_t)((int64_t)(mid + (1u << 28)) >> 29) + w[4 * i + 3]);
+    out[i] = (int64_t)((top << (3 + s)) + (uint64_t)((int64_t)(mid + half) >> (29 - s)) + w[4 * i + 3]);
   }
 }
 

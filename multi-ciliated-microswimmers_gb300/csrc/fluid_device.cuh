@@ -444,8 +444,8 @@ __device__ __forceinline__ void apply_map_f64(const double* par, double& vx, dou
   } else {
 #pragma unroll
     for (int q = 0; q < 9; ++q) {
-      const Limbs p = word_limbs(w[q + q / 3]);
-      A[q] = from_fixed((int64_t)((uint64_t)(int64_t)p.h << 32) + p.l, kMapBits);
+      const Limbs p = q ? word_limbs(w[q + q / 3]) : first_limbs(w[0]);
+      A[q] = from_fixed((int64_t)((uint64_t)(int64_t)p.h << 32) + p.l, kMapBits - word_scale(w[0]));
     }
 #pragma unroll
     for (int q = 0; q < 3; ++q) b[q] = from_fixed((int64_t)w[4 * q + 3], kOutBits);

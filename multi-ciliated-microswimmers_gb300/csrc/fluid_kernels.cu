@@ -269,7 +269,7 @@ __device__ __noinline__ unsigned map_f64(const CellSums& t, long cid, float gf, 
 // The sums' part: factor and mean velocity.  False if the cell takes the
 // float64 form, whose words it has written to par.
 __device__ __forceinline__ bool cell_factor(double4 s, uint32_t w, long cid, const StepArgs& a, double* par, int64_t& sc,
-                                            int64_t* u, uint64_t& ke, double& ke_rest, unsigned& errbits, bool& gfail) {
+                                            int& scale, int64_t* u, uint64_t& ke, double& ke_rest, unsigned& errbits, bool& gfail) {
   const int nf = cnt_fluid(w), nb = cnt_beads(w);
   int num = nf + nb, sk = -1;
   double M = (double)num;
@@ -311,6 +311,7 @@ __device__ __forceinline__ bool cell_factor(double4 s, uint32_t w, long cid, con
   }
   int64_t inv = 0, top = 0, erel = 0;
   sc = 1ll << kAxisBits;
+  scale = 0;
   if (nb == 0 && num < 256) {
     inv = __ldg(g_inv_n.x + num);  // M = num without beads
     top = mean_top(ebits, num);
@@ -323,8 +324,25 @@ __device__ __forceinline__ bool cell_factor(double4 s, uint32_t w, long cid, con
     fit = cell_energy(p, kin, ebits, inv, top, num == 1, u, erel);
     if (fit && num > 1) {
       const double e = from_fixed(erel, ebits);
-      const double f = a.inj_gamma ? thermostat_factor(injected_gamma(a, cid, errbits), e) : thermostat_factor(gf, e);
-      fit = to_fixed<60, 1>(f, sc);
+      double f;
+      if (a.inj_gamma) {
+        const double g = injected_gamma(a, cid, errbits);
+        f = thermostat_factor(g, e);
+        fit = g < kGammaMax;
+      } else {
+        f = thermostat_factor(gf, e);
+        fit = gf < kGammaMax;
+      }
+      const int hi = __double2hiint(f);
+      if (hi >= 1024 << 20) {  // 2 and more: a quarter of it, where the sums leave room
+#pragma unroll
+        for (int q = 0; q < 3; ++q) fit = fit && u[q] < kMeanMaxHot && u[q] > -kMeanMaxHot;
+        f = __hiloint2double(hi - (2 << 20), __double2loint(f));
+        scale = 2;
+      } else {
+        fit = true;
+      }
+      fit = to_fixed<60, 1>(f, sc) && fit;
     }
   }
   if (!fit) {
@@ -351,9 +369,9 @@ __device__ __forceinline__ void cell_rotation(long cid, const StepArgs& a, int64
   }
   rotation_fixed(r, kCosAlpha, kSinAlpha, R);
 }
-__device__ __forceinline__ void store_row(double* par, int i, const int64_t* row, int64_t sc, const int64_t* u) {
+__device__ __forceinline__ void store_row(double* par, int i, const int64_t* row, int64_t sc, int scale, const int64_t* u) {
   uint64_t w[4];
-  map_row(i, row, sc, u, w);
+  map_row(i, row, sc, u, w, scale);
   ulonglong2* p = reinterpret_cast<ulonglong2*>(par + 4 * i);
   p[0] = make_ulonglong2(w[0], w[1]);
   p[1] = make_ulonglong2(w[2], w[3]);
@@ -363,10 +381,11 @@ __device__ __forceinline__ void store_row(double* par, int i, const int64_t* row
 __device__ __forceinline__ void collision_map(double4 s, uint32_t w, long cid, const StepArgs& a, double* par, uint64_t& ke,
                                               double& ke_rest, unsigned& errbits, bool& gfail) {
   int64_t R[9], u[3], sc;
-  if (!cell_factor(s, w, cid, a, par, sc, u, ke, ke_rest, errbits, gfail)) return;
+  int scale;
+  if (!cell_factor(s, w, cid, a, par, sc, scale, u, ke, ke_rest, errbits, gfail)) return;
   cell_rotation(cid, a, R);
 #pragma unroll
-  for (int i = 0; i < 3; ++i) store_row(par, i, R + 3 * i, sc, u);
+  for (int i = 0; i < 3; ++i) store_row(par, i, R + 3 * i, sc, scale, u);
 }
 
 // The block's sum of fixed-point energies (units of 2^-40, each thread's below
@@ -469,7 +488,7 @@ constexpr int kPairCTAs = 10;  // per SM
 __global__ void __launch_bounds__(kCellThreads, kPairCTAs) k_cell_pairs_f64(CellsF64 c, StepArgs a) {
   __shared__ BlockEnergy s_e;
   __shared__ int64_t s_R[2][3][32], s_u[2][3][32], s_sc[2][32];
-  __shared__ int s_fits[2][32];
+  __shared__ int s_fits[2][32];  // 1 + the map's scale, or 0
   energy_begin(s_e);
   chain_begin();
   const int lane = threadIdx.x & 31;
@@ -485,7 +504,7 @@ __global__ void __launch_bounds__(kCellThreads, kPairCTAs) k_cell_pairs_f64(Cell
     double* par = c.par + 12 * cid;
     int64_t R[9], u[3] = {0, 0, 0}, sc = 0;
     if (sums) {
-      int fits = 0;
+      int fits = 0, scale = 0;
       if (cid < c.ncell) {
         const uint32_t w = __ldcg(c.cnt + cid);
         const double2* p = reinterpret_cast<const double2*>(c.sum + cid);
@@ -494,7 +513,9 @@ __global__ void __launch_bounds__(kCellThreads, kPairCTAs) k_cell_pairs_f64(Cell
           c.sum[cid] = make_double4(0.0, 0.0, 0.0, 0.0);
           c.cnt[cid] = 0u;
           if (!(a.premapped && cnt_beads(w) > 0))  // else mapped by k_bead_maps_f64
-            fits = cell_factor(make_double4(lo.x, lo.y, hi.x, hi.y), w, cid, a, par, sc, u, ke, ke_rest, errbits, gfail);
+            fits = cell_factor(make_double4(lo.x, lo.y, hi.x, hi.y), w, cid, a, par, sc, scale, u, ke, ke_rest, errbits, gfail)
+                       ? 1 + scale
+                       : 0;
         }
       }
       s_fits[b][lane] = fits;
@@ -512,16 +533,17 @@ __global__ void __launch_bounds__(kCellThreads, kPairCTAs) k_cell_pairs_f64(Cell
     }
     __syncthreads();
     if (!s_fits[b][lane]) continue;
+    const int scale = s_fits[b][lane] - 1;
     if (sums) {
 #pragma unroll
       for (int q = 0; q < 3; ++q) R[q] = s_R[b][q][lane];
-      store_row(par, 0, R, sc, u);
+      store_row(par, 0, R, sc, scale, u);
     } else {
       sc = s_sc[b][lane];
 #pragma unroll
       for (int q = 0; q < 3; ++q) u[q] = s_u[b][q][lane];
-      store_row(par, 1, R + 3, sc, u);
-      store_row(par, 2, R + 6, sc, u);
+      store_row(par, 1, R + 3, sc, scale, u);
+      store_row(par, 2, R + 6, sc, scale, u);
     }
   }
   if (gfail) errbits |= kErrGammaLoop;
