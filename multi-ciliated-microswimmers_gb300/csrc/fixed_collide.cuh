@@ -260,7 +260,25 @@ MPCD_HD void apply_words(const uint64_t* w, const int64_t* v, int64_t* out) {
 
 // sum of v_i^2 in units of 2^-52, v_i in units of 2^-58 with |v_i| < 16
 constexpr int kSquareBits = 52;
-constexpr int kEnergyBits = 40;  // of the sums of kinetic energies
+// A sum of such squares, or of cells' kinetic energies in units of 2^-55: 96 bits,
+// every addend whole, so that the sum is exact whatever the number of addends.
+struct EnergySum {
+  uint64_t lo = 0;
+  uint32_t hi = 0;
+};
+MPCD_HD void energy_add(EnergySum& e, uint64_t lo, uint32_t hi) {
+  e.lo += lo;
+  e.hi += hi + (e.lo < lo ? 1u : 0u);
+}
+constexpr int kCellEnergyBits = 55;
+MPCD_HD void energy_add_cell(EnergySum& e, int64_t kin, int bits) {  // of kinetic_fixed
+  const int sh = kCellEnergyBits - bits;
+  energy_add(e, (uint64_t)kin << sh, sh ? (uint32_t)((uint64_t)kin >> (64 - sh)) : 0u);
+}
+MPCD_HD double energy_value(const EnergySum& e, int bits) {
+  const double unit = 1.0 / (double)(1ull << bits);
+  return (double)e.lo * unit + (double)e.hi * (18446744073709551616.0 * unit);
+}
 MPCD_HD int64_t square_words(Limbs x, Limbs y, Limbs z) {
   const int64_t top = wide(x.h, x.h) + wide(y.h, y.h) + wide(z.h, z.h);
   const int64_t mid = wide(x.h, x.l) + wide(y.h, y.l) + wide(z.h, z.l);

@@ -264,12 +264,12 @@ __device__ __noinline__ unsigned map_f64(const CellSums& t, long cid, float gf, 
 // 140-247) as twelve words (fixed_collide.cuh): in fixed point when the
 // cell's numbers fit, else as float64 factor, axis and mean velocity, in two
 // parts that need nothing of each other.  The cell's sum m v^2 before the
-// collision goes to the sums of ke (units of 2^-40) or ke_rest.
+// collision goes to the sums of ke or ke_rest.
 //
 // The sums' part: factor and mean velocity.  False if the cell takes the
 // float64 form, whose words it has written to par.
 __device__ __forceinline__ bool cell_factor(double4 s, uint32_t w, long cid, const StepArgs& a, double* par, int64_t& sc,
-                                            int& scale, int64_t* u, uint64_t& ke, double& ke_rest, unsigned& errbits, bool& gfail) {
+                                            int& scale, int64_t* u, EnergySum& ke, double& ke_rest, unsigned& errbits, bool& gfail) {
   const int nf = cnt_fluid(w), nb = cnt_beads(w);
   int num = nf + nb, sk = -1;
   double M = (double)num;
@@ -304,7 +304,7 @@ __device__ __forceinline__ bool cell_factor(double4 s, uint32_t w, long cid, con
   int64_t kin = 0;
   const int ebits = kinetic_fixed(s.w, kin);
   if (ebits) {
-    ke += (uint64_t)((kin + (1ll << (ebits - kEnergyBits - 1))) >> (ebits - kEnergyBits));
+    energy_add_cell(ke, kin, ebits);
   } else {
     ke_rest += s.w;
     fit = false;
@@ -378,7 +378,7 @@ __device__ __forceinline__ void store_row(double* par, int i, const int64_t* row
 }
 
 // The whole map by one thread.
-__device__ __forceinline__ void collision_map(double4 s, uint32_t w, long cid, const StepArgs& a, double* par, uint64_t& ke,
+__device__ __forceinline__ void collision_map(double4 s, uint32_t w, long cid, const StepArgs& a, double* par, EnergySum& ke,
                                               double& ke_rest, unsigned& errbits, bool& gfail) {
   int64_t R[9], u[3], sc;
   int scale;
@@ -388,10 +388,10 @@ __device__ __forceinline__ void collision_map(double4 s, uint32_t w, long cid, c
   for (int i = 0; i < 3; ++i) store_row(par, i, R + 3 * i, sc, scale, u);
 }
 
-// The block's sum of fixed-point energies (units of 2^-40, each thread's below
-// 2^58) and a float64 rest, added to *dst with the given sign by the warp that
-// comes last: no barrier at the end of a block, whose other warps would wait
-// there for the slowest (0.8 to 1.1 of 12 cycles per instruction before).
+// The block's sum of fixed-point energies (units of 2^-bits) and a float64 rest,
+// added to *dst with the given sign by the warp that comes last: no barrier at
+// the end of a block, whose other warps would wait there for the slowest (0.8 to
+// 1.1 of 12 cycles per instruction before).
 struct BlockEnergy {
   double sum;
   unsigned warps;
@@ -403,13 +403,16 @@ __device__ __forceinline__ void energy_begin(BlockEnergy& b) {
   }
   __syncthreads();
 }
-__device__ __forceinline__ void energy_end(BlockEnergy& b, uint64_t ke, double rest, double sign, double* dst) {
+__device__ __forceinline__ void energy_end(BlockEnergy& b, EnergySum ke, int bits, double rest, double sign, double* dst) {
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) ke += __shfl_xor_sync(0xffffffffu, ke, o);
+  for (int o = 16; o > 0; o >>= 1) {
+    const uint64_t lo = __shfl_xor_sync(0xffffffffu, ke.lo, o);
+    energy_add(ke, lo, __shfl_xor_sync(0xffffffffu, ke.hi, o));
+  }
   if (rest != 0.0) atomicAdd(&b.sum, rest);
   __syncwarp();
   if ((threadIdx.x & 31) == 0) {
-    atomicAdd(&b.sum, (double)ke * (1.0 / (double)(1ull << kEnergyBits)));
+    atomicAdd(&b.sum, energy_value(ke, bits));
     __threadfence_block();
     if (atomicAdd(&b.warps, 1u) == (blockDim.x >> 5) - 1) {
       __threadfence_block();
@@ -417,11 +420,6 @@ __device__ __forceinline__ void energy_end(BlockEnergy& b, uint64_t ke, double r
       if (tot != 0.0) atomicAdd(dst, sign * tot);
     }
   }
-}
-// before a thread's fixed-point sum can outgrow energy_end
-__device__ __forceinline__ void flush_ke(uint64_t& ke, double& rest) {
-  rest += (double)ke * (1.0 / (double)(1ull << kEnergyBits));
-  ke = 0;
 }
 
 // ============================================================== float64 ===
@@ -437,9 +435,8 @@ __global__ void __launch_bounds__(kCellThreads, 12) k_cell_params_f64(CellsF64 c
   __shared__ BlockEnergy s_e;
   energy_begin(s_e);
   chain_begin();
-  uint64_t ke = 0;
+  EnergySum ke;
   double ke_rest = 0.0;
-  int rounds = 0;
   unsigned errbits = 0;
   bool gfail = false;
   constexpr int kU = 2;
@@ -466,15 +463,11 @@ __global__ void __launch_bounds__(kCellThreads, 12) k_cell_params_f64(CellsF64 c
       c.cnt[cid] = 0u;
       if (a.premapped && cnt_beads(w[u]) > 0) continue;  // mapped by k_bead_maps_f64
       collision_map(sm[u], w[u], cid, a, c.par + 12 * cid, ke, ke_rest, errbits, gfail);
-      if (++rounds == (1 << 6)) {  // a cell's energy is below 2^52 units
-        flush_ke(ke, ke_rest);
-        rounds = 0;
-      }
     }
   }
   if (gfail) errbits |= kErrGammaLoop;
   if (errbits) atomicOr(a.err, errbits);
-  energy_end(s_e, ke, ke_rest, 1.0, a.diss);
+  energy_end(s_e, ke, kCellEnergyBits, ke_rest, 1.0, a.diss);
 }
 
 // The same by pairs of warps, 32 cells a CTA: one warp makes count, sums, Gamma
@@ -493,9 +486,8 @@ __global__ void __launch_bounds__(kCellThreads, kPairCTAs) k_cell_pairs_f64(Cell
   chain_begin();
   const int lane = threadIdx.x & 31;
   const bool sums = threadIdx.x < 32;  // the warp of the sums; the other makes the rotations
-  uint64_t ke = 0;
+  EnergySum ke;
   double ke_rest = 0.0;
-  int rounds = 0;
   unsigned errbits = 0;
   bool gfail = false;
   int b = 0;  // two sets of words: one barrier per round
@@ -522,10 +514,6 @@ __global__ void __launch_bounds__(kCellThreads, kPairCTAs) k_cell_pairs_f64(Cell
       s_sc[b][lane] = sc;
 #pragma unroll
       for (int q = 0; q < 3; ++q) s_u[b][q][lane] = u[q];
-      if (++rounds == (1 << 6)) {  // a cell's energy is below 2^52 units
-        flush_ke(ke, ke_rest);
-        rounds = 0;
-      }
     } else if (cid < c.ncell) {
       cell_rotation(cid, a, R);
 #pragma unroll
@@ -548,7 +536,7 @@ __global__ void __launch_bounds__(kCellThreads, kPairCTAs) k_cell_pairs_f64(Cell
   }
   if (gfail) errbits |= kErrGammaLoop;
   if (errbits) atomicOr(a.err, errbits);
-  energy_end(s_e, ke, ke_rest, 1.0, a.diss);
+  energy_end(s_e, ke, kCellEnergyBits, ke_rest, 1.0, a.diss);
 }
 
 // Walls along z (NOSLIP / SLIP, src/libcilia/mpcd.cpp:346-376): the channel is
@@ -671,9 +659,8 @@ __global__ void __launch_bounds__(kFluidThreads, 8) k_fluid_step_f64(FluidF64 f,
   __shared__ BlockEnergy s_e;
   energy_begin(s_e);
   chain_begin();
-  uint64_t ke = 0;  // sum of v'^2 in units of 2^-40, and the rest
+  EnergySum ke;  // sum of v'^2, and the rest
   double ke_rest = 0.0;
-  int rounds = 0;
   unsigned bad = 0;
   for (I i = (I)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (I)gridDim.x * blockDim.x) {
     const uint32_t cp = f.cell[i];
@@ -706,7 +693,7 @@ __global__ void __launch_bounds__(kFluidThreads, 8) k_fluid_step_f64(FluidF64 f,
     if (fit) {
       const Limbs wx = split_limbs(y[0] << 2), wy = split_limbs(y[1] << 2), wz = split_limbs(y[2] << 2);
       const int64_t k2 = square_words(wx, wy, wz);
-      ke += (uint64_t)((k2 + 2048) >> 12);
+      energy_add(ke, (uint64_t)k2, 0u);
       if (kick) {
         const int64_t yk = y[0] + a.xkick;
         K = from_fixed(square_words(split_limbs(yk << 2), wy, wz), kSquareBits);
@@ -768,10 +755,6 @@ __global__ void __launch_bounds__(kFluidThreads, 8) k_fluid_step_f64(FluidF64 f,
       oz = t.o[2];
       bad |= t.bad;
     }
-    if (++rounds == (1 << 8)) {  // a particle's energy is below 2^50 units
-      flush_ke(ke, ke_rest);
-      rounds = 0;
-    }
     // bin with the next shift
     const uint32_t cn =
         (uint32_t)shifted(ix, ox, a.xta_next[0], Lx) +
@@ -788,7 +771,7 @@ __global__ void __launch_bounds__(kFluidThreads, 8) k_fluid_step_f64(FluidF64 f,
     f.vz[i] = vz;
   }
   if (bad) atomicOr(a.err, bad);
-  energy_end(s_e, ke, ke_rest, -1.0, a.diss);
+  energy_end(s_e, ke, kSquareBits, ke_rest, -1.0, a.diss);
 }
 
 __global__ void k_bin_fluid_f64(FluidF64 f, CellsF64 c, StepArgs a) {
@@ -1603,7 +1586,7 @@ __global__ void k_gather_fluid(F f, const uint32_t* at, long d0, long d1, bool v
 __global__ void k_bead_maps_f64(MDState m, CellsF64 c, StepArgs a, uint32_t* claim, uint32_t tag) {
   __shared__ BlockEnergy s_e;
   energy_begin(s_e);
-  uint64_t ke = 0;
+  EnergySum ke;
   double ke_rest = 0.0;
   unsigned errbits = 0;
   bool gfail = false;
@@ -1618,11 +1601,10 @@ __global__ void k_bead_maps_f64(MDState m, CellsF64 c, StepArgs a, uint32_t* cla
     const uint32_t w = c.cnt[cid];
     if (w == 0) continue;
     collision_map(c.sum[cid], w, cid, a, c.par + 12 * cid, ke, ke_rest, errbits, gfail);
-    flush_ke(ke, ke_rest);
   }
   if (gfail) errbits |= kErrGammaLoop;
   if (errbits) atomicOr(a.err, errbits);
-  energy_end(s_e, ke, ke_rest, 1.0, a.diss);
+  energy_end(s_e, ke, kCellEnergyBits, ke_rest, 1.0, a.diss);
 }
 
 __global__ void k_bead_maps_f32(MDState m, CellsF32 c, StepArgs a, uint32_t* claim, uint32_t tag) {
