@@ -74,8 +74,9 @@ __device__ __forceinline__ void wrap_cell(int& i, int L) {
   }
 }
 
-// an unwrapped coordinate (any finite value below about 1e9) as cell and offset
-__device__ __forceinline__ void split_coord(double x, int L, int& i, uint64_t& o, unsigned& bad) {
+// an unwrapped coordinate (any finite value below about 1e9), counted from cell i0, as
+// cell and offset
+__device__ __forceinline__ void split_coord(double x, int L, int& i, uint64_t& o, unsigned& bad, int i0 = 0) {
   if (!(x > -1.0e9 && x < 1.0e9)) {  // non-finite: keep the particle in its cell and report
     o = kOffOne / 2;
     bad |= kErrCellRange;
@@ -89,7 +90,7 @@ __device__ __forceinline__ void split_coord(double x, int L, int& i, uint64_t& o
     i += 1;  // x was a tiny negative number: x - floor(x) rounded to 1
   else
     o = offset_from_double(d);
-  i %= L;
+  i = (i + i0) % L;
   if (i < 0) i += L;
 }
 
@@ -101,7 +102,8 @@ __device__ __forceinline__ void stream_coord(int& i, uint64_t& o, double v, cons
     i += c;
     wrap_cell(i, L);
   } else {
-    split_coord((double)i + fma(v, a.h, offset_to_double(o)), L, i, o, bad);
+    const int i0 = i;  // the offset alone: added to a cell index it would lose the index's bits
+    split_coord(fma(v, a.h, offset_to_double(o)), L, i, o, bad, i0);
   }
 }
 
