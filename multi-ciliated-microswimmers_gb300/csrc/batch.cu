@@ -1250,7 +1250,8 @@ int mpcd_batch_get_beads(mpcd_batch* b, int r, long nb, double* pos, double* vel
       BK(cudaHostAlloc((void**)&b->h_beads, 6 * kPinnedBeads * sizeof(double), cudaHostAllocMapped | cudaHostAllocPortable));
     double* d = nullptr;
     BK(cudaHostGetDevicePointer((void**)&d, b->h_beads, 0));
-    b->launches_total += launch_store_beads(b->md, s0, nb, d, d + 3 * nb, nullptr, nullptr, b->s0);
+    BK(launch_store_beads(b->md, s0, nb, d, d + 3 * nb, nullptr, nullptr, b->s0));
+    ++b->launches_total;
     BK(cudaStreamSynchronize(b->s0));
     if (pos) std::memcpy(pos, b->h_beads, bytes);
     if (vel) std::memcpy(vel, b->h_beads + 3 * nb, bytes);
@@ -1264,7 +1265,8 @@ int mpcd_batch_get_beads(mpcd_batch* b, int r, long nb, double* pos, double* vel
     b->beads_cap = nb;
   }
   double *dpos = b->d_beads, *dvel = dpos + 3 * (size_t)nb;
-  b->launches_total += launch_store_beads(b->md, s0, nb, dpos, dvel, nullptr, nullptr, b->s0);
+  BK(launch_store_beads(b->md, s0, nb, dpos, dvel, nullptr, nullptr, b->s0));
+  ++b->launches_total;
   touch_pages(pos, bytes);
   touch_pages(vel, bytes);
   if (pos) BK(cudaMemcpyAsync(pos, dpos, bytes, cudaMemcpyDeviceToHost, b->s0));

@@ -1041,7 +1041,8 @@ int read_fluid(mpcd_engine* h, const F& f, double* pos, double* vel) {
     return cudaMemcpyAsync(to + 3 * d0, from + 3 * d0, 3 * (size_t)(d1 - d0) * sizeof(double), cudaMemcpyDeviceToHost, s);
   };
   if (n < kPartsMin) {
-    h->launches += launch_store_fluid(f, dpos, dvel, h->d_status, h->d_err, h->stream);
+    CK(launch_store_fluid(f, dpos, dvel, h->d_status, h->d_err, h->stream));
+    ++h->launches;
     if (pos) CK(copy(pos, dpos, 0, n, h->stream));
     if (vel) CK(copy(vel, dvel, 0, n, h->stream));
     return MPCD_OK;
@@ -1049,7 +1050,8 @@ int read_fluid(mpcd_engine* h, const F& f, double* pos, double* vel) {
   if (!h->scopy) CK(cudaStreamCreateWithFlags(&h->scopy, cudaStreamNonBlocking));
   for (cudaEvent_t& ev : h->ev_part)
     if (!ev) CK(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
-  h->launches += launch_find_particles(f, h->d_rank, h->d_status, h->d_err, h->stream);
+  CK(launch_find_particles(f, h->d_rank, h->d_status, h->d_err, h->stream));
+  ++h->launches;
   // a small part first, so that the copies begin early
   struct Part {
     bool velocity;
@@ -1059,8 +1061,8 @@ int read_fluid(mpcd_engine* h, const F& f, double* pos, double* vel) {
   int k = 0;
   for (const Part& p : parts) {
     if (p.velocity ? !vel : !pos) continue;
-    h->launches +=
-        launch_gather_fluid(f, h->d_rank, p.d0, p.d1, p.velocity, p.velocity ? dvel : dpos, h->d_status, h->stream);
+    CK(launch_gather_fluid(f, h->d_rank, p.d0, p.d1, p.velocity, p.velocity ? dvel : dpos, h->d_status, h->stream));
+    ++h->launches;
     CK(cudaEventRecord(h->ev_part[k++], h->stream));
   }
   k = 0;
@@ -1164,7 +1166,8 @@ int mpcd_get_beads(mpcd_engine* h, long nb, double* pos, double* vel) {
       CK(cudaHostAlloc((void**)&h->h_beads, 6 * kPinnedBeads * sizeof(double), cudaHostAllocMapped | cudaHostAllocPortable));
     double* d = nullptr;
     CK(cudaHostGetDevicePointer((void**)&d, h->h_beads, 0));
-    h->launches += launch_store_beads(h->md, 0, nb, d, d + 3 * nb, h->d_status, h->d_err, h->stream);
+    CK(launch_store_beads(h->md, 0, nb, d, d + 3 * nb, h->d_status, h->d_err, h->stream));
+    ++h->launches;
     CK(cudaStreamSynchronize(h->stream));
     if (pos) std::memcpy(pos, h->h_beads, bytes);
     if (vel) std::memcpy(vel, h->h_beads + 3 * nb, bytes);
@@ -1172,7 +1175,8 @@ int mpcd_get_beads(mpcd_engine* h, long nb, double* pos, double* vel) {
   }
   if (int rc = stage_buffer(h, nb)) return rc;
   double *dpos = h->d_stage, *dvel = dpos + 3 * (size_t)nb;
-  h->launches += launch_store_beads(h->md, 0, nb, dpos, dvel, h->d_status, h->d_err, h->stream);
+  CK(launch_store_beads(h->md, 0, nb, dpos, dvel, h->d_status, h->d_err, h->stream));
+  ++h->launches;
   touch_pages(pos, bytes);
   touch_pages(vel, bytes);
   if (pos) CK(cudaMemcpyAsync(pos, dpos, bytes, cudaMemcpyDeviceToHost, h->stream));

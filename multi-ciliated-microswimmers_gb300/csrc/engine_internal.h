@@ -336,9 +336,11 @@ inline void touch_pages(void* p, size_t bytes) {
   for (size_t i = 0; i < bytes; i += 4096) c[i] = 0;
   if (bytes) c[bytes - 1] = 0;
 }
+// The read-backs' kernels; a launch that was refused leaves no trace in what is
+// read, so that these say so themselves.
 // positions and velocities of the nb beads whose slots begin at s0, in bead
 // order; status may be null
-int launch_store_beads(const MDState& m, long s0, long nb, double* pos, double* vel, unsigned* status,
+cudaError_t launch_store_beads(const MDState& m, long s0, long nb, double* pos, double* vel, unsigned* status,
                        const unsigned* err, cudaStream_t s);
 // Swimmers of up to this many beads are read through pinned host memory that
 // the kernel writes and the host copies from, larger ones by two copies of the
@@ -347,11 +349,11 @@ int launch_store_beads(const MDState& m, long s0, long nb, double* pos, double* 
 constexpr long kPinnedBeads = 3072;
 // read-back into the caller's order (status: {bad id, error word} in host memory)
 template <typename F>
-int launch_store_fluid(const F& f, double* pos, double* vel, unsigned* status, const unsigned* err, cudaStream_t s);
+cudaError_t launch_store_fluid(const F& f, double* pos, double* vel, unsigned* status, const unsigned* err, cudaStream_t s);
 template <typename F>
-int launch_find_particles(const F& f, uint32_t* at, unsigned* status, const unsigned* err, cudaStream_t s);
+cudaError_t launch_find_particles(const F& f, uint32_t* at, unsigned* status, const unsigned* err, cudaStream_t s);
 template <typename F>
-int launch_gather_fluid(const F& f, const uint32_t* at, long d0, long d1, bool velocity, double* out, unsigned* status,
+cudaError_t launch_gather_fluid(const F& f, const uint32_t* at, long d0, long d1, bool velocity, double* out, unsigned* status,
                         cudaStream_t s);
 // observables from the binned cell sums (float64 path; valid while the sums
 // are those of the last binning): out[10], part[7 * kObsBlocks], counter zeroed once

@@ -1739,7 +1739,7 @@ int launch_spheres_update(RigidSphereDev* sph, int n, double* acc, double* fsum,
 // channel 37.7 to 36.0, 80 x 71 x 89 232 to 227.  Not beside an MD launch, where an
 // event lies between the two.
 template <typename... P, typename... A>
-void launch_in_chain(void (*kernel)(P...), int grid, int threads, cudaStream_t s, bool chained, const A&... args) {
+cudaError_t launch_in_chain(void (*kernel)(P...), int grid, int threads, cudaStream_t s, bool chained, const A&... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(threads);
@@ -1749,7 +1749,7 @@ void launch_in_chain(void (*kernel)(P...), int grid, int threads, cudaStream_t s
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = chained ? 1 : 0;
-  cudaLaunchKernelEx(&cfg, kernel, args...);
+  return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
 int launch_collision_draws(int nc, uint64_t seed, uint64_t step, long n, double* gamma, double* axis, unsigned* err,
@@ -1946,33 +1946,28 @@ int launch_convert_offsets(long n, uint64_t* o, bool integers, cudaStream_t s) {
   k_convert_offsets<<<grid_for(n), kThreads, 0, s>>>(n, o, integers);
   return 1;
 }
-int launch_store_beads(const MDState& m, long s0, long nb, double* pos, double* vel, unsigned* status,
+cudaError_t launch_store_beads(const MDState& m, long s0, long nb, double* pos, double* vel, unsigned* status,
                        const unsigned* err, cudaStream_t s) {
-  k_store_beads<<<grid_for(3 * nb, 128), 128, 0, s>>>(m, s0, (int)nb, pos, vel, status, err);
-  return 1;
+  return launch_in_chain(k_store_beads, grid_for(3 * nb, 128), 128, s, false, m, s0, (int)nb, pos, vel, status, err);
 }
 template <typename F>
-int launch_store_fluid(const F& f, double* pos, double* vel, unsigned* status, const unsigned* err, cudaStream_t s) {
-  if (f.n == 0) return 0;
-  launch_in_chain(k_store_fluid<F>, grid_for(f.n), kThreads, s, true, f, pos, vel, status, err);
-  return 1;
+cudaError_t launch_store_fluid(const F& f, double* pos, double* vel, unsigned* status, const unsigned* err, cudaStream_t s) {
+  return launch_in_chain(k_store_fluid<F>, grid_for(f.n), kThreads, s, true, f, pos, vel, status, err);
 }
 template <typename F>
-int launch_find_particles(const F& f, uint32_t* at, unsigned* status, const unsigned* err, cudaStream_t s) {
-  launch_in_chain(k_find_particles<F>, grid_for(f.n, kThreads, 8), kThreads, s, true, f, at, status, err);
-  return 1;
+cudaError_t launch_find_particles(const F& f, uint32_t* at, unsigned* status, const unsigned* err, cudaStream_t s) {
+  return launch_in_chain(k_find_particles<F>, grid_for(f.n, kThreads, 8), kThreads, s, true, f, at, status, err);
 }
 template <typename F>
-int launch_gather_fluid(const F& f, const uint32_t* at, long d0, long d1, bool velocity, double* out, unsigned* status,
+cudaError_t launch_gather_fluid(const F& f, const uint32_t* at, long d0, long d1, bool velocity, double* out, unsigned* status,
                         cudaStream_t s) {
-  if (d1 <= d0) return 0;
-  k_gather_fluid<<<grid_for(d1 - d0, kThreads, 8), kThreads, 0, s>>>(f, at, d0, d1, velocity, out, status);
-  return 1;
+  return launch_in_chain(k_gather_fluid<F>, grid_for(d1 - d0, kThreads, 8), kThreads, s, false, f, at, d0, d1, velocity, out,
+                         status);
 }
 #define MPCD_READ_BACK(F)                                                                                        \
-  template int launch_store_fluid(const F&, double*, double*, unsigned*, const unsigned*, cudaStream_t);         \
-  template int launch_find_particles(const F&, uint32_t*, unsigned*, const unsigned*, cudaStream_t);             \
-  template int launch_gather_fluid(const F&, const uint32_t*, long, long, bool, double*, unsigned*, cudaStream_t)
+  template cudaError_t launch_store_fluid(const F&, double*, double*, unsigned*, const unsigned*, cudaStream_t);         \
+  template cudaError_t launch_find_particles(const F&, uint32_t*, unsigned*, const unsigned*, cudaStream_t);             \
+  template cudaError_t launch_gather_fluid(const F&, const uint32_t*, long, long, bool, double*, unsigned*, cudaStream_t)
 MPCD_READ_BACK(FluidF64);
 MPCD_READ_BACK(FluidF32);
 #undef MPCD_READ_BACK
