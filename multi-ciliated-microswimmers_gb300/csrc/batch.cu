@@ -510,6 +510,13 @@ std::string plan_replica(mpcd_batch* b, Replica& R) {
 int upload_md(mpcd_batch* b, int r, Replica& R) {
   const MDPlan& pl = R.plan;
   MDState& m = b->md;
+  if (R.nb > kPinnedBeads && b->beads_cap < R.nb) {  // what its read-back uses
+    cudaFree(b->d_beads);
+    b->d_beads = nullptr;
+    b->beads_cap = 0;
+    BK(cudaMalloc((void**)&b->d_beads, 6 * (size_t)R.nb * sizeof(double)));
+    b->beads_cap = R.nb;
+  }
   if (pl.ntiles > 0) {
     const long sb = R.tile0 * (long)b->T;
     const long ns = pl.nslots;
@@ -678,6 +685,9 @@ int mpcd_batch_create(const mpcd_batch_params* params, mpcd_batch** out) {
     if ((e = cudaEventCreateWithFlags(&b->ev_join[g], cudaEventDisableTiming)) != cudaSuccess) return bail(e, "event");
   }
   if ((e = cudaEventCreateWithFlags(&b->ev_fork, cudaEventDisableTiming)) != cudaSuccess) return bail(e, "event");
+  if ((e = cudaHostAlloc((void**)&b->h_beads, 6 * kPinnedBeads * sizeof(double),
+                         cudaHostAllocMapped | cudaHostAllocPortable)) != cudaSuccess)
+    return bail(e, "alloc");
   b->npart_pages = (p.max_particles + kPartPage - 1) / kPartPage;
   b->ncell_pages = (p.max_cells + kCellPage - 1) / kCellPage;
   b->part_cap = b->npart_pages * kPartPage;
@@ -1246,8 +1256,6 @@ int mpcd_batch_get_beads(mpcd_batch* b, int r, long nb, double* pos, double* vel
   const size_t bytes = 3 * (size_t)nb * sizeof(double);
   const long s0 = R->tile0 * (long)b->T;
   if (nb <= kPinnedBeads) {
-    if (!b->h_beads)
-      BK(cudaHostAlloc((void**)&b->h_beads, 6 * kPinnedBeads * sizeof(double), cudaHostAllocMapped | cudaHostAllocPortable));
     double* d = nullptr;
     BK(cudaHostGetDevicePointer((void**)&d, b->h_beads, 0));
     BK(launch_store_beads(b->md, s0, nb, d, d + 3 * nb, nullptr, nullptr, b->s0));
@@ -1256,13 +1264,6 @@ int mpcd_batch_get_beads(mpcd_batch* b, int r, long nb, double* pos, double* vel
     if (pos) std::memcpy(pos, b->h_beads, bytes);
     if (vel) std::memcpy(vel, b->h_beads + 3 * nb, bytes);
     return MPCD_OK;
-  }
-  if (b->beads_cap < nb) {
-    cudaFree(b->d_beads);
-    b->d_beads = nullptr;
-    b->beads_cap = 0;
-    BK(cudaMalloc((void**)&b->d_beads, 6 * (size_t)nb * sizeof(double)));
-    b->beads_cap = nb;
   }
   double *dpos = b->d_beads, *dvel = dpos + 3 * (size_t)nb;
   BK(launch_store_beads(b->md, s0, nb, dpos, dvel, nullptr, nullptr, b->s0));

@@ -273,7 +273,17 @@ void free_md(MDState& m) {
   m.bar = bar;
 }
 
+// Fluids of at least this many particles are read in parts, each copied while
+// the next is gathered (64^3 x 10: 0.92 to 0.78 ms, 80 x 71 x 89 x 10: 1.86 to 1.49 of
+// which 1.3 are the link; 32^3 x 10 0.136 instead of 0.130: one launch below)
+constexpr long kPartsMin = 1l << 20;
+
 int alloc_fluid(mpcd_engine* h, long n) {
+  if (n >= kPartsMin) {  // what the read-back in parts uses
+    if (!h->scopy) CK(cudaStreamCreateWithFlags(&h->scopy, cudaStreamNonBlocking));
+    for (cudaEvent_t& ev : h->ev_part)
+      if (!ev) CK(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+  }
   // the same particle count: the arrays are kept (the load rewrites every one)
   const bool f64 = h->p.precision == MPCD_FP64;
   if (h->d_rank && (f64 ? (h->f64.id && h->f64tmp.id && h->f64.n == n && h->f64tmp.n == n)
@@ -353,6 +363,18 @@ int check_launch(mpcd_engine* h, const char* what) {
   return MPCD_OK;
 }
 
+int stage_buffer(mpcd_engine* h, long n) {
+  const size_t need = 6 * (size_t)(n > 0 ? n : 1);
+  if (need > h->stage_cap) {
+    cudaFree(h->d_stage);
+    h->d_stage = nullptr;
+    h->stage_cap = 0;
+    CK(dalloc(&h->d_stage, need));
+    h->stage_cap = need;
+  }
+  return MPCD_OK;
+}
+
 // Build the MD device layout (md_plan.cu plans it on the host; this uploads
 // it into freshly allocated device arrays).
 int build_md(mpcd_engine* h) {
@@ -361,6 +383,12 @@ int build_md(mpcd_engine* h) {
   if (h->nb == 0) {
     h->md_dirty = false;
     return MPCD_OK;
+  }
+  // what the bead read-back uses
+  if (h->nb > kPinnedBeads) {
+    if (int rc = stage_buffer(h, h->nb)) return rc;
+  } else if (!h->h_beads) {
+    CK(cudaHostAlloc((void**)&h->h_beads, 6 * kPinnedBeads * sizeof(double), cudaHostAllocMapped | cudaHostAllocPortable));
   }
   MDInput in;
   in.nb = h->nb;
@@ -976,17 +1004,6 @@ struct Staging {
   double* d = nullptr;
   unsigned* flag = nullptr;
 };
-int stage_buffer(mpcd_engine* h, long n) {
-  const size_t need = 6 * (size_t)(n > 0 ? n : 1);
-  if (need > h->stage_cap) {
-    cudaFree(h->d_stage);
-    h->d_stage = nullptr;
-    h->stage_cap = 0;
-    CK(dalloc(&h->d_stage, need));
-    h->stage_cap = need;
-  }
-  return MPCD_OK;
-}
 int staging(mpcd_engine* h, long n, Staging& st) {
   if (int rc = stage_buffer(h, n)) return rc;
   if (!h->d_stage_flag) CK(dalloc(&h->d_stage_flag, 1));
@@ -1027,11 +1044,6 @@ int mpcd_set_fluid(mpcd_engine* h, long n, const double* pos, const double* vel)
 
 }  // extern "C"
 namespace {
-// Fluids of at least this many particles are read in parts, each copied while
-// the next is gathered (64^3 x 10: 0.92 to 0.78 ms, 80 x 71 x 89 x 10: 1.86 to 1.49 of
-// which 1.3 are the link; 32^3 x 10 0.136 instead of 0.130: one launch below)
-constexpr long kPartsMin = 1l << 20;
-
 template <typename F>
 int read_fluid(mpcd_engine* h, const F& f, double* pos, double* vel) {
   const long n = f.n;
@@ -1047,9 +1059,6 @@ int read_fluid(mpcd_engine* h, const F& f, double* pos, double* vel) {
     if (vel) CK(copy(vel, dvel, 0, n, h->stream));
     return MPCD_OK;
   }
-  if (!h->scopy) CK(cudaStreamCreateWithFlags(&h->scopy, cudaStreamNonBlocking));
-  for (cudaEvent_t& ev : h->ev_part)
-    if (!ev) CK(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
   CK(launch_find_particles(f, h->d_rank, h->d_status, h->d_err, h->stream));
   ++h->launches;
   // a small part first, so that the copies begin early
@@ -1162,8 +1171,6 @@ int mpcd_get_beads(mpcd_engine* h, long nb, double* pos, double* vel) {
   const size_t bytes = 3 * (size_t)nb * sizeof(double);
   h->h_status[0] = h->h_status[1] = 0u;
   if (nb <= kPinnedBeads) {
-    if (!h->h_beads)
-      CK(cudaHostAlloc((void**)&h->h_beads, 6 * kPinnedBeads * sizeof(double), cudaHostAllocMapped | cudaHostAllocPortable));
     double* d = nullptr;
     CK(cudaHostGetDevicePointer((void**)&d, h->h_beads, 0));
     CK(launch_store_beads(h->md, 0, nb, d, d + 3 * nb, h->d_status, h->d_err, h->stream));
@@ -1173,7 +1180,6 @@ int mpcd_get_beads(mpcd_engine* h, long nb, double* pos, double* vel) {
     if (vel) std::memcpy(vel, h->h_beads + 3 * nb, bytes);
     return report_error(h, h->h_status[1]);
   }
-  if (int rc = stage_buffer(h, nb)) return rc;
   double *dpos = h->d_stage, *dvel = dpos + 3 * (size_t)nb;
   CK(launch_store_beads(h->md, 0, nb, dpos, dvel, h->d_status, h->d_err, h->stream));
   ++h->launches;
