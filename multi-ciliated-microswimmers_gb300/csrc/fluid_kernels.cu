@@ -118,32 +118,10 @@ constexpr InvTable make_inv_table() {
 }
 __device__ const InvTable g_inv_n = make_inv_table();
 
-// Free-running rotation axis of the float64 path: the direction drawn in
-// float (cos theta = 2u - 1, phi = 2 pi u', as generate_collision_matrix,
-// src/libcilia/mpcd.cpp:269-284), normalised in float64 so that the rotation
-// is orthogonal to float64 precision.  |r|^2 = 1 + e with |e| of a few float
-// roundings: two Newton steps for 1/sqrt from 1 (y1 = 1.5 - n2/2 is within
-// 3e^2/8, y2 within float64 rounding) on the FMA chain instead of the general
-// reciprocal square root.
-__device__ __forceinline__ void draw_axis_f64(uint64_t seed, uint64_t step, uint32_t cid, double& rx, double& ry,
-                                              double& rz) {
-  const u32x4 r = draw4(seed, step, kStreamCell, cid, 0u);
-  const float ct = 2.0f * u01_flt(r.y) - 1.0f;
-  const float st = sqrtf(fmaxf(0.0f, 1.0f - ct * ct));
-  float sp, cp;
-  sincospif(2.0f * u01_flt(r.x), &sp, &cp);
-  rx = (double)(st * cp);
-  ry = (double)(st * sp);
-  rz = (double)ct;
-  const double n2 = fma(rx, rx, fma(ry, ry, rz * rz));
-  const double y1 = fma(-0.5, n2, 1.5);
-  const double y2 = y1 * fma(-0.5, (n2 * y1) * y1, 1.5);
-  rx *= y2;
-  ry *= y2;
-  rz *= y2;
-}
-
-// the same direction in units of 2^-60
+// Free-running rotation axis of the float64 path in units of 2^-60: the direction
+// drawn in float (cos theta = 2u - 1, phi = 2 pi u', as generate_collision_matrix,
+// src/libcilia/mpcd.cpp:269-284), normalised to more than float64 precision so that
+// the rotation is orthogonal to it.
 __device__ __forceinline__ void draw_axis_fixed(uint64_t seed, uint64_t step, uint32_t cid, int64_t* r) {
   const u32x4 q = draw4(seed, step, kStreamCell, cid, 0u);
   const float ct = 2.0f * u01_flt(q.y) - 1.0f;
@@ -154,6 +132,15 @@ __device__ __forceinline__ void draw_axis_fixed(uint64_t seed, uint64_t step, ui
   r[1] = axis_fixed(st * sp);
   r[2] = axis_fixed(ct);
   axis_normalise(r);
+}
+// the same axis as the nearest float64 numbers
+__device__ __forceinline__ void draw_axis_f64(uint64_t seed, uint64_t step, uint32_t cid, double& rx, double& ry,
+                                              double& rz) {
+  int64_t r[3];
+  draw_axis_fixed(seed, step, cid, r);
+  rx = from_fixed(r[0], kAxisBits);
+  ry = from_fixed(r[1], kAxisBits);
+  rz = from_fixed(r[2], kAxisBits);
 }
 
 // The thermostat factor sqrt(g / (erel / 2)) = 2g / sqrt(2g erel): one
