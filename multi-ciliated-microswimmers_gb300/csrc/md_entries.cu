@@ -23,16 +23,16 @@
 // The chain of one substep: packets arrive -> one entry -> a bead's sum ->
 // Verlet -> packets leave.  The entries between the tile's own beads are
 // evaluated by the first warps while the last warps poll.  The launch is
-// latency bound (51 dependent evaluations of about 2.7 us; issue slots, pipes
+// latency bound (51 dependent evaluations of about 2.6 us; issue slots, pipes
 // and DRAM mostly idle): a packet takes 250-600 ns from one SM to another,
 // an entry about 0.4 us, a bead's sum and Verlet step 0.4 us, and the round of
 // the sphere centre's tile (its 642 beads' packets, written elsewhere since the
-// last read, take about 0.9 us to fetch, its sum's last tree 0.12) alternates
+// last read, take about 0.9 us to fetch) alternates
 // with the patches' rounds.
 //
-// MD per launch timed alone, this kernel / md_df.cu: swimmer64 146 / 217 us in
-// double-float, 134 / 196 with float springs; a 700-bead swimmer 135 / 187;
-// swimmer128 with float springs 227 / 431 (there a tile of 256 slots has two
+// MD per launch timed alone, this kernel / md_df.cu: swimmer64 138 / 217 us in
+// double-float, 127 / 196 with float springs; a 700-bead swimmer 133 / 187;
+// swimmer128 with float springs 223 / 431 (there a tile of 256 slots has two
 // lanes per slot, and its springs follow one another; here 152 tiles of three
 // cilia or 151 sphere beads).  Running sums of the entries in any order took
 // 122, 114, 117 and 213 us.
@@ -209,30 +209,37 @@ __device__ __forceinline__ void slot_sum(int lanes, const float2* F, int step, i
   else
     lane_sums<2 / HALVES, kFloat>(F, step, lanes * step, rows, h, l);
 }
-// The sums of three components over a warp by md_df.cu's xor tree (16 first, every lane
-// adding its partner's value to its own) as lane `src` ends with them.  Only the
-// lanes on src's side of a level count for the next one: the others take a
-// component over, added from src's side.  x ends in lane src, y in src ^ 8, z in
-// src ^ 16.
-__device__ __forceinline__ void shfl_acc(float& h, float& l, float gh, float gl, bool first, int o) {
-  const float bh = __shfl_xor_sync(0xffffffffu, gh, o), bl = __shfl_xor_sync(0xffffffffu, gl, o);
-  float al = first ? l : bl;
-  df_acc(h, al, bh, first ? bl : l);  // the high parts' sum and its error do not depend on the order
-  l = al;
-}
-__device__ __forceinline__ void warp_tree(const float (&s)[6], int lane, int src, float& h, float& l) {
-  const bool a = ((lane ^ src) & 16) == 0, b = ((lane ^ src) & 8) == 0;
-  // src's half adds x and y, the other z
-  float xh = a ? s[0] : s[4], xl = a ? s[1] : s[5], yh = s[2], yl = s[3];
-  shfl_acc(xh, xl, a ? s[4] : s[0], a ? s[5] : s[1], a, 16);
-  shfl_acc(yh, yl, s[2], s[3], true, 16);
-  // src's quarter goes on with x, its neighbour with y
-  const bool y = a && !b;
-  h = y ? yh : xh;
-  l = y ? yl : xl;
-  shfl_acc(h, l, !a ? xh : (y ? xh : yh), !a ? xl : (y ? xl : yl), !y, 8);
+// The sum of n slots' sums w[0 .. n) as a warp of md_df.cu makes it (lane l adds l,
+// l + 32, ... and the lanes are combined by a xor tree, 16 first, each adding its
+// partner's value to its own), as its lane `src` ends with it.  By the eight lanes
+// of a group: t stands for the four of that warp's lanes whose low bits are src's xor t.
+// The sum is in the group's lane 0.
+__device__ __forceinline__ void slots_tree(const float2* w, int n, int src, int t, float& h, float& l) {
+  const int c = src ^ t;
+  auto strided = [&](int k, float& sh, float& sl) {
+    sh = sl = 0.f;
+    if (k < n) {
+      sh = w[k].x;
+      sl = w[k].y;
+    }
+#pragma unroll 1
+    for (k += 32; k < n; k += 32) df_acc(sh, sl, w[k].x, w[k].y);
+  };
+  float ah, al, bh, bl, ch, cl, dh, dl;
+  strided(c, ah, al);
+  strided(c ^ 16, bh, bl);
+  strided(c ^ 8, ch, cl);
+  strided(c ^ 24, dh, dl);
+  df_acc(ah, al, bh, bl);
+  df_acc(ch, cl, dh, dl);
+  df_acc(ah, al, ch, cl);
 #pragma unroll
-  for (int o = 4; o > 0; o >>= 1) shfl_acc(h, l, h, l, true, o);
+  for (int o = 4; o > 0; o >>= 1) {
+    const float oh = __shfl_xor_sync(0xffffffffu, ah, o), ol = __shfl_xor_sync(0xffffffffu, al, o);
+    df_acc(ah, al, oh, ol);
+  }
+  h = ah;
+  l = al;
 }
 
 // md_df.cu adds the slots of a bead with more than this many by a warp's tree,
@@ -318,7 +325,7 @@ __device__ void md_entries_body(const MDState& m, const MDStepArgs& a, Bin bin) 
 #pragma unroll
   for (int j = 0; j < NC; ++j) {
     const int c = tid / HALVES + j * nthr;
-    ck[j] = solo ? c : c / T;  // a solo tile's bead: the first warp
+    ck[j] = solo ? ((tid & 7) || j ? 3 : tid >> 3) : c / T;  // a solo tile's bead: lanes 0, 8, 16
     cq[j] = solo ? 0 : c - ck[j] * T;
     cmv[j] = ck[j] < 3 ? m.moves[base + cq[j]] : -1;  // 1 moves, 0 fixed, -1 none
   }
@@ -499,6 +506,10 @@ __device__ void md_entries_body(const MDState& m, const MDStepArgs& a, Bin bin) 
     Packet d[6];
     uint2 sc1 = make_uint2(0, 0), sc2 = sc1;
     if (solo && tid >= 32 && si < nent) {
+      // not at once: the polls' loads stand in the way of the first warp's shared
+      // memory and shuffles (64^3 swimmer 143 to 138 us per launch, with float springs 133
+      // to 127; 130 ns and more 142, 127)
+      __nanosleep(80);
       sc1 = s_code[si];
       sc2 = s_code[si2];
       receive_two(m.qp[e & 1], m.nslots, a.tag0 + (uint32_t)e, s_hslot[(int)(sc1.x >> 16) - T],
@@ -636,33 +647,21 @@ __device__ void md_entries_body(const MDState& m, const MDStepArgs& a, Bin bin) 
     // slots and warps sum it, then the Verlet step
     const bool last = e == a.n;
     const dfloat c = e == 0 || last ? dt2 : dt;
-    float ssum[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    float ssh = 0.f, ssl = 0.f;  // a solo tile's coordinate tid / 8, in lanes 0, 8 and 16
     if (solo && warp == 0) {
-      const bool tree = solo_slots > kTreeRun;
-      const int k0 = tree ? lane32 : 0, kstep = tree ? 32 : 1;
-      for (int k = k0; k < solo_slots; k += kstep) {
-#pragma unroll
-        for (int q = 0; q < 3; ++q) {
-          const float2 p = s_fx[q * fw + solo_slots * lanes * wmax + k];
-          df_acc(ssum[2 * q], ssum[2 * q + 1], p.x, p.y);
-        }
-      }
-      __syncwarp();
-      if (tree) {
-        float h, l;
-        warp_tree(ssum, lane32, solo_src, h, l);
-        // the owner of a coordinate fetches it
-        const int from = ck[0] < 3 ? solo_src ^ (8 * ck[0]) : lane32;  // x, y, z: src, src ^ 8, src ^ 16
-        ssum[0] = ssum[2] = ssum[4] = __shfl_sync(0xffffffffu, h, from);
-        ssum[1] = ssum[3] = ssum[5] = __shfl_sync(0xffffffffu, l, from);
+      const float2* w = s_fx + min(lane32 >> 3, 2) * fw + lanes * wmax * solo_slots;
+      if (solo_slots > kTreeRun) {
+        slots_tree(w, solo_slots, solo_src, lane32 & 7, ssh, ssl);
+      } else {
+        for (int k = 0; k < solo_slots; ++k) df_acc(ssh, ssl, w[k].x, w[k].y);
       }
     }
 #pragma unroll
     for (int j = 0; j < NC; ++j) {
       float th = 0.f, tl = 0.f;
       if (solo) {
-        th = ck[j] == 0 ? ssum[0] : (ck[j] == 1 ? ssum[2] : ssum[4]);
-        tl = ck[j] == 0 ? ssum[1] : (ck[j] == 1 ? ssum[3] : ssum[5]);
+        th = ssh;
+        tl = ssl;
       } else {
         const float2* F = s_fx + fat[j];
         uint32_t shape = fshape[j];
