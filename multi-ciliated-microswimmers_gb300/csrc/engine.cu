@@ -475,14 +475,9 @@ int build_md(mpcd_engine* h) {
   CK(dalloc(&m.vz, ns));
   CK(dalloc(&m.moves, ns));
   CK(dalloc(&m.slot_of, ns));
-  CK(dalloc(&m.prim, ns));
-  CK(dalloc(&m.nhelp, ns));
-  CK(dalloc(&m.tile_help, m.ntiles));
-  CK(dalloc(&m.sp_start, ns + 1));
   CK(dalloc(&m.halo, pl.halo.size()));
   CK(dalloc(&m.halo_start, m.ntiles + 1));
   CK(dalloc(&m.diag, nbond));
-  CK(dalloc(&m.tile_react, m.ntiles));
   m.ncil = (int)ncil;
   CK(dalloc(&m.cil, ncil));
   CK(dalloc(&m.midpnt, ncil));
@@ -501,11 +496,19 @@ int build_md(mpcd_engine* h) {
   CK(up(m.vz, pl.VZ.data(), ns * 8));
   CK(up(m.moves, pl.mv.data(), ns * 4));
   CK(up(m.slot_of, pl.slot_of.data(), pl.slot_of.size() * 4));
-  CK(up(m.prim, pl.prim.data(), ns * 4));
-  CK(up(m.nhelp, pl.nhelp.data(), ns * 4));
-  CK(up(m.tile_help, pl.thelp.data(), m.ntiles * 4));
-  CK(up(m.sp_start, pl.start.data(), (ns + 1) * 4));
-  if (nspk && !m.de) {  // the entries kernel keeps them in its own tables
+  if (!m.de) {  // slots and springs; the entries kernel has tables of its own
+    CK(dalloc(&m.prim, ns));
+    CK(dalloc(&m.nhelp, ns));
+    CK(dalloc(&m.tile_help, m.ntiles));
+    CK(dalloc(&m.sp_start, ns + 1));
+    CK(dalloc(&m.tile_react, m.ntiles));
+    CK(up(m.prim, pl.prim.data(), ns * 4));
+    CK(up(m.nhelp, pl.nhelp.data(), ns * 4));
+    CK(up(m.tile_help, pl.thelp.data(), m.ntiles * 4));
+    CK(up(m.sp_start, pl.start.data(), (ns + 1) * 4));
+    CK(up(m.tile_react, pl.tile_react.data(), m.ntiles * 4));
+  }
+  if (nspk && !m.de) {
     CK(dalloc(&m.sp_other, nspk));
     CK(dalloc(&m.sp_local, nspk));
     CK(dalloc(&m.sp_kind, nspk));
@@ -519,7 +522,6 @@ int build_md(mpcd_engine* h) {
     CK(up(m.sp_rest, pl.srest.data(), nspk * 8));
     CK(up(m.sp_m2k, pl.sm2k.data(), nspk * 8));
   }
-  CK(up(m.tile_react, pl.tile_react.data(), m.ntiles * 4));
   if (ncil) {
     CK(up(m.cil, pl.cd.data(), ncil * sizeof(CiliumDev)));
     CK(up(m.midpnt, pl.mid.data(), ncil * 8));
