@@ -46,6 +46,14 @@ MPCD_HD uint64_t mul_hi64(uint64_t a, uint64_t b) {
 #endif
 }
 
+// The bits of the float nearest to x (ties to even, as a conversion rounds), for
+// 2^-100 <= x < 2^100: the conversion itself is a float64 instruction.
+MPCD_HD uint32_t nearest_float_bits(double x) {
+  const uint64_t u = f64_bits(x);
+  const uint64_t w = u + 0x0fffffffu + ((u >> 29) & 1u);
+  return (uint32_t)((w - (896ull << 52)) >> 29);
+}
+
 // o in [0, 1) to the nearest unit (exact for o >= 2^-7: 53 bits end above 2^-60)
 MPCD_HD uint64_t offset_from_double(double o) {
   const uint64_t k = (uint64_t)rint(o * (double)kOffOne);

@@ -4,6 +4,8 @@
 
 #include <cuda_runtime.h>
 
+#include "fixed_offset.cuh"
+
 #ifndef MPCD_HD
 #define MPCD_HD __host__ __device__ __forceinline__
 #endif
@@ -224,7 +226,7 @@ __device__ __forceinline__ double rsqrt_f64(double x) {
   const uint32_t hi = (uint32_t)__double2hiint(x);
   double y;
   if (hi - (923u << 20) < (200u << 20)) {  // 2^-100 .. 2^100
-    const uint32_t b = __float_as_uint(rsqrtf(__uint_as_float(((hi - (896u << 20)) << 3) | ((uint32_t)__double2loint(x) >> 29))));
+    const uint32_t b = __float_as_uint(rsqrtf(__uint_as_float(nearest_float_bits(x))));
     y = __hiloint2double((int)((b >> 3) + (896u << 20)), (int)(b << 29));
   } else {
     y = (double)rsqrtf((float)x);
