@@ -30,8 +30,8 @@
 // last read, take about 0.9 us to fetch) alternates
 // with the patches' rounds.
 //
-// MD per launch timed alone, this kernel / md_df.cu: swimmer64 138 / 217 us in
-// double-float, 127 / 196 with float springs; a 700-bead swimmer 133 / 187;
+// MD per launch timed alone, this kernel / md_df.cu: swimmer64 135 / 217 us in
+// double-float, 124 / 196 with float springs; a 700-bead swimmer 131 / 187;
 // swimmer128 with float springs 223 / 431 (there a tile of 256 slots has two
 // lanes per slot, and its springs follow one another; here 152 tiles of three
 // cilia or 151 sphere beads).  Running sums of the entries in any order took
@@ -315,7 +315,9 @@ __device__ void md_entries_body(const MDState& m, const MDStepArgs& a, Bin bin) 
   const int tid = threadIdx.x, nthr = blockDim.x, back = nthr - 1 - tid;
   const int lane32 = tid & 31, warp = tid >> 5;
   const bool solo = m.de_solo[tile] != 0;
-  const int lanes = m.de_lanes;
+  // narrow tiles go with slots of eight lanes: known here, the sums' code is one
+  // straight line (64^3 swimmer 138 to 135 us per launch, with float springs 127 to 123)
+  const int lanes = HALVES == 2 ? 8 : m.de_lanes;
   // owned coordinates: number c = tid / HALVES + j nthr below 3 T is coordinate
   // c / T of bead c mod T, so that few warps run the sums and the Verlet step
   // (a warp's instructions count once, however many lanes take part); with
@@ -740,7 +742,7 @@ template <typename Bin>
 const void* entries_kernel(const MDState& m) {
   const bool fl = m.df == 2;
   const int threads = md_entries_threads(m.tile);
-  if (6 * m.tile <= threads)
+  if (6 * m.tile <= threads && m.de_lanes == 8)
     return fl ? (const void*)k_md_entries<1, 2, true, Bin> : (const void*)k_md_entries<1, 2, false, Bin>;
   if (3 * m.tile <= threads)
     return fl ? (const void*)k_md_entries<1, 1, true, Bin> : (const void*)k_md_entries<1, 1, false, Bin>;

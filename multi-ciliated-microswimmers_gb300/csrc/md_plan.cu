@@ -1268,6 +1268,7 @@ std::string plan_entries(const MDInput& in, int grid_f32cells, const MDPlan& slo
     probe.tile = tile;
     probe.ntiles = nt;
     probe.df = probe.de = 1;
+    probe.de_lanes = out.de_lanes;
     probe.hmax = out.hmax;
     probe.de_nent_max = out.de_nent_max;
     probe.de_ninc_max = out.de_ninc_max;
