@@ -68,13 +68,13 @@ METRIC = "MPCD particle-steps/s"
 # DRAM bytes (read + write) per fluid particle of one fluid_step launch, from
 # one ncu capture on swimmer64 (profiles/fluid_step_swimmer64.md); the traffic
 # grows in proportion to the particles, so it is scaled to the workload.
-TRAFFIC_B_PER_PARTICLE = {"fp64": 107.7, "fp32": 48.7}
+TRAFFIC_B_PER_PARTICLE = {"fp64": 100.8, "fp32": 48.7}
 # the replica batch's fluid pass on the 64-replica ensemble
 # (profiles/batch_fluid_ensemble64.md: 2,389.7 MB for 34,273,280 particles)
 BATCH_TRAFFIC_B_PER_PARTICLE = 2389.7e6 / 34273280
 # FP64 pipe of the same captures (sm__pipe_fp64_cycles_active, of peak, active);
 # the float64 fluid step computes in 64-bit fixed point and is not bound by it
-FP64_PIPE_ACTIVE = {"fp64": 0.187, "fp32": 0.014}
+FP64_PIPE_ACTIVE = {"fp64": 0.159, "fp32": 0.014}
 # algorithmic bytes per particle-step: read + write of the reference's state
 # (float64: 3 position + 4 velocity/mass doubles; float32 split: two float4)
 BYTES_PER_PARTICLE = {"fp64": 112, "fp32": 64}

@@ -274,8 +274,9 @@ void free_md(MDState& m) {
 }
 
 // Fluids of at least this many particles are read in parts, each copied while
-// the next is gathered (64^3 x 10: 0.92 to 0.78 ms, 80 x 71 x 89 x 10: 1.86 to 1.49 of
-// which 1.3 are the link; 32^3 x 10 0.136 instead of 0.130: one launch below)
+// the next is gathered, smaller ones by one launch.  In parts / by one launch, us:
+// 0.33 M particles 139 / 125, 0.64 M 219 / 215, 0.85 M 272 / 292, 1.04 M 326 / 362, 1.76 M
+// 526 / 616, 2.62 M 756 / 946 (they cross near 0.7 M)
 constexpr long kPartsMin = 1l << 20;
 
 int alloc_fluid(mpcd_engine* h, long n) {
@@ -407,11 +408,11 @@ int build_md(mpcd_engine* h) {
   in.nbond = (long)h->newlen.size();
   in.newlen = h->newlen.data();
   in.oldlen = h->oldlen.data();
-  // -1: the grid kernel of md_df.cu (faster on GB300 than the float64 kernel
+  // -1: the double-float grid kernels (faster on GB300 than the float64 kernels
   // and than the split-arithmetic cluster kernel for one box), with
   // double-float springs for the float64 path and float springs on the same
-  // double-float positions for the float32 split path (swimmer64 MD 0.204
-  // against 0.215 ms, swimmer128 0.423 against 0.526)
+  // double-float positions for the float32 split path (swimmer64 MD 0.124 ms
+  // against 0.135)
   // contact forces between cilia run on the float64 grid kernel only
   const int arith = h->repel != 0.0 ? 0 : h->p.md_split < 0 ? (h->p.precision == MPCD_FP32 ? 3 : 2) : h->p.md_split;
   if (arith > 5) return fail(h, MPCD_EINVAL, "md_split must be -1 or 0 to 5");
@@ -1418,11 +1419,11 @@ int mpcd_step(mpcd_engine* h, const mpcd_inject* inj) {
     // round of particles per thread, two in float64): as they retire, the
     // higher-priority MD CTAs take their place, and the fluid CTAs fill what
     // the MD leaves of every SM.  Per step, short-lived CTAs against a
-    // persistent grid: swimmer64 223 us against 224 (float64; 268 with half
-    // the grid), 489 against 522 (float64, IEEE springs), 145 against 153
+    // persistent grid: swimmer64 218 us against 234 (float64; 277 with a quarter
+    // of the grid), 399 against 423 (float64, IEEE springs), 153 against 162
     // (split precision).  MD CTAs of 512 threads leave registers for one fluid
     // CTA: the pass runs after them, best on its persistent grid (20 k beads
-    // in 128^3: 581 against 628).  Alone: persistent, in float64 two rounds of
+    // in 128^3: 594 against 645).  Alone: persistent, in float64 two rounds of
     // the CTAs that fit.
     ProfScope ps(h, MPCD_K_FLUID);
     const bool wide = h->md.de && md_entries_threads(h->md.tile) > 384;

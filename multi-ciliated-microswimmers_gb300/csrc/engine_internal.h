@@ -344,8 +344,9 @@ cudaError_t launch_store_beads(const MDState& m, long s0, long nb, double* pos, 
                        const unsigned* err, cudaStream_t s);
 // Swimmers of up to this many beads are read through pinned host memory that
 // the kernel writes and the host copies from, larger ones by two copies of the
-// copy engine (2 x 24 KB: 12 us against 19; 2 x 123 KB: 24 against 20, the
-// host reads what the device has just written at 14 GB/s)
+// copy engine.  Pinned / copies, us per read: 1000 beads 20 / 33, 2000 23 / 34, 3000 26 / 35,
+// 5000 33 / 39, 8000 44 / 41 (the host reads what the device has just written at 14
+// GB/s; they cross near 6 k)
 constexpr long kPinnedBeads = 3072;
 // read-back into the caller's order (status: {bad id, error word} in host memory)
 template <typename F>

@@ -11,13 +11,15 @@
 // All quantities are two's-complement integers times a power of two chosen so
 // that the thermal range has bits to spare: velocities and mean velocities in
 // units of 2^-58, new velocities 2^-56, map entries 2^-59, axis components and
-// the thermostat factor 2^-60.  A rounding is half a unit of these, against
-// 2^-54 for float64 numbers of one half and more, so results are at least as close to the exact ones as
-// the float64 form's wherever the terms of a sum are of order one.  What does
-// not fit (velocities of 16 thermal velocities and more, mean velocities of 8,
-// thermostat factors of 8 (of 2 where the mean velocity is 2), kinetic energies of a cell of 4096, momenta of 512,
-// cells colder than 1/16, non-finite values) takes the float64 form, about half
-// as fast; a warp with one such particle makes both.  The factor's limit is what
+// the thermostat factor 2^-60, a cell's kinetic energy and momentum 2^-55 (2^-50 and
+// 2^-52 from 128 on).  What enters is truncated (less than one unit), a product is
+// within one unit, against half of 2^-53 for float64 numbers of one half and more:
+// results are at least as close to the exact ones as the float64 form's wherever
+// the terms of a sum are of order one.  What does not fit (velocities of 16
+// thermal velocities and more, mean velocities of 8, thermostat factors of 8, of 2
+// where the mean velocity is 2, kinetic energies of a cell of 4096, momenta of
+// 512, cells colder than 1/16, non-finite values) takes the float64 form, about
+// half as fast; a warp with one such particle makes both.  The factor's limit is what
 // counts at low densities: with 2 in place of 8, 4 % of the particles of a box with
 // three per cell were beyond it, in half of the warps, and 0.1 % with ten per cell
 // (64^3 cells, us per step, limit 2 / limit 8 / all in float64: two per cell 92 / 58 / 77,

@@ -2,9 +2,11 @@
 // operations on them that the fluid pass needs, in integer arithmetic.
 //
 // An offset o in [0, 1) is the integer k = o 2^60.  GB300 completes about one
-// float64 operation per clock and SM against 64 integer ones, and the fluid
-// pass is bound by its float64 pipe; streaming (x += v h), the wrap into the
-// next cell and the comparison with the grid shift need none of it this way.
+// float64 operation per clock and SM against 64 integer ones, and in float64 the
+// fluid pass is bound by that pipe; streaming (x += v h), the wrap into the next cell
+// and the comparison with the grid shift need none of it this way.  An offset that
+// is not a multiple of 2^-60 (below 2^-7, so only in the first row of cells, where a
+// position has more bits) is rounded to one when it is uploaded.
 // The displacement v h is the truncated high part of the exact product of the
 // two float64 significands, so its error is below 2 units of 2^-60 where the
 // fused multiply-add on a float64 offset rounds to 2^-54 (offsets of one half

@@ -277,12 +277,6 @@ __device__ __forceinline__ void sphere_virtual(const RigidSphereDev& S, const do
   p[2] += dm * us[2];
 }
 
-// Split-precision collision map of one cell (MPCD::next_tstep,
-// src/libcilia/mpcd.cpp:140-247): mean velocity, relative kinetic energy, the
-// MBS thermostat factor from a Gamma(3(N-1)/2) draw and the rotation about a
-// random axis, written as three float4 rows (A row, b) of v' = A v + b.  The
-// cell's sum m v^2 before the collision goes into ldiss.  `cid` keys the
-// generator (the cell's index within its own box).
 // The virtual particles of a cell on a sphere's surface or in a wall layer, up
 // to rho = 10 (src/libcilia/mpcd.cpp:175-198); returns the sphere or -1.  Not
 // inlined: the common path fits the instruction cache better without it.
@@ -315,6 +309,12 @@ static __device__ __noinline__ int add_virtual_f32(float4& s, float& M, int& num
   return sk;
 }
 
+// Split-precision collision map of one cell (MPCD::next_tstep,
+// src/libcilia/mpcd.cpp:140-247): mean velocity, relative kinetic energy, the
+// MBS thermostat factor from a Gamma(3(N-1)/2) draw and the rotation about a
+// random axis, written as two float4 {axis, factor} and {mean velocity, 0}.  The
+// cell's sum m v^2 before the collision goes into ldiss.  `cid` keys the
+// generator (the cell's index within its own box).
 __device__ __forceinline__ void cell_map_f32(const float4 s0, const uint32_t w, const uint32_t cid, const uint64_t seed,
                                              const uint64_t step, const float mb, const double* inj_gamma,
                                              const double* inj_axis, float4* par_out, float& ldiss, unsigned& errbits,

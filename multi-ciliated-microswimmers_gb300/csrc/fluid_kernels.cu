@@ -417,7 +417,7 @@ __device__ __forceinline__ void energy_end(BlockEnergy& b, EnergySum ke, int bit
 // per cell (1890 instructions, 12 cycles each at six warps per scheduler); the
 // float64 form kept that pipe 73 % busy.  64-thread blocks fill the SMs in the
 // finest steps (24 warps with 80 registers; five blocks of 128: 36 us, eight
-// with 64 registers: 43).  64^3 cells 48 to 31 us, 80 x 71 x 89 96 to 51.  For
+// with 64 registers: 43).  64^3 cells 48 to 31 us, 80 x 71 x 89 96 to 50.  For
 // boxes beyond one wave of the pair form below.
 constexpr int kCellThreads = 64;
 __global__ void __launch_bounds__(kCellThreads, 12) k_cell_params_f64(CellsF64 c, StepArgs a) {
@@ -462,10 +462,10 @@ __global__ void __launch_bounds__(kCellThreads, 12) k_cell_params_f64(CellsF64 c
 // The same by pairs of warps, 32 cells a CTA: one warp makes count, sums, Gamma
 // draw and thermostat factor, the other axis and rotation, and both the rows of
 // the map: half the chain, for twice the warps.  That pays while all pairs are
-// on the SMs at once (10 CTAs of 92 registers each): per step 36^3 cells 30.8
-// us against 31.9, 32^3 26.1 / 27.5, the channel (24 x 21 x 37) 33.0 / 36.0, 8^3
-// 12.4 / 13.2; beyond, the one-thread form does: 40^3 39.0 against 41.3, 64^3
-// cells 31 us against 41.
+// on the SMs at once (10 CTAs of 92 registers each): per step 36^3 cells 29.2
+// us against 29.9, 32^3 24.9 / 25.3, the channel (24 x 21 x 37) 31.1 / 32.8, 8^3
+// 8.8 / 10.2; beyond, the one-thread form does: 40^3 36.5 against 38.8, 64^3
+// cells 29 us against 41.
 constexpr int kPairCTAs = 10;  // per SM
 __global__ void __launch_bounds__(kCellThreads, kPairCTAs) k_cell_pairs_f64(CellsF64 c, StepArgs a) {
   __shared__ BlockEnergy s_e;
@@ -633,10 +633,10 @@ __device__ __forceinline__ void add_to_cell(double* sum, uint32_t cell, double v
 // Collision, kinetic energy, streaming, wrap and the comparison with the grid
 // shift run in 64-bit fixed point (fixed_collide.cuh, fixed_offset.cuh); float64
 // appears only as the stored velocity and in the atomic sums, which the L2
-// adds.  Nothing is saturated now (issue 52 %, the L1 data path 59 %, crossbar
-// 50 %); 32 warps of 64 registers per SM did best (24 of 80: 107 us), and
-// fetching the next particle ahead brought nothing.  64^3 x 10: 116 us with the
-// collision in float64 to 98; 80 x 71 x 89 x 10: 234 to 177; 32^3 x 10: 21.
+// adds.  Nothing is saturated (issue 61 %, the L1 data path 69 %); 32 warps of 64
+// registers per SM did best (24 of 80: 107 us against 98), and fetching the next
+// particle ahead brought nothing.  64^3 x 10: 116 us with the collision in float64,
+// 94 now; 80 x 71 x 89 x 10: 234, 171; 32^3 x 10: 20.
 // Walls and spheres are instantiations of their own; between walls only a
 // particle that would leave the channel takes the bounce-back.
 constexpr int kFluidThreads = 128;
