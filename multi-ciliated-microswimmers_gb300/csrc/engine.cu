@@ -427,16 +427,20 @@ int build_md(mpcd_engine* h) {
   const char* mt = std::getenv("MPCD_MD_MIN_TILE");
   const int min_tile = mt ? std::max(0, std::min(256, std::atoi(mt))) : 0;
   const int f32cells = h->p.precision == MPCD_FP32 ? 1 : 0;
-  const std::string why = plan_md(in, MDForce{}, allow_cluster, false, f32cells, pl, min_tile);
-  if (!why.empty()) return fail(h, MPCD_EINVAL, why);
   // double-float arithmetic: the entries layout (md_entries.cu) where the bead
   // set fits it, with the same results.  MPCD_MD_SLOTS=1 keeps the slot layout
   // (tests of that kernel)
   const char* slots = std::getenv("MPCD_MD_SLOTS");
-  if (in.df && !in.pair && !(slots && std::atoi(slots) != 0)) {
+  const bool entries = in.df && !in.pair && !(slots && std::atoi(slots) != 0);
+  std::string why = plan_md(in, MDForce{}, allow_cluster, false, f32cells, pl, min_tile, entries);
+  if (why.empty() && entries) {
     MDPlan de;
-    if (plan_entries(in, f32cells, pl, de, min_tile).empty()) pl = std::move(de);
+    if (plan_entries(in, f32cells, pl, de, min_tile).empty())
+      pl = std::move(de);
+    else
+      why = plan_md(in, MDForce{}, allow_cluster, false, f32cells, pl, min_tile);
   }
+  if (!why.empty()) return fail(h, MPCD_EINVAL, why);
   if (const char* ps = std::getenv("MPCD_MD_PLAN_STATS"); ps && std::atoi(ps) && pl.pair) {
     // the pair layout's per-tile sizes: force entries (of them reaching only
     // the tile), halo, incidences, hubs reached

@@ -179,7 +179,7 @@ std::string plan_pair_tables(MDPlan& out, const std::vector<int>& hubs) {
 }  // namespace
 
 std::string plan_md(const MDInput& in, const MDForce& force, bool allow_cluster, bool no_react, int grid_f32cells,
-                    MDPlan& out, int min_tile) {
+                    MDPlan& out, int min_tile, bool layout_only) {
   // springs per helper slot: the longest serial spring chain of any thread.
   // Odd, so that the helper slots' spring lists start in different
   // shared-memory banks.
@@ -220,10 +220,10 @@ std::string plan_md(const MDInput& in, const MDForce& force, bool allow_cluster,
   std::vector<int> run_id(nb, -1);
   for (long b = 0, r = 0; b < nb; ++b)
     if (owner[b] < 0) run_id[b] = (b > 0 && owner[b - 1] < 0) ? run_id[b - 1] : (int)r++;
-  std::vector<int> bstart(nb + 1, 0), blist(nsp);
-  for (long i = 0; i < nsp; ++i) bstart[in.sp_t[i] + 1]++;
-  for (long b = 0; b < nb; ++b) bstart[b + 1] += bstart[b];
-  {
+  std::vector<int> bstart(nb + 1, 0), blist(layout_only ? 0 : nsp);  // springs by bead
+  if (!layout_only) {
+    for (long i = 0; i < nsp; ++i) bstart[in.sp_t[i] + 1]++;
+    for (long b = 0; b < nb; ++b) bstart[b + 1] += bstart[b];
     std::vector<int> fillp(bstart.begin(), bstart.end() - 1);
     for (long i = 0; i < nsp; ++i) blist[fillp[in.sp_t[i]]++] = (int)i;
   }
@@ -460,7 +460,7 @@ std::string plan_md(const MDInput& in, const MDForce& force, bool allow_cluster,
       // list (helper slots) instead of reactions
       bool any_hub = false;
       for (long b = 0; b < nb && !any_hub; ++b) any_hub = hub[b] != 0;
-      if (any_hub && !no_react) return plan_md(in, force, allow_cluster, true, grid_f32cells, out, min_tile);
+      if (any_hub && !no_react) return plan_md(in, force, allow_cluster, true, grid_f32cells, out, min_tile, layout_only);
       return "the MD bead set needs more than 16 tiles of the fixed layout";
     }
     tile = force.tile;
@@ -515,7 +515,7 @@ std::string plan_md(const MDInput& in, const MDForce& force, bool allow_cluster,
     }
     for (long i = 0; i < nsp && !bad; ++i)
       if (react[i] && slot_of[in.sp_t[i]] / tile != slot_of[in.sp_o[i]] / tile) bad = true;
-    if (bad) return plan_md(in, force, allow_cluster, true, grid_f32cells, out, min_tile);
+    if (bad) return plan_md(in, force, allow_cluster, true, grid_f32cells, out, min_tile, layout_only);
   }
   // Hubs of the pair kernel: a bead outside the cilia with more than
   // kPairLong springs, each with an exact reverse partner (a sphere's centre,
@@ -610,14 +610,17 @@ std::string plan_md(const MDInput& in, const MDForce& force, bool allow_cluster,
   std::vector<int> pos(start.begin(), start.end() - 1);
   const long nspk = start[ns];  // springs kept
   out.so.assign(nspk, 0);
-  out.sk.assign(nspk, 0);
-  out.sr.assign(nspk, 0);
-  out.srest.assign(nspk, 0.0);
-  out.sm2k.assign(nspk, 0.0);
+  if (!layout_only) {
+    out.sk.assign(nspk, 0);
+    out.sr.assign(nspk, 0);
+    out.srest.assign(nspk, 0.0);
+    out.sm2k.assign(nspk, 0.0);
+  }
   for (long i = 0; i < nsp; ++i) {
     if (sslot[i] < 0) continue;
     const int d = pos[sslot[i]]++;
     out.so[d] = slot_of[in.sp_o[i]];
+    if (layout_only) continue;
     out.sk[d] = in.sp_k[i] | (react[i] ? kSpringReact : 0);
     out.sr[d] = in.sp_r[i];
     out.srest[d] = in.sp_rest[i];
@@ -661,14 +664,28 @@ std::string plan_md(const MDInput& in, const MDForce& force, bool allow_cluster,
       hub_at[slot_of[b]] = 1;
       hub_slots.push_back(slot_of[b]);
     }
-  out.sl.assign(nspk, 0);
+  if (!layout_only) out.sl.assign(nspk, 0);
   out.hstart.assign(out.ntiles + 1, 0);
   out.df_runs.clear();
   out.df_run_start.assign(1, 0);
   out.df_single.clear();
   out.df_single_start.assign(1, 0);
   int hmax = 0;
-  for (int t = 0; t < out.ntiles; ++t) {
+  if (layout_only) {  // the largest halo
+    std::vector<int> stamp(ns, -1);
+    for (int t = 0; t < out.ntiles; ++t) {
+      const int b0 = t * tile, b1 = b0 + tile;
+      int n = 0;
+      for (int d = start[b0]; d < start[b1]; ++d) {
+        const int o = out.so[d];
+        if ((o >= b0 && o < b1) || stamp[o] == t) continue;
+        stamp[o] = t;
+        ++n;
+      }
+      hmax = std::max(hmax, n);
+    }
+  }
+  for (int t = 0; t < out.ntiles && !layout_only; ++t) {
     const int b0 = t * tile, b1 = b0 + tile;
     std::vector<int> ext;
     for (int s2 = start[b0]; s2 < start[b1]; ++s2)
@@ -735,7 +752,16 @@ std::string plan_md(const MDInput& in, const MDForce& force, bool allow_cluster,
     std::vector<long> idx;
     std::vector<int> so, sk, sr, slv;
     std::vector<double> srest, sm2k;
-    for (int sl_ = 0; sl_ < ns; ++sl_) {
+    if (layout_only) {  // the checks of the codes below
+      if (tile + hmax > (1 << 16)) return "an MD tile is too large for packed spring codes";
+      for (long i = 0; i < nsp; ++i) {
+        if (sslot[i] < 0 || (in.sp_k[i] & 3) < MPCD_SPRING_BOND) continue;
+        const int t = sslot[i] / tile, lref = in.sp_r[i] - out.df_b0[t];
+        if (lref < 0 || lref >= out.df_nb[t]) return "a bond spring refers to a bond outside its tile's cilia";
+        if (lref >= (1 << 14)) return "an MD tile is too large for packed spring codes";
+      }
+    }
+    for (int sl_ = 0; sl_ < ns && !layout_only; ++sl_) {
       const int a0 = start[sl_], a1 = start[sl_ + 1];
       idx.clear();
       for (int k = a0; k < a1; ++k)
@@ -776,7 +802,7 @@ std::string plan_md(const MDInput& in, const MDForce& force, bool allow_cluster,
   if (in.pair) {
     if (!out.df) return "the pair kernel needs the double-float grid layout";
     const std::string e = plan_pair_tables(out, hub_slots);
-    if (e == "hub") return plan_md(in, force, allow_cluster, true, grid_f32cells, out, min_tile);  // no hubs then
+    if (e == "hub") return plan_md(in, force, allow_cluster, true, grid_f32cells, out, min_tile, layout_only);  // no hubs then
     if (!e.empty()) return e;
     out.pair = in.pair;
   }
@@ -814,14 +840,20 @@ std::string plan_md(const MDInput& in, const MDForce& force, bool allow_cluster,
     }
     if (!md_cluster_feasible(probe)) {
       if (forced) return "the fixed cluster layout does not fit on the device";
-      return plan_md(in, force, false, no_react, grid_f32cells, out, min_tile);  // grid layout instead
+      return plan_md(in, force, false, no_react, grid_f32cells, out, min_tile, layout_only);  // grid layout instead
     }
   } else {
     const int cap = md_max_coresident_blocks(probe, grid_f32cells);
+    if (layout_only) {  // the halo's copy lists, not made here, may decide: all of them then
+      probe.df_nsingle_max = hmax;
+      probe.df_nrun_max = hmax;
+      if (md_max_coresident_blocks(probe, grid_f32cells) != cap)
+        return plan_md(in, force, allow_cluster, no_react, grid_f32cells, out, min_tile);
+    }
     if (out.ntiles > cap) {
       // a large bead set: wider tiles (fewer CTAs; the double-float kernel
       // then runs four, then two lanes per slot)
-      if (tile < 256) return plan_md(in, force, allow_cluster, no_react, grid_f32cells, out, tile < 128 ? 128 : 256);
+      if (tile < 256) return plan_md(in, force, allow_cluster, no_react, grid_f32cells, out, tile < 128 ? 128 : 256, layout_only);
       return "MD tiles exceed the co-resident CTA limit of the device";
     }
   }

@@ -100,7 +100,9 @@ std::string plan_entries(const MDInput& in, int grid_f32cells, const MDPlan& slo
 // `grid_f32cells` selects the co-resident limit checked for the grid layout.
 // `min_tile`: the narrowest grid-layout tile to consider (0: as narrow as the
 // widest cilium allows); a grid that is not co-resident is re-planned wider.
+// `layout_only` (a double-float grid layout): the slots, with the same checks, but
+// not the springs' tables.
 std::string plan_md(const MDInput& in, const MDForce& force, bool allow_cluster, bool no_react, int grid_f32cells,
-                    MDPlan& out, int min_tile = 0);
+                    MDPlan& out, int min_tile = 0, bool layout_only = false);
 
 }  // namespace mpcd

@@ -73,3 +73,35 @@ def test_long_lists_agree_bit_for_bit(springs, precision, min_tile, monkeypatch)
         e.close()
     assert np.abs(got[0][1][hub]).max() > 0
     assert np.array_equal(got[0][0], got[1][0]) and np.array_equal(got[0][1], got[1][1])
+
+
+def test_a_bead_set_beyond_the_pair_layout_runs_on_the_slot_kernel(monkeypatch):
+    """Six beads with 200 springs each: four get a tile of their own, the others'
+    slots are more than the pair kernel adds in order."""
+    rng = np.random.default_rng(9)
+    nb, hubs, springs = 1300, 6, 200
+    pos = rng.uniform(4, 28, (nb, 3))
+    t, o = [], []
+    for h in range(hubs):
+        other = hubs + h * springs + np.arange(springs)
+        t += [np.full(springs, h), other]
+        o += [other, np.full(springs, h)]
+    t, o = np.concatenate(t).astype(np.int32), np.concatenate(o).astype(np.int32)
+    rest = np.sqrt(((pos[t] - pos[o]) ** 2).sum(axis=1)) * 1.02
+    k = np.full(len(t), 1.5)
+    ip, dp = ctypes.POINTER(ctypes.c_int), ctypes.POINTER(ctypes.c_double)
+    z = np.zeros(len(t), dtype=np.int32)
+    got = []
+    for slots in ("0", "1"):
+        monkeypatch.setenv("MPCD_MD_SLOTS", slots)
+        e = cg.Engine(32, tstep=0.1, ststep=0.002)
+        e.set_fluid(np.array([[0.5, 0.5, 0.5]]), np.zeros((1, 3)))
+        e.set_beads(pos, np.zeros((nb, 3)))
+        assert cg.lib().mpcd_set_springs(e.handle, len(t), t.ctypes.data_as(ip), o.ctypes.data_as(ip), z.ctypes.data_as(ip),
+                                         z.ctypes.data_as(ip), rest.ctypes.data_as(dp), k.ctypes.data_as(dp)) == 0
+        e.run(1)
+        got.append((e.beads(nb), e.md_layout()))
+        e.close()
+    assert got[0][1] == got[1][1]  # one layout
+    assert np.abs(got[0][0][1]).max() > 0
+    assert np.array_equal(got[0][0][0], got[1][0][0]) and np.array_equal(got[0][0][1], got[1][0][1])
