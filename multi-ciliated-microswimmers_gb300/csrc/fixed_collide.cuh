@@ -102,7 +102,7 @@ MPCD_HD int64_t mul_sh(Limbs a, Limbs b) {
 constexpr int kVelBits = 58;         // velocities that go in, up to 16; mean velocities
 constexpr int kMapBits = 59;         // entries of A
 constexpr int kAxisBits = 60;        // axis components, thermostat factor
-constexpr int kOutBits = 56;         // velocities that come out: up to 92 with the limits below
+constexpr int kOutBits = 56;         // velocities that come out, below 128 (apply_words)
 constexpr int64_t kMeanMax = 1ll << 61;  // 8, mean velocities
 constexpr int64_t kMeanMaxHot = 1ll << 59;  // 2, where the thermostat factor is 2 or more
 constexpr float kGammaMax = 4096.f;         // and the Gamma variate there

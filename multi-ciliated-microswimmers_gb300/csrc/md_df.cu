@@ -1,6 +1,10 @@
 // MD substeps of one MPC step for the float64 path, in double-float
 // arithmetic on the FP32 pipes.
 //
+// The general form: every bead set whose layout fits the device can run here.
+// Those that fit the layout of md_entries.cu (a thread per spring pair, about 60 %
+// of the time) run there, with the same results bit for bit.
+//
 // Same integrator and forces as md_kernels.cu (velocity Verlet of
 // src/libcilia/mdobject.cpp:36-72 inside the loop of src/simulation.cpp:217-265;
 // springs of src/cilia.cpp:127-239, src/sphere.cpp:87-119, src/clami.cpp:188-198)
